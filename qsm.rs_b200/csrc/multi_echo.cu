@@ -221,7 +221,7 @@ void linear_fit_device(qsm_ctx* ctx, const double* ph, const double* mg, const d
   // index (p/100 * count) truncated, clamped to count - 1 (multi_echo.rs:789-790)
   long long idx = (long long)((pct / 100.0) * (double)count);
   if (idx > count - 1) idx = count - 1;
-  const double thr = select_ranks(ctx, resid, sel, N, {idx})[0];
+  const double thr = select_ranks(ctx, resid, sel, N, count, {idx})[0];
   LaunchScope ls(ctx, "reliability");
   k_reliability<<<grid1d(N), 256, 0, ctx->stream>>>(N, mask, resid, thr, reliability);
   ls.done();
