@@ -5,6 +5,8 @@
 
 #include <algorithm>
 #include <cstring>
+#include <system_error>
+#include <thread>
 
 namespace qsm {
 
@@ -70,6 +72,12 @@ void* ws_get(qsm_ctx* ctx, const std::string& name, size_t bytes) {
   }
   b.epoch = ctx->epoch;
   return b.p;
+}
+
+void* ws_scratch_get(qsm_ctx* ctx, const std::string& name, size_t bytes) {
+  auto it = ctx->ws.find(name);
+  if (it != ctx->ws.end()) it->second.epoch = 0;  // earlier pointers of this call are dead
+  return ws_get(ctx, name, bytes);
 }
 
 bool stream_capturing(qsm_ctx* ctx) {
@@ -246,26 +254,52 @@ void check_finite(double v, const char* name) {
   if (!std::isfinite(v)) throw QsmError(QSM_ERR_INVALID_ARGUMENT, std::string(name) + " is not finite");
 }
 
-void h2d(qsm_ctx* ctx, void* dst, const void* src, size_t bytes) {
-  QSM_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
-}
-void d2h(qsm_ctx* ctx, void* dst, const void* src, size_t bytes) {
-  QSM_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-}
 void sync(qsm_ctx* ctx) { QSM_CUDA(cudaStreamSynchronize(ctx->stream)); }
 
 namespace {
-void ensure_pinned(qsm_ctx* ctx) {
-  for (int k = 0; k < 2; ++k) {
-    if (!ctx->pinned[k]) {
-      if (cudaHostAlloc(&ctx->pinned[k], kStageBytes, cudaHostAllocDefault) != cudaSuccess) {
-        (void)cudaGetLastError();
-        ctx->pinned[k] = nullptr;
-        throw QsmError(QSM_ERR_ALLOC, "pinned staging allocation failed");
-      }
-    }
-    if (!ctx->pinned_ev[k]) QSM_CUDA(cudaEventCreateWithFlags(&ctx->pinned_ev[k], cudaEventDisableTiming));
+// Host memory the driver would have to stage itself (neither page-locked nor managed).
+bool pageable(const void* p) {
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return true;
   }
+  return at.type == cudaMemoryTypeUnregistered;
+}
+
+void ensure_pinned(qsm_ctx* ctx) {
+  if (!ctx->pinned && cudaHostAlloc(&ctx->pinned, 2 * kStageThreads * kStageChunk, cudaHostAllocDefault) != cudaSuccess) {
+    (void)cudaGetLastError();
+    ctx->pinned = nullptr;
+    throw QsmError(QSM_ERR_ALLOC, "pinned staging allocation failed");
+  }
+  while (ctx->pinned_ev.size() < 2 * (size_t)kStageThreads) {
+    cudaEvent_t e = nullptr;
+    QSM_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    ctx->pinned_ev.push_back(e);
+  }
+}
+
+// work(worker) on kStageThreads threads (worker 0 here, and those that cannot be started);
+// the first CUDA error of any is thrown.
+template <class F> void stage_workers(qsm_ctx* ctx, const F& work) {
+  cudaError_t err[kStageThreads];
+  auto run = [&](int w) {
+    err[w] = cudaSetDevice(ctx->device);
+    if (err[w] == cudaSuccess) err[w] = work(w);
+  };
+  std::vector<std::thread> th;
+  th.reserve(kStageThreads);
+  int started = 1;
+  try {
+    for (; started < kStageThreads; ++started) th.emplace_back(run, started);
+  } catch (const std::system_error&) {
+  }
+  run(0);
+  for (int w = started; w < kStageThreads; ++w) run(w);
+  for (auto& t : th) t.join();
+  for (int w = 0; w < kStageThreads; ++w)
+    if (err[w] != cudaSuccess) throw QsmError(QSM_ERR_CUDA, std::string("staged copy: ") + cudaGetErrorString(err[w]));
 }
 }  // namespace
 
@@ -273,39 +307,59 @@ void staged_h2d(qsm_ctx* ctx, void* dst, const void* src, size_t bytes) {
   ensure_pinned(ctx);
   const uint8_t* s = static_cast<const uint8_t*>(src);
   uint8_t* d = static_cast<uint8_t*>(dst);
-  bool used[2] = {false, false};
-  for (size_t off = 0, c = 0; off < bytes; off += kStageBytes, ++c) {
-    const int k = (int)(c % 2);
-    const size_t n = std::min(kStageBytes, bytes - off);
-    if (used[k]) QSM_CUDA(cudaEventSynchronize(ctx->pinned_ev[k]));  // this slot's previous DMA is done
-    std::memcpy(ctx->pinned[k], s + off, n);
-    QSM_CUDA(cudaMemcpyAsync(d + off, ctx->pinned[k], n, cudaMemcpyHostToDevice, ctx->stream));
-    QSM_CUDA(cudaEventRecord(ctx->pinned_ev[k], ctx->stream));
-    used[k] = true;
-  }
-  sync(ctx);
+  stage_workers(ctx, [&](int w) -> cudaError_t {
+    int k = 0;
+    for (size_t off = (size_t)w * kStageChunk; off < bytes; off += kStageThreads * kStageChunk, k ^= 1) {
+      const int slot = 2 * w + k;
+      uint8_t* p = static_cast<uint8_t*>(ctx->pinned) + slot * kStageChunk;
+      const size_t n = std::min(kStageChunk, bytes - off);
+      cudaError_t e = cudaEventSynchronize(ctx->pinned_ev[slot]);  // the slot's last DMA
+      if (e != cudaSuccess) return e;
+      std::memcpy(p, s + off, n);
+      e = cudaMemcpyAsync(d + off, p, n, cudaMemcpyHostToDevice, ctx->stream);
+      if (e == cudaSuccess) e = cudaEventRecord(ctx->pinned_ev[slot], ctx->stream);
+      if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+  });
 }
 
 void staged_d2h(qsm_ctx* ctx, void* dst, const void* src, size_t bytes) {
   ensure_pinned(ctx);
   const uint8_t* s = static_cast<const uint8_t*>(src);
   uint8_t* d = static_cast<uint8_t*>(dst);
-  const size_t nchunks = (bytes + kStageBytes - 1) / kStageBytes;
-  auto issue = [&](size_t c) {
-    const int k = (int)(c % 2);
-    const size_t off = c * kStageBytes;
-    QSM_CUDA(cudaMemcpyAsync(ctx->pinned[k], s + off, std::min(kStageBytes, bytes - off), cudaMemcpyDeviceToHost,
-                             ctx->stream));
-    QSM_CUDA(cudaEventRecord(ctx->pinned_ev[k], ctx->stream));
-  };
-  if (nchunks > 0) issue(0);
-  for (size_t c = 0; c < nchunks; ++c) {
-    if (c + 1 < nchunks) issue(c + 1);  // the other slot was drained in the previous step
-    const int k = (int)(c % 2);
-    QSM_CUDA(cudaEventSynchronize(ctx->pinned_ev[k]));
-    const size_t off = c * kStageBytes;
-    std::memcpy(d + off, ctx->pinned[k], std::min(kStageBytes, bytes - off));
-  }
+  stage_workers(ctx, [&](int w) -> cudaError_t {
+    const size_t step = kStageThreads * kStageChunk;
+    auto issue = [&](size_t off, int k) -> cudaError_t {
+      const int slot = 2 * w + k;
+      cudaError_t e = cudaMemcpyAsync(static_cast<uint8_t*>(ctx->pinned) + slot * kStageChunk, s + off,
+                                      std::min(kStageChunk, bytes - off), cudaMemcpyDeviceToHost, ctx->stream);
+      return e == cudaSuccess ? cudaEventRecord(ctx->pinned_ev[slot], ctx->stream) : e;
+    };
+    size_t off = (size_t)w * kStageChunk;
+    int k = 0;
+    if (off < bytes) {
+      const cudaError_t e = issue(off, 0);
+      if (e != cudaSuccess) return e;
+    }
+    for (; off < bytes; off += step, k ^= 1) {
+      cudaError_t e = off + step < bytes ? issue(off + step, k ^ 1) : cudaSuccess;
+      if (e == cudaSuccess) e = cudaEventSynchronize(ctx->pinned_ev[2 * w + k]);
+      if (e != cudaSuccess) return e;
+      std::memcpy(d + off, static_cast<uint8_t*>(ctx->pinned) + (2 * w + k) * kStageChunk,
+                  std::min(kStageChunk, bytes - off));
+    }
+    return cudaSuccess;
+  });
+}
+
+void h2d(qsm_ctx* ctx, void* dst, const void* src, size_t bytes) {
+  if (bytes >= kStageMin && pageable(src)) staged_h2d(ctx, dst, src, bytes);
+  else QSM_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
+}
+void d2h(qsm_ctx* ctx, void* dst, const void* src, size_t bytes) {
+  if (bytes >= kStageMin && pageable(dst)) staged_d2h(ctx, dst, src, bytes);
+  else QSM_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
 }
 
 void LaunchScope::done() {
@@ -378,10 +432,8 @@ qsm_status qsm_ctx_destroy(qsm_ctx* ctx) {
   for (auto& kv : ctx->twiddles) cudaFree(kv.second);
   for (auto& kv : ctx->tables) cudaFree(kv.second);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
-  for (int k = 0; k < 2; ++k) {
-    if (ctx->pinned[k]) cudaFreeHost(ctx->pinned[k]);
-    if (ctx->pinned_ev[k]) cudaEventDestroy(ctx->pinned_ev[k]);
-  }
+  if (ctx->pinned) cudaFreeHost(ctx->pinned);
+  for (cudaEvent_t e : ctx->pinned_ev) cudaEventDestroy(e);
   delete ctx;
   return QSM_OK;
 }

@@ -52,9 +52,14 @@ std::vector<double> poisson_axis(int n, double vs) {
   return q;
 }
 
-template <typename S> const S* table(qsm_ctx* ctx, const std::string& key, const std::vector<double>& v) {
-  std::vector<S> h(v.begin(), v.end());
-  return (const S*)upload_table(ctx, key + (sizeof(S) == 4 ? ":f" : ":d"), h.data(), h.size() * sizeof(S));
+// The table cached under the key, or make() uploaded.
+template <typename S, class Make> const S* table(qsm_ctx* ctx, const std::string& key, const Make& make) {
+  const std::string full = key + (sizeof(S) == 4 ? ":f" : ":d");
+  auto it = ctx->tables.find(full);
+  if (it != ctx->tables.end()) return (const S*)it->second;
+  const std::vector<double> v = make();
+  const std::vector<S> h(v.begin(), v.end());
+  return (const S*)upload_table(ctx, full, h.data(), h.size() * sizeof(S));
 }
 
 std::string k(const char* what, int n, double vs) {
@@ -67,15 +72,15 @@ std::string k(const char* what, int n, double vs) {
 
 template <typename S> KSpaceT<S> make_kspace_t(qsm_ctx* ctx, const GridDims& d, const double bdir[3]) {
   KSpaceT<S> K;
-  K.fx = table<S>(ctx, k("freq", d.nx, d.vsx), fftfreq(d.nx, d.vsx));
-  K.fy = table<S>(ctx, k("freq", d.ny, d.vsy), fftfreq(d.ny, d.vsy));
-  K.fz = table<S>(ctx, k("freq", d.nz, d.vsz), fftfreq(d.nz, d.vsz));
-  K.lx = table<S>(ctx, k("lap", d.nx, d.vsx), lapneg_axis(d.nx, d.vsx));
-  K.ly = table<S>(ctx, k("lap", d.ny, d.vsy), lapneg_axis(d.ny, d.vsy));
-  K.lz = table<S>(ctx, k("lap", d.nz, d.vsz), lapneg_axis(d.nz, d.vsz));
-  K.qx = table<S>(ctx, k("poi", d.nx, d.vsx), poisson_axis(d.nx, d.vsx));
-  K.qy = table<S>(ctx, k("poi", d.ny, d.vsy), poisson_axis(d.ny, d.vsy));
-  K.qz = table<S>(ctx, k("poi", d.nz, d.vsz), poisson_axis(d.nz, d.vsz));
+  K.fx = table<S>(ctx, k("freq", d.nx, d.vsx), [&] { return fftfreq(d.nx, d.vsx); });
+  K.fy = table<S>(ctx, k("freq", d.ny, d.vsy), [&] { return fftfreq(d.ny, d.vsy); });
+  K.fz = table<S>(ctx, k("freq", d.nz, d.vsz), [&] { return fftfreq(d.nz, d.vsz); });
+  K.lx = table<S>(ctx, k("lap", d.nx, d.vsx), [&] { return lapneg_axis(d.nx, d.vsx); });
+  K.ly = table<S>(ctx, k("lap", d.ny, d.vsy), [&] { return lapneg_axis(d.ny, d.vsy); });
+  K.lz = table<S>(ctx, k("lap", d.nz, d.vsz), [&] { return lapneg_axis(d.nz, d.vsz); });
+  K.qx = table<S>(ctx, k("poi", d.nx, d.vsx), [&] { return poisson_axis(d.nx, d.vsx); });
+  K.qy = table<S>(ctx, k("poi", d.ny, d.vsy), [&] { return poisson_axis(d.ny, d.vsy); });
+  K.qz = table<S>(ctx, k("poi", d.nz, d.vsz), [&] { return poisson_axis(d.nz, d.vsz); });
   K.nyqx = (d.nx % 2 == 0) ? d.nx / 2 : -1;
   K.nyqy = (d.ny % 2 == 0) ? d.ny / 2 : -1;
   K.nyqz = (d.nz % 2 == 0) ? d.nz / 2 : -1;
