@@ -2,10 +2,11 @@
 // V-SHARP) on the GPU, plus the pipeline dispatcher run_bg_removal.
 //
 // Mask erosion decides "SMV(mask) > delta" with delta within ~1e-8 of a rational
-// count/total for realistic kernels, so the mask convolution always runs in double
-// (FP64 transform error ~1e-15) whatever the context precision; field filtering runs
-// in the working precision.
+// count/total for realistic kernels: it is decided by exact counts (smv.cu), and the sphere
+// kernel's multipliers are evaluated in double, whatever the context precision; field
+// filtering runs in the working precision.
 #include "functors.cuh"
+#include "smv.h"
 #include "solvers.h"
 
 #include <algorithm>
@@ -13,40 +14,66 @@
 
 namespace qsm {
 
+// Rust % on f64 is the truncated fmod; out of line, so that its loop costs the callers no
+// registers
+__device__ __noinline__ double turn_remainder(double x) { return fmod(x, 2.0 * kPi); }
+
 __device__ __forceinline__ double wrap_pi(double x) {
-  // src/unwrap/laplacian.rs:21-30 (Rust % on f64 is the truncated fmod)
+  // src/unwrap/laplacian.rs:21-30
   const double two_pi = 2.0 * kPi;
-  double y = fmod(x, two_pi);
+  // differences of wrapped phases lie within a turn, where the remainder is x itself
+  double y = x;
+  if (!(fabs(x) < two_pi)) y = turn_remainder(x);
   if (y > kPi) y -= two_pi;
   else if (y < -kPi) y += two_pi;
   return y;
 }
 
-// Wrapped 7-point Laplacian (periodic), masked, evaluated in double on the fly as
-// the X-pass input (src/unwrap/laplacian.rs:34-78, 146-149).
-template <typename T> struct LoadWrappedLap {
-  const double* ph;
-  const uint8_t* mask;
-  int nx, ny, nz;
-  double dx2, dy2, dz2;
-  __device__ __forceinline__ T operator()(int row, int e) const {
-    const long long sy = nx, sz = (long long)nx * ny;
-    const long long i = (long long)row * nx + e;
-    if (mask[i] == 0) return T(0);
-    const int j = row % ny, k = row / ny;
-    const long long ip = (e + 1 < nx) ? i + 1 : i - (nx - 1);
-    const long long im = (e > 0) ? i - 1 : i + (nx - 1);
-    const long long jp = (j + 1 < ny) ? i + sy : i - (ny - 1) * sy;
-    const long long jm = (j > 0) ? i - sy : i + (ny - 1) * sy;
-    const long long kp = (k + 1 < nz) ? i + sz : i - (long long)(nz - 1) * sz;
-    const long long km = (k > 0) ? i - sz : i + (long long)(nz - 1) * sz;
-    const double u = ph[i];
-    const double lx = (wrap_pi(ph[ip] - u) - wrap_pi(u - ph[im])) * dx2;
-    const double ly = (wrap_pi(ph[jp] - u) - wrap_pi(u - ph[jm])) * dy2;
-    const double lz = (wrap_pi(ph[kp] - u) - wrap_pi(u - ph[km])) * dz2;
-    return (T)(lx + ly + lz);
+// Wrapped 7-point Laplacian (periodic), masked, in double (src/unwrap/laplacian.rs:34-78,
+// 146-149), into working precision.  32x8 (x, y) tiles, each thread marching zchunk planes
+// with the z neighbours in registers, x neighbours by shuffle.  A pass of its own: inside
+// the X transform's loader every row element was a copy of this code with its six fmod
+// loops, and the X pass ran 265 us at 256x256x176, 250 with the loops skipped; this kernel
+// and the plain X pass take 94 us together.
+template <typename T>
+__global__ void __launch_bounds__(256)
+    k_wrapped_lap(int nx, int ny, int nz, int zchunk, double dx2, double dy2, double dz2, const double* __restrict__ ph,
+                  const uint8_t* __restrict__ mask, T* __restrict__ lap) {
+  const int lane = threadIdx.x & 31;
+  const int e = blockIdx.x * 32 + lane, j = blockIdx.y * 8 + (threadIdx.x >> 5);
+  if (j >= ny) return;  // whole warps
+  const bool in = e < nx;
+  const int i = in ? e : nx - 1;
+  const int k0 = blockIdx.z * zchunk, k1 = min(nz, k0 + zchunk);
+  const long long sz = (long long)nx * ny;
+  const int ip = i + 1 < nx ? i + 1 : 0, im = i > 0 ? i - 1 : nx - 1;
+  const double* row = ph + (long long)j * nx;
+  const double* rowp = ph + (long long)(j + 1 < ny ? j + 1 : 0) * nx + i;
+  const double* rowm = ph + (long long)(j > 0 ? j - 1 : ny - 1) * nx + i;
+  double um = row[(k0 > 0 ? k0 - 1 : nz - 1) * sz + i];
+  double u = row[k0 * sz + i];
+  for (int k = k0; k < k1; ++k) {
+    const long long b = k * sz;
+    const double up = row[(k + 1 < nz ? k + 1 : 0) * sz + i];
+    const double yp = rowp[b], ym = rowm[b];
+    double xp = __shfl_down_sync(0xffffffffu, u, 1), xm = __shfl_up_sync(0xffffffffu, u, 1);
+    if (lane == 31 || i + 1 >= nx) xp = row[b + ip];
+    if (lane == 0) xm = row[b + im];
+    const bool on = in && mask[b + (long long)j * nx + i] != 0;
+    if (in) {
+      T v = T(0);
+      if (on) {
+        const double lx = (wrap_pi(xp - u) - wrap_pi(u - xm)) * dx2;
+        const double ly = (wrap_pi(yp - u) - wrap_pi(u - ym)) * dy2;
+        const double lz = (wrap_pi(up - u) - wrap_pi(u - um)) * dz2;
+        v = (T)(lx + ly + lz);
+      }
+      lap[b + (long long)j * nx + i] = v;
+    }
+    um = u;
+    u = up;
   }
-};
+}
 
 // Poisson solve multiplier 1/lambda, 0 where |lambda| <= 1e-20 (src/unwrap/laplacian.rs:91-117)
 template <typename T> struct OpPoisson {
@@ -59,118 +86,56 @@ template <typename T> struct OpPoisson {
   }
 };
 
-// Normalised binary sphere at wrap-centred coordinates (src/kernels/smv.rs:19-67).
-// The inclusion test is evaluated without FMA contraction so that it matches the
-// reference's dx*dx + dy*dy + dz*dz <= r^2 exactly.
-struct SphereGeom {
-  int nx, ny, nz;
-  double vsx, vsy, vsz, r2, norm;
-};
-__host__ __device__ __forceinline__ double sph_coord(int i, int n, double vs) {
-  const int c = (i <= n / 2) ? i : i - n;
-  return (double)c * vs;
-}
-__device__ __forceinline__ bool sph_inside(const SphereGeom& s, int i, int j, int k) {
-  const double dx = sph_coord(i, s.nx, s.vsx), dy = sph_coord(j, s.ny, s.vsy), dz = sph_coord(k, s.nz, s.vsz);
-  const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-  return d2 <= s.r2;
-}
-struct LoadSphere {
-  SphereGeom s;
-  __device__ __forceinline__ double operator()(int row, int e) const {
-    const int j = row % s.ny, k = row / s.ny;
-    return sph_inside(s, e, j, k) ? s.norm : 0.0;
-  }
-};
-
-SphereGeom sphere_geom(const GridDims& d, double radius) {
-  SphereGeom s;
-  s.nx = d.nx;
-  s.ny = d.ny;
-  s.nz = d.nz;
-  s.vsx = d.vsx;
-  s.vsy = d.vsy;
-  s.vsz = d.vsz;
-  s.r2 = radius * radius;
-  // count the sphere's voxels on the host over the per-axis candidates
-  auto axis = [&](int n, double vs) {
-    std::vector<double> v;
-    for (int i = 0; i < n; ++i) {
-      const double c = sph_coord(i, n, vs);
-      if (c * c <= s.r2) v.push_back(c);
-    }
-    return v;
-  };
-  std::vector<double> ax = axis(d.nx, d.vsx), ay = axis(d.ny, d.vsy), az = axis(d.nz, d.vsz);
-  double count = 0.0;
-  for (double dz : az)
-    for (double dy : ay)
-      for (double dx : ax) {
-        volatile double a = dx * dx;
-        volatile double b = dy * dy;
-        volatile double c = dz * dz;
-        volatile double ab = a + b;
-        volatile double d2 = ab + c;
-        if (d2 <= s.r2) count += 1.0;
-      }
-  s.norm = count > 0.0 ? 1.0 / count : 0.0;
-  return s;
-}
-
-// pre/post multiply by Re(S) from a double spectrum (the SMV kernel transform)
-template <typename T> struct OpMulS {
+// Multiplier array applied as a pass's elements are fetched.
+template <typename T> struct OpPreMult {
   using C = cplx_t<T>;
-  const double2* S;
-  int one_minus;  // 1: multiply by (1 - S), 0: by S
-  __device__ __forceinline__ T m(long long idx) const {
-    const double s = S[idx].x;
-    return (T)(one_minus ? 1.0 - s : s);
-  }
-  __device__ __forceinline__ C pre(C v, int, int, int, long long idx) const { return cscale(v, m(idx)); }
+  const T* m;
+  static constexpr bool kNoPost = true;
+  __device__ __forceinline__ C pre(C v, int, int, int, long long idx) const { return cscale(v, __ldg(m + idx)); }
   __device__ __forceinline__ C post(C v, int, int, int, long long) const { return v; }
-  __device__ __forceinline__ C mid(C v, int, int, int, long long idx) const { return cscale(v, m(idx)); }
 };
 
-// SHARP deconvolution: |1 - S| < thr -> 0, else X / (1 - S) (src/bgremove/sharp.rs:111-119,
-// vsharp.rs:147-156)
-template <typename T> struct OpDeconvS {
-  using C = cplx_t<T>;
-  const double2* S;
-  double thr;
-  __device__ __forceinline__ C mid(C v, int, int, int, long long idx) const {
-    const double oms = 1.0 - S[idx].x;
-    if (fabs(oms) < thr) return mk<C>(T(0), T(0));
-    return cscale(v, (T)(1.0 / oms));
-  }
-};
-
-// eroded = (v/N > delta) (src/kernels/smv.rs:100-104)
-struct StoreThreshold {
-  uint8_t* out;
-  int nx;
-  double scale, delta;
-  __device__ __forceinline__ void operator()(int row, int e, double v) {
-    out[(long long)row * nx + e] = (v * scale > delta) ? 1 : 0;
-  }
-  __device__ __forceinline__ void finish() {}
-};
-
-// V-SHARP first-hit selection (src/bgremove/vsharp.rs:168-176)
+// V-SHARP first-hit selection (src/bgremove/vsharp.rs:168-176): the voxels that this
+// radius is the first to keep
 template <typename T> struct StoreSelect {
-  const uint8_t* eroded;
-  uint8_t* final_mask;
+  const uint8_t* first;
+  const uint8_t* taken;
+  const unsigned* row_hits;  // bit idx mod 32: some voxel of the row is kept first by idx
   T* local;
-  int nx;
+  int nx, idx;
   T scale;
+  static constexpr bool kRowFilter = true;
+  __device__ __forceinline__ bool wants_row(int row) const { return (__ldg(row_hits + row) >> (idx & 31)) & 1u; }
   __device__ __forceinline__ void operator()(int row, int e, T v) {
     const long long i = (long long)row * nx + e;
-    if (eroded[i] == 1 && final_mask[i] == 0) {
-      local[i] = v * scale;
-      final_mask[i] = 1;
-    }
+    if (__ldg(first + i) == idx && __ldg(taken + i) == 0) local[i] = v * scale;
   }
   __device__ __forceinline__ void finish() {}
 };
+
+// eroded = 1 where the only sphere keeps the voxel
+__global__ void k_first_to_mask(long long n, const uint8_t* first, uint8_t* mask) {
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+    mask[i] = first[i] == 0 ? 1 : 0;
+}
+// row_hits[row] = the set of first[] values (mod 32) in the row; one warp per row
+__global__ void __launch_bounds__(256)
+    k_row_hits(int nx, int nrows, const uint8_t* __restrict__ first, unsigned* __restrict__ hits) {
+  for (int row = blockIdx.x * 8 + (threadIdx.x >> 5); row < nrows; row += gridDim.x * 8) {
+    unsigned h = 0u;
+    for (int e = threadIdx.x & 31; e < nx; e += 32) {
+      const unsigned f = first[(long long)row * nx + e];
+      if (f != 255u) h |= 1u << (f & 31u);
+    }
+    h = __reduce_or_sync(0xffffffffu, h);
+    if ((threadIdx.x & 31) == 0) hits[row] = h;
+  }
+}
+// taken |= some sphere keeps the voxel
+__global__ void k_first_taken(long long n, const uint8_t* __restrict__ first, uint8_t* __restrict__ taken) {
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+    if (first[i] != 255) taken[i] = 1;
+}
 
 // SMV: local = eroded == 1 ? field - SMV(field) : 0 (src/bgremove/smv.rs:50-56)
 template <typename T> struct StoreSmvLocal {
@@ -181,7 +146,7 @@ template <typename T> struct StoreSmvLocal {
   T scale;
   __device__ __forceinline__ void operator()(int row, int e, T v) {
     const long long i = (long long)row * nx + e;
-    out[i] = eroded[i] == 1 ? field[i] - (double)(v * scale) : 0.0;
+    out[i] = __ldg(eroded + i) == 1 ? __ldg(field + i) - (double)(v * scale) : 0.0;
   }
   __device__ __forceinline__ void finish() {}
 };
@@ -195,18 +160,13 @@ void forward3(qsm_ctx* ctx, const Fft3<T>& f, const Load& ld, cplx_t<T>* dst) {
   run_yz<T, -1, 2>(ctx, f, dst, dst, OpId<T>{}, nullptr);
 }
 
-// S = FFT(smv_kernel(r)) in double (src/kernels/smv.rs:19-67 + src/fft.rs:514-520)
-void smv_spectrum(qsm_ctx* ctx, const Fft3<double>& f64, const GridDims& d, double radius, double2* S) {
-  forward3<double>(ctx, f64, LoadSphere{sphere_geom(d, radius)}, S);
-}
-
-// eroded = IFFT(Fm * S) > delta, all in double
-void erode_smv(qsm_ctx* ctx, const Fft3<double>& f64, const GridDims& d, const double2* Fm, const double2* S,
-               double delta, uint8_t* eroded) {
-  double2* tmp = ws<double2>(ctx, "bg.tmp64", (size_t)f64.g.hsize());
-  run_yz<double, +1, 2>(ctx, f64, Fm, tmp, OpMulS<double>{S, 0}, nullptr);
-  run_yz<double, +1, 1>(ctx, f64, tmp, tmp, OpId<double>{}, nullptr);
-  run_x_c2r<double>(ctx, f64, tmp, StoreThreshold{eroded, d.nx, 1.0 / (double)d.n, delta}, nullptr);
+// eroded = mean of the mask over the sphere > delta (src/kernels/smv.rs:73-105)
+void smv_erode(qsm_ctx* ctx, const GridDims& d, const uint8_t* mask, const SmvSphere& s, double delta,
+               uint8_t* eroded) {
+  smv_erode_first(ctx, d, mask, {s}, delta, eroded);
+  LaunchScope ls(ctx, "smv_mask");
+  k_first_to_mask<<<grid1d(d.n), 256, 0, ctx->stream>>>(d.n, eroded, eroded);
+  ls.done();
 }
 
 // 1 - sqrt(1e-7), src/bgremove/sharp.rs:79 and vsharp.rs:129
@@ -217,68 +177,81 @@ template <typename T>
 void sharp_impl(qsm_ctx* ctx, const GridDims& d, const double* field, const uint8_t* mask, double threshold,
                 double radius, double* out_local, uint8_t* out_mask) {
   using C = cplx_t<T>;
-  Fft3<double> f64 = make_fft3<double>(ctx, d);
   Fft3<T> f = make_fft3<T>(ctx, d);
   const size_t H = (size_t)f.g.hsize();
-  double2* S = ws<double2>(ctx, "bg.S", H);
-  double2* Fm = ws<double2>(ctx, "bg.Fm", H);
+  T* m = ws<T>(ctx, "bg.mult", H);
   C* spec = ws<C>(ctx, "spec", H);
   T* g = ws<T>(ctx, "bg.img", (size_t)d.n);
-  smv_spectrum(ctx, f64, d, radius, S);
-  forward3<double>(ctx, f64, LoadCast<uint8_t, double>{mask, d.nx}, Fm);
-  erode_smv(ctx, f64, d, Fm, S, sharp_delta(), out_mask);
+  const SmvSphere s = smv_sphere(d, radius);
+  smv_erode(ctx, d, mask, s, sharp_delta(), out_mask);
   const T scale = (T)(1.0 / (double)d.n);
   // high-pass, mask
+  smv_multiplier<T>(ctx, f, s, kSmvOneMinusS, 0.0, m);
   run_x_r2c<T>(ctx, f, spec, LoadCast<double, T>{field, d.nx}, nullptr);
   run_yz<T, -1, 1>(ctx, f, spec, spec, OpId<T>{}, nullptr);
-  run_z_fused<T>(ctx, f, spec, spec, OpMulS<T>{S, 1}, nullptr);
+  run_z_fused_m<T>(ctx, f, spec, spec, m, nullptr);
   run_yz<T, +1, 1>(ctx, f, spec, spec, OpId<T>{}, nullptr);
   run_x_c2r<T>(ctx, f, spec, StoreMaskEqOne<T>{g, out_mask, d.nx, scale}, nullptr);
-  // deconvolve, mask
+  // SHARP deconvolution: |1 - S| < thr -> 0, else X / (1 - S) (sharp.rs:111-119), mask
+  smv_multiplier<T>(ctx, f, s, kSmvDeconv, threshold, m);
   run_x_r2c<T>(ctx, f, spec, LoadCast<T, T>{g, d.nx}, nullptr);
   run_yz<T, -1, 1>(ctx, f, spec, spec, OpId<T>{}, nullptr);
-  run_z_fused<T>(ctx, f, spec, spec, OpDeconvS<T>{S, threshold}, nullptr);
+  run_z_fused_m<T>(ctx, f, spec, spec, m, nullptr);
   run_yz<T, +1, 1>(ctx, f, spec, spec, OpId<T>{}, nullptr);
   run_x_c2r<T>(ctx, f, spec, StoreMaskedF64<T>{out_local, out_mask, d.nx, scale}, nullptr);
 }
 
-// V-SHARP (src/bgremove/vsharp.rs:88-199), radii already sorted descending, >= 2
+// V-SHARP (src/bgremove/vsharp.rs:88-199), radii already sorted descending, >= 2.  The
+// erosions of all radii are one distance transform (smv.cu), so the radius that keeps each
+// voxel first is known before any field is filtered; a radius then costs its multiplier
+// and one inverse transform.
 template <typename T>
 void vsharp_impl(qsm_ctx* ctx, const GridDims& d, const double* field, const uint8_t* mask,
                  const std::vector<double>& radii, double threshold, qsm_progress_fn progress, void* user,
                  double* out_local, uint8_t* out_mask) {
   using C = cplx_t<T>;
-  Fft3<double> f64 = make_fft3<double>(ctx, d);
   Fft3<T> f = make_fft3<T>(ctx, d);
   const size_t H = (size_t)f.g.hsize();
   const size_t N = (size_t)d.n;
-  double2* S0 = ws<double2>(ctx, "bg.S0", H);
-  double2* S = ws<double2>(ctx, "bg.S", H);
-  double2* Fm = ws<double2>(ctx, "bg.Fm", H);
+  T* m = ws<T>(ctx, "bg.mult", H);
   C* Ff = ws<C>(ctx, "bg.Ff", H);
   C* tmp = ws<C>(ctx, "bg.tmpT", H);
-  uint8_t* eroded = ws<uint8_t>(ctx, "bg.eroded", N);
+  uint8_t* first = ws<uint8_t>(ctx, "bg.first", N);
+  unsigned* hits = ws<unsigned>(ctx, "bg.row_hits", (size_t)d.ny * d.nz);
   T* local = ws<T>(ctx, "bg.img", N);
   QSM_CUDA(cudaMemsetAsync(out_mask, 0, N, ctx->stream));
   QSM_CUDA(cudaMemsetAsync(local, 0, N * sizeof(T), ctx->stream));
-  forward3<double>(ctx, f64, LoadCast<uint8_t, double>{mask, d.nx}, Fm);
   forward3<T>(ctx, f, LoadCast<double, T>{field, d.nx}, Ff);
   const T scale = (T)(1.0 / (double)d.n);
   const double delta = sharp_delta();
-  for (size_t idx = 0; idx < radii.size(); ++idx) {
-    if (progress) progress(user, idx + 1, radii.size());
-    double2* Sr = (idx == 0) ? S0 : S;
-    smv_spectrum(ctx, f64, d, radii[idx], Sr);
-    erode_smv(ctx, f64, d, Fm, Sr, delta, eroded);
-    run_yz<T, +1, 2, true>(ctx, f, Ff, tmp, OpMulS<T>{Sr, 1}, nullptr);
-    run_yz<T, +1, 1>(ctx, f, tmp, tmp, OpId<T>{}, nullptr);
-    run_x_c2r<T>(ctx, f, tmp, StoreSelect<T>{eroded, out_mask, local, d.nx, scale}, nullptr);
+  std::vector<SmvSphere> spheres;
+  for (double r : radii) spheres.push_back(smv_sphere(d, r));
+  constexpr size_t kGroup = 254;  // radii per erosion call
+  for (size_t g0 = 0; g0 < radii.size(); g0 += kGroup) {
+    const size_t g1 = std::min(radii.size(), g0 + kGroup);
+    smv_erode_first(ctx, d, mask, std::vector<SmvSphere>(spheres.begin() + g0, spheres.begin() + g1), delta, first);
+    {
+      LaunchScope ls(ctx, "vsharp_rows");
+      k_row_hits<<<x_rows_grid(f.g), 256, 0, ctx->stream>>>(d.nx, d.ny * d.nz, first, hits);
+      ls.done();
+    }
+    for (size_t idx = g0; idx < g1; ++idx) {
+      if (progress) progress(user, idx + 1, radii.size());
+      smv_multiplier<T>(ctx, f, spheres[idx], kSmvOneMinusS, 0.0, m);
+      run_yz<T, +1, 2, true>(ctx, f, Ff, tmp, OpPreMult<T>{m}, nullptr);
+      run_yz<T, +1, 1>(ctx, f, tmp, tmp, OpId<T>{}, nullptr);
+      run_x_c2r<T>(ctx, f, tmp, StoreSelect<T>{first, out_mask, hits, local, d.nx, (int)(idx - g0), scale}, nullptr);
+    }
+    LaunchScope ls(ctx, "vsharp_mask");
+    k_first_taken<<<grid1d(d.n), 256, 0, ctx->stream>>>(d.n, first, out_mask);
+    ls.done();
   }
-  // deconvolution with the largest kernel's inverse
+  // deconvolution with the largest kernel's inverse (vsharp.rs:147-156)
   C* spec = ws<C>(ctx, "spec", H);
+  smv_multiplier<T>(ctx, f, spheres[0], kSmvDeconv, threshold, m);
   run_x_r2c<T>(ctx, f, spec, LoadCast<T, T>{local, d.nx}, nullptr);
   run_yz<T, -1, 1>(ctx, f, spec, spec, OpId<T>{}, nullptr);
-  run_z_fused<T>(ctx, f, spec, spec, OpDeconvS<T>{S0, threshold}, nullptr);
+  run_z_fused_m<T>(ctx, f, spec, spec, m, nullptr);
   run_yz<T, +1, 1>(ctx, f, spec, spec, OpId<T>{}, nullptr);
   run_x_c2r<T>(ctx, f, spec, StoreMaskedF64<T>{out_local, out_mask, d.nx, scale}, nullptr);
 }
@@ -288,18 +261,16 @@ template <typename T>
 void smv_impl(qsm_ctx* ctx, const GridDims& d, const double* field, const uint8_t* mask, double radius,
               double* out_local, uint8_t* out_mask) {
   using C = cplx_t<T>;
-  Fft3<double> f64 = make_fft3<double>(ctx, d);
   Fft3<T> f = make_fft3<T>(ctx, d);
   const size_t H = (size_t)f.g.hsize();
-  double2* S = ws<double2>(ctx, "bg.S", H);
-  double2* Fm = ws<double2>(ctx, "bg.Fm", H);
+  T* m = ws<T>(ctx, "bg.mult", H);
   C* spec = ws<C>(ctx, "spec", H);
-  smv_spectrum(ctx, f64, d, radius, S);
-  forward3<double>(ctx, f64, LoadCast<uint8_t, double>{mask, d.nx}, Fm);
-  erode_smv(ctx, f64, d, Fm, S, 1.0 - 1e-10, out_mask);
+  const SmvSphere s = smv_sphere(d, radius);
+  smv_erode(ctx, d, mask, s, 1.0 - 1e-10, out_mask);
+  smv_multiplier<T>(ctx, f, s, kSmvS, 0.0, m);
   run_x_r2c<T>(ctx, f, spec, LoadCast<double, T>{field, d.nx}, nullptr);
   run_yz<T, -1, 1>(ctx, f, spec, spec, OpId<T>{}, nullptr);
-  run_z_fused<T>(ctx, f, spec, spec, OpMulS<T>{S, 0}, nullptr);
+  run_z_fused_m<T>(ctx, f, spec, spec, m, nullptr);
   run_yz<T, +1, 1>(ctx, f, spec, spec, OpId<T>{}, nullptr);
   run_x_c2r<T>(ctx, f, spec, StoreSmvLocal<T>{field, out_mask, out_local, d.nx, (T)(1.0 / (double)d.n)}, nullptr);
 }
@@ -358,12 +329,12 @@ template <typename T> struct StoreIsmv {
   double acc[1];
   __device__ __forceinline__ void operator()(int row, int e, T v) {
     const long long i = (long long)row * nx + e;
-    const double er = (double)eroded[i];
-    const double fld = field[i];
-    const double m0 = mask[i] != 0 ? 1.0 : 0.0;
+    const double er = (double)__ldg(eroded + i);
+    const double fld = __ldg(field + i);
+    const double m0 = __ldg(mask + i) != 0 ? 1.0 : 0.0;
     const T fn = (T)(er * (double)(v * scale) + fld * (m0 - er));
     out[i] = fn;
-    const double f0 = prev ? (double)prev[i] : fld * er;
+    const double f0 = prev ? (double)__ldg(prev + i) : fld * er;
     const double dd = f0 - (double)fn;
     acc[0] += dd * dd;
   }
@@ -390,52 +361,29 @@ __global__ void k_ismv_out(long long N, const double* __restrict__ field, const 
 }
 
 template <typename T>
-__global__ void k_re_spectrum(long long H, const double2* __restrict__ S, T* __restrict__ out) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < H; i += (long long)gridDim.x * blockDim.x)
-    out[i] = (T)S[i].x;
-}
-
-template <typename T> struct OpMulRe {
-  using C = cplx_t<T>;
-  const T* m;
-  __device__ __forceinline__ C mid(C v, int, int, int, long long idx) const { return cscale(v, m[idx]); }
-};
-
-template <typename T> struct LoadVol {
-  const T* p;
-  int nx;
-  __device__ __forceinline__ T operator()(int row, int e) const { return p[(long long)row * nx + e]; }
-};
-
-template <typename T>
 void ismv_impl(qsm_ctx* ctx, const GridDims& d, const double* field, const uint8_t* mask,
                const qsm_ismv_params& p, qsm_progress_fn progress, void* user, double* out_local,
                uint8_t* out_mask) {
   using C = cplx_t<T>;
-  Fft3<double> f64 = make_fft3<double>(ctx, d);
   Fft3<T> f = make_fft3<T>(ctx, d);
   const size_t H = (size_t)f.g.hsize();
   const long long N = d.n;
   const std::string pre = sizeof(T) == 4 ? "ismv32." : "ismv64.";
-  double2* S = ws<double2>(ctx, "bg.S", H);
-  double2* Fm = ws<double2>(ctx, "bg.Fm", H);
   T* Sr = ws<T>(ctx, pre + "Sr", H);
   C* spec = ws<C>(ctx, pre + "spec", H);
   T* fb[2] = {ws<T>(ctx, pre + "f0", (size_t)N), ws<T>(ctx, pre + "f1", (size_t)N)};
   IsmvState* st = ws<IsmvState>(ctx, pre + "state", 1);
-  double* partials = ws<double>(ctx, pre + "partials", (size_t)kMaxPersistentBlocks);
+  double* partials = ws<double>(ctx, pre + "partials", x_partials(f, 1));
   QSM_CUDA(cudaMemsetAsync(st, 0, sizeof(IsmvState), ctx->stream));
-  smv_spectrum(ctx, f64, d, p.radius, S);
-  forward3<double>(ctx, f64, LoadCast<uint8_t, double>{mask, d.nx}, Fm);
-  erode_smv(ctx, f64, d, Fm, S, 1.0 - 1e-10, out_mask);  // ismv.rs:166-169
+  const SmvSphere sphere = smv_sphere(d, p.radius);
+  smv_multiplier<T>(ctx, f, sphere, kSmvS, 0.0, Sr);
+  smv_erode(ctx, d, mask, sphere, 1.0 - 1e-10, out_mask);  // ismv.rs:166-169
   {
     LaunchScope ls(ctx, "ismv_init");
-    k_re_spectrum<T><<<grid1d((long long)H), 256, 0, ctx->stream>>>((long long)H, S, Sr);
     k_ismv_init<T><<<grid1d(N), 256, 0, ctx->stream>>>(N, field, out_mask, p.tol, p.max_iter, fb[0], st, partials);
     ls.done();
   }
   const int* done = &st->done;
-  const bool use_m = zm_tile_width<T>(d.nz, f.pz.m, f.pz.T) > 0;
   const T scale = (T)(1.0 / (double)N);
   const int maxi = (int)std::min<size_t>(p.max_iter, (size_t)1 << 30);
   // iteration k reads fb[(k-1) % 2] and writes fb[k % 2]
@@ -443,10 +391,9 @@ void ismv_impl(qsm_ctx* ctx, const GridDims& d, const double* field, const uint8
     const T* in = fb[(k - 1) % 2];
     StoreIsmv<T> store{fb[k % 2], k == 1 ? nullptr : in, field, mask, out_mask, d.nx, scale, st, partials, maxi,
                        {0.0}};
-    run_x_r2c<T>(ctx, f, spec, LoadVol<T>{in, d.nx}, done);
+    run_x_r2c<T>(ctx, f, spec, LoadCast<T, T>{in, d.nx}, done);
     run_yz<T, -1, 1>(ctx, f, spec, spec, OpId<T>{}, done);
-    if (use_m) run_z_fused_m<T>(ctx, f, spec, spec, Sr, done);
-    else run_z_fused<T>(ctx, f, spec, spec, OpMulRe<T>{Sr}, done);
+    run_z_fused_m<T>(ctx, f, spec, spec, Sr, done);
     run_yz<T, +1, 1>(ctx, f, spec, spec, OpId<T>{}, done);
     run_x_c2r<T>(ctx, f, spec, store, done);
   };
@@ -527,9 +474,18 @@ void unwrap_impl(qsm_ctx* ctx, const GridDims& d, const double* phase, const uin
   Fft3<T> f = make_fft3<T>(ctx, d);
   KSpace K = make_kspace(ctx, d, nullptr);
   C* spec = ws<C>(ctx, "spec", (size_t)f.g.hsize());
-  LoadWrappedLap<T> ld{phase, mask, d.nx, d.ny, d.nz, 1.0 / (d.vsx * d.vsx), 1.0 / (d.vsy * d.vsy),
-                       1.0 / (d.vsz * d.vsz)};
-  run_x_r2c<T>(ctx, f, spec, ld, nullptr);
+  T* lap = ws<T>(ctx, sizeof(T) == 4 ? "unwrap.lap32" : "unwrap.lap64", (size_t)d.n);
+  {
+    // about 24 blocks per SM
+    const int gx = (d.nx + 31) / 32, gy = (d.ny + 7) / 8;
+    const long long zc = std::max<long long>(1, 24LL * sm_count(ctx) / ((long long)gx * gy));
+    const int zchunk = (int)((d.nz + zc - 1) / zc);
+    LaunchScope ls(ctx, "wrapped_lap");
+    k_wrapped_lap<T><<<dim3(gx, gy, (d.nz + zchunk - 1) / zchunk), 256, 0, ctx->stream>>>(
+        d.nx, d.ny, d.nz, zchunk, 1.0 / (d.vsx * d.vsx), 1.0 / (d.vsy * d.vsy), 1.0 / (d.vsz * d.vsz), phase, mask, lap);
+    ls.done();
+  }
+  run_x_r2c<T>(ctx, f, spec, LoadCast<T, T>{lap, d.nx}, nullptr);
   run_yz<T, -1, 1>(ctx, f, spec, spec, OpId<T>{}, nullptr);
   run_z_fused<T>(ctx, f, spec, spec, OpPoisson<T>{K}, nullptr);
   run_yz<T, +1, 1>(ctx, f, spec, spec, OpId<T>{}, nullptr);

@@ -15,6 +15,7 @@
 //   p     : p = r + beta p
 // replayed as a CUDA graph of one iteration, polled every 8 iterations.
 #include "functors.cuh"
+#include "smv.h"
 #include "solvers.h"
 
 #include <algorithm>
@@ -22,10 +23,9 @@
 
 namespace qsm {
 
-// helpers defined in bgremove.cu
-void smv_spectrum(qsm_ctx* ctx, const Fft3<double>& f64, const GridDims& d, double radius, double2* S);
-void erode_smv(qsm_ctx* ctx, const Fft3<double>& f64, const GridDims& d, const double2* Fm, const double2* S,
-               double delta, uint8_t* eroded);
+// defined in bgremove.cu
+void smv_erode(qsm_ctx* ctx, const GridDims& d, const uint8_t* mask, const SmvSphere& s, double delta,
+               uint8_t* eroded);
 double sharp_delta();
 
 namespace {
@@ -38,19 +38,6 @@ struct CgState {
   double rsold, alpha, beta, bnorm, tol;
 };
 
-// multiplier array pointwise op for the in-kernel Z pass (long axes)
-template <typename T> struct OpMulArr {
-  using C = cplx_t<T>;
-  const T* m;
-  __device__ __forceinline__ C mid(C v, int, int, int, long long idx) const { return cscale(v, m[idx]); }
-};
-
-template <typename T> struct LoadImg {
-  const T* p;
-  int nx;
-  __device__ __forceinline__ T operator()(int row, int e) const { return p[(long long)row * nx + e]; }
-};
-
 // out = w * v / N (w null: 1)
 template <typename T> struct StoreWeighted {
   T* out;
@@ -60,7 +47,7 @@ template <typename T> struct StoreWeighted {
   __device__ __forceinline__ void operator()(int row, int e, T v) {
     const long long i = (long long)row * nx + e;
     const T y = v * invn;
-    out[i] = w ? w[i] * y : y;
+    out[i] = w ? __ldg(w + i) * y : y;
   }
   __device__ __forceinline__ void finish() {}
 };
@@ -81,14 +68,15 @@ template <typename T> struct StoreCgA {
   double acc[2];
   __device__ __forceinline__ void operator()(int row, int e, T v) {
     const long long i = (long long)row * nx + e;
-    const T xi = x ? x[i] : T(0);
+    const T xi = x ? __ldg(x + i) : T(0);
     const T ax = v * invn + lambda * xi;
     if (mode == 0) {
-      const T r = b[i] - ax;
+      const T bi = __ldg(b + i);
+      const T r = bi - ax;
       out[i] = r;
       p_out[i] = r;
       acc[0] += (double)r * (double)r;
-      acc[1] += (double)b[i] * (double)b[i];
+      acc[1] += (double)bi * (double)bi;
     } else {
       out[i] = ax;
       acc[0] += (double)xi * (double)ax;
@@ -164,13 +152,6 @@ __global__ void k_half_from_full(Geom g, const double* __restrict__ K, T* __rest
   }
 }
 
-// 1 - Re(S) on the half spectrum (RESHARP's DKER, src/bgremove/resharp.rs:71-72)
-template <typename T>
-__global__ void k_one_minus_re(long long H, const double2* __restrict__ S, T* __restrict__ out) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < H; i += (long long)gridDim.x * blockDim.x)
-    out[i] = (T)(1.0 - S[i].x);
-}
-
 template <typename Tin, typename Tout>
 __global__ void k_convert(long long N, const Tin* __restrict__ in, Tout* __restrict__ out) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x)
@@ -186,12 +167,11 @@ __global__ void k_masked_out(long long N, const T* __restrict__ x, const uint8_t
 
 // y = Re IFFT(K * FFT(x)) then the store functor
 template <typename T, class Load, class Store>
-void k_filter(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* spec, const T* Kh, bool use_m, const Load& ld,
-              const Store& st, const int* done) {
+void k_filter(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* spec, const T* Kh, const Load& ld, const Store& st,
+              const int* done) {
   run_x_r2c<T>(ctx, f, spec, ld, done);
   run_yz<T, -1, 1>(ctx, f, spec, spec, OpId<T>{}, done);
-  if (use_m) run_z_fused_m<T>(ctx, f, spec, spec, Kh, done);
-  else run_z_fused<T>(ctx, f, spec, spec, OpMulArr<T>{Kh}, done);
+  run_z_fused_m<T>(ctx, f, spec, spec, Kh, done);
   run_yz<T, +1, 1>(ctx, f, spec, spec, OpId<T>{}, done);
   run_x_c2r<T>(ctx, f, spec, st, done);
 }
@@ -213,7 +193,7 @@ size_t cg_normal_impl(qsm_ctx* ctx, const GridDims& d, const T* Kh, const T* w, 
   T* ap = ws<T>(ctx, nm("ap"), (size_t)N);
   T* t = ws<T>(ctx, nm("t"), (size_t)N);
   C* spec = ws<C>(ctx, nm("spec"), (size_t)f.g.hsize());
-  double* partials = ws<double>(ctx, nm("partials"), (size_t)kMaxPersistentBlocks * 2);
+  double* partials = ws<double>(ctx, nm("partials"), x_partials(f, 2));
   CgState* st = ws<CgState>(ctx, nm("state"), 1);
   {
     CgState s0{};
@@ -221,7 +201,6 @@ size_t cg_normal_impl(qsm_ctx* ctx, const GridDims& d, const T* Kh, const T* w, 
     h2d(ctx, st, &s0, sizeof(s0));
   }
   const int* done = &st->done;
-  const bool use_m = zm_tile_width<T>(d.nz, f.pz.m, f.pz.T) > 0;
   const T invn = (T)(1.0 / (double)N);
   const T lam = (T)lambda;
   // x = x0
@@ -231,8 +210,8 @@ size_t cg_normal_impl(qsm_ctx* ctx, const GridDims& d, const T* Kh, const T* w, 
     ls.done();
   }
   auto apply_a = [&](const T* in, const StoreCgA<T>& store) {
-    k_filter<T>(ctx, f, spec, Kh, use_m, LoadImg<T>{in, d.nx}, StoreWeighted<T>{t, w, d.nx, invn}, done);
-    k_filter<T>(ctx, f, spec, Kh, use_m, LoadImg<T>{t, d.nx}, store, done);
+    k_filter<T>(ctx, f, spec, Kh, LoadCast<T, T>{in, d.nx}, StoreWeighted<T>{t, w, d.nx, invn}, done);
+    k_filter<T>(ctx, f, spec, Kh, LoadCast<T, T>{t, d.nx}, store, done);
   };
   // r = b - A x0; p = r (src/solvers/cg.rs:50-60)
   apply_a(x, StoreCgA<T>{r, p, x, b, d.nx, invn, lam, 0, st, partials, {0.0, 0.0}});
@@ -305,17 +284,11 @@ void resharp_impl(qsm_ctx* ctx, const GridDims& d, const double* field, const ui
                   const qsm_resharp_params& p, qsm_progress_fn progress, void* user, double* out_local,
                   uint8_t* out_mask) {
   using C = cplx_t<T>;
-  Fft3<double> f64 = make_fft3<double>(ctx, d);
   Fft3<T> f = make_fft3<T>(ctx, d);
   const long long N = d.n;
   const size_t H = (size_t)f.g.hsize();
-  double2* S = ws<double2>(ctx, "bg.S", H);
-  double2* Fm = ws<double2>(ctx, "bg.Fm", H);
-  smv_spectrum(ctx, f64, d, p.radius, S);
-  run_x_r2c<double>(ctx, f64, Fm, LoadCast<uint8_t, double>{mask, d.nx}, nullptr);
-  run_yz<double, -1, 1>(ctx, f64, Fm, Fm, OpId<double>{}, nullptr);
-  run_yz<double, -1, 2>(ctx, f64, Fm, Fm, OpId<double>{}, nullptr);
-  erode_smv(ctx, f64, d, Fm, S, sharp_delta(), out_mask);
+  const SmvSphere sphere = smv_sphere(d, p.radius);
+  smv_erode(ctx, d, mask, sphere, sharp_delta(), out_mask);
   const char* pre = sizeof(T) == 4 ? "rs32." : "rs64.";
   auto nm = [&](const char* s) { return std::string(pre) + s; };
   T* Kh = ws<T>(ctx, nm("dker"), H);
@@ -325,18 +298,17 @@ void resharp_impl(qsm_ctx* ctx, const GridDims& d, const double* field, const ui
   T* t = ws<T>(ctx, nm("t"), (size_t)N);
   T* x = ws<T>(ctx, nm("x"), (size_t)N);
   C* spec = ws<C>(ctx, nm("spec"), H);
+  smv_multiplier<T>(ctx, f, sphere, kSmvOneMinusS, 0.0, Kh);  // DKER, src/bgremove/resharp.rs:71-72
   {
     LaunchScope ls(ctx, "resharp_setup");
-    k_one_minus_re<T><<<grid1d((long long)H), 256, 0, ctx->stream>>>((long long)H, S, Kh);
     k_convert<uint8_t, T><<<grid1d(N), 256, 0, ctx->stream>>>(N, out_mask, w);
     k_convert<double, T><<<grid1d(N), 256, 0, ctx->stream>>>(N, field, fld);
     ls.done();
   }
   // b = H^T H field (resharp.rs:84-85)
-  const bool use_m = zm_tile_width<T>(d.nz, f.pz.m, f.pz.T) > 0;
   const T invn = (T)(1.0 / (double)N);
-  k_filter<T>(ctx, f, spec, Kh, use_m, LoadImg<T>{fld, d.nx}, StoreWeighted<T>{t, w, d.nx, invn}, nullptr);
-  k_filter<T>(ctx, f, spec, Kh, use_m, LoadImg<T>{t, d.nx}, StoreWeighted<T>{b, nullptr, d.nx, invn}, nullptr);
+  k_filter<T>(ctx, f, spec, Kh, LoadCast<T, T>{fld, d.nx}, StoreWeighted<T>{t, w, d.nx, invn}, nullptr);
+  k_filter<T>(ctx, f, spec, Kh, LoadCast<T, T>{t, d.nx}, StoreWeighted<T>{b, nullptr, d.nx, invn}, nullptr);
   cg_normal_impl<T>(ctx, d, Kh, w, p.tik_reg, b, nullptr, p.tol, p.max_iter, progress, user, x);
   LaunchScope ls(ctx, "resharp_out");
   k_masked_out<T><<<grid1d(N), 256, 0, ctx->stream>>>(N, x, out_mask, out_local);

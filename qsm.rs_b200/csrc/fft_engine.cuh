@@ -366,6 +366,40 @@ template <int N, int TT, int R0, int R1, int R2> struct FixedPlan {
   X(162, 18, 9, 9, 2) X(168, 12, 8, 7, 3) X(180, 15, 15, 12, 1) X(200, 14, 8, 5, 5)               \
   X(216, 18, 12, 6, 3) X(224, 16, 16, 7, 2) X(225, 15, 15, 15, 1) X(240, 16, 16, 15, 1)
 
+// The remaining lengths from 32 to 384 with prime factors up to 13, compiled for the passes
+// without functors only (more_plans.cuh); four lists, one per translation unit.
+#define QSM_FIXED_PLANS_MORE_0(X) \
+  X(32, 2, 16, 2, 1) X(39, 3, 13, 3, 1) X(45, 3, 15, 3, 1) X(52, 4, 13, 4, 1) \
+  X(60, 4, 15, 4, 1) X(70, 7, 10, 7, 1) X(88, 8, 11, 8, 1) X(104, 8, 13, 8, 1) \
+  X(121, 11, 11, 11, 1) X(140, 10, 7, 5, 4) X(156, 13, 13, 12, 1) X(182, 14, 13, 7, 2) \
+  X(198, 18, 11, 6, 3) X(231, 21, 11, 7, 3) X(245, 18, 7, 7, 5) X(264, 24, 11, 6, 4) \
+  X(280, 20, 8, 7, 5) X(297, 33, 11, 9, 3) X(315, 23, 15, 7, 3) X(330, 30, 15, 11, 2) \
+  X(350, 35, 10, 7, 5) X(363, 33, 11, 11, 3)
+
+#define QSM_FIXED_PLANS_MORE_1(X) \
+  X(33, 3, 11, 3, 1) X(40, 3, 8, 5, 1) X(48, 4, 12, 4, 1) X(54, 6, 9, 6, 1) \
+  X(63, 7, 9, 7, 1) X(77, 7, 11, 7, 1) X(91, 7, 13, 7, 1) X(105, 8, 15, 7, 1) \
+  X(126, 11, 7, 6, 3) X(143, 13, 13, 11, 1) X(165, 15, 15, 11, 1) X(189, 21, 9, 7, 3) \
+  X(208, 16, 16, 13, 1) X(234, 20, 13, 6, 3) X(250, 25, 10, 5, 5) X(270, 23, 15, 6, 3) \
+  X(286, 26, 13, 11, 2) X(300, 20, 15, 5, 4) X(320, 22, 8, 8, 5) X(336, 24, 16, 7, 3) \
+  X(351, 39, 13, 9, 3) X(364, 28, 13, 7, 4)
+
+#define QSM_FIXED_PLANS_MORE_2(X) \
+  X(35, 3, 7, 5, 1) X(42, 4, 7, 6, 1) X(49, 4, 7, 7, 1) X(55, 5, 11, 5, 1) \
+  X(65, 5, 13, 5, 1) X(78, 7, 13, 6, 1) X(98, 7, 7, 7, 2) X(110, 11, 11, 10, 1) \
+  X(130, 13, 13, 10, 1) X(147, 11, 7, 7, 3) X(169, 13, 13, 13, 1) X(195, 15, 15, 13, 1) \
+  X(210, 15, 15, 7, 2) X(242, 22, 11, 11, 2) X(252, 21, 12, 7, 3) X(273, 21, 13, 7, 3) \
+  X(288, 24, 12, 12, 2) X(308, 28, 11, 7, 4) X(324, 36, 12, 9, 3) X(338, 26, 13, 13, 2) \
+  X(352, 32, 16, 11, 2) X(375, 25, 15, 5, 5)
+
+#define QSM_FIXED_PLANS_MORE_3(X) \
+  X(36, 3, 12, 3, 1) X(44, 4, 11, 4, 1) X(50, 5, 10, 5, 1) X(56, 4, 8, 7, 1) \
+  X(66, 6, 11, 6, 1) X(84, 7, 12, 7, 1) X(99, 11, 11, 9, 1) X(117, 13, 13, 9, 1) \
+  X(132, 12, 12, 11, 1) X(154, 14, 11, 7, 2) X(175, 13, 7, 5, 5) X(196, 14, 7, 7, 4) \
+  X(220, 20, 11, 5, 4) X(243, 27, 9, 9, 3) X(260, 20, 13, 5, 4) X(275, 25, 11, 5, 5) \
+  X(294, 25, 7, 7, 6) X(312, 24, 13, 8, 3) X(325, 25, 13, 5, 5) X(343, 25, 7, 7, 7) \
+  X(360, 24, 15, 8, 3) X(378, 42, 9, 7, 6)
+
 // The runtime stages of a plan's length-m transform, reading through fetch (first
 // stage) and writing through emit (last stage).
 template <int DIR, typename C, class SA, class Fetch, class Emit>
@@ -417,18 +451,6 @@ __device__ __noinline__ void fft_pencil_direct(const FftPlan1D* plp, int t, bool
     if constexpr (DST_G) gdst[base + e * stride] = v;
     else sp[sa(e)] = v;
   };
-  // Compile-time plans only for the contiguous (X) passes in single precision:
-  // inlining every plan into the strided Y/Z engine, or into the double-precision
-  // engine, raises the register count past the occupancy budget.
-  if constexpr (!std::is_same<SA, SAStrided>::value && sizeof(C) == 8) {
-#define QSM_TRY_FIXED(N_, T_, R0_, R1_, R2_)                                                \
-    if (FixedPlan<N_, T_, R0_, R1_, R2_>::matches(pl)) {                                    \
-      FixedPlan<N_, T_, R0_, R1_, R2_>::template run<DIR>(t, active, sp, sa, tw, fetch, emit); \
-      return;                                                                               \
-    }
-    QSM_FIXED_PLANS(QSM_TRY_FIXED)
-#undef QSM_TRY_FIXED
-  }
   run_stages<DIR>(pl, t, active, sp, sa, tw, fetch, emit);
 }
 

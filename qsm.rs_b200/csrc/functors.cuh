@@ -14,6 +14,17 @@ template <typename Tin, typename T> struct LoadCast {
   __device__ __forceinline__ const Tin* row_begin(int row) const { return p + (long long)row * nx; }
 };
 
+// product of two arrays
+template <typename Ta, typename T> struct LoadProduct {
+  const Ta* a;
+  const T* b;
+  int nx;
+  __device__ __forceinline__ T operator()(int row, int e) const {
+    const long long i = (long long)row * nx + e;
+    return (T)((double)__ldg(a + i) * (double)__ldg(b + i));
+  }
+};
+
 // value where mask != 0, else 0
 template <typename Tin, typename T> struct LoadMasked {
   const Tin* p;
@@ -25,7 +36,33 @@ template <typename Tin, typename T> struct LoadMasked {
   }
 };
 
+// A loader that only reads an array of the working precision, and its array.
+template <typename T> struct PlainLoad<T, LoadCast<T, T>> : std::true_type {};
+
 // ----------------------------------------------------------------- stores --
+// out[i] = v * scale in working precision
+template <typename T> struct StoreReal {
+  T* __restrict__ out;
+  int nx;
+  T scale;
+  __device__ __forceinline__ void operator()(int row, int e, T v) { out[(long long)row * nx + e] = v * scale; }
+  __device__ __forceinline__ void finish() {}
+};
+template <typename T> struct PlainStore<T, StoreReal<T>> : std::true_type {};
+
+// out[i] = mask[i] != 0 ? v*scale : 0 in working precision
+template <typename T> struct StoreMaskedT {
+  T* __restrict__ out;
+  const uint8_t* __restrict__ mask;
+  int nx;
+  T scale;
+  __device__ __forceinline__ void operator()(int row, int e, T v) {
+    const long long i = (long long)row * nx + e;
+    out[i] = __ldg(mask + i) != 0 ? v * scale : T(0);
+  }
+  __device__ __forceinline__ void finish() {}
+};
+
 // out[i] = mask[i] != 0 ? v*scale : 0, written as double
 template <typename T> struct StoreMaskedF64 {
   double* __restrict__ out;

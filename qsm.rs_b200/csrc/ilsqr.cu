@@ -310,7 +310,8 @@ template <typename T> struct OpLsqrOut {
     return Scalars{mode == 0 ? -st->alpha : -st->beta, mode == 0 ? st->su : st->sv};
   }
   // post() with the old value and the scalars already in hand (same arithmetic)
-  __device__ __forceinline__ C post_old(C v, int ix, int iy, int iz, C oldv, const Scalars& s, double& acc) const {
+  __device__ __forceinline__ C post_old(C v, int ix, int iy, int iz, long long, C oldv, const Scalars& s,
+                                        double& acc) const {
     C r = cscale(v, (T)dip(K, ix, iy, iz));
     if (mode <= 1) {
       const C o = cscale(oldv, (T)s.sc);
@@ -484,14 +485,6 @@ template <typename T> struct LoadScaled {  // x * s (s = deferred scale in the s
   int nx;
   __device__ __forceinline__ T operator()(int row, int e) const { return p[(long long)row * nx + e] * (T)*s; }
 };
-template <typename T> struct StoreScaledReal {
-  T* out;
-  int nx;
-  T invn;
-  __device__ __forceinline__ void operator()(int row, int e, T v) { out[(long long)row * nx + e] = v * invn; }
-  __device__ __forceinline__ void finish() {}
-};
-
 // v = Re IFFT(...)/N - beta*v (ilsqr.rs:1260-1276 then :425-427), with ||v||^2; the
 // last block runs the LSMR recurrences (ilsqr.rs:433-492).  init: v = A^T u only.
 template <typename T> struct StoreLsmrV {
@@ -964,7 +957,7 @@ void ilsqr_impl(qsm_ctx* ctx, const GridDims& d, const double* f, const uint8_t*
     ls.done();
   }
   run_iterations(ctx, p.max_iter, mdone, [&]() {
-    mic_chain(LoadScaled<T>{vv, &mst->sv, d.nx}, StoreScaledReal<T>{rq, d.nx, invn});
+    mic_chain(LoadScaled<T>{vv, &mst->sv, d.nx}, StoreReal<T>{rq, d.nx, invn});
     {
       LaunchScope ls(ctx, "lsmr_grad");
       k_lsmr_grad<T, T><<<grid1d(N), 256, 0, ctx->stream>>>(d.nx, d.ny, d.nz, hx, hy, hz, rq, wg, u3, mst, partials, 0);

@@ -4,6 +4,7 @@
 
 #include "internal.h"
 #include "passes.cuh"
+#include "two_factor.cuh"
 
 namespace qsm {
 
@@ -13,7 +14,15 @@ template <typename T> struct Fft3 {
   const cplx_t<T>* twx;
   const cplx_t<T>* twy;
   const cplx_t<T>* twz;
+  TwoFactor<T> tfx{}, tfy{}, tfz{};  // two-factor passes of each axis (n = 0: none)
+  T* xstage = nullptr;  // buffer of the runtime-engine X passes (null: the context's own)
 };
+
+// The two-factor form of a length (two_factor.cu), n = 0 when it has none.
+template <typename T> TwoFactor<T> make_two_factor(qsm_ctx* ctx, int n);
+// Its radices and blocks, and its host table (tw).
+template <typename T> TwoFactor<T> plan_two_factor(int n);
+template <typename T> std::vector<cplx_t<T>> two_factor_table(const TwoFactor<T>& ax);
 
 // Point each Bluestein plan at the chirp and kernel spectrum that follow the stage
 // twiddles in its table.
@@ -40,6 +49,9 @@ template <typename T> Fft3<T> make_fft3(qsm_ctx* ctx, const GridDims& d) {
   f.twy = (const cplx_t<T>*)twiddle_table(ctx, f.py, dbl);
   f.twz = (const cplx_t<T>*)twiddle_table(ctx, f.pz, dbl);
   attach_tables(f);
+  f.tfx = make_two_factor<T>(ctx, d.nx);
+  f.tfy = make_two_factor<T>(ctx, d.ny);
+  f.tfz = make_two_factor<T>(ctx, d.nz);
   return f;
 }
 
@@ -89,64 +101,134 @@ template <typename T> inline long long x_blocks(const Fft3<T>& f) {
   return (npairs + P - 1) / P;
 }
 
-// Compile-time X kernels (float) for the lengths of QSM_FIXED_PLANS (and of
-// QSM_FIXED_PLANS_WIDE when W); false when the plan is not one of them.
+constexpr int kMaxPersistentBlocks = 4096;
+
+// ------------------------------------------------------- two-factor launches --
+// Two buffers of a tile (rows of `stride` elements) and the twiddle table.
+template <typename T> inline size_t tf_smem(int n, int stride) { return (2 * (size_t)stride + 1) * n * sizeof(cplx_t<T>); }
+// Whether a pass over this axis takes the two-factor kernels (stride: tf_cols, or
+// tf_x_stride for X passes).
+template <typename T> inline bool tf_usable(const qsm_ctx* ctx, const TwoFactor<T>& ax, int stride) {
+  return compiled_plans(ctx) && ax.n > 0 && tf_smem<T>(ax.n, stride) <= 227u * 1024u;
+}
+template <typename T> inline unsigned tf_x_grid(long long rows) {
+  const long long b = (rows + tf_cols<T>() - 1) / tf_cols<T>();
+  return (unsigned)(b < kMaxPersistentBlocks ? b : kMaxPersistentBlocks);
+}
+// Multiplier array as a Z-pass operator (spectrum layout).
+template <typename T> struct OpMultArray {
+  using C = cplx_t<T>;
+  const T* m;
+  __device__ __forceinline__ C mid(C v, int, int, int, long long idx) const { return cscale(v, __ldg(m + idx)); }
+};
+
+// Doubles that K sums per block of an X pass may fill (grid_sum_last), whichever kernel runs.
+template <typename T> inline size_t x_partials(const Fft3<T>& f, int K) {
+  const long long b = x_blocks(f);
+  return (size_t)(b > kMaxPersistentBlocks ? b : kMaxPersistentBlocks) * K;
+}
+
+// Pencils per block of the compile-time X passes: as many whole pencils as 256 threads hold.
+// A pencil's threads are not rounded up to a divisor of a warp (as the runtime engine's
+// are): at 21 threads per pencil (length 189) a third of each block idled.
+template <class FP> constexpr int x_fx_pencils() { return FP::T >= 256 ? 1 : 256 / FP::T; }
+template <class FP> inline unsigned x_fx_blocks(long long pencils) {
+  return (unsigned)((pencils + x_fx_pencils<FP>() - 1) / x_fx_pencils<FP>());
+}
+
+// One compile-time X pass (k_x_r2c_fx / k_x_c2r_fx, FP a FixedPlan).
+template <typename T, class FP, bool DEAD, class Load>
+bool launch_x_r2c_fx(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* spec, const Load& ld, const int* done) {
+  constexpr int P = x_fx_pencils<FP>();
+  const size_t smem = (size_t)(x_tw_len<T>(FP::n) + P * x_rowlen<T>(FP::n)) * sizeof(cplx_t<T>);
+  auto kern = k_x_r2c_fx<T, FP, Load, DEAD>;
+  ensure_smem(kern, smem);
+  LaunchScope ls(ctx, "fft_x_r2c");
+  kern<<<x_fx_blocks<FP>(((long long)f.g.nrows() + 1) / 2), dim3(FP::T, P), smem, ctx->stream>>>(f.g, f.twx, spec, ld, done);
+  ls.done();
+  return true;
+}
+template <typename T, class FP, bool DEAD, class Store>
+bool launch_x_c2r_fx(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* spec, const Store& st, const int* done) {
+  constexpr int P = x_fx_pencils<FP>();
+  const size_t smem = (size_t)(x_tw_len<T>(FP::n) + P * x_rowlen<T>(FP::n)) * sizeof(cplx_t<T>);
+  auto kern = k_x_c2r_fx<T, FP, Store, DEAD>;
+  ensure_smem(kern, smem);
+  LaunchScope ls(ctx, "fft_x_c2r");
+  kern<<<x_fx_blocks<FP>(((long long)f.g.nrows() + 1) / 2), dim3(FP::T, P), smem, ctx->stream>>>(f.g, f.twx, spec, st, done);
+  ls.done();
+  return true;
+}
+
+// Compile-time X kernels with the functor inside: in float for the lengths of
+// QSM_FIXED_PLANS, and with W in both precisions for QSM_FIXED_PLANS_WIDE too; false when
+// the plan is not one of them.
 template <typename T, bool W, bool DEAD, class Load>
 bool run_x_r2c_fixed(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* spec, const Load& ld, const int* done) {
   if (!compiled_plans(ctx)) return false;
-  if constexpr (!std::is_same<T, float>::value && !W) {
-    return false;
-  } else {
-    using C = cplx_t<T>;
 #define QSM_TRY_XR(N_, T_, R0_, R1_, R2_)                                                          \
-    if (FixedPlan<N_, T_, R0_, R1_, R2_>::matches(f.px)) {                                         \
-      using FP = FixedPlan<N_, T_, R0_, R1_, R2_>;                                                 \
-      const int Tt = x_block_t(T_);                                                                \
-      const int P = x_pencils_per_block<T>(T_);                                                    \
-      const size_t smem = (size_t)(x_tw_len<T>(N_) + P * x_rowlen<T>(N_)) * sizeof(C);            \
-      auto kern = k_x_r2c_fx<T, FP, Load, DEAD>;                                                   \
-      ensure_smem(kern, smem);                                                                     \
-      LaunchScope ls(ctx, "fft_x_r2c");                                                            \
-      kern<<<(unsigned)x_blocks(f), dim3(Tt, P), smem, ctx->stream>>>(f.g, f.twx, spec, ld, done); \
-      ls.done();                                                                                   \
-      return true;                                                                                 \
-    }
+  if (FixedPlan<N_, T_, R0_, R1_, R2_>::matches(f.px))                                             \
+    return launch_x_r2c_fx<T, FixedPlan<N_, T_, R0_, R1_, R2_>, DEAD>(ctx, f, spec, ld, done);
+  if constexpr (std::is_same<T, float>::value || W) {
     QSM_FIXED_PLANS(QSM_TRY_XR)
-    if constexpr (W) {
-      QSM_FIXED_PLANS_WIDE(QSM_TRY_XR)
-    }
-#undef QSM_TRY_XR
-    return false;
   }
+  if constexpr (W) {
+    QSM_FIXED_PLANS_WIDE(QSM_TRY_XR)
+  }
+#undef QSM_TRY_XR
+  return false;
 }
 
 template <typename T, bool W, bool DEAD, class Store>
 bool run_x_c2r_fixed(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* spec, const Store& st, const int* done) {
   if (!compiled_plans(ctx)) return false;
-  if constexpr (!std::is_same<T, float>::value && !W) {
-    return false;
-  } else {
-    using C = cplx_t<T>;
 #define QSM_TRY_XC(N_, T_, R0_, R1_, R2_)                                                          \
-    if (FixedPlan<N_, T_, R0_, R1_, R2_>::matches(f.px)) {                                         \
-      using FP = FixedPlan<N_, T_, R0_, R1_, R2_>;                                                 \
-      const int Tt = x_block_t(T_);                                                                \
-      const int P = x_pencils_per_block<T>(T_);                                                    \
-      const size_t smem = (size_t)(x_tw_len<T>(N_) + P * x_rowlen<T>(N_)) * sizeof(C);            \
-      auto kern = k_x_c2r_fx<T, FP, Store, DEAD>;                                                  \
-      ensure_smem(kern, smem);                                                                     \
-      LaunchScope ls(ctx, "fft_x_c2r");                                                            \
-      kern<<<(unsigned)x_blocks(f), dim3(Tt, P), smem, ctx->stream>>>(f.g, f.twx, spec, st, done); \
-      ls.done();                                                                                   \
-      return true;                                                                                 \
-    }
+  if (FixedPlan<N_, T_, R0_, R1_, R2_>::matches(f.px))                                             \
+    return launch_x_c2r_fx<T, FixedPlan<N_, T_, R0_, R1_, R2_>, DEAD>(ctx, f, spec, st, done);
+  if constexpr (std::is_same<T, float>::value || W) {
     QSM_FIXED_PLANS(QSM_TRY_XC)
-    if constexpr (W) {
-      QSM_FIXED_PLANS_WIDE(QSM_TRY_XC)
-    }
-#undef QSM_TRY_XC
-    return false;
   }
+  if constexpr (W) {
+    QSM_FIXED_PLANS_WIDE(QSM_TRY_XC)
+  }
+#undef QSM_TRY_XC
+  return false;
+}
+
+// Compile-time X passes between a real array and a half spectrum for every listed length
+// (plain_x32.cu, plain_x64.cu, more_*.cu); x_plain_has says whether the axis is one of them.
+template <typename T>
+bool x_plain_r2c(qsm_ctx* ctx, const Fft3<T>& f, const T* in, cplx_t<T>* spec, const int* done);
+template <typename T>
+bool x_plain_c2r(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* spec, T* out, T scale, const int* done);
+bool plan_listed(const FftPlan1D& pl);
+// Loaders and stores that are just such arrays (functors.cuh).
+template <typename T, class Load> struct PlainLoad : std::false_type {};
+template <typename T, class Store> struct PlainStore : std::false_type {};
+
+// Runtime-engine X passes over plain arrays (real rows, half spectra, full complex rows),
+// compiled once (plain_rt.cu).
+template <typename T>
+void run_x_r2c_rt(qsm_ctx* ctx, const Fft3<T>& f, const T* in, cplx_t<T>* spec, const int* done);
+template <typename T>
+void run_x_c2r_rt(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* spec, T* out, T scale, const int* done);
+template <typename T, int DIR>
+void run_x_c2c_rt(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* rows, const int* done);
+
+// Buffers of the runtime-engine X passes, between the caller's functor and the engine.
+template <typename T> T* x_stage(qsm_ctx* ctx, const Fft3<T>& f) {
+  return f.xstage ? f.xstage : ws_scratch<T>(ctx, sizeof(T) == 4 ? "x.stage32" : "x.stage64", (size_t)f.g.nvox());
+}
+template <typename T> cplx_t<T>* x_stage_c(qsm_ctx* ctx, const Fft3<T>& f) {
+  return ws_scratch<cplx_t<T>>(ctx, sizeof(T) == 4 ? "x.stagec32" : "x.stagec64", (size_t)f.g.hsize());
+}
+// A listed length with a functor that no compile-time kernel carries: the functor as a pass
+// of its own around the plain kernel, except in small volumes, where the launch costs more
+// than the two-factor kernel (functor inside) loses.
+template <typename T> inline bool x_use_stage(const Fft3<T>& f) { return f.g.nvox() > (1LL << 20); }
+inline unsigned x_rows_grid(const Geom& g) {
+  const long long b = ((long long)g.nrows() + 7) / 8;
+  return (unsigned)(b < 1184 ? b : 1184);
 }
 
 // DEAD (compile-time kernels only): the pass reads ld's rows for the last time and drops
@@ -154,15 +236,34 @@ bool run_x_c2r_fixed(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* spec, cons
 template <typename T, bool W = false, bool DEAD = false, class Load>
 void run_x_r2c(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* spec, const Load& ld, const int* done) {
   if (run_x_r2c_fixed<T, W, DEAD>(ctx, f, spec, ld, done)) return;
-  using C = cplx_t<T>;
-  const int Tt = x_block_t(f.px.T);
-  const int P = x_pencils_per_block<T>(f.px.T);
-  const size_t smem = (size_t)(f.px.m + P * x_rowlen<T>(f.px.m)) * sizeof(C);
-  auto kern = f.px.m != f.px.n ? k_x_r2c<T, Load, true> : k_x_r2c<T, Load, false>;
-  ensure_smem(kern, smem);
-  LaunchScope ls(ctx, "fft_x_r2c");
-  kern<<<(unsigned)x_blocks(f), dim3(Tt, P), smem, ctx->stream>>>(f.g, f.px, f.twx, spec, ld, done);
-  ls.done();
+  const bool listed = compiled_plans(ctx) && plan_listed(f.px);
+  if constexpr (PlainLoad<T, Load>::value) {
+    if (listed) {
+      x_plain_r2c<T>(ctx, f, ld.p, spec, done);
+      return;
+    }
+  }
+  if (tf_usable(ctx, f.tfx, tf_x_stride<T>()) && !(listed && x_use_stage(f))) {
+    const size_t smem = tf_smem<T>(f.tfx.n, tf_x_stride<T>());
+    auto kern = k_x_r2c_tf<T, Load>;
+    ensure_smem(kern, smem);
+    LaunchScope ls(ctx, "fft_x_r2c");
+    kern<<<tf_x_grid<T>(((long long)f.g.nrows() + 1) / 2), kTfThreads, smem, ctx->stream>>>(f.g, f.tfx, spec, ld, done);
+    ls.done();
+    return;
+  }
+  if constexpr (PlainLoad<T, Load>::value) {
+    run_x_r2c_rt<T>(ctx, f, ld.p, spec, done);
+    return;
+  }
+  T* st = x_stage(ctx, f);
+  {
+    LaunchScope ls(ctx, "x_load");
+    k_x_load<T, T, Load><<<x_rows_grid(f.g), 256, 0, ctx->stream>>>(f.g, f.g.nx, ld, st, done);
+    ls.done();
+  }
+  if (listed) x_plain_r2c<T>(ctx, f, st, spec, done);
+  else run_x_r2c_rt<T>(ctx, f, st, spec, done);
 }
 
 // DEAD (compile-time kernels only): the pass reads the half spectrum for the last time and
@@ -170,14 +271,31 @@ void run_x_r2c(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* spec, const Load& ld, 
 template <typename T, bool W = false, bool DEAD = false, class Store>
 void run_x_c2r(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* spec, const Store& st, const int* done) {
   if (run_x_c2r_fixed<T, W, DEAD>(ctx, f, spec, st, done)) return;
-  using C = cplx_t<T>;
-  const int Tt = x_block_t(f.px.T);
-  const int P = x_pencils_per_block<T>(f.px.T);
-  const size_t smem = (size_t)(f.px.m + P * x_rowlen<T>(f.px.m)) * sizeof(C);
-  auto kern = f.px.m != f.px.n ? k_x_c2r<T, Store, true> : k_x_c2r<T, Store, false>;
-  ensure_smem(kern, smem);
-  LaunchScope ls(ctx, "fft_x_c2r");
-  kern<<<(unsigned)x_blocks(f), dim3(Tt, P), smem, ctx->stream>>>(f.g, f.px, f.twx, spec, st, done);
+  const bool listed = compiled_plans(ctx) && plan_listed(f.px);
+  if constexpr (PlainStore<T, Store>::value) {
+    if (listed) {
+      x_plain_c2r<T>(ctx, f, spec, st.out, st.scale, done);
+      return;
+    }
+  }
+  if (tf_usable(ctx, f.tfx, tf_x_stride<T>()) && !(listed && x_use_stage(f))) {
+    const size_t smem = tf_smem<T>(f.tfx.n, tf_x_stride<T>());
+    auto kern = k_x_c2r_tf<T, Store>;
+    ensure_smem(kern, smem);
+    LaunchScope ls(ctx, "fft_x_c2r");
+    kern<<<tf_x_grid<T>(((long long)f.g.nrows() + 1) / 2), kTfThreads, smem, ctx->stream>>>(f.g, f.tfx, spec, st, done);
+    ls.done();
+    return;
+  }
+  if constexpr (PlainStore<T, Store>::value) {
+    run_x_c2r_rt<T>(ctx, f, spec, st.out, st.scale, done);
+    return;
+  }
+  T* buf = x_stage(ctx, f);
+  if (listed) x_plain_c2r<T>(ctx, f, spec, buf, T(1), done);
+  else run_x_c2r_rt<T>(ctx, f, spec, buf, T(1), done);
+  LaunchScope ls(ctx, "x_store");
+  k_x_store<T, T, Store><<<x_rows_grid(f.g), 256, 0, ctx->stream>>>(f.g, f.g.nx, buf, st, done);
   ls.done();
 }
 
@@ -208,14 +326,12 @@ void run_x_full(qsm_ctx* ctx, const Fft3<T>& f, const Load& ld, const Mid& mid, 
 #define QSM_TRY_XF(N_, T_, R0_, R1_, R2_)                                                          \
     if (FixedPlan<N_, T_, R0_, R1_, R2_>::matches(f.px)) {                                         \
       using FP = FixedPlan<N_, T_, R0_, R1_, R2_>;                                                 \
-      const int Tt = x_block_t(T_);                                                                \
-      const int P = x_pencils_per_block<T>(T_);                                                    \
+      constexpr int P = x_fx_pencils<FP>();                                                        \
       const size_t smem = (size_t)(x_tw_len<T>(N_) + P * x_rowlen<T>(N_)) * sizeof(C);            \
       auto kern = k_x_full_fx<T, FP, D1, D2, Load, Mid, Store>;                                    \
       ensure_smem(kern, smem);                                                                     \
-      const long long blocks = ((long long)f.g.nrows() + P - 1) / P;                              \
       LaunchScope ls(ctx, name);                                                                   \
-      kern<<<(unsigned)blocks, dim3(Tt, P), smem, ctx->stream>>>(f.g, f.twx, ld, mid, st, done);   \
+      kern<<<x_fx_blocks<FP>(f.g.nrows()), dim3(T_, P), smem, ctx->stream>>>(f.g, f.twx, ld, mid, st, done);   \
       ls.done();                                                                                   \
       return;                                                                                      \
     }
@@ -223,17 +339,30 @@ void run_x_full(qsm_ctx* ctx, const Fft3<T>& f, const Load& ld, const Mid& mid, 
 #undef QSM_TRY_XF
     }
   }
-  if ((f.px.n + f.px.T - 1) / f.px.T > kFftEmax)
-    throw QsmError(QSM_ERR_UNSUPPORTED_SIZE, "x length outside the per-thread register budget");
-  const int Tt = x_block_t(f.px.T);
-  const int P = x_pencils_per_block<T>(f.px.T);
-  const size_t smem = (size_t)(f.px.m + P * x_rowlen<T>(f.px.m)) * sizeof(C);
-  auto kern = f.px.m != f.px.n ? k_x_full<T, D1, D2, Load, Mid, Store, true>
-                                : k_x_full<T, D1, D2, Load, Mid, Store, false>;
-  ensure_smem(kern, smem);
-  const long long blocks = ((long long)f.g.nrows() + P - 1) / P;
-  LaunchScope ls(ctx, name);
-  kern<<<(unsigned)blocks, dim3(Tt, P), smem, ctx->stream>>>(f.g, f.px, f.twx, ld, mid, st, done);
+  if (tf_usable(ctx, f.tfx, tf_x_stride<T>())) {
+    const size_t smem = tf_smem<T>(f.tfx.n, tf_x_stride<T>());
+    auto kern = k_x_full_tf<T, D1, D2, Load, Mid, Store>;
+    ensure_smem(kern, smem);
+    LaunchScope ls(ctx, name);
+    kern<<<tf_x_grid<T>(f.g.nrows()), kTfThreads, smem, ctx->stream>>>(f.g, f.tfx, ld, mid, st, done);
+    ls.done();
+    return;
+  }
+  C* rows = x_stage_c(ctx, f);
+  {
+    LaunchScope ls(ctx, "x_load");
+    k_x_load<T, C, Load><<<x_rows_grid(f.g), 256, 0, ctx->stream>>>(f.g, f.g.pitch, ld, rows, done);
+    ls.done();
+  }
+  if constexpr (D1 != 0) run_x_c2c_rt<T, D1>(ctx, f, rows, done);
+  {
+    LaunchScope ls(ctx, "x_mid");
+    k_x_mid<T, Mid><<<x_rows_grid(f.g), 256, 0, ctx->stream>>>(f.g, mid, rows, done);
+    ls.done();
+  }
+  if constexpr (D2 != 0) run_x_c2c_rt<T, D2>(ctx, f, rows, done);
+  LaunchScope ls(ctx, "x_store");
+  k_x_store<T, C, Store><<<x_rows_grid(f.g), 256, 0, ctx->stream>>>(f.g, f.g.pitch, rows, st, done);
   ls.done();
 }
 
@@ -292,25 +421,6 @@ template <typename T> inline size_t dx_smem(int n, int P) {
 
 template <typename T> inline size_t yz_smem(int n, int P) {
   return (size_t)(((n + 7) & ~7) + 2 * (size_t)n * P) * sizeof(cplx_t<T>);
-}
-
-// Tile width for a Y/Z pass: 128-byte rows, halved while the block (P x T threads)
-// does not fit on an SM (long axes: many threads, registers, shared memory).
-template <typename T, class K> int yz_tile_width(K kernel, int n, int Tn) {
-  constexpr int kMinP = 16 / (int)sizeof(cplx_t<T>) > 0 ? 16 / (int)sizeof(cplx_t<T>) : 1;
-  for (int P = yz_cols<T>(); P >= kMinP; P /= 2) {
-    if (P * Tn > 1024) continue;
-    const size_t smem = yz_smem<T>(n, P);
-    if (smem > 227u * 1024u) continue;
-    ensure_smem(kernel, smem);
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, P * Tn, smem) != cudaSuccess) {
-      (void)cudaGetLastError();
-      continue;
-    }
-    if (per_sm >= 1) return P;
-  }
-  throw QsmError(QSM_ERR_UNSUPPORTED_SIZE, "axis of length " + std::to_string(n) + " does not fit one tile");
 }
 
 // Columns per tile of the compile-time Y/Z passes: 128-byte tile rows (16 float or 8
@@ -384,54 +494,6 @@ bool fx_launch_ok(qsm_ctx* ctx, K kern, int threads, size_t smem, unsigned* grid
   return true;
 }
 
-// One compile-time Y/Z pass (k_pass_yz_dx, FP a FixedPlan) in launch shape `shape`.
-// scoped: count and (when profiling) time the launch under the pass's name.
-template <typename T, int DIR, int AXIS, class FP>
-bool launch_yz_fx(qsm_ctx* ctx, const Fft3<T>& f, int shape, const cplx_t<T>* src, cplx_t<T>* dst,
-                  const int* done, bool scoped) {
-  const cplx_t<T>* tw = (AXIS == 1) ? f.twy : f.twz;
-  auto kern = k_pass_yz_dx<T, DIR, FP, fx_cols<T>()>;
-  const size_t smem = dx_smem<T>(FP::n, fx_cols<T>());
-  const TileWalk w = tile_walk(f, AXIS, fx_cols<T>(), (shape & kTuneEdge) != 0);
-  unsigned grid = 0;
-  if (!fx_launch_ok(ctx, kern, fx_cols<T>() * FP::T, smem, &grid, w.ntiles, (shape & kTuneBlockPerTile) != 0,
-                    tune_bpsm(shape)))
-    return false;
-  if (!scoped) {
-    kern<<<grid, dim3(fx_cols<T>(), FP::T), smem, ctx->stream>>>(f.g, w, tw, src, dst, done);
-    return true;
-  }
-  LaunchScope ls(ctx, AXIS == 1 ? (DIR < 0 ? "fft_y_fwd" : "fft_y_inv") : (DIR < 0 ? "fft_z_fwd" : "fft_z_inv"));
-  kern<<<grid, dim3(fx_cols<T>(), FP::T), smem, ctx->stream>>>(f.g, w, tw, src, dst, done);
-  ls.done();
-  return true;
-}
-
-// Compile-time Y/Z kernels (fx_cols<T>() columns per tile) for the axis lengths of
-// QSM_FIXED_PLANS (and QSM_FIXED_PLANS_WIDE when W); returns false when the plan is not
-// one of them.
-template <typename T, int DIR, int AXIS, bool W>
-bool run_yz_fixed(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const int* done) {
-  if (!compiled_plans(ctx)) return false;
-  {
-    const FftPlan1D& pl = (AXIS == 1) ? f.py : f.pz;
-#define QSM_TRY_YZ(N_, T_, R0_, R1_, R2_)                                                         \
-    if (FixedPlan<N_, T_, R0_, R1_, R2_>::matches(pl) && fx_cols<T>() * T_ <= 1024) {                   \
-      using FP = FixedPlan<N_, T_, R0_, R1_, R2_>;                                                \
-      const int shape = tuned_shape(ctx, yz_tune_key<T>("yz_fx", f, AXIS, DIR));                  \
-      return launch_yz_fx<T, DIR, AXIS, FP>(ctx, f, shape, src, dst, done, true);                 \
-    }
-    QSM_FIXED_PLANS(QSM_TRY_YZ)
-    if constexpr (W) {
-      QSM_FIXED_PLANS_WIDE(QSM_TRY_YZ)
-    }
-#undef QSM_TRY_YZ
-    return false;
-  }
-}
-
-constexpr int kMaxPersistentBlocks = 4096;
-
 // One compile-time operator pass: k_pass_yz_dx_old when the op's epilogue reads a second
 // array (ACC only), k_pass_yz_st_op when its pre hook wants a staged tile, else
 // k_pass_yz_dx_op.  False when the block does not fit.
@@ -487,93 +549,50 @@ bool run_yz_op_fixed(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_
   }
 }
 
-// AXIS 1 = y, 2 = z; DIR -1 forward, +1 inverse; W adds QSM_FIXED_PLANS_WIDE for plain
-// passes and the compile-time operator pass (QSM_FIXED_PLANS) for the others.
-template <typename T, int DIR, int AXIS, bool W = false, class Op>
-void run_yz(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const Op& op, const int* done) {
-  if constexpr (IsPlainOp<Op>::value) {
-    if (run_yz_fixed<T, DIR, AXIS, W>(ctx, f, src, dst, done)) return;
-  } else if constexpr (W) {
-    if (run_yz_op_fixed<T, DIR, AXIS, false>(ctx, f, src, dst, op, nullptr, nullptr, done,
-                                             AXIS == 1 ? (DIR < 0 ? "fft_y_fwd" : "fft_y_inv")
-                                                       : (DIR < 0 ? "fft_z_fwd" : "fft_z_inv")))
-      return;
-  }
-  const FftPlan1D& pl = (AXIS == 1) ? f.py : f.pz;
-  const cplx_t<T>* tw = (AXIS == 1) ? f.twy : f.twz;
-  auto kern = pl.m != pl.n ? k_pass_yz<T, DIR, AXIS, Op, true> : k_pass_yz<T, DIR, AXIS, Op, false>;
-  const int P = yz_tile_width<T>(kern, pl.m, pl.T);
-  const size_t smem = yz_smem<T>(pl.m, P);
-  const TileWalk w = tile_walk(f, AXIS, P);
-  const unsigned grid = persistent_grid(ctx, kern, P * pl.T, smem, w.ntiles);
-  LaunchScope ls(ctx, AXIS == 1 ? (DIR < 0 ? "fft_y_fwd" : "fft_y_inv") : (DIR < 0 ? "fft_z_fwd" : "fft_z_inv"));
-  kern<<<grid, dim3(P, pl.T), smem, ctx->stream>>>(f.g, pl, w, tw, src, dst, op, done);
-  ls.done();
-}
-
-// Y/Z pass with an FP64 accumulation in its post hook (k_pass_yz_acc).  `partials`
-// holds at least kMaxPersistentBlocks doubles; `counter` is 0 between launches.
-template <typename T, int DIR, int AXIS, bool W = false, class Op>
-void run_yz_acc(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const Op& op,
-                double* partials, unsigned* counter, const int* done, const char* name) {
-  if constexpr (W) {
-    if (run_yz_op_fixed<T, DIR, AXIS, true>(ctx, f, src, dst, op, partials, counter, done, name)) return;
-  }
-  const FftPlan1D& pl = (AXIS == 1) ? f.py : f.pz;
-  const cplx_t<T>* tw = (AXIS == 1) ? f.twy : f.twz;
-  auto kern = pl.m != pl.n ? k_pass_yz_acc<T, DIR, AXIS, Op, true> : k_pass_yz_acc<T, DIR, AXIS, Op, false>;
-  const int P = yz_tile_width<T>(kern, pl.m, pl.T);
-  const size_t smem = yz_smem<T>(pl.m, P);
-  const TileWalk w = tile_walk(f, AXIS, P);
-  unsigned grid = persistent_grid(ctx, kern, P * pl.T, smem, w.ntiles);
-  if (grid > (unsigned)kMaxPersistentBlocks) grid = kMaxPersistentBlocks;
+// Two-factor Y/Z pass; false when the axis does not use it.
+template <typename T, int DIR, int AXIS, bool ACC, class Op>
+bool run_yz_tf(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const Op& op, double* partials,
+               unsigned* counter, const int* done, const char* name) {
+  const TwoFactor<T>& ax = AXIS == 1 ? f.tfy : f.tfz;
+  if (!tf_usable(ctx, ax, tf_cols<T>())) return false;
+  const size_t smem = tf_smem<T>(ax.n, tf_cols<T>());
+  auto kern = k_pass_yz_tf<T, DIR, AXIS, Op, ACC>;
+  ensure_smem(kern, smem);
+  const TileWalk w = tile_walk(f, AXIS, tf_cols<T>());
+  unsigned grid = persistent_grid(ctx, kern, kTfThreads, smem, w.ntiles);
+  if (ACC && grid > (unsigned)kMaxPersistentBlocks) grid = kMaxPersistentBlocks;
   LaunchScope ls(ctx, name);
-  kern<<<grid, dim3(P, pl.T), smem, ctx->stream>>>(f.g, pl, w, tw, src, dst, op, partials, counter, done);
-  ls.done();
-}
-
-// n multiplier rows, m tile-buffer rows (m = n except for Bluestein plans)
-template <typename T> inline size_t zm_smem(int n, int m, int P) {
-  return yz_smem<T>(m, P) + 2 * (((size_t)n * P + 3) & ~(size_t)3) * sizeof(T);
-}
-
-// Tile width of the multiplier-array Z pass, 0 when no width fits (very long axes).
-template <typename T> int zm_tile_width(int n, int m, int Tn) {
-  auto kern = m != n ? k_z_fused_m<T, true> : k_z_fused_m<T, false>;
-  for (int p = yz_cols<T>(); p >= 16 / (int)sizeof(T); p /= 2) {
-    if (p * Tn > 1024 || zm_smem<T>(n, m, p) > 227u * 1024u) continue;
-    ensure_smem(kern, zm_smem<T>(n, m, p));
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, p * Tn, zm_smem<T>(n, m, p)) != cudaSuccess) {
-      (void)cudaGetLastError();
-      continue;
-    }
-    if (per_sm >= 1) return p;
-  }
-  return 0;
-}
-
-// One compile-time multiplier Z pass (k_z_fused_m_fx, FP a FixedPlan) in launch shape
-// `shape`; scoped as in launch_yz_fx.
-template <typename T, class FP>
-bool launch_zm_fx(qsm_ctx* ctx, const Fft3<T>& f, int shape, const cplx_t<T>* src, cplx_t<T>* dst, const T* mult,
-                  const int* done, bool scoped) {
-  auto kfx = k_z_fused_m_fx<T, FP, kZmCols>;
-  const size_t smem = zm_smem<T>(FP::n, FP::n, kZmCols);
-  const TileWalk w = tile_walk(f, 2, kZmCols, (shape & kTuneEdge) != 0);
-  unsigned grid = 0;
-  if (!fx_launch_ok(ctx, kfx, kZmCols * FP::T, smem, &grid, w.ntiles, (shape & kTuneBlockPerTile) != 0,
-                    tune_bpsm(shape)))
-    return false;
-  if (!scoped) {
-    kfx<<<grid, dim3(kZmCols, FP::T), smem, ctx->stream>>>(f.g, w, f.twz, src, dst, mult, done);
-    return true;
-  }
-  LaunchScope ls(ctx, "fft_z_fused");
-  kfx<<<grid, dim3(kZmCols, FP::T), smem, ctx->stream>>>(f.g, w, f.twz, src, dst, mult, done);
+  kern<<<grid, kTfThreads, smem, ctx->stream>>>(f.g, ax, w, src, dst, op, partials, counter, done);
   ls.done();
   return true;
 }
+// Two-factor fused Z pass; false when the axis does not use it.
+template <typename T, class Op>
+bool run_z_fused_tf(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const Op& op,
+                    const int* done) {
+  if (!tf_usable(ctx, f.tfz, tf_cols<T>())) return false;
+  const size_t smem = tf_smem<T>(f.tfz.n, tf_cols<T>());
+  auto kern = k_z_fused_tf<T, Op>;
+  ensure_smem(kern, smem);
+  const TileWalk w = tile_walk(f, 2, tf_cols<T>());
+  const unsigned grid = persistent_grid(ctx, kern, kTfThreads, smem, w.ntiles);
+  LaunchScope ls(ctx, "fft_z_fused");
+  kern<<<grid, kTfThreads, smem, ctx->stream>>>(f.g, f.tfz, w, src, dst, op, done);
+  ls.done();
+  return true;
+}
+
+// Plain passes (plain_y*.cu, plain_z*.cu, plain_rt.cu: instantiated once): the compile-time
+// kernel for the lengths of QSM_FIXED_PLANS and QSM_FIXED_PLANS_WIDE, the two-factor
+// kernel, or the runtime engine.
+template <typename T, int DIR, int AXIS>
+void run_yz_plain(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const int* done);
+template <typename T, int DIR, int AXIS>
+void run_yz_rt(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const int* done);
+// Z forward -> precomputed real multiplier array (spectrum layout) -> Z inverse.
+template <typename T>
+void run_z_fused_m(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const T* mult,
+                   const int* done);
 
 // Tune the launch shape of the compile-time Y/Z pass (DIR, AXIS) and of the multiplier
 // Z pass for grid f, running the candidates in place on `scratch` (a half spectrum of f
@@ -583,111 +602,117 @@ bool launch_zm_fx(qsm_ctx* ctx, const Fft3<T>& f, int shape, const cplx_t<T>* sr
 // where it runs: after the pass that fills the L2-resident spectrum, not back to back
 // with itself.  No-op when the lengths have no compile-time pass, the shapes are cached,
 // the autotuner is off or the stream is capturing.
-template <typename T, int DIR, int AXIS, bool W>
-void tune_yz_fixed(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* scratch, const std::function<void()>* chain = nullptr) {
-  {
-    if (!compiled_plans(ctx)) return;
-    const std::string key = yz_tune_key<T>("yz_fx", f, AXIS, DIR);
-    if (!autotune_due(ctx, key)) return;
-    const FftPlan1D& pl = (AXIS == 1) ? f.py : f.pz;
-#define QSM_TUNE_YZ(N_, T_, R0_, R1_, R2_)                                                        \
-    if (FixedPlan<N_, T_, R0_, R1_, R2_>::matches(pl) && fx_cols<T>() * T_ <= 1024) {                   \
-      using FP = FixedPlan<N_, T_, R0_, R1_, R2_>;                                                \
-      auto kern = k_pass_yz_dx<T, DIR, FP, fx_cols<T>()>;                                              \
-      const size_t smem = dx_smem<T>(FP::n, fx_cols<T>());                                             \
-      ensure_smem(kern, smem);                                                                    \
-      const auto cands = yz_candidates(f, fx_cols<T>(), kern, fx_cols<T>() * FP::T, smem);                  \
-      if (chain != nullptr)                                                                       \
-        autotune_pick(ctx, key, cands, [&](int c) { ctx->tuned[key] = TuneRec{c, {}}; (*chain)(); }, 3, 4); \
-      else                                                                                        \
-        autotune_pick(ctx, key, cands, [&](int c) {                                               \
-          launch_yz_fx<T, DIR, AXIS, FP>(ctx, f, c, scratch, scratch, nullptr, false);             \
-        });                                                                                       \
-      return;                                                                                     \
-    }
-    QSM_FIXED_PLANS(QSM_TUNE_YZ)
-    if constexpr (W) {
-      QSM_FIXED_PLANS_WIDE(QSM_TUNE_YZ)
-    }
-#undef QSM_TUNE_YZ
-  }
-}
-
-template <typename T, bool W>
+template <typename T, int DIR, int AXIS>
+void tune_yz_fixed(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* scratch, const std::function<void()>* chain = nullptr);
+template <typename T>
 void tune_z_fused_m(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* scratch, T* mscratch,
-                    const std::function<void()>* chain = nullptr) {
-  if constexpr (std::is_same<T, float>::value) {
-    if (!compiled_plans(ctx)) return;
-    const std::string key = yz_tune_key<T>("zm_fx", f, 2, -1);
-    if (!autotune_due(ctx, key)) return;
-    const FftPlan1D& pl = f.pz;
-#define QSM_TUNE_ZM(N_, T_, R0_, R1_, R2_)                                                        \
-    if (FixedPlan<N_, T_, R0_, R1_, R2_>::matches(pl) && kZmCols * T_ <= 1024) {                   \
-      using FP = FixedPlan<N_, T_, R0_, R1_, R2_>;                                                \
-      auto kfx = k_z_fused_m_fx<T, FP, kZmCols>;                                                  \
-      const size_t smem = zm_smem<T>(FP::n, FP::n, kZmCols);                                      \
-      ensure_smem(kfx, smem);                                                                     \
-      const auto cands = yz_candidates(f, kZmCols, kfx, kZmCols * FP::T, smem);                   \
-      if (chain != nullptr)                                                                       \
-        autotune_pick(ctx, key, cands, [&](int c) { ctx->tuned[key] = TuneRec{c, {}}; (*chain)(); }, 3, 4); \
-      else                                                                                        \
-        autotune_pick(ctx, key, cands, [&](int c) {                                               \
-          launch_zm_fx<T, FP>(ctx, f, c, scratch, scratch, mscratch, nullptr, false);              \
-        });                                                                                       \
-      return;                                                                                     \
-    }
-    QSM_FIXED_PLANS(QSM_TUNE_ZM)
-    if constexpr (W) {
-      QSM_FIXED_PLANS_WIDE(QSM_TUNE_ZM)
-    }
-#undef QSM_TUNE_ZM
+                    const std::function<void()>* chain = nullptr);
+
+#define QSM_MORE_DECLARE(G_)                                                                                      \
+  template <typename T, int DIR, int AXIS>                                                                        \
+  bool more_yz_##G_(qsm_ctx*, const Fft3<T>&, const cplx_t<T>*, cplx_t<T>*, const int*);                           \
+  template <typename T>                                                                                           \
+  bool more_zm_##G_(qsm_ctx*, const Fft3<T>&, const cplx_t<T>*, cplx_t<T>*, const T*, const int*);                 \
+  template <typename T> bool more_xr_##G_(qsm_ctx*, const Fft3<T>&, const T*, cplx_t<T>*, const int*);             \
+  template <typename T> bool more_xc_##G_(qsm_ctx*, const Fft3<T>&, const cplx_t<T>*, T*, T, const int*);
+QSM_MORE_DECLARE(0)
+QSM_MORE_DECLARE(1)
+QSM_MORE_DECLARE(2)
+QSM_MORE_DECLARE(3)
+#undef QSM_MORE_DECLARE
+
+inline const char* yz_name(int axis, int dir) {
+  return axis == 1 ? (dir < 0 ? "fft_y_fwd" : "fft_y_inv") : (dir < 0 ? "fft_z_fwd" : "fft_z_inv");
+}
+inline unsigned spec_grid(const Geom& g) { return (unsigned)(g.nrows() < 2368 ? g.nrows() : 2368); }
+
+// The hooks of a pass as elementwise passes (those that do something) around the plain
+// transform.
+template <typename T, int DIR, int AXIS, class Op>
+void run_yz_hooks(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const Op& op, const int* done) {
+  if constexpr (!NoPre<Op>::value) {
+    LaunchScope ls(ctx, "yz_pre");
+    k_spec_pre<T, Op><<<spec_grid(f.g), 128, 0, ctx->stream>>>(f.g, src, dst, op, done);
+    ls.done();
+    src = dst;
+  }
+  run_yz_plain<T, DIR, AXIS>(ctx, f, src, dst, done);
+  if constexpr (!NoPost<Op>::value) {
+    LaunchScope ls(ctx, "yz_post");
+    k_spec_post<T, Op><<<spec_grid(f.g), 128, 0, ctx->stream>>>(f.g, dst, op, done);
+    ls.done();
   }
 }
 
-// Z fused pass with a precomputed real multiplier array (spectrum layout); W adds
-// QSM_FIXED_PLANS_WIDE.
-template <typename T, bool W = false>
-void run_z_fused_m(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const T* mult,
-                   const int* done) {
-  const FftPlan1D& pl = f.pz;
-  if constexpr (std::is_same<T, float>::value) {
-    if (compiled_plans(ctx)) {
-#define QSM_TRY_ZM(N_, T_, R0_, R1_, R2_)                                                         \
-    if (FixedPlan<N_, T_, R0_, R1_, R2_>::matches(pl) && kZmCols * T_ <= 1024) {                   \
-      using FP = FixedPlan<N_, T_, R0_, R1_, R2_>;                                                \
-      const int shape = tuned_shape(ctx, yz_tune_key<T>("zm_fx", f, 2, -1));                      \
-      if (launch_zm_fx<T, FP>(ctx, f, shape, src, dst, mult, done, true)) return;                 \
-    }
-    QSM_FIXED_PLANS(QSM_TRY_ZM)
+// AXIS 1 = y, 2 = z; DIR -1 forward, +1 inverse.  Passes with hooks take the compile-time
+// operator kernel when W (QSM_FIXED_PLANS); at other listed lengths the hooks run as passes
+// of their own around the compile-time transform, and elsewhere inside the two-factor kernel.
+template <typename T, int DIR, int AXIS, bool W = false, class Op>
+void run_yz(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const Op& op, const int* done) {
+  if constexpr (IsPlainOp<Op>::value) {
+    run_yz_plain<T, DIR, AXIS>(ctx, f, src, dst, done);
+  } else {
     if constexpr (W) {
-      QSM_FIXED_PLANS_WIDE(QSM_TRY_ZM)
+      if (run_yz_op_fixed<T, DIR, AXIS, false>(ctx, f, src, dst, op, nullptr, nullptr, done, yz_name(AXIS, DIR))) return;
     }
-#undef QSM_TRY_ZM
-    }
+    const bool listed = compiled_plans(ctx) && plan_listed(AXIS == 1 ? f.py : f.pz);
+    if (!listed && run_yz_tf<T, DIR, AXIS, false>(ctx, f, src, dst, op, nullptr, nullptr, done, yz_name(AXIS, DIR))) return;
+    run_yz_hooks<T, DIR, AXIS>(ctx, f, src, dst, op, done);
   }
-  auto kern = pl.m != pl.n ? k_z_fused_m<T, true> : k_z_fused_m<T, false>;
-  const int P = zm_tile_width<T>(pl.n, pl.m, pl.T);
-  if (P == 0) throw QsmError(QSM_ERR_UNSUPPORTED_SIZE, "z axis does not fit one multiplier tile");
-  const size_t smem = zm_smem<T>(pl.n, pl.m, P);
-  const TileWalk w = tile_walk(f, 2, P);
-  const unsigned grid = persistent_grid(ctx, kern, P * pl.T, smem, w.ntiles);
-  LaunchScope ls(ctx, "fft_z_fused");
-  kern<<<grid, dim3(P, pl.T), smem, ctx->stream>>>(f.g, pl, w, f.twz, src, dst, mult, done);
+}
+
+// Y/Z pass with an FP64 accumulation in its post hook (as k_pass_yz_tf, ACC).  `partials`
+// holds at least kMaxPersistentBlocks doubles; `counter` is 0 between launches.
+template <typename T, int DIR, int AXIS, bool W = false, class Op>
+void run_yz_acc(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const Op& op,
+                double* partials, unsigned* counter, const int* done, const char* name) {
+  if constexpr (W) {
+    if (run_yz_op_fixed<T, DIR, AXIS, true>(ctx, f, src, dst, op, partials, counter, done, name)) return;
+  }
+  const bool listed = compiled_plans(ctx) && plan_listed(AXIS == 1 ? f.py : f.pz);
+  if (!listed && run_yz_tf<T, DIR, AXIS, true>(ctx, f, src, dst, op, partials, counter, done, name)) return;
+  // dst may be the op's old vector: the transform goes through a buffer of its own
+  cplx_t<T>* t = x_stage_c(ctx, f);
+  if constexpr (!NoPre<Op>::value) {
+    LaunchScope ls(ctx, "yz_pre");
+    k_spec_pre<T, Op><<<spec_grid(f.g), 128, 0, ctx->stream>>>(f.g, src, t, op, done);
+    ls.done();
+    src = t;
+  }
+  run_yz_plain<T, DIR, AXIS>(ctx, f, src, t, done);
+  LaunchScope ls(ctx, name);
+  k_spec_post_acc<T, Op><<<spec_grid(f.g), 128, 0, ctx->stream>>>(f.g, t, dst, op, partials, counter, done);
   ls.done();
 }
 
+// The real multiplier of op.mid as an array (spectrum layout).
+template <typename T, class Op>
+void spec_multiplier(qsm_ctx* ctx, const Fft3<T>& f, const Op& op, T* out, const int* done) {
+  LaunchScope ls(ctx, "z_mult");
+  k_spec_mult<T, Op><<<dim3((unsigned)f.g.ny, (unsigned)f.g.nz), 128, 0, ctx->stream>>>(f.g, op, out, done);
+  ls.done();
+}
+
+// Z forward -> op.mid -> Z inverse, op.mid a real multiplier (v -> m v).  Listed lengths
+// evaluate it once into an array for the compile-time multiplier pass (`array` false where
+// no buffer may be allocated); else the two-factor kernel evaluates it in the pass.
 template <typename T, class Op>
 void run_z_fused(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const Op& op,
-                 const int* done) {
-  const FftPlan1D& pl = f.pz;
-  auto kern = pl.m != pl.n ? k_z_fused<T, Op, true> : k_z_fused<T, Op, false>;
-  const int P = yz_tile_width<T>(kern, pl.m, pl.T);
-  const size_t smem = yz_smem<T>(pl.m, P);
-  const TileWalk w = tile_walk(f, 2, P);
-  const unsigned grid = persistent_grid(ctx, kern, P * pl.T, smem, w.ntiles);
-  LaunchScope ls(ctx, "fft_z_fused");
-  kern<<<grid, dim3(P, pl.T), smem, ctx->stream>>>(f.g, pl, w, f.twz, src, dst, op, done);
-  ls.done();
+                 const int* done, bool array = true) {
+  if (array && compiled_plans(ctx) && plan_listed(f.pz)) {
+    T* m = ws_scratch<T>(ctx, sizeof(T) == 4 ? "z.mult32" : "z.mult64", (size_t)f.g.hsize());
+    spec_multiplier<T>(ctx, f, op, m, done);
+    run_z_fused_m<T>(ctx, f, src, dst, m, done);
+    return;
+  }
+  if (run_z_fused_tf(ctx, f, src, dst, op, done)) return;
+  run_yz_plain<T, -1, 2>(ctx, f, src, dst, done);
+  {
+    LaunchScope ls(ctx, "z_mid");
+    k_spec_mid<T, Op><<<spec_grid(f.g), 128, 0, ctx->stream>>>(f.g, dst, op, done);
+    ls.done();
+  }
+  run_yz_plain<T, +1, 2>(ctx, f, dst, dst, done);
 }
 
 // ---------------------------------------------------------------------------

@@ -137,11 +137,27 @@ extern "C" qsm_status qsm_tkd_device_noalloc(const double* d_local_field, const 
     K.by = bdir[1] / bn;
     K.bz = bdir[2] / bn;
 
+    // two-factor tables where they still fit; otherwise the runtime-engine X passes go
+    // through the output buffer
+    TwoFactor<double>* axes[3] = {&f.tfx, &f.tfy, &f.tfz};
+    for (int a = 0; a < 3; ++a) {
+      TwoFactor<double> ax = plan_two_factor<double>(ns[a]);
+      if (ax.n == 0) continue;
+      const std::vector<double2> h = two_factor_table(ax);
+      const size_t bytes = round256(h.size() * sizeof(double2));
+      if ((size_t)(cur - base) + bytes > kNoAllocScratchBytes) continue;
+      QSM_CUDA(cudaMemcpyAsync(cur, h.data(), h.size() * sizeof(double2), cudaMemcpyHostToDevice, local.stream));
+      ax.tw = reinterpret_cast<const double2*>(cur);
+      cur += bytes;
+      *axes[a] = ax;
+    }
+    f.xstage = d_out_chi;
+
     // the same chain as qsm_tkd_device in double (src/inversion/tkd.rs:48-99); the
     // spectrum is fully written by the first pass, so nothing needs clearing
     run_x_r2c<double>(&local, f, spec, LoadCast<double, double>{d_local_field, d.nx}, nullptr);
     run_yz<double, -1, 1>(&local, f, spec, spec, OpId<double>{}, nullptr);
-    run_z_fused<double>(&local, f, spec, spec, OpTkd<double>{K, params->threshold, 0}, nullptr);
+    run_z_fused<double>(&local, f, spec, spec, OpTkd<double>{K, params->threshold, 0}, nullptr, false);
     run_yz<double, +1, 1>(&local, f, spec, spec, OpId<double>{}, nullptr);
     run_x_c2r<double>(&local, f, spec, StoreMaskedF64<double>{d_out_chi, d_mask, d.nx, 1.0 / (double)d.n}, nullptr);
     QSM_CUDA(cudaStreamSynchronize(local.stream));

@@ -83,12 +83,12 @@ __device__ __forceinline__ void l2_discard_lines(const void* lo, const void* hi,
 // ---------------------------------------------------------------------------
 // X forward: real rows -> half spectrum.  blockDim = (Tb, P) with Tb >= plan T
 // (threads t >= T idle, so blocks stay whole warps); P pencils (row pairs).
-// A thread holds at most kFftEmax elements of a row (T >= n/16), so the loader's
-// global reads are issued as one unrolled batch before any is consumed.
+// A thread holds at most kFftEmax elements of a row (T >= n/16), so its global reads are
+// issued as one unrolled batch before any is consumed.
 // ---------------------------------------------------------------------------
-template <typename T, class Load, bool BL>
+template <typename T, bool BL>
 __global__ void k_x_r2c(Geom g, const __grid_constant__ FftPlan1D pl, const cplx_t<T>* __restrict__ twg,
-                        cplx_t<T>* __restrict__ spec, Load ld, const int* __restrict__ done) {
+                        cplx_t<T>* __restrict__ spec, const T* __restrict__ in, const int* __restrict__ done) {
   using C = cplx_t<T>;
   if (done != nullptr && *done) return;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -116,8 +116,8 @@ __global__ void k_x_r2c(Geom g, const __grid_constant__ FftPlan1D pl, const cplx
       va[c] = T(0);
       vb[c] = T(0);
       if (active && e < n) {
-        va[c] = ld((int)a, e);
-        if (hasb) vb[c] = ld((int)b, e);
+        va[c] = in[a * g.nx + e];
+        if (hasb) vb[c] = in[b * g.nx + e];
       }
     }
 #pragma unroll
@@ -142,16 +142,12 @@ __global__ void k_x_r2c(Geom g, const __grid_constant__ FftPlan1D pl, const cplx
 }
 
 // ---------------------------------------------------------------------------
-// X pass over full complex rows (complex-to-complex spectra: [nz][ny][pitch] with all
-// nx columns valid).  Per row: load -> FFT(D1) -> mid -> FFT(D2) -> store, where a
-// direction of 0 skips that transform.  One row per pencil; blockDim = (Tb, P).
-//   Load : C operator()(int row, int e)
-//   Mid  : C operator()(C v, int row, int e)
-//   Store: void operator()(int row, int e, C v); void finish()
+// X transform of full complex rows in place (complex-to-complex spectra: [nz][ny][pitch]
+// with all nx columns valid).  One row per pencil; blockDim = (Tb, P).
 // ---------------------------------------------------------------------------
-template <typename T, int D1, int D2, class Load, class Mid, class Store, bool BL>
-__global__ void k_x_full(Geom g, const __grid_constant__ FftPlan1D pl, const cplx_t<T>* __restrict__ twg, Load ld,
-                         Mid mid, Store st0, const int* __restrict__ done) {
+template <typename T, int DIR, bool BL>
+__global__ void k_x_c2c(Geom g, const __grid_constant__ FftPlan1D pl, const cplx_t<T>* __restrict__ twg,
+                        cplx_t<T>* __restrict__ rows, const int* __restrict__ done) {
   using C = cplx_t<T>;
   if (done != nullptr && *done) return;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -167,48 +163,58 @@ __global__ void k_x_full(Geom g, const __grid_constant__ FftPlan1D pl, const cpl
   const bool active = row < g.nrows() && t < pl.T;
   C* sp = sm + threadIdx.y * rowlen;
   SAPadded<PadG<T>::G> sa;
-  {
-    C v[kFftEmax];
-#pragma unroll
-    for (int c = 0; c < kFftEmax; ++c) {
-      const int e = t + c * pl.T;
-      v[c] = mk<C>(T(0), T(0));
-      if (active && e < n) v[c] = ld((int)row, e);
-    }
-#pragma unroll
-    for (int c = 0; c < kFftEmax; ++c) {
-      const int e = t + c * pl.T;
-      if (active && e < n) sp[sa(e)] = v[c];
-    }
-  }
-  __syncthreads();
-  if constexpr (D1 != 0) fft_pencil<D1, C, SAPadded<PadG<T>::G>, false, false, BL>(&pl, t, active, sp, sa, tw, nullptr, nullptr, 0, 0);
   if (active)
-    for (int e = t; e < n; e += pl.T) sp[sa(e)] = mid(sp[sa(e)], (int)row, e);
+    for (int e = t; e < n; e += pl.T) sp[sa(e)] = rows[row * g.pitch + e];
   __syncthreads();
-  if constexpr (D2 != 0) fft_pencil<D2, C, SAPadded<PadG<T>::G>, false, false, BL>(&pl, t, active, sp, sa, tw, nullptr, nullptr, 0, 0);
+  fft_pencil<DIR, C, SAPadded<PadG<T>::G>, false, false, BL>(&pl, t, active, sp, sa, tw, nullptr, nullptr, 0, 0);
+  if (active)
+    for (int e = t; e < n; e += pl.T) rows[row * g.pitch + e] = sp[sa(e)];
+}
+
+// Elementwise halves of a runtime-engine X pass: the loader's rows to an array of row
+// pitch `pitch`, the mid hook over complex rows, and the array to the store functor.  A
+// warp takes whole rows.
+template <typename T, typename V, class Load>
+__global__ void __launch_bounds__(256)
+    k_x_load(Geom g, int pitch, Load ld, V* __restrict__ out, const int* __restrict__ done) {
+  if (done != nullptr && *done) return;
+  const int lane = threadIdx.x & 31;
+  for (int row = blockIdx.x * 8 + (threadIdx.x >> 5); row < g.nrows(); row += gridDim.x * 8)
+#pragma unroll 4
+    for (int e = lane; e < g.nx; e += 32) out[(long long)row * pitch + e] = ld(row, e);
+}
+template <typename T, class Mid>
+__global__ void __launch_bounds__(256)
+    k_x_mid(Geom g, Mid mid, cplx_t<T>* __restrict__ rows, const int* __restrict__ done) {
+  if (done != nullptr && *done) return;
+  const int lane = threadIdx.x & 31;
+  for (int row = blockIdx.x * 8 + (threadIdx.x >> 5); row < g.nrows(); row += gridDim.x * 8)
+    for (int e = lane; e < g.nx; e += 32) {
+      cplx_t<T>* q = rows + (long long)row * g.pitch + e;
+      *q = mid(*q, row, e);
+    }
+}
+template <typename T, typename V, class Store>
+__global__ void __launch_bounds__(256)
+    k_x_store(Geom g, int pitch, const V* in, Store st0, const int* __restrict__ done) {
+  if (done != nullptr && *done) return;
+  const int lane = threadIdx.x & 31;
   Store st = st0;
-  {
-    C v[kFftEmax];
-#pragma unroll
-    for (int c = 0; c < kFftEmax; ++c) {
-      const int e = t + c * pl.T;
-      if (active && e < n) v[c] = sp[sa(e)];
-    }
-#pragma unroll
-    for (int c = 0; c < kFftEmax; ++c) {
-      const int e = t + c * pl.T;
-      if (active && e < n) st((int)row, e, v[c]);
-    }
+  for (int row = blockIdx.x * 8 + (threadIdx.x >> 5); row < g.nrows(); row += gridDim.x * 8) {
+#pragma unroll 4
+    for (int e = lane; e < g.nx; e += 32) st(row, e, __ldcg(in + (long long)row * pitch + e));
   }
   st.finish();
 }
 
-// Compile-time form of k_x_full with both transforms (FP a FixedPlan): the first
-// transform's first stage fetches through the loader, its last stage applies the mid
-// hook and passes the values in registers to the second transform (the reversed plan),
-// whose last stage hands its values straight to the store functor, so a row makes three
-// shared-memory round trips fewer than in k_x_full.  Every element of a row is fetched
+// Compile-time X pass over full complex rows with both transforms (FP a FixedPlan), per
+// row load -> FFT(D1) -> mid -> FFT(D2) -> store:
+//   Load : C operator()(int row, int e)
+//   Mid  : C operator()(C v, int row, int e)
+//   Store: void operator()(int row, int e, C v); void finish()
+// The first transform's first stage fetches through the loader, its last stage applies the
+// mid hook and passes the values in registers to the second transform (the reversed plan),
+// whose last stage hands its values straight to the store functor.  Every element of a row is fetched
 // in the first stage, before any store of that row, so the loader and the store may
 // address the same rows.
 template <typename T, class FP, int D1, int D2, class Load, class Mid, class Store>
@@ -251,9 +257,10 @@ __global__ void k_x_full_fx(Geom g, const cplx_t<T>* __restrict__ twg, Load ld, 
 // ---------------------------------------------------------------------------
 constexpr int kXHalfMax = 9;
 
-template <typename T, class Store, bool BL>
+template <typename T, bool BL>
 __global__ void k_x_c2r(Geom g, const __grid_constant__ FftPlan1D pl, const cplx_t<T>* __restrict__ twg,
-                        const cplx_t<T>* __restrict__ spec, Store st0, const int* __restrict__ done) {
+                        const cplx_t<T>* __restrict__ spec, T* __restrict__ out, T scale,
+                        const int* __restrict__ done) {
   using C = cplx_t<T>;
   if (done != nullptr && *done) return;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -302,7 +309,6 @@ __global__ void k_x_c2r(Geom g, const __grid_constant__ FftPlan1D pl, const cplx
   }
   __syncthreads();
   fft_pencil<+1, C, SAPadded<PadG<T>::G>, false, false, BL>(&pl, t, active, sp, sa, tw, nullptr, nullptr, 0, 0);
-  Store st = st0;
   {
     C v[kFftEmax];
 #pragma unroll
@@ -314,12 +320,11 @@ __global__ void k_x_c2r(Geom g, const __grid_constant__ FftPlan1D pl, const cplx
     for (int c = 0; c < kFftEmax; ++c) {
       const int e = t + c * pl.T;
       if (active && e < n) {
-        st((int)a, e, v[c].x);
-        if (hasb) st((int)b, e, v[c].y);
+        out[a * g.nx + e] = v[c].x * scale;
+        if (hasb) out[b * g.nx + e] = v[c].y * scale;
       }
     }
   }
-  st.finish();
 }
 
 // ---------------------------------------------------------------------------
@@ -328,7 +333,7 @@ __global__ void k_x_c2r(Geom g, const __grid_constant__ FftPlan1D pl, const cplx
 // rebuild of the two half-spectrum rows (c2r), and the c2r's last stage hands its
 // values straight to the store functor, so each pass makes one shared-memory round
 // trip fewer than k_x_r2c / k_x_c2r and runs with constant loop bounds.
-// blockDim = (Tb >= FP::T, P) as for the runtime kernels.
+// blockDim = (FP::T, P).
 // DEAD: the pass reads its input for the last time (r2c: the loader's rows, through
 // ld.row_begin; c2r: the half spectrum), so each block drops the L2 lines of its rows
 // (l2_discard_lines) once it has read them, instead of leaving them dirty.
@@ -379,6 +384,11 @@ __global__ void k_x_r2c_fx(Geom g, const cplx_t<T>* __restrict__ twg, cplx_t<T>*
   }
 }
 
+// Stores that take only some rows (wants_row(row)): a block none of whose rows is wanted
+// returns before it reads the spectrum.
+template <class Store, class = void> struct RowFilter : std::false_type {};
+template <class Store> struct RowFilter<Store, std::void_t<decltype(Store::kRowFilter)>> : std::bool_constant<Store::kRowFilter> {};
+
 template <typename T, class FP, class Store, bool DEAD = false>
 __global__ void k_x_c2r_fx(Geom g, const cplx_t<T>* __restrict__ twg, const cplx_t<T>* __restrict__ spec, Store st0,
                            const int* __restrict__ done) {
@@ -395,8 +405,13 @@ __global__ void k_x_c2r_fx(Geom g, const cplx_t<T>* __restrict__ twg, const cplx
   const int p = threadIdx.y;
   const int nrows = g.nrows();
   const int a = 2 * (blockIdx.x * blockDim.y + p), b = a + 1;
-  const bool active = a < nrows && t < TT;
+  bool active = a < nrows && t < TT;
   const bool hasb = b < nrows;
+  if constexpr (RowFilter<Store>::value) {
+    const bool want = active && (st0.wants_row(a) || (hasb && st0.wants_row(b)));
+    if (!__syncthreads_or(want)) return;
+    active = want;
+  }
   C* sp = sm + p * x_rowlen<T>(N);
   SAPadded<PadG<T>::G> sa;
   const C* ra = spec + (long long)a * g.pitch;
@@ -522,14 +537,11 @@ __device__ __forceinline__ void issue_tile(const C* __restrict__ src, C* buf, co
 // Register cap of the tiled Y/Z kernels: three 256-thread CTAs per SM in single
 // precision, three 128-thread CTAs in double.
 template <typename T> struct YzRegCap { static constexpr int value = sizeof(T) == 4 ? 80 : 128; };
-// The fused Z kernels run two transforms around a pointwise op; under the Y/Z cap they
-// spill (float: ~0.1 KB, double: ~1.5 KB per thread), so they get a larger one.
-template <typename T> struct ZRegCap { static constexpr int value = sizeof(T) == 4 ? 128 : 168; };
 
-template <typename T, int DIR, int AXIS, class Op, bool BL>
+template <typename T, int DIR, bool BL>
 __global__ void __maxnreg__(YzRegCap<T>::value)
     k_pass_yz(Geom g, const __grid_constant__ FftPlan1D pl, TileWalk w, const cplx_t<T>* __restrict__ twg,
-                          const cplx_t<T>* src, cplx_t<T>* dst, Op op, const int* __restrict__ done) {
+              const cplx_t<T>* src, cplx_t<T>* dst, const int* __restrict__ done) {
   using C = cplx_t<T>;
   if (done != nullptr && *done) return;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -559,27 +571,7 @@ __global__ void __maxnreg__(YzRegCap<T>::value)
     const int col = tx * P + px;
     const bool active = col < g.nxh;
     const long long base = col + (long long)outer * w.ostride;
-    C* sp = cur + px;
-    if constexpr (IsPlainOp<Op>::value) {
-      fft_pencil<DIR, C, SAStrided, false, true, BL>(&pl, t, active, sp, sa, tw, nullptr, dst, base, w.estride);
-    } else {
-      if (active) {
-        for (int e = t; e < n; e += pl.T) {
-          const long long idx = base + e * w.estride;
-          sp[sa(e)] = (AXIS == 1) ? op.pre(sp[sa(e)], col, e, outer, idx) : op.pre(sp[sa(e)], col, outer, e, idx);
-        }
-      }
-      __syncthreads();
-      fft_pencil<DIR, C, SAStrided, false, false, BL>(&pl, t, active, sp, sa, tw, nullptr, nullptr, 0, 0);
-      if (active) {
-        for (int e = t; e < n; e += pl.T) {
-          const long long idx = base + e * w.estride;
-          const C v = sp[sa(e)];
-          dst[idx] = (AXIS == 1) ? op.post(v, col, e, outer, idx) : op.post(v, col, outer, e, idx);
-        }
-      }
-      __syncthreads();
-    }
+    fft_pencil<DIR, C, SAStrided, false, true, BL>(&pl, t, active, cur + px, sa, tw, nullptr, dst, base, w.estride);
   }
   cp_async_wait<0>();
 }
@@ -653,64 +645,58 @@ __device__ __forceinline__ bool grid_sum_last(double (&a)[K], double* __restrict
   return true;
 }
 
-// Y/Z pass whose post hook also accumulates one FP64 value per element
-// (post(v, ix, iy, iz, idx, acc) returns the value to store).  The block that
-// finishes last reduces the sums and runs op.last(total) on its thread 0.
-template <typename T, int DIR, int AXIS, class Op, bool BL>
-__global__ void __maxnreg__(YzRegCap<T>::value)
-    k_pass_yz_acc(Geom g, const __grid_constant__ FftPlan1D pl, TileWalk w, const cplx_t<T>* __restrict__ twg,
-                  const cplx_t<T>* src, cplx_t<T>* dst, Op op, double* __restrict__ partials, unsigned* counter,
-                  const int* __restrict__ done) {
-  using C = cplx_t<T>;
-  if (done != nullptr && *done) return;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  C* tw = reinterpret_cast<C*>(smraw);
-  const int n = pl.n;
-  const int m = pl.m;  // rows of a tile buffer: n, or the Bluestein convolution length
-  const int P = blockDim.x;
-  C* buf0 = tw + ((m + 7) & ~7);
-  C* buf1 = buf0 + (size_t)m * P;
-  const int tid = threadIdx.x + threadIdx.y * blockDim.x;
-  for (int i = tid; i < m; i += blockDim.x * blockDim.y) tw[i] = twg[i];
-  const int px = threadIdx.x;
-  const int t = threadIdx.y;
-  SAStrided sa{P};
-  double acc[1] = {0.0};
-  int tile = blockIdx.x;
-  if (tile < w.ntiles) issue_tile(src, buf0, g, w, tile, n, P);
-  cp_async_commit();
-  for (int it = 0; tile < w.ntiles; tile += gridDim.x, ++it) {
-    C* cur = (it & 1) ? buf1 : buf0;
-    C* nxt = (it & 1) ? buf0 : buf1;
-    const int next = tile + gridDim.x;
-    if (next < w.ntiles) issue_tile(src, nxt, g, w, next, n, P);
-    cp_async_commit();
-    cp_async_wait<1>();
-    __syncthreads();
-    const int tx = tile % w.ntx, outer = tile / w.ntx;
-    const int col = tx * P + px;
-    const bool active = col < g.nxh;
-    const long long base = col + (long long)outer * w.ostride;
-    C* sp = cur + px;
-    if (active) {
-      for (int e = t; e < n; e += pl.T) {
-        const long long idx = base + e * w.estride;
-        sp[sa(e)] = (AXIS == 1) ? op.pre(sp[sa(e)], col, e, outer, idx) : op.pre(sp[sa(e)], col, outer, e, idx);
-      }
-    }
-    __syncthreads();
-    fft_pencil<DIR, C, SAStrided, false, false, BL>(&pl, t, active, sp, sa, tw, nullptr, nullptr, 0, 0);
-    if (active) {
-      for (int e = t; e < n; e += pl.T) {
-        const long long idx = base + e * w.estride;
-        const C v = sp[sa(e)];
-        dst[idx] = (AXIS == 1) ? op.post(v, col, e, outer, idx, acc[0]) : op.post(v, col, outer, e, idx, acc[0]);
-      }
-    }
-    __syncthreads();
+// Operators with an identity pre or post hook (kNoPre, kNoPost).
+template <class Op, class = void> struct NoPre : std::false_type {};
+template <class Op> struct NoPre<Op, std::void_t<decltype(Op::kNoPre)>> : std::bool_constant<Op::kNoPre> {};
+template <class Op, class = void> struct NoPost : std::false_type {};
+template <class Op> struct NoPost<Op, std::void_t<decltype(Op::kNoPost)>> : std::bool_constant<Op::kNoPost> {};
+
+// Elementwise hooks of a spectrum (hook order and coordinates as the Y/Z passes); a block
+// walks rows.
+template <typename T, class F> __device__ __forceinline__ void spec_each(const Geom& g, const F& f) {
+  for (int row = blockIdx.x; row < g.nrows(); row += gridDim.x) {
+    const int iz = row / g.ny, iy = row - iz * g.ny;
+    const long long r = (long long)row * g.pitch;
+    for (int ix = threadIdx.x; ix < g.nxh; ix += blockDim.x) f(ix, iy, iz, r + ix);
   }
-  cp_async_wait<0>();
-  if (grid_sum_last<1>(acc, partials, counter) && tid == 0) op.last(acc[0]);
+}
+template <typename T, class Op>
+__global__ void __launch_bounds__(128)
+    k_spec_pre(Geom g, const cplx_t<T>* src, cplx_t<T>* dst, Op op, const int* __restrict__ done) {
+  if (done != nullptr && *done) return;
+  spec_each<T>(g, [&](int ix, int iy, int iz, long long i) { dst[i] = op.pre(src[i], ix, iy, iz, i); });
+}
+template <typename T, class Op>
+__global__ void __launch_bounds__(128) k_spec_post(Geom g, cplx_t<T>* dst, Op op, const int* __restrict__ done) {
+  if (done != nullptr && *done) return;
+  spec_each<T>(g, [&](int ix, int iy, int iz, long long i) { dst[i] = op.post(dst[i], ix, iy, iz, i); });
+}
+template <typename T, class Op>
+__global__ void __launch_bounds__(128) k_spec_mid(Geom g, cplx_t<T>* dst, Op op, const int* __restrict__ done) {
+  if (done != nullptr && *done) return;
+  spec_each<T>(g, [&](int ix, int iy, int iz, long long i) { dst[i] = op.mid(dst[i], ix, iy, iz, i); });
+}
+// The real multiplier of op.mid as an array (spectrum layout, padding columns 0); one block
+// per row.
+template <typename T, class Op>
+__global__ void __launch_bounds__(128)
+    k_spec_mult(Geom g, Op op, T* __restrict__ out, const int* __restrict__ done) {
+  if (done != nullptr && *done) return;
+  using C = cplx_t<T>;
+  const int iy = blockIdx.x, iz = blockIdx.y;
+  const long long row = ((long long)iz * g.ny + iy) * g.pitch;
+  for (int ix = threadIdx.x; ix < g.pitch; ix += 128)
+    out[row + ix] = ix < g.nxh ? op.mid(mk<C>(T(1), T(0)), ix, iy, iz, row + ix).x : T(0);
+}
+// The block that finishes last reduces the sums and runs op.last(total) on its thread 0.
+template <typename T, class Op>
+__global__ void __launch_bounds__(128)
+    k_spec_post_acc(Geom g, const cplx_t<T>* src, cplx_t<T>* dst, Op op, double* __restrict__ partials,
+                    unsigned* counter, const int* __restrict__ done) {
+  if (done != nullptr && *done) return;
+  double acc[1] = {0.0};
+  spec_each<T>(g, [&](int ix, int iy, int iz, long long i) { dst[i] = op.post(src[i], ix, iy, iz, i, acc[0]); });
+  if (grid_sum_last<1>(acc, partials, counter) && threadIdx.x == 0) op.last(acc[0]);
 }
 
 // ------------------------------------------------------------------------------
@@ -734,11 +720,6 @@ template <int P> struct SAStridedC {
   __device__ __forceinline__ int operator()(int e) const { return e * P; }
 };
 
-template <typename T, class FP, int P>
-__global__ void __launch_bounds__(P* FP::T, (P * FP::T <= 256 ? 3 : 1))
-    k_z_fused_m_fx(Geom g, TileWalk w, const cplx_t<T>* __restrict__ twg, const cplx_t<T>* src, cplx_t<T>* dst,
-                   const T* __restrict__ mult, const int* __restrict__ done);
-
 // Real multiplier tile (same tile walk, element size sizeof(T)), 16-byte chunks.
 template <typename T>
 __device__ __forceinline__ void issue_mtile(const T* __restrict__ src, T* buf, const Geom& g, const TileWalk& w,
@@ -758,63 +739,6 @@ __device__ __forceinline__ void issue_mtile(const T* __restrict__ src, T* buf, c
     const T* gp = src + base + (long long)e * w.estride + (ok ? ch * kPer : 0);
     cp_async16(buf + e * P + ch * kPer, gp, ok);
   }
-}
-
-// Z forward -> multiply by a precomputed real multiplier -> Z inverse.  The
-// multiplier (spectrum layout, real) is staged with the spectrum tile, so the
-// pointwise step is one shared-memory read per element.  Needs P*sizeof(T) >= 16.
-template <typename T, bool BL>
-__global__ void __maxnreg__(ZRegCap<T>::value) k_z_fused_m(Geom g, const __grid_constant__ FftPlan1D pl, TileWalk w,
-                            const cplx_t<T>* __restrict__ twg, const cplx_t<T>* src, cplx_t<T>* dst,
-                            const T* __restrict__ mult, const int* __restrict__ done) {
-  using C = cplx_t<T>;
-  if (done != nullptr && *done) return;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  C* tw = reinterpret_cast<C*>(smraw);
-  const int n = pl.n;
-  const int m = pl.m;  // rows of a tile buffer: n, or the Bluestein convolution length
-  const int P = blockDim.x;
-  C* buf0 = tw + ((m + 7) & ~7);
-  C* buf1 = buf0 + (size_t)m * P;
-  T* mb0 = reinterpret_cast<T*>(buf1 + (size_t)m * P);
-  T* mb1 = mb0 + (((size_t)n * P + 3) & ~(size_t)3);
-  const int tid = threadIdx.x + threadIdx.y * blockDim.x;
-  for (int i = tid; i < m; i += blockDim.x * blockDim.y) tw[i] = twg[i];
-  const int px = threadIdx.x;
-  const int t = threadIdx.y;
-  SAStrided sa{P};
-  int tile = blockIdx.x;
-  if (tile < w.ntiles) {
-    issue_tile(src, buf0, g, w, tile, n, P);
-    issue_mtile(mult, mb0, g, w, tile, n, P);
-  }
-  cp_async_commit();
-  for (int it = 0; tile < w.ntiles; tile += gridDim.x, ++it) {
-    C* cur = (it & 1) ? buf1 : buf0;
-    C* nxt = (it & 1) ? buf0 : buf1;
-    T* mcur = (it & 1) ? mb1 : mb0;
-    T* mnxt = (it & 1) ? mb0 : mb1;
-    const int next = tile + gridDim.x;
-    if (next < w.ntiles) {
-      issue_tile(src, nxt, g, w, next, n, P);
-      issue_mtile(mult, mnxt, g, w, next, n, P);
-    }
-    cp_async_commit();
-    cp_async_wait<1>();
-    __syncthreads();
-    const int tx = tile % w.ntx, iy = tile / w.ntx;
-    const int col = tx * P + px;
-    const bool active = col < g.nxh;
-    const long long base = col + (long long)iy * w.ostride;
-    C* sp = cur + px;
-    fft_pencil<-1, C, SAStrided, false, false, BL>(&pl, t, active, sp, sa, tw, nullptr, nullptr, 0, 0);
-    if (active) {
-      for (int e = t; e < n; e += pl.T) sp[sa(e)] = cscale(sp[sa(e)], mcur[e * P + px]);
-    }
-    __syncthreads();
-    fft_pencil<+1, C, SAStrided, false, true, BL>(&pl, t, active, sp, sa, tw, nullptr, dst, base, w.estride);
-  }
-  cp_async_wait<0>();
 }
 
 // Compile-time Y/Z pass (FP a FixedPlan, P columns per tile) in direct-fetch form: the
@@ -1016,8 +940,8 @@ __global__ void __launch_bounds__(P* FP::T, yz_dx_min_blocks<T, P * FP::T>())
       for (int e = t; e < n; e += FP::T) {
         const long long idx = base + e * w.estride;
         const C o = osrc != nullptr ? obuf[e * P + px] : mk<C>(T(0), T(0));
-        dst[idx] = (AXIS == 1) ? op.post_old(sp[sa(e)], col, e, outer, o, sc, acc[0])
-                               : op.post_old(sp[sa(e)], col, outer, e, o, sc, acc[0]);
+        dst[idx] = (AXIS == 1) ? op.post_old(sp[sa(e)], col, e, outer, idx, o, sc, acc[0])
+                               : op.post_old(sp[sa(e)], col, outer, e, idx, o, sc, acc[0]);
       }
     }
     __syncthreads();  // the next tile's copies and transform overwrite both buffers
@@ -1037,14 +961,15 @@ template <int THREADS, int BUDGET = 512> constexpr int zm_min_blocks() {
 // blocks, at most 102 registers) where that compiles without spills, as for the 176-point
 // benchmark axis (TV-ADMM 256x256x176: 2 us per iteration less); 512 for the lengths whose
 // plan spilled at 640 (ptxas: 4-92 bytes per thread).
-template <int N> constexpr int zm_budget() {
+template <typename T, int N> constexpr int zm_budget() {
+  if (sizeof(T) == 8) return 384;  // twice the registers per value (168 at 128 threads)
   return (N == 75 || N == 125 || N == 128 || N == 135 || N == 150 || N == 180 || N == 216 || N == 224 ||
           N == 225 || N == 240 || N == 256)
              ? 512
              : 640;
 }
 template <typename T, class FP, int P>
-__global__ void __launch_bounds__(P* FP::T, zm_min_blocks<P * FP::T, zm_budget<FP::n>()>())
+__global__ void __launch_bounds__(P* FP::T, zm_min_blocks<P * FP::T, zm_budget<T, FP::n>()>())
     k_z_fused_m_fx(Geom g, TileWalk w, const cplx_t<T>* __restrict__ twg, const cplx_t<T>* src, cplx_t<T>* dst,
                    const T* __restrict__ mult, const int* __restrict__ done) {
   using C = cplx_t<T>;
@@ -1097,52 +1022,6 @@ __global__ void __launch_bounds__(P* FP::T, zm_min_blocks<P * FP::T, zm_budget<F
     C v[kFftEmax];
     FP::template run_v<-1>(v, t, active, sp, sa, tw, fetch, keep);
     ReversePlan<FP>::type::template run_v<+1>(v, t, active, sp, sa, tw, in_regs, emit);
-  }
-  cp_async_wait<0>();
-}
-
-// Z forward -> Op::mid pointwise -> Z inverse, tiled like k_pass_yz (outer = y).
-template <typename T, class Op, bool BL>
-__global__ void __maxnreg__(ZRegCap<T>::value)
-    k_z_fused(Geom g, const __grid_constant__ FftPlan1D pl, TileWalk w, const cplx_t<T>* __restrict__ twg,
-                          const cplx_t<T>* src, cplx_t<T>* dst, Op op, const int* __restrict__ done) {
-  using C = cplx_t<T>;
-  if (done != nullptr && *done) return;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  C* tw = reinterpret_cast<C*>(smraw);
-  const int n = pl.n;
-  const int m = pl.m;  // rows of a tile buffer: n, or the Bluestein convolution length
-  const int P = blockDim.x;
-  C* buf0 = tw + ((m + 7) & ~7);
-  C* buf1 = buf0 + (size_t)m * P;
-  const int tid = threadIdx.x + threadIdx.y * blockDim.x;
-  for (int i = tid; i < m; i += blockDim.x * blockDim.y) tw[i] = twg[i];
-  const int px = threadIdx.x;
-  const int t = threadIdx.y;
-  SAStrided sa{P};
-  int tile = blockIdx.x;
-  if (tile < w.ntiles) issue_tile(src, buf0, g, w, tile, n, P);
-  cp_async_commit();
-  for (int it = 0; tile < w.ntiles; tile += gridDim.x, ++it) {
-    C* cur = (it & 1) ? buf1 : buf0;
-    C* nxt = (it & 1) ? buf0 : buf1;
-    const int next = tile + gridDim.x;
-    if (next < w.ntiles) issue_tile(src, nxt, g, w, next, n, P);
-    cp_async_commit();
-    cp_async_wait<1>();
-    __syncthreads();
-    const int tx = tile % w.ntx, iy = tile / w.ntx;
-    const int col = tx * P + px;
-    const bool active = col < g.nxh;
-    const long long base = col + (long long)iy * w.ostride;
-    C* sp = cur + px;
-    fft_pencil<-1, C, SAStrided, false, false, BL>(&pl, t, active, sp, sa, tw, nullptr, nullptr, 0, 0);
-    if (active) {
-#pragma unroll 1
-      for (int e = t; e < n; e += pl.T) sp[sa(e)] = op.mid(sp[sa(e)], col, iy, e, base + e * w.estride);
-    }
-    __syncthreads();
-    fft_pencil<+1, C, SAStrided, false, true, BL>(&pl, t, active, sp, sa, tw, nullptr, dst, base, w.estride);
   }
   cp_async_wait<0>();
 }

@@ -86,38 +86,11 @@ __global__ void k_rts_mult(Geom g, KSpace K, double delta, double mu, double rho
   }
 }
 
-// in-kernel form of the same multiplier (very long z axes)
-template <typename T> struct OpRtsMul {
-  using C = cplx_t<T>;
-  KSpace K;
-  double delta, mu, rho;
-  __device__ __forceinline__ C mid(C v, int ix, int iy, int iz, long long) const {
-    const KSpace& k = K;
-    const double m = K.sym(ix, iy, iz, [&](double kx, double ky, double kz, int a, int b, int c) {
-      double mm = 0.0;
-      return rts_inv_a(k, k.dipole(kx, ky, kz), a, b, c, delta, mu, rho, &mm);
-    });
-    return cscale(v, (T)m);
-  }
-};
-
 template <typename T>
 __global__ void k_sub(long long N, const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ out) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x)
     out[i] = a[i] - b[i];
 }
-
-template <typename T> struct StoreMaskedT {
-  T* out;
-  const uint8_t* mask;
-  int nx;
-  T scale;
-  __device__ __forceinline__ void operator()(int row, int e, T v) {
-    const long long i = (long long)row * nx + e;
-    out[i] = mask[i] != 0 ? v * scale : T(0);
-  }
-  __device__ __forceinline__ void finish() {}
-};
 
 }  // namespace
 
@@ -125,9 +98,11 @@ template <typename T>
 void rts_impl(qsm_ctx* ctx, const GridDims& d, const double* f, const uint8_t* mask, const double bdir[3],
               const qsm_rts_params& p, qsm_progress_fn progress, void* user, double* out) {
   const std::string pre = sizeof(T) == 4 ? "rts32." : "rts64.";
+  if ((size_t)plan_or_throw(d.nz).m * 36 * sizeof(T) / sizeof(float) > 227u * 1024u && d.nz > 1024)
+    throw QsmError(QSM_ERR_UNSUPPORTED_SIZE, "z axis too long for the RTS multiplier tiles");
   TvState* st = ws<TvState>(ctx, pre + "state", 1);
   TvVol<T> v;
-  tv_alloc<T>(ctx, v, pre, d, bdir, 1.0, 1.0 / p.rho, st, mask, out);
+  tv_alloc<T>(ctx, v, pre, d, 1.0 / p.rho, st, mask, out);
   const KSpace K = make_kspace(ctx, d, bdir);
   T* x1 = ws<T>(ctx, pre + "x1", (size_t)d.n);
   // step 1: x_1 = mask * Re IFFT(F(f) * c(D))
@@ -150,7 +125,6 @@ void rts_impl(qsm_ctx* ctx, const GridDims& d, const double* f, const uint8_t* m
     k_rts_mult<T><<<grid1d(v.f.g.hsize()), 256, 0, ctx->stream>>>(v.f.g, K, p.delta, p.mu, p.rho, v.mult);
     ls.done();
   }
-  if (!v.use_mult) throw QsmError(QSM_ERR_UNSUPPORTED_SIZE, "z axis too long for the RTS multiplier tiles");
   ctx->tv_last_iters = tv_run<T>(ctx, v, p.max_iter, p.tol, progress, user);
 }
 

@@ -184,8 +184,7 @@ void tv_unrolled_impl(qsm_ctx* ctx, const GridDims& d, const double* f, const ui
       if (!have_vbar && j != K) throw QsmError(QSM_ERR_CUDA, "adjoint sweep out of order");
       run_x_r2c<T>(ctx, v.f, v.spec, ld, nullptr);
       run_yz<T, -1, 1>(ctx, v.f, v.spec, v.spec, OpId<T>{}, nullptr);
-      if (v.use_mult) run_z_fused_m<T>(ctx, v.f, v.spec, v.spec, v.mult, nullptr);
-      else run_z_fused<T>(ctx, v.f, v.spec, v.spec, v.mul, nullptr);
+      run_z_fused_m<T>(ctx, v.f, v.spec, v.spec, v.mult, nullptr);
       run_yz<T, +1, 1>(ctx, v.f, v.spec, v.spec, OpId<T>{}, nullptr);
       run_x_c2r<T>(ctx, v.f, v.spec, StoreReal<T>{w, d.nx, v.scale}, nullptr);
       // adjoint of U_i from S_i = (y_i, u_{i-1})

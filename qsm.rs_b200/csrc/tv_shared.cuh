@@ -35,21 +35,6 @@ template <typename T> struct OpAdmmRhs {
   }
 };
 
-// per-iteration multiplier rho * sym(inv_a) (admm.rs:105-108), working precision
-template <typename T> struct OpAdmmMul {
-  using C = cplx_t<T>;
-  KSpaceT<T> K;
-  T rho;
-  __device__ __forceinline__ C mid(C v, int ix, int iy, int iz, long long) const {
-    const KSpaceT<T>& k = K;
-    const T r = rho;
-    const T ia = K.sym(ix, iy, iz, [&](T kx, T ky, T kz, int a, int b, int c) {
-      return admm_inv_a<T>(k, kx, ky, kz, a, b, c, r);
-    });
-    return cscale(v, r * ia);
-  }
-};
-
 // Per-iteration multiplier rho*sym(inv_a) as a real half-spectrum array (spectrum
 // layout, padding columns 0), evaluated once per solve in double.
 template <typename T>
@@ -70,14 +55,6 @@ __global__ void k_admm_mult(Geom g, KSpace K, double rho, T* __restrict__ out) {
     out[i] = (T)m;
   }
 }
-
-template <typename T> struct StoreReal {
-  T* __restrict__ out;
-  int nx;
-  T scale;
-  __device__ __forceinline__ void operator()(int row, int e, T v) { out[(long long)row * nx + e] = v * scale; }
-  __device__ __forceinline__ void finish() {}
-};
 
 struct TvState {
   int done;       // 1 once relative_change < tol
@@ -668,7 +645,6 @@ __global__ void k_tv_out(long long N, const T* __restrict__ x0, const T* __restr
 template <typename T> struct TvVol {
   GridDims d;
   Fft3<T> f;
-  OpAdmmMul<T> mul;
   T* x0;
   T* yb[2];
   T* ub[2];
@@ -679,7 +655,7 @@ template <typename T> struct TvVol {
   TvState* st;
   dim3 sgrid;
   int zchunk;
-  bool vec, use_mult;
+  bool vec;
   bool staged = false;  // k_tv_step_s for the full update (unweighted, 16-byte vectors)
   dim3 sgrid_s;
   int zchunk_s = 0;
@@ -700,12 +676,11 @@ extern template void tv_tune<double>(qsm_ctx*, const TvVol<double>&);
 // constants; `thr` is the shrink threshold.  The only work enqueued is the launch-shape
 // tuning of a grid the context has not seen (tv_tune), which overwrites the new buffers.
 template <typename T>
-void tv_alloc(qsm_ctx* ctx, TvVol<T>& v, const std::string& pre, const GridDims& d, const double bdir[3],
-              double rho_mul, double thr, TvState* st, const uint8_t* d_mask, double* d_out) {
+void tv_alloc(qsm_ctx* ctx, TvVol<T>& v, const std::string& pre, const GridDims& d, double thr, TvState* st,
+              const uint8_t* d_mask, double* d_out) {
   using C = cplx_t<T>;
   v.d = d;
   v.f = make_fft3<T>(ctx, d);
-  v.mul = OpAdmmMul<T>{make_kspace_t<T>(ctx, d, bdir), (T)rho_mul};
   const long long N = d.n;
   const long long H = v.f.g.hsize();
   auto nm = [&](const char* s) { return pre + s; };
@@ -747,7 +722,6 @@ void tv_alloc(qsm_ctx* ctx, TvVol<T>& v, const std::string& pre, const GridDims&
   v.mask = d_mask;
   v.out = d_out;
   v.mult = ws<T>(ctx, pre + "mult", (size_t)v.f.g.hsize());
-  v.use_mult = zm_tile_width<T>(d.nz, v.f.pz.m, v.f.pz.T) > 0;
   tv_tune(ctx, v);
 }
 
@@ -767,7 +741,7 @@ template <typename T> void tv_init_state(qsm_ctx* ctx, const TvVol<T>& v, double
 template <typename T>
 void tv_setup(qsm_ctx* ctx, TvVol<T>& v, const std::string& pre, const GridDims& d, const double* d_f,
               const uint8_t* d_mask, const double bdir[3], const qsm_tv_params& p, TvState* st, double* d_out) {
-  tv_alloc<T>(ctx, v, pre, d, bdir, p.rho, p.lambda / p.rho, st, d_mask, d_out);
+  tv_alloc<T>(ctx, v, pre, d, p.lambda / p.rho, st, d_mask, d_out);
   const KSpace K64 = make_kspace(ctx, d, bdir);
   const long long H = v.f.g.hsize();
   run_x_r2c<T>(ctx, v.f, v.spec, LoadCast<double, T>{d_f, d.nx}, nullptr);
@@ -776,8 +750,6 @@ void tv_setup(qsm_ctx* ctx, TvVol<T>& v, const std::string& pre, const GridDims&
   run_yz<T, +1, 1>(ctx, v.f, v.spec, v.spec, OpId<T>{}, nullptr);
   run_x_c2r<T>(ctx, v.f, v.spec, StoreReal<T>{v.x0, d.nx, v.scale}, nullptr);
   tv_init_state<T>(ctx, v, p.tol);
-  // precomputed multiplier tiles need P*sizeof(T) >= 16 (always true for the
-  // 128-byte tiles; narrow tiles of very long z axes use the in-kernel multiplier)
   LaunchScope ls(ctx, "admm_mult");
   k_admm_mult<T><<<grid1d(H), 256, 0, ctx->stream>>>(v.f.g, K64, p.rho, v.mult);
   ls.done();
@@ -814,10 +786,9 @@ template <typename T> void tv_step_launch(qsm_ctx* ctx, const TvVol<T>& v, int q
 // while the stencil streams.
 template <typename T> void tv_fft(qsm_ctx* ctx, const TvVol<T>& v, int q, const int* done) {
   run_x_r2c<T, true, true>(ctx, v.f, v.spec, LoadCast<T, T>{v.div, v.d.nx}, done);
-  run_yz<T, -1, 1, true>(ctx, v.f, v.spec, v.spec, OpId<T>{}, done);
-  if (v.use_mult) run_z_fused_m<T, true>(ctx, v.f, v.spec, v.spec, v.mult, done);
-  else run_z_fused<T>(ctx, v.f, v.spec, v.spec, v.mul, done);
-  run_yz<T, +1, 1, true>(ctx, v.f, v.spec, v.spec, OpId<T>{}, done);
+  run_yz<T, -1, 1>(ctx, v.f, v.spec, v.spec, OpId<T>{}, done);
+  run_z_fused_m<T>(ctx, v.f, v.spec, v.spec, v.mult, done);
+  run_yz<T, +1, 1>(ctx, v.f, v.spec, v.spec, OpId<T>{}, done);
   run_x_c2r<T, true, true>(ctx, v.f, v.spec, StoreReal<T>{v.yb[q], v.d.nx, v.scale}, done);
 }
 extern template void tv_fft<float>(qsm_ctx*, const TvVol<float>&, int, const int*);
@@ -842,9 +813,9 @@ template <typename T> void tv_tune(qsm_ctx* ctx, const TvVol<T>& v) {
     tv_step_launch(ctx, v, 0, 0);
     tv_fft(ctx, v, 0, nullptr);
   };
-  tune_yz_fixed<T, -1, 1, true>(ctx, v.f, v.spec, &chain);
-  tune_yz_fixed<T, +1, 1, true>(ctx, v.f, v.spec, &chain);
-  if (v.use_mult) tune_z_fused_m<T, true>(ctx, v.f, v.spec, v.mult, &chain);
+  tune_yz_fixed<T, -1, 1>(ctx, v.f, v.spec, &chain);
+  tune_yz_fixed<T, +1, 1>(ctx, v.f, v.spec, &chain);
+  tune_z_fused_m<T>(ctx, v.f, v.spec, v.mult, &chain);
 }
 
 template <typename T> void tv_iter(qsm_ctx* ctx, const TvVol<T>& v, int q) {
