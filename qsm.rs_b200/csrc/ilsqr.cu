@@ -1,22 +1,28 @@
 // iLSQR dipole inversion (src/inversion/ilsqr.rs:1307-1351) -> (chi, xsa, xfs, xlsqr).
 //
 // Step 1, lsqr_step (ilsqr.rs:953-1030).  Laplacian weights w (mask-adaptive stencil,
-//   thresholds at the 60th / 99.9th percentile by exact radix selection), b = D*FFT(w*f),
-//   then complex LSQR (ilsqr.rs:177-321, relative-residual stop) on k-space vectors with
-//   A = A^H = D*FFT(w*Re IFFT(D*x)).  The vectors are full complex spectra: D is not
-//   symmetric under k -> -k on even-length Nyquist planes and the reference iterates on
-//   the whole complex vector.  One application of A is five passes,
-//     Z inv (pre: *s*D) -> Y inv -> X [inv, w*Re/N, fwd] -> Y fwd -> Z fwd (post: *D - c*old)
+//   thresholds at the 60th / 99.9th percentile by exact selection), b = D*FFT(w*f), then
+//   complex LSQR (ilsqr.rs:177-321, relative-residual stop) on k-space vectors with
+//   A = A^H = D*FFT(w*Re IFFT(D*x)).  D is not symmetric under k -> -k on even-length
+//   Nyquist planes, so the reference iterates on the whole complex vector; but b and every
+//   output of A are D times the spectrum of a real image, and so is every vector of the
+//   iteration.  The solver therefore holds h = m G on the half spectrum, where D G is the
+//   reference's vector and m(k) = sqrt((D(k)^2 + D(-k)^2)/2).  D G -> m G keeps norms
+//   (summing |h|^2 with c = 2, or 1 on the self-paired columns), and with it
+//     A: h -> m FFT(w IFFT(m h)),
+//   so this is the same iteration on half the values.  One application is five passes,
+//     Z inv (pre: *s*m) -> Y inv -> X [c2r, w/N, r2c] -> Y fwd -> Z fwd (post: *m - c*old)
 //   where s is the deferred 1/beta or 1/alpha of the input vector and the Z fwd pass
 //   also accumulates the FP64 norm of its output.  The block that finishes that pass
 //   last completes the norm and runs the scalar recurrence on the device, so one LSQR
 //   iteration (two applications and the x/w update) is 11 launches without a host
-//   synchronisation, replayed as a CUDA graph.
+//   synchronisation, replayed as a CUDA graph.  (On full spectra an application took 1.85 ms
+//   in FP64 at 384x384x256, and on half spectra 1.04 ms.)
 // Step 2, fastqsm_step (ilsqr.rs:1037-1167).  F = FFT(f); k-space weights |D|^0.001
 //   normalised by the 1st/30th percentiles of all values; the SMV (r = 3) kernel
-//   spectrum; Eq. 9/11 filtering chains with the masked real part taken in the fused X
-//   pass between inverse and forward transforms; TKD (t0 = 1/8, sign(+0) = +1) and the
-//   2x2 least-squares fit over all voxels (FP64 sums).
+//   spectrum; the Eq. 9/11 filters and the TKD (t0 = 1/8, sign(+0) = +1) are real k-space
+//   factors followed by the real part, hence half-spectrum chains with the symmetrised
+//   factor; and the 2x2 least-squares fit over all voxels (FP64 sums).
 // Step 3, susceptibility_artifacts_step (ilsqr.rs:1174-1289).  Gradient weights from
 //   the mask-adaptive gradient of xfs (percentiles 50 / 70 per component); LSMR
 //   (ilsqr.rs:344-517) on real vectors.  Its k-space mask mic = |D| < 0.1 acts through
@@ -26,6 +32,7 @@
 // Step 4: chi = mask * (xlsqr - xsa).
 #include "functors.cuh"
 #include "select.h"
+#include "smv.h"
 #include "solvers.h"
 
 #include <algorithm>
@@ -165,59 +172,6 @@ template <typename T> struct StoreSpecRow {
   __device__ __forceinline__ void operator()(int row, int e, cplx_t<T> v) { s[(long long)row * pitch + e] = v; }
   __device__ __forceinline__ void finish() {}
 };
-// real image value (optionally times a second real array) as a complex row element
-template <typename Tin, typename T> struct LoadRealProduct {
-  const Tin* a;
-  const T* b;  // may be null
-  int nx;
-  __device__ __forceinline__ cplx_t<T> operator()(int row, int e) const {
-    const long long i = (long long)row * nx + e;
-    double v = (double)a[i];
-    if (b != nullptr) v = (double)b[i] * v;
-    return mk<cplx_t<T>>((T)v, T(0));
-  }
-};
-// SMV sphere image (src/kernels/smv.rs:19-67) as a complex row element
-struct SphereImg {
-  int nx, ny, nz;
-  double vsx, vsy, vsz, r2, norm;
-};
-__device__ __forceinline__ double sphere_coord(int i, int n, double vs) { return (double)((i <= n / 2) ? i : i - n) * vs; }
-template <typename T> struct LoadSphereC {
-  SphereImg s;
-  __device__ __forceinline__ cplx_t<T> operator()(int row, int e) const {
-    const int j = row % s.ny, k = row / s.ny;
-    const double dx = sphere_coord(e, s.nx, s.vsx), dy = sphere_coord(j, s.ny, s.vsy), dz = sphere_coord(k, s.nz, s.vsz);
-    const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-    return mk<cplx_t<T>>((T)(d2 <= s.r2 ? s.norm : 0.0), T(0));
-  }
-};
-SphereImg sphere_img(const GridDims& d, double radius) {
-  SphereImg s{d.nx, d.ny, d.nz, d.vsx, d.vsy, d.vsz, radius * radius, 0.0};
-  auto axis = [&](int n, double vs) {
-    std::vector<double> v;
-    for (int i = 0; i < n; ++i) {
-      const double c = (double)((i <= n / 2) ? i : i - n) * vs;
-      if (c * c <= s.r2) v.push_back(c);
-    }
-    return v;
-  };
-  const std::vector<double> ax = axis(d.nx, d.vsx), ay = axis(d.ny, d.vsy), az = axis(d.nz, d.vsz);
-  double count = 0.0;
-  for (double dz : az)
-    for (double dy : ay)
-      for (double dx : ax) {
-        volatile double a = dx * dx;
-        volatile double b = dy * dy;
-        volatile double c = dz * dz;
-        volatile double ab = a + b;
-        volatile double d2 = ab + c;
-        if (d2 <= s.r2) count += 1.0;
-      }
-  s.norm = count > 0.0 ? 1.0 / count : 0.0;
-  return s;
-}
-
 // w * Re(v)/N as a real row element (lsqr_step's apply_a, ilsqr.rs:1000-1003)
 template <typename T> struct MidWeightRe {
   const T* w;
@@ -227,28 +181,6 @@ template <typename T> struct MidWeightRe {
     return mk<cplx_t<T>>(w[(long long)row * nx + e] * (v.x * invn), T(0));
   }
 };
-// mask ? Re(v)/N : 0 as a real row element (fastqsm_step, ilsqr.rs:1093-1100)
-template <typename T> struct MidMaskRe {
-  const uint8_t* m;
-  int nx;
-  T invn;
-  __device__ __forceinline__ cplx_t<T> operator()(cplx_t<T> v, int row, int e) const {
-    return mk<cplx_t<T>>(m[(long long)row * nx + e] != 0 ? v.x * invn : T(0), T(0));
-  }
-};
-// out[i] = mask ? Re(v)/N : 0
-template <typename T, typename Tout> struct StoreMaskRe {
-  Tout* out;
-  const uint8_t* m;
-  int nx;
-  T invn;
-  __device__ __forceinline__ void operator()(int row, int e, cplx_t<T> v) {
-    const long long i = (long long)row * nx + e;
-    out[i] = m[i] != 0 ? (Tout)(v.x * invn) : Tout(0);
-  }
-  __device__ __forceinline__ void finish() {}
-};
-
 // ====================================================================== LSQR ==
 struct LsqrState {
   int done;   // every later kernel returns at once
@@ -259,6 +191,40 @@ struct LsqrState {
   double su, sv;  // deferred scales of u and v: 1/beta and 1/alpha (1 when zero)
   double rho_bar, phi_bar, bnorm, t1, t2, tol;
 };
+
+// The scalar recurrence after the norm of an application's output (modes as OpLsqrOut).
+__device__ inline void lsqr_last(LsqrState* st, int mode, double total) {
+  const double nrm = sqrt(total);
+  if (mode == 0 || mode == 2) {
+    st->beta = nrm;
+    st->su = nrm > 0.0 ? 1.0 / nrm : 1.0;
+    if (mode == 2) {
+      st->bnorm = nrm;
+      st->phi_bar = nrm;
+    }
+    return;
+  }
+  st->alpha = nrm;
+  st->sv = nrm > 0.0 ? 1.0 / nrm : 1.0;
+  if (mode == 3) {
+    st->rho_bar = nrm;
+    if (nrm * st->beta == 0.0) st->done = 1;
+    return;
+  }
+  // Givens rotation and step lengths, src/inversion/ilsqr.rs:261-290
+  const double alpha = nrm, beta = st->beta;
+  const double rho = sqrt(st->rho_bar * st->rho_bar + beta * beta);
+  const double c = st->rho_bar / rho;
+  const double s = beta / rho;
+  const double theta = s * alpha;
+  st->rho_bar = -c * alpha;
+  const double phi = c * st->phi_bar;
+  st->phi_bar *= s;
+  st->t1 = phi / rho;
+  st->t2 = -theta / rho;
+  st->iters += 1;
+  if (st->phi_bar / (st->bnorm + 1e-20) <= st->tol) st->stop = 1;
+}
 
 __device__ __forceinline__ double dip(const KSpace& K, int ix, int iy, int iz) {
   return K.dipole(__ldg(K.fx + ix), __ldg(K.fy + iy), __ldg(K.fz + iz));
@@ -320,39 +286,158 @@ template <typename T> struct OpLsqrOut {
     acc += (double)r.x * (double)r.x + (double)r.y * (double)r.y;
     return r;
   }
-  __device__ void last(double total) const {
-    const double nrm = sqrt(total);
-    if (mode == 0 || mode == 2) {
-      st->beta = nrm;
-      st->su = nrm > 0.0 ? 1.0 / nrm : 1.0;
-      if (mode == 2) {
-        st->bnorm = nrm;
-        st->phi_bar = nrm;
-      }
-      return;
-    }
-    st->alpha = nrm;
-    st->sv = nrm > 0.0 ? 1.0 / nrm : 1.0;
-    if (mode == 3) {
-      st->rho_bar = nrm;
-      if (nrm * st->beta == 0.0) st->done = 1;
-      return;
-    }
-    // Givens rotation and step lengths, src/inversion/ilsqr.rs:261-290
-    const double alpha = nrm, beta = st->beta;
-    const double rho = sqrt(st->rho_bar * st->rho_bar + beta * beta);
-    const double c = st->rho_bar / rho;
-    const double s = beta / rho;
-    const double theta = s * alpha;
-    st->rho_bar = -c * alpha;
-    const double phi = c * st->phi_bar;
-    st->phi_bar *= s;
-    st->t1 = phi / rho;
-    st->t2 = -theta / rho;
-    st->iters += 1;
-    if (st->phi_bar / (st->bnorm + 1e-20) <= st->tol) st->stop = 1;
+  __device__ void last(double total) const { lsqr_last(st, mode, total); }
+};
+
+// v * s * m: the input of A, s its deferred scale
+template <typename T> struct OpScaleM {
+  using C = cplx_t<T>;
+  const T* m;
+  const double* s;
+  static constexpr bool kNoPost = true;
+  __device__ __forceinline__ C pre(C v, int, int, int, long long idx) const {
+    return cscale(cscale(v, (T)__ldg(s)), __ldg(m + idx));
+  }
+  __device__ __forceinline__ C post(C v, int, int, int, long long) const { return v; }
+};
+
+// Z forward epilogue of an application of A on half spectra; modes as OpLsqrOut.
+template <typename T> struct OpLsqrHalf {
+  using C = cplx_t<T>;
+  const T* m;
+  int nx;
+  const C* old;
+  LsqrState* st;
+  int mode;
+  static constexpr bool kReadsOld = true;
+  static constexpr bool kNoPre = true;
+  struct Scalars {
+    double coef, sc;
+  };
+  __device__ __forceinline__ C pre(C v, int, int, int, long long) const { return v; }
+  __device__ __forceinline__ const C* old_src() const { return mode <= 1 ? old : nullptr; }
+  __device__ __forceinline__ Scalars scalars() const {
+    if (mode > 1) return Scalars{0.0, 0.0};
+    return Scalars{mode == 0 ? -st->alpha : -st->beta, mode == 0 ? st->su : st->sv};
+  }
+  __device__ __forceinline__ C post_old(C v, int ix, int, int, long long idx, C oldv, const Scalars& s,
+                                        double& acc) const {
+    C r = cscale(v, __ldg(m + idx));
+    if (mode <= 1) r = cadd(r, cscale(cscale(oldv, (T)s.sc), (T)s.coef));
+    const double c = (ix == 0 || 2 * ix == nx) ? 1.0 : 2.0;
+    acc += c * ((double)r.x * (double)r.x + (double)r.y * (double)r.y);
+    return r;
+  }
+  __device__ __forceinline__ C post(C v, int ix, int iy, int iz, long long idx, double& acc) const {
+    return post_old(v, ix, iy, iz, idx, mode <= 1 ? old[idx] : v, scalars(), acc);
+  }
+  __device__ void last(double total) const { lsqr_last(st, mode, total); }
+};
+
+// m = sqrt(sym(D^2)), and sym(D) / m (0 where m is), which takes h to the reference's
+// spectrum under the real part
+template <typename T> struct OpHalfD {
+  using C = cplx_t<T>;
+  KSpace K;
+  int ratio;
+  __device__ __forceinline__ C mid(C v, int ix, int iy, int iz, long long) const {
+    const KSpace& k = K;
+    const double m = sqrt(K.sym(ix, iy, iz, [&](double kx, double ky, double kz, int, int, int) {
+      const double d = k.dipole(kx, ky, kz);
+      return d * d;
+    }));
+    if (!ratio) return cscale(v, (T)m);
+    const double d = K.sym(ix, iy, iz, [&](double kx, double ky, double kz, int, int, int) { return k.dipole(kx, ky, kz); });
+    return cscale(v, (T)(m > 0.0 ? d / m : 0.0));
   }
 };
+
+// X pass of an application of A: half spectrum -> real rows -> * w / N -> half spectrum, in
+// place (FP a FixedPlan).  Two rows are one complex pencil; the inverse transform's last
+// stage weights its values in registers and hands them to the forward transform (the
+// reversed plan), whose results are split into the two half spectra.
+template <typename T, class FP>
+__global__ void k_x_weight_fx(Geom g, const cplx_t<T>* __restrict__ twg, cplx_t<T>* __restrict__ spec,
+                              const T* __restrict__ w, T invn, const int* __restrict__ done) {
+  using C = cplx_t<T>;
+  constexpr int N = FP::n, TT = FP::T, NXH = N / 2 + 1;
+  if (done != nullptr && *done) return;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  constexpr bool TWP = x_tw_padded<T>();
+  C* tw = reinterpret_cast<C*>(smraw);
+  C* sm = tw + x_tw_len<T>(N);
+  const int tid = threadIdx.x + threadIdx.y * blockDim.x;
+  for (int i = tid; i < N; i += blockDim.x * blockDim.y) tw[TWP ? tw_pad(i) : i] = twg[i];
+  const int t = threadIdx.x;
+  const int nrows = g.nrows();
+  const int a = 2 * (blockIdx.x * blockDim.y + threadIdx.y), b = a + 1;
+  const bool active = a < nrows && t < TT;
+  const bool hasb = b < nrows;
+  C* sp = sm + threadIdx.y * x_rowlen<T>(N);
+  SAPadded<PadG<T>::G> sa;
+  C* ra = spec + (long long)a * g.pitch;
+  C* rb = spec + (long long)b * g.pitch;
+  auto fetch = [&](int e) -> C {
+    const bool lo = e <= N / 2;
+    const int k = lo ? e : N - e;
+    C xa = ra[k];
+    C xb = hasb ? rb[k] : mk<C>(T(0), T(0));
+    if (k == 0 || 2 * k == N) {
+      xa.y = T(0);
+      xb.y = T(0);
+    }
+    return lo ? mk<C>(xa.x - xb.y, xa.y + xb.x) : mk<C>(xa.x + xb.y, xb.x - xa.y);
+  };
+  const T* wa = w + (long long)a * N;
+  auto hook = [&](int e, C x) -> C {
+    return mk<C>(__ldg(wa + e) * (x.x * invn), hasb ? __ldg(wa + N + e) * (x.y * invn) : T(0));
+  };
+  auto emit = [&](int e, C v) { sp[sa(e)] = v; };
+  C v[kFftEmax];
+  EmitInRegs<decltype(hook)> keep{hook};
+  FetchInRegs in_regs;
+  FP::template run_v<+1, TWP>(v, t, active, sp, sa, tw, fetch, keep);
+  ReversePlan<FP>::type::template run_v<-1, TWP>(v, t, active, sp, sa, tw, in_regs, emit);
+  if (active) {
+    const T half = T(0.5);
+#pragma unroll
+    for (int c = 0; c < (NXH + TT - 1) / TT; ++c) {
+      const int k = t + c * TT;
+      if (k < NXH) {
+        const C zk = sp[sa(k)];
+        const C zn = sp[sa(k == 0 ? 0 : N - k)];
+        ra[k] = mk<C>((zk.x + zn.x) * half, (zk.y - zn.y) * half);
+        if (hasb) rb[k] = mk<C>((zk.y + zn.y) * half, (zn.x - zk.x) * half);
+      }
+    }
+  }
+}
+
+// The same over any length; `img` is a real volume for lengths without the compile-time
+// kernel.
+template <typename T>
+void run_x_weight(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* spec, const T* w, T invn, T* img, const int* done) {
+  if (compiled_plans(ctx)) {
+#define QSM_TRY_XW(N_, T_, R0_, R1_, R2_)                                                                        \
+    if (FixedPlan<N_, T_, R0_, R1_, R2_>::matches(f.px)) {                                                       \
+      using FP = FixedPlan<N_, T_, R0_, R1_, R2_>;                                                               \
+      constexpr int P = x_fx_pencils<FP>();                                                                      \
+      const size_t smem = (size_t)(x_tw_len<T>(N_) + P * x_rowlen<T>(N_)) * sizeof(cplx_t<T>);                   \
+      auto kern = k_x_weight_fx<T, FP>;                                                                          \
+      ensure_smem(kern, smem);                                                                                   \
+      LaunchScope ls(ctx, "fft_x_lsqr");                                                                         \
+      kern<<<x_fx_blocks<FP>(((long long)f.g.nrows() + 1) / 2), dim3(T_, P), smem, ctx->stream>>>(               \
+          f.g, f.twx, spec, w, invn, done);                                                                      \
+      ls.done();                                                                                                 \
+      return;                                                                                                    \
+    }
+    QSM_FIXED_PLANS(QSM_TRY_XW)
+    QSM_FIXED_PLANS_WIDE(QSM_TRY_XW)
+#undef QSM_TRY_XW
+  }
+  run_x_c2r<T>(ctx, f, spec, StoreReal<T>{img, f.g.nx, invn}, done);
+  run_x_r2c<T>(ctx, f, spec, LoadProduct<T, T>{img, w, f.g.nx}, done);
+}
 
 template <typename T>
 __global__ void k_lsqr_init_w(long long n, const cplx_t<T>* __restrict__ v, cplx_t<T>* __restrict__ w,
@@ -380,50 +465,43 @@ __global__ void k_lsqr_update(long long n, cplx_t<T>* __restrict__ x, cplx_t<T>*
 }
 
 // ============================================================ FastQSM ops ==
-// Eq. 9/11 filter x*wfs + x*h*(1 - wfs) with wfs = clamp((|D|^n - lo)/(hi - lo)),
-// src/inversion/ilsqr.rs:739-757, 1080-1088
-template <typename T> struct FsFilter {
+// Eq. 9/11 filter wfs + h*(1 - wfs) with wfs = clamp((|D|^n - lo)/(hi - lo)),
+// src/inversion/ilsqr.rs:739-757, 1080-1088; with sign: times sign(D) (ilsqr.rs:1057-1060)
+template <typename T> struct OpFsFilter {
   using C = cplx_t<T>;
   KSpace K;
-  const cplx_t<T>* h;  // SMV kernel spectrum (real part used)
+  const T* h;  // SMV kernel spectrum (even, real)
   double n_exp, lo, range;
-  __device__ __forceinline__ C apply(C x, int ix, int iy, int iz, long long idx) const {
-    double w = pow(fabs(dip(K, ix, iy, iz)), n_exp);
-    if (range > 1e-20) w = (w - lo) / range;
-    w = fmin(fmax(w, 0.0), 1.0);
-    const T wt = (T)w, hh = h[idx].x;
-    return cadd(cscale(x, wt), cscale(cscale(x, hh), T(1) - wt));
-  }
-};
-// pre of the first inverse Z pass: x = F*sign(D) (ilsqr.rs:1057-1060), then the filter
-template <typename T> struct OpFsFirst {
-  using C = cplx_t<T>;
-  FsFilter<T> F;
-  __device__ __forceinline__ C pre(C v, int ix, int iy, int iz, long long idx) const {
-    const double d = dip(F.K, ix, iy, iz);
-    const T sg = d > 0.0 ? T(1) : (d < 0.0 ? T(-1) : T(0));
-    return F.apply(cscale(v, sg), ix, iy, iz, idx);
-  }
-  __device__ __forceinline__ C post(C v, int, int, int, long long) const { return v; }
-};
-template <typename T> struct OpFsMid {
-  using C = cplx_t<T>;
-  FsFilter<T> F;
+  int with_sign;
   __device__ __forceinline__ C mid(C v, int ix, int iy, int iz, long long idx) const {
-    return F.apply(v, ix, iy, iz, idx);
+    const double hh = (double)__ldg(h + idx), ne = n_exp, l = lo, rg = range;
+    const int sgn = with_sign;
+    const KSpace& k = K;
+    const double m = K.sym(ix, iy, iz, [&](double kx, double ky, double kz, int, int, int) {
+      const double d = k.dipole(kx, ky, kz);
+      double w = pow(fabs(d), ne);
+      if (rg > 1e-20) w = (w - l) / rg;
+      w = fmin(fmax(w, 0.0), 1.0);
+      const double r = w + hh * (1.0 - w);
+      return sgn ? (d > 0.0 ? r : (d < 0.0 ? -r : 0.0)) : r;
+    });
+    return cscale(v, (T)m);
   }
 };
-// pre: F * inv_d with inv_d = signum(D)/t0 where |D| < t0, else 1/D (ilsqr.rs:1118-1126)
+// inv_d = signum(D)/t0 where |D| < t0, else 1/D (ilsqr.rs:1118-1126)
 template <typename T> struct OpTkdInv {
   using C = cplx_t<T>;
   KSpace K;
   double t0;
-  __device__ __forceinline__ C pre(C v, int ix, int iy, int iz, long long) const {
-    const double d = dip(K, ix, iy, iz);
-    const double inv = fabs(d) < t0 ? copysign(1.0, d) / t0 : 1.0 / d;
-    return cscale(v, (T)inv);
+  __device__ __forceinline__ C mid(C v, int ix, int iy, int iz, long long) const {
+    const double t = t0;
+    const KSpace& k = K;
+    const double m = K.sym(ix, iy, iz, [&](double kx, double ky, double kz, int, int, int) {
+      const double d = k.dipole(kx, ky, kz);
+      return fabs(d) < t ? copysign(1.0, d) / t : 1.0 / d;
+    });
+    return cscale(v, (T)m);
   }
-  __device__ __forceinline__ C post(C v, int, int, int, long long) const { return v; }
 };
 
 // sums of xfs, xtkd, xfs^2, xfs*xtkd over all voxels (ilsqr.rs:1141-1146)
@@ -755,20 +833,19 @@ void ilsqr_impl(qsm_ctx* ctx, const GridDims& d, const double* f, const uint8_t*
     sync(ctx);
     return;
   }
-  Fft3<T> ff = make_fft3_full<T>(ctx, d);
   Fft3<T> fh = make_fft3<T>(ctx, d);
   KSpace K = make_kspace(ctx, d, bdir);
-  const long long NF = ff.g.hsize();
+  const long long NH = fh.g.hsize();
   const T invn = (T)(1.0 / (double)N);
-  double* partials = ws<double>(ctx, nm("partials"), (size_t)kMaxPersistentBlocks * 4);
+  double* partials = ws<double>(ctx, nm("partials"), std::max(x_partials(fh, 1), (size_t)kMaxPersistentBlocks * 4));
   unsigned* counter = ws<unsigned>(ctx, nm("counter"), 1);
   QSM_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned), ctx->stream));
-  C* t = ws<C>(ctx, nm("t"), (size_t)NF);
-  C* ub = ws<C>(ctx, nm("u"), (size_t)NF);
-  C* vb = ws<C>(ctx, nm("v"), (size_t)NF);
-  C* wb = ws<C>(ctx, nm("w"), (size_t)NF);
-  C* xb = ws<C>(ctx, nm("x"), (size_t)NF);
-  for (C* b : {t, ub, vb, wb, xb}) QSM_CUDA(cudaMemsetAsync(b, 0, sizeof(C) * NF, ctx->stream));
+  C* t = ws<C>(ctx, nm("t"), (size_t)NH);
+  C* ub = ws<C>(ctx, nm("u"), (size_t)NH);
+  C* vb = ws<C>(ctx, nm("v"), (size_t)NH);
+  C* wb = ws<C>(ctx, nm("w"), (size_t)NH);
+  C* xb = ws<C>(ctx, nm("x"), (size_t)NH);
+  for (C* b : {t, ub, vb, wb, xb}) QSM_CUDA(cudaMemsetAsync(b, 0, sizeof(C) * NH, ctx->stream));
   double* dwork = ws<double>(ctx, nm("dwork"), (size_t)(3 * N));
   const double hx2 = 1.0 / (d.vsx * d.vsx), hy2 = 1.0 / (d.vsy * d.vsy), hz2 = 1.0 / (d.vsz * d.vsz);
 
@@ -793,60 +870,61 @@ void ilsqr_impl(qsm_ctx* ctx, const GridDims& d, const double* f, const uint8_t*
     h2d(ctx, lst, &init, sizeof(init));
   }
   const int* ldone = &lst->done;
+  T* mult = ws<T>(ctx, nm("m"), (size_t)NH);  // m, then sym(D)/m, then LSMR's k-space mask
+  T* img = ws<T>(ctx, nm("img"), (size_t)N);
+  spec_multiplier<T>(ctx, fh, OpHalfD<T>{K, 0}, mult, nullptr);
   // b = D * FFT(w*f) -> u, beta = ||b||
-  run_x_full<T, -1, 0>(ctx, ff, LoadRealProduct<double, T>{f, wl, d.nx}, MidId<T>{}, StoreSpecRow<T>{t, ff.g.pitch},
-                       nullptr, "fft_x_c2c");
-  run_yz<T, -1, 1>(ctx, ff, t, t, OpId<T>{}, nullptr);
-  run_yz_acc<T, -1, 2, true>(ctx, ff, t, ub, OpLsqrOut<T>{K, nullptr, lst, 2}, partials, counter, nullptr, "fft_z_lsqr");
+  run_x_r2c<T>(ctx, fh, t, LoadProduct<double, T>{f, wl, d.nx}, nullptr);
+  run_yz<T, -1, 1>(ctx, fh, t, t, OpId<T>{}, nullptr);
+  run_yz_acc<T, -1, 2, true>(ctx, fh, t, ub, OpLsqrHalf<T>{mult, d.nx, nullptr, lst, 2}, partials, counter, nullptr,
+                             "fft_z_lsqr");
   // y = A(s*x) written to dst with the given epilogue mode
   auto apply_a = [&](const C* x, const double* s, C* dst, const C* old, int mode) {
-    // compile-time staged pass (a direct-fetch first stage with the dipole scale in its
-    // loads ran 309 against 256 us at 384x384x256 in float, 619 against 450 us in double)
-    run_yz<T, +1, 2, true>(ctx, ff, x, t, OpScaleD<T>{K, s}, ldone);
-    run_yz<T, +1, 1>(ctx, ff, t, t, OpId<T>{}, ldone);
-    run_x_full<T, +1, -1, true>(ctx, ff, LoadSpecRow<T>{t, ff.g.pitch}, MidWeightRe<T>{wl, d.nx, invn},
-                          StoreSpecRow<T>{t, ff.g.pitch}, ldone, "fft_x_lsqr");
-    run_yz<T, -1, 1>(ctx, ff, t, t, OpId<T>{}, ldone);
-    run_yz_acc<T, -1, 2, true>(ctx, ff, t, dst, OpLsqrOut<T>{K, old, lst, mode}, partials, counter, ldone, "fft_z_lsqr");
+    run_yz<T, +1, 2, true>(ctx, fh, x, t, OpScaleM<T>{mult, s}, ldone);
+    run_yz<T, +1, 1>(ctx, fh, t, t, OpId<T>{}, ldone);
+    run_x_weight<T>(ctx, fh, t, wl, invn, img, ldone);
+    run_yz<T, -1, 1>(ctx, fh, t, t, OpId<T>{}, ldone);
+    run_yz_acc<T, -1, 2, true>(ctx, fh, t, dst, OpLsqrHalf<T>{mult, d.nx, old, lst, mode}, partials, counter, ldone,
+                               "fft_z_lsqr");
   };
   // v = A^H u, alpha; w = v
   apply_a(ub, &lst->su, vb, nullptr, 3);
   {
     LaunchScope ls(ctx, "lsqr_init");
-    k_lsqr_init_w<T><<<grid1d(NF), 256, 0, ctx->stream>>>(NF, vb, wb, lst);
+    k_lsqr_init_w<T><<<grid1d(NH), 256, 0, ctx->stream>>>(NH, vb, wb, lst);
     ls.done();
   }
-  const unsigned ugrid = grid1d(NF);
+  const unsigned ugrid = grid1d(NH);
   run_iterations(ctx, 50, ldone, [&]() {  // maxit_lsqr, ilsqr.rs:967
     apply_a(vb, &lst->sv, ub, ub, 0);
     apply_a(ub, &lst->su, vb, vb, 1);
     LaunchScope ls(ctx, "lsqr_update");
-    k_lsqr_update<T><<<ugrid, 256, 0, ctx->stream>>>(NF, xb, wb, vb, lst, partials);
+    k_lsqr_update<T><<<ugrid, 256, 0, ctx->stream>>>(NH, xb, wb, vb, lst, partials);
     ls.done();
   });
-  // xlsqr = mask * Re IFFT(x)
-  run_yz<T, +1, 2>(ctx, ff, xb, t, OpId<T>{}, nullptr);
-  run_yz<T, +1, 1>(ctx, ff, t, t, OpId<T>{}, nullptr);
-  run_x_full<T, +1, 0>(ctx, ff, LoadSpecRow<T>{t, ff.g.pitch}, MidId<T>{}, StoreMaskRe<T, double>{xlsqr, mask, d.nx, invn},
-                       nullptr, "fft_x_c2c");
+  // xlsqr = mask * Re IFFT(D G_x), D G_x = sym(D)/m h_x under the real part
+  spec_multiplier<T>(ctx, fh, OpHalfD<T>{K, 1}, mult, nullptr);
+  {
+    LsqrState one{};
+    one.su = 1.0;
+    h2d(ctx, lst, &one, sizeof(one));
+  }
+  run_yz<T, +1, 2, true>(ctx, fh, xb, t, OpScaleM<T>{mult, &lst->su}, nullptr);
+  run_yz<T, +1, 1>(ctx, fh, t, t, OpId<T>{}, nullptr);
+  run_x_c2r<T>(ctx, fh, t, StoreMaskedF64<T>{xlsqr, mask, d.nx, invn}, nullptr);
 
   // ------------------------------------------------------------- step 2 --
   report(2);
   // step 2 runs in TD; with TD == T its buffers are step 1's (same names, same sizes)
-  Fft3<TD> ffd = make_fft3_full<TD>(ctx, d);
+  Fft3<TD> fd = make_fft3<TD>(ctx, d);
   const TD invnd = (TD)(1.0 / (double)N);
-  CD* Fb = ws<CD>(ctx, nmd("v"), (size_t)NF);  // FFT(f)
-  CD* hs = ws<CD>(ctx, nmd("u"), (size_t)NF);  // SMV kernel spectrum
-  CD* td = ws<CD>(ctx, nmd("t"), (size_t)NF);
-  run_x_full<TD, -1, 0>(ctx, ffd, LoadRealProduct<double, TD>{f, nullptr, d.nx}, MidId<TD>{},
-                       StoreSpecRow<TD>{Fb, ffd.g.pitch}, nullptr, "fft_x_c2c");
-  run_yz<TD, -1, 1>(ctx, ffd, Fb, Fb, OpId<TD>{}, nullptr);
-  run_yz<TD, -1, 2>(ctx, ffd, Fb, Fb, OpId<TD>{}, nullptr);
-  run_x_full<TD, -1, 0>(ctx, ffd, LoadSphereC<TD>{sphere_img(d, 3.0)}, MidId<TD>{}, StoreSpecRow<TD>{hs, ffd.g.pitch},
-                       nullptr, "fft_x_c2c");
-  run_yz<TD, -1, 1>(ctx, ffd, hs, hs, OpId<TD>{}, nullptr);
-  run_yz<TD, -1, 2>(ctx, ffd, hs, hs, OpId<TD>{}, nullptr);
-  FsFilter<TD> filt{K, hs, 0.001, 0.0, 0.0};
+  CD* Fb = ws<CD>(ctx, nmd("v"), (size_t)NH);  // FFT(f) along x and y
+  CD* td = ws<CD>(ctx, nmd("t"), (size_t)NH);
+  TD* hs = ws<TD>(ctx, nmd("h"), (size_t)NH);  // SMV kernel spectrum (r = 3)
+  smv_multiplier<TD>(ctx, fd, smv_sphere(d, 3.0), kSmvS, 0.0, hs);
+  run_x_r2c<TD>(ctx, fd, Fb, LoadCast<double, TD>{f, d.nx}, nullptr);
+  run_yz<TD, -1, 1>(ctx, fd, Fb, Fb, OpId<TD>{}, nullptr);
+  OpFsFilter<TD> filt{K, hs, 0.001, 0.0, 0.0, 1};
   {
     LaunchScope ls(ctx, "ilsqr_dipole_pow");
     k_dipole_pow<<<grid1d(N), 256, 0, ctx->stream>>>(K, d.nx, d.ny, d.nz, 0.001, dwork);
@@ -858,19 +936,18 @@ void ilsqr_impl(qsm_ctx* ctx, const GridDims& d, const double* f, const uint8_t*
   TD* xfs_raw = ws<TD>(ctx, nmd("xfs_raw"), (size_t)N);
   TD* xtkd = ws<TD>(ctx, nmd("xtkd"), (size_t)N);
   TD* xfs = ws<TD>(ctx, nmd("xfs"), (size_t)N);
-  run_yz<TD, +1, 2>(ctx, ffd, Fb, td, OpFsFirst<TD>{filt}, nullptr);
-  run_yz<TD, +1, 1>(ctx, ffd, td, td, OpId<TD>{}, nullptr);
-  run_x_full<TD, +1, -1>(ctx, ffd, LoadSpecRow<TD>{td, ffd.g.pitch}, MidMaskRe<TD>{mask, d.nx, invnd},
-                        StoreSpecRow<TD>{td, ffd.g.pitch}, nullptr, "fft_x_fastqsm");
-  run_yz<TD, -1, 1>(ctx, ffd, td, td, OpId<TD>{}, nullptr);
-  run_z_fused<TD>(ctx, ffd, td, td, OpFsMid<TD>{filt}, nullptr);
-  run_yz<TD, +1, 1>(ctx, ffd, td, td, OpId<TD>{}, nullptr);
-  run_x_full<TD, +1, 0>(ctx, ffd, LoadSpecRow<TD>{td, ffd.g.pitch}, MidId<TD>{}, StoreMaskRe<TD, TD>{xfs_raw, mask, d.nx, invnd},
-                       nullptr, "fft_x_c2c");
-  run_yz<TD, +1, 2>(ctx, ffd, Fb, td, OpTkdInv<TD>{K, 1.0 / 8.0}, nullptr);
-  run_yz<TD, +1, 1>(ctx, ffd, td, td, OpId<TD>{}, nullptr);
-  run_x_full<TD, +1, 0>(ctx, ffd, LoadSpecRow<TD>{td, ffd.g.pitch}, MidId<TD>{}, StoreMaskRe<TD, TD>{xtkd, mask, d.nx, invnd},
-                       nullptr, "fft_x_c2c");
+  run_z_fused<TD>(ctx, fd, Fb, td, filt, nullptr);
+  run_yz<TD, +1, 1>(ctx, fd, td, td, OpId<TD>{}, nullptr);
+  run_x_c2r<TD>(ctx, fd, td, StoreMaskedT<TD>{xfs, mask, d.nx, invnd}, nullptr);
+  run_x_r2c<TD>(ctx, fd, td, LoadCast<TD, TD>{xfs, d.nx}, nullptr);
+  run_yz<TD, -1, 1>(ctx, fd, td, td, OpId<TD>{}, nullptr);
+  filt.with_sign = 0;
+  run_z_fused<TD>(ctx, fd, td, td, filt, nullptr);
+  run_yz<TD, +1, 1>(ctx, fd, td, td, OpId<TD>{}, nullptr);
+  run_x_c2r<TD>(ctx, fd, td, StoreMaskedT<TD>{xfs_raw, mask, d.nx, invnd}, nullptr);
+  run_z_fused<TD>(ctx, fd, Fb, td, OpTkdInv<TD>{K, 1.0 / 8.0}, nullptr);
+  run_yz<TD, +1, 1>(ctx, fd, td, td, OpId<TD>{}, nullptr);
+  run_x_c2r<TD>(ctx, fd, td, StoreMaskedT<TD>{xtkd, mask, d.nx, invnd}, nullptr);
   {
     double* sums = ws<double>(ctx, nmd("sums"), 4);
     LaunchScope ls(ctx, "fastqsm_sums");
@@ -919,7 +996,7 @@ void ilsqr_impl(qsm_ctx* ctx, const GridDims& d, const double* f, const uint8_t*
     h2d(ctx, mst, &init, sizeof(init));
   }
   const int* mdone = &mst->done;
-  // N-length LSMR vectors reuse the idle LSQR buffers (each holds 2*NF >= 2N reals)
+  // N-length LSMR vectors reuse the idle LSQR buffers (each holds 2*NH >= N reals)
   T* vv = reinterpret_cast<T*>(vb);
   T* hh = reinterpret_cast<T*>(wb);
   T* hbar = reinterpret_cast<T*>(xb);
@@ -929,10 +1006,11 @@ void ilsqr_impl(qsm_ctx* ctx, const GridDims& d, const double* f, const uint8_t*
   C* spec = ws<C>(ctx, nm("lsmr_spec"), (size_t)fh.g.hsize());
   QSM_CUDA(cudaMemsetAsync(spec, 0, sizeof(C) * fh.g.hsize(), ctx->stream));
   const T hx = (T)(1.0 / d.vsx), hy = (T)(1.0 / d.vsy), hz = (T)(1.0 / d.vsz);
+  spec_multiplier<T>(ctx, fh, OpMic<T>{K}, mult, nullptr);
   auto mic_chain = [&](const auto& load, const auto& store) {
     run_x_r2c<T>(ctx, fh, spec, load, mdone);
     run_yz<T, -1, 1>(ctx, fh, spec, spec, OpId<T>{}, mdone);
-    run_z_fused<T>(ctx, fh, spec, spec, OpMic<T>{K}, mdone);
+    run_z_fused_m<T>(ctx, fh, spec, spec, mult, mdone);
     run_yz<T, +1, 1>(ctx, fh, spec, spec, OpId<T>{}, mdone);
     run_x_c2r<T>(ctx, fh, spec, store, mdone);
   };
