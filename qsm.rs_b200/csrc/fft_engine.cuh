@@ -314,7 +314,7 @@ template <int N, int TT, int R0, int R1, int R2> struct ReversePlan<FixedPlan<N,
 };
 
 template <int N, int TT, int R0, int R1, int R2> struct FixedPlan {
-  static constexpr int n = N, T = TT;
+  static constexpr int n = N, T = TT, r0 = R0;
   static __host__ __device__ constexpr bool matches(const FftPlan1D& pl) {
     return pl.n == N && pl.m == N && pl.T == TT && pl.radix[0] == R0 && pl.radix[1] == R1 &&
            (R2 == 1 ? pl.nstages == 2 : (pl.nstages == 3 && pl.radix[2] == R2));

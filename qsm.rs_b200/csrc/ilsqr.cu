@@ -374,7 +374,7 @@ __global__ void k_x_weight_fx(Geom g, const cplx_t<T>* __restrict__ twg, cplx_t<
   const bool active = a < nrows && t < TT;
   const bool hasb = b < nrows;
   C* sp = sm + threadIdx.y * x_rowlen<T>(N);
-  SAPadded<PadG<T>::G> sa;
+  SAPadded<x_pad<T, FP>()> sa;
   C* ra = spec + (long long)a * g.pitch;
   C* rb = spec + (long long)b * g.pitch;
   auto fetch = [&](int e) -> C {
@@ -421,12 +421,12 @@ void run_x_weight(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* spec, const T* w, T
 #define QSM_TRY_XW(N_, T_, R0_, R1_, R2_)                                                                        \
     if (FixedPlan<N_, T_, R0_, R1_, R2_>::matches(f.px)) {                                                       \
       using FP = FixedPlan<N_, T_, R0_, R1_, R2_>;                                                               \
-      constexpr int P = x_fx_pencils<FP>();                                                                      \
+      const int P = x_fx_pencils<FP>(ctx, ((long long)f.g.nrows() + 1) / 2);                                     \
       const size_t smem = (size_t)(x_tw_len<T>(N_) + P * x_rowlen<T>(N_)) * sizeof(cplx_t<T>);                   \
       auto kern = k_x_weight_fx<T, FP>;                                                                          \
       ensure_smem(kern, smem);                                                                                   \
       LaunchScope ls(ctx, "fft_x_lsqr");                                                                         \
-      kern<<<x_fx_blocks<FP>(((long long)f.g.nrows() + 1) / 2), dim3(T_, P), smem, ctx->stream>>>(               \
+      kern<<<x_fx_blocks(((long long)f.g.nrows() + 1) / 2, P), dim3(T_, P), smem, ctx->stream>>>(                  \
           f.g, f.twx, spec, w, invn, done);                                                                      \
       ls.done();                                                                                                 \
       return;                                                                                                    \

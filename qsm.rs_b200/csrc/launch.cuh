@@ -128,34 +128,41 @@ template <typename T> inline size_t x_partials(const Fft3<T>& f, int K) {
   return (size_t)(b > kMaxPersistentBlocks ? b : kMaxPersistentBlocks) * K;
 }
 
-// Pencils per block of the compile-time X passes: as many whole pencils as 256 threads hold.
-// A pencil's threads are not rounded up to a divisor of a warp (as the runtime engine's
-// are): at 21 threads per pencil (length 189) a third of each block idled.
-template <class FP> constexpr int x_fx_pencils() { return FP::T >= 256 ? 1 : 256 / FP::T; }
-template <class FP> inline unsigned x_fx_blocks(long long pencils) {
-  return (unsigned)((pencils + x_fx_pencils<FP>() - 1) / x_fx_pencils<FP>());
+int sm_count_of(int device);  // multiprocessor count, cached per device under a lock
+inline int sm_count(qsm_ctx* ctx) { return sm_count_of(ctx->device); }
+
+// Pencils per block of the compile-time X passes: as many whole pencils as 256 threads
+// hold, halved (down to two warps) while the grid is under two blocks per SM: at 64^3 a
+// block of 64 four-thread pencils left 32 blocks for 148 SMs.  A pencil's threads are not
+// rounded up to a divisor of a warp (as the runtime engine's are): at 21 threads per pencil
+// (length 189) a third of each block idled.
+template <class FP> inline int x_fx_pencils(qsm_ctx* ctx, long long pencils) {
+  int P = FP::T >= 256 ? 1 : 256 / FP::T;
+  while (P > 1 && P / 2 * FP::T >= 64 && (pencils + P - 1) / P < 2LL * sm_count(ctx)) P /= 2;
+  return P;
 }
+inline unsigned x_fx_blocks(long long pencils, int P) { return (unsigned)((pencils + P - 1) / P); }
 
 // One compile-time X pass (k_x_r2c_fx / k_x_c2r_fx, FP a FixedPlan).
 template <typename T, class FP, bool DEAD, class Load>
 bool launch_x_r2c_fx(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* spec, const Load& ld, const int* done) {
-  constexpr int P = x_fx_pencils<FP>();
+  const int P = x_fx_pencils<FP>(ctx, ((long long)f.g.nrows() + 1) / 2);
   const size_t smem = (size_t)(x_tw_len<T>(FP::n) + P * x_rowlen<T>(FP::n)) * sizeof(cplx_t<T>);
   auto kern = k_x_r2c_fx<T, FP, Load, DEAD>;
   ensure_smem(kern, smem);
   LaunchScope ls(ctx, "fft_x_r2c");
-  kern<<<x_fx_blocks<FP>(((long long)f.g.nrows() + 1) / 2), dim3(FP::T, P), smem, ctx->stream>>>(f.g, f.twx, spec, ld, done);
+  kern<<<x_fx_blocks(((long long)f.g.nrows() + 1) / 2, P), dim3(FP::T, P), smem, ctx->stream>>>(f.g, f.twx, spec, ld, done);
   ls.done();
   return true;
 }
 template <typename T, class FP, bool DEAD, class Store>
 bool launch_x_c2r_fx(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* spec, const Store& st, const int* done) {
-  constexpr int P = x_fx_pencils<FP>();
+  const int P = x_fx_pencils<FP>(ctx, ((long long)f.g.nrows() + 1) / 2);
   const size_t smem = (size_t)(x_tw_len<T>(FP::n) + P * x_rowlen<T>(FP::n)) * sizeof(cplx_t<T>);
   auto kern = k_x_c2r_fx<T, FP, Store, DEAD>;
   ensure_smem(kern, smem);
   LaunchScope ls(ctx, "fft_x_c2r");
-  kern<<<x_fx_blocks<FP>(((long long)f.g.nrows() + 1) / 2), dim3(FP::T, P), smem, ctx->stream>>>(f.g, f.twx, spec, st, done);
+  kern<<<x_fx_blocks(((long long)f.g.nrows() + 1) / 2, P), dim3(FP::T, P), smem, ctx->stream>>>(f.g, f.twx, spec, st, done);
   ls.done();
   return true;
 }
@@ -326,12 +333,12 @@ void run_x_full(qsm_ctx* ctx, const Fft3<T>& f, const Load& ld, const Mid& mid, 
 #define QSM_TRY_XF(N_, T_, R0_, R1_, R2_)                                                          \
     if (FixedPlan<N_, T_, R0_, R1_, R2_>::matches(f.px)) {                                         \
       using FP = FixedPlan<N_, T_, R0_, R1_, R2_>;                                                 \
-      constexpr int P = x_fx_pencils<FP>();                                                        \
+      const int P = x_fx_pencils<FP>(ctx, f.g.nrows());                                            \
       const size_t smem = (size_t)(x_tw_len<T>(N_) + P * x_rowlen<T>(N_)) * sizeof(C);            \
       auto kern = k_x_full_fx<T, FP, D1, D2, Load, Mid, Store>;                                    \
       ensure_smem(kern, smem);                                                                     \
       LaunchScope ls(ctx, name);                                                                   \
-      kern<<<x_fx_blocks<FP>(f.g.nrows()), dim3(T_, P), smem, ctx->stream>>>(f.g, f.twx, ld, mid, st, done);   \
+      kern<<<x_fx_blocks(f.g.nrows(), P), dim3(T_, P), smem, ctx->stream>>>(f.g, f.twx, ld, mid, st, done);   \
       ls.done();                                                                                   \
       return;                                                                                      \
     }
@@ -367,9 +374,6 @@ void run_x_full(qsm_ctx* ctx, const Fft3<T>& f, const Load& ld, const Mid& mid, 
 }
 
 template <typename T> inline int yz_cols() { return sizeof(T) == 4 ? 16 : 8; }
-
-int sm_count_of(int device);  // multiprocessor count, cached per device under a lock
-inline int sm_count(qsm_ctx* ctx) { return sm_count_of(ctx->device); }
 
 // Persistent grid: as many CTAs as fit on the device at once, capped by the work.
 template <class K> unsigned persistent_grid(qsm_ctx* ctx, K kernel, int threads, size_t smem, long long work) {

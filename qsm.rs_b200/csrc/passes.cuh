@@ -36,6 +36,13 @@ template <typename T> struct PadG;
 template <> struct PadG<float> { static constexpr int G = 16; };
 template <> struct PadG<double> { static constexpr int G = 8; };
 
+// Row skew of the compile-time X passes.  Thread j of the first stage writes elements
+// j * R0 + r: one gap per 16 puts a radix-16 stage's 16-byte writes on distinct banks (one
+// per 8 left them two-way), and one per 8 does for the others.
+template <typename T, class FP> constexpr int x_pad() {
+  return sizeof(T) == 8 && FP::r0 == 16 ? 16 : PadG<T>::G;
+}
+
 template <typename T> __host__ __device__ inline int x_rowlen(int n) { return n + n / PadG<T>::G + 1; }
 // Twiddle table of the compile-time X passes: padded (tw_pad) in double, where it took
 // iLSQR's FP64 X pass at length 384 from 523 to 504 us; dense in float, where the extra
@@ -234,7 +241,7 @@ __global__ void k_x_full_fx(Geom g, const cplx_t<T>* __restrict__ twg, Load ld, 
   const int row = blockIdx.x * blockDim.y + threadIdx.y;
   const bool active = row < g.nrows() && t < TT;
   C* sp = sm + threadIdx.y * x_rowlen<T>(N);
-  SAPadded<PadG<T>::G> sa;
+  SAPadded<x_pad<T, FP>()> sa;
   Store st = st0;
   auto fetch_g = [&](int e) -> C { return ld(row, e); };
   auto emit_g = [&](int e, C v) { st(row, e, v); };
@@ -357,7 +364,7 @@ __global__ void k_x_r2c_fx(Geom g, const cplx_t<T>* __restrict__ twg, cplx_t<T>*
   const bool active = a < nrows && t < TT;
   const bool hasb = b < nrows;
   C* sp = sm + p * x_rowlen<T>(N);
-  SAPadded<PadG<T>::G> sa;
+  SAPadded<x_pad<T, FP>()> sa;
   auto fetch = [&](int e) -> C { return mk<C>(ld(a, e), hasb ? ld(b, e) : T(0)); };
   auto emit = [&](int e, C v) { sp[sa(e)] = v; };
   FP::template run<-1, TWP>(t, active, sp, sa, tw, fetch, emit);
@@ -413,7 +420,7 @@ __global__ void k_x_c2r_fx(Geom g, const cplx_t<T>* __restrict__ twg, const cplx
     active = want;
   }
   C* sp = sm + p * x_rowlen<T>(N);
-  SAPadded<PadG<T>::G> sa;
+  SAPadded<x_pad<T, FP>()> sa;
   const C* ra = spec + (long long)a * g.pitch;
   const C* rb = spec + (long long)b * g.pitch;
   // z[e] = A[e] + i B[e] from the two half spectra (A, B Hermitian)
@@ -705,15 +712,16 @@ __global__ void __launch_bounds__(128)
 // bounds, j mod Ns, twiddle strides and shared-memory addressing fold into constants.
 // Plain copies (k_pass_yz_dx) and the multiplier Z pass (k_z_fused_m_fx).
 // ------------------------------------------------------------------------------
-// Resident blocks per SM the compile-time Y/Z passes are compiled for: four blocks of
-// up to 256 threads in float (64 registers; no plan of the two lists spills more than 4
+// Resident blocks per SM the compile-time Y/Z passes are compiled for: in float 1024 threads
+// of blocks of 129 to 256 (64 registers; no plan of the two lists spills more than 4
 // bytes, and with the five-block multiplier Z pass the TV-ADMM iteration at 256x256x176
-// went from 0.1956 to 0.1941 ms); in double (twice the registers
-// per value) three blocks of up to 128 threads and two of up to 256, so the long plans
-// (384: 208 threads) do not spill.
+// went from 0.1956 to 0.1941 ms), in double (twice the registers per value) about 384, and
+// two blocks of up to 256 so the long plans (384: 208 threads) do not spill.  Smaller blocks
+// get proportionally more, or the short lengths' latency shows: three 64-thread blocks of
+// the 128-point double pass kept 7.6 warps per SM.
 template <typename T, int THREADS> constexpr int yz_dx_min_blocks() {
-  if constexpr (sizeof(T) == 4) return THREADS <= 256 ? 4 : 1;
-  else return THREADS <= 128 ? 3 : (THREADS <= 256 ? 2 : 1);
+  if constexpr (sizeof(T) == 4) return THREADS <= 64 ? 10 : THREADS <= 128 ? 6 : THREADS <= 256 ? 4 : 1;
+  else return THREADS <= 64 ? 6 : THREADS <= 96 ? 4 : THREADS <= 128 ? 3 : (THREADS <= 256 ? 2 : 1);
 }
 
 template <int P> struct SAStridedC {
