@@ -124,20 +124,28 @@ template <typename T> struct OpMultArray {
 
 // Doubles that K sums per block of an X pass may fill (grid_sum_last), whichever kernel runs.
 template <typename T> inline size_t x_partials(const Fft3<T>& f, int K) {
-  const long long b = x_blocks(f);
+  // blocks of the runtime engine; the compile-time kernels' are half as large, with room for
+  // a pencil count that does not fill them
+  const long long b = 4 * x_blocks(f);
   return (size_t)(b > kMaxPersistentBlocks ? b : kMaxPersistentBlocks) * K;
 }
 
 int sm_count_of(int device);  // multiprocessor count, cached per device under a lock
 inline int sm_count(qsm_ctx* ctx) { return sm_count_of(ctx->device); }
 
-// Pencils per block of the compile-time X passes: as many whole pencils as 256 threads
-// hold, halved (down to two warps) while the grid is under two blocks per SM: at 64^3 a
-// block of 64 four-thread pencils left 32 blocks for 148 SMs.  A pencil's threads are not
-// rounded up to a divisor of a warp (as the runtime engine's are): at 21 threads per pencil
-// (length 189) a third of each block idled.
+// Threads a block of the compile-time X passes aims at.  Blocks of 128 overlap each other's
+// barriers better than blocks of 256 (double: r2c at 189x231x165 47.0 to 42.8 us, c2r 43.5 to
+// 38.8 us, at 160x192x160 25.9 to 23.0 and 24.9 to 20.9 us; float c2r at 256x256x176 24.9 to
+// 23.4 us, r2c unchanged); at 64 the twiddle table of each block costs that again (43.6 and
+// 39.7 us, 23.4 and 21.3 us).
+constexpr int kXThreads = 128;
+// Pencils per block: as many whole pencils as kXThreads threads hold, halved (down to two
+// warps) while the grid is under two blocks per SM: at 64^3 a block of 64 four-thread pencils
+// left 32 blocks for 148 SMs.  A pencil's threads are not rounded up to a divisor of a warp
+// (as the runtime engine's are): at 21 threads per pencil (length 189) a third of each block
+// idled.
 template <class FP> inline int x_fx_pencils(qsm_ctx* ctx, long long pencils) {
-  int P = FP::T >= 256 ? 1 : 256 / FP::T;
+  int P = FP::T >= kXThreads ? 1 : kXThreads / FP::T;
   while (P > 1 && P / 2 * FP::T >= 64 && (pencils + P - 1) / P < 2LL * sm_count(ctx)) P /= 2;
   return P;
 }

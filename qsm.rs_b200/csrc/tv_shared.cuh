@@ -527,10 +527,11 @@ __global__ void __launch_bounds__(kStepBX* kStepBY, 2)
   cp_async_commit();
   double sd = 0.0, sx = 0.0;
   for (int k = k0; k < k1; ++k) {
+    cp_async_wait<1>();  // the stages of planes k - 1 and k have landed
+    __syncthreads();
+    // slot s(k + 2) = s(k - 2) was last read before this barrier
     if (k + 2 < k1) issue(k + 2);
     cp_async_commit();
-    cp_async_wait<2>();  // the stages of planes k - 1 and k have landed
-    __syncthreads();
     const Slot& Sp = slot(k - 1);  // x0, y at plane k
     const Slot& Sk = slot(k);      // x0, y at plane k + 1; y_{i-2}, u at plane k
     const long long c = (long long)k * sz + rowj + i;
@@ -594,7 +595,6 @@ __global__ void __launch_bounds__(kStepBX* kStepBY, 2)
     }
     uz_km = uz;
     x_km = x_k;
-    __syncthreads();  // slot s(k - 1) is refilled by the next iteration
   }
   cp_async_wait<0>();
   __shared__ int am_last;
