@@ -293,7 +293,7 @@ struct Box {
 // sub-volume extraction: phase as float, both masks
 __global__ void k_tgv_extract(Box b, int nx, int ny, const double* __restrict__ phase, const uint8_t* __restrict__ m0,
                               const uint8_t* __restrict__ me, float* __restrict__ ph, uint8_t* __restrict__ m0s,
-                              uint8_t* __restrict__ mes) {
+                              uint8_t* __restrict__ mes, uint8_t* __restrict__ mk) {
   const long long N = b.n();
   for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < N; s += (long long)gridDim.x * blockDim.x) {
     const int i = (int)(s % b.bx), j = (int)((s / b.bx) % b.by), k = (int)(s / ((long long)b.bx * b.by));
@@ -301,6 +301,7 @@ __global__ void k_tgv_extract(Box b, int nx, int ny, const double* __restrict__ 
     ph[s] = (float)phase[f];
     m0s[s] = m0[f];
     mes[s] = me[f];
+    mk[s] = (uint8_t)((m0[f] != 0 ? 1 : 0) | (me[f] != 0 ? 2 : 0));
   }
 }
 
@@ -351,8 +352,7 @@ __global__ void k_tgv_sub_mean(long long N, const uint8_t* __restrict__ m0, cons
 // ============================================================ iteration ==
 struct TgvArrays {
   const float* lphi;
-  const uint8_t* m0;
-  const uint8_t* me;
+  const uint8_t* mk;  // 1: mask0, 2: the eroded mask that holds it
   float* eta;
   float* p[3];
   float* q[6];  // xx, xy, xz, yy, yz, zz
@@ -374,62 +374,87 @@ struct TgvFlag {
   int pad;
 };
 
-// masked Neumann Laplacian at s (apply_laplacian_inplace, tgv.rs:780-824); the caller
-// handles mask0 == 0
-template <class F>
-__device__ __forceinline__ float lap_neumann(const F& a, long long s, int i, int j, int k, const Box& b, long long sxy,
-                                             const TgvScalars& c) {
-  const float a0 = a(s);
-  const float xm = i > 0 ? a(s - 1) : a0, xp = i + 1 < b.bx ? a(s + 1) : a0;
-  const float ym = j > 0 ? a(s - b.bx) : a0, yp = j + 1 < b.by ? a(s + b.bx) : a0;
-  const float zm = k > 0 ? a(s - sxy) : a0, zp = k + 1 < b.bz ? a(s + sxy) : a0;
-  return c.hx2 * (xm - 2.0f * a0 + xp) + c.hy2 * (ym - 2.0f * a0 + yp) + c.hz2 * (zm - 2.0f * a0 + zp);
-}
+// The primal and dual kernels run 32x4 (x, y) tiles, each thread marching through
+// `zchunk` planes of one (i, j) column: no index division, and the y/z neighbours of a
+// voxel are the tile's own recent loads (L1) rather than another block's (L2).  Both wait on
+// loads, not on HBM (208 bytes a voxel of the mask, 4 of 6.65 TB/s at 256x256x176), so warps
+// count: eight blocks of four warps per SM fit 64 registers without spills.  An iteration
+// there takes 203 us; 226 at 32x8 tiles with three blocks (80 registers), 215 with four, 214
+// at 32x2, 267 at 48 registers (spills); 268 before the running sums and with the voxels
+// outside the masks read and written.
+constexpr int kTgvBX = 32, kTgvBY = 4;
+constexpr int kTgvBlocks = 8;  // resident per SM
+// Chunks of z: enough that the tiles make about kTgvChunks blocks per SM, for the ends of the
+// ellipsoid's columns are idle (16: 227 us, 32: 210, 48: 203, 64 and 96: 204).
+constexpr int kTgvChunks = 48;
 
-// 27-point stencil at an interior voxel (apply_stencil, tgv.rs:667-713; dk, dj, di order)
-template <class F>
-__device__ __forceinline__ float stencil27(const F& a, long long s, long long bx, long long sxy, const TgvConst& K) {
-  float sum = 0.0f;
-#pragma unroll
-  for (int dk = 0; dk < 3; ++dk)
+// Sums of the 27-point stencil (apply_stencil, tgv.rs:667-713; dk, dj, di order) along a
+// column: the nine values of a plane end the sum of the plane below, continue their own
+// plane's and begin that of the plane above, so each is loaded once instead of three times
+// (27 loads a voxel kept the load units, not HBM, busy).
+struct Stencil27 {
+  float below = 0.0f, own = 0.0f;  // planes k and k + 1 before plane k + 1 is added
+  // Plane k + 1 around a (element s of it); returns the sum of plane k.  c: its centre,
+  // x and y neighbours.
+  __device__ __forceinline__ float add(const float* __restrict__ a, unsigned s, unsigned bx, const TgvConst& K, float c[5]) {
+    float v[9];
 #pragma unroll
     for (int dj = 0; dj < 3; ++dj)
 #pragma unroll
-      for (int di = 0; di < 3; ++di)
-        sum += K.st[(di * 3 + dj) * 3 + dk] * a(s + (di - 1) + (dj - 1) * bx + (dk - 1) * sxy);
-  return sum;
-}
+      for (int di = 0; di < 3; ++di) v[dj * 3 + di] = a[s + dj * bx - bx + di - 1];
+    float above = 0.0f;
+#pragma unroll
+    for (int dj = 0; dj < 3; ++dj)
+#pragma unroll
+      for (int di = 0; di < 3; ++di) {
+        const float x = v[dj * 3 + di];
+        below += K.st[(di * 3 + dj) * 3 + 2] * x;
+        own += K.st[(di * 3 + dj) * 3 + 1] * x;
+        above += K.st[(di * 3 + dj) * 3 + 0] * x;
+      }
+    c[0] = v[4];
+    c[1] = v[3];
+    c[2] = v[5];
+    c[3] = v[1];
+    c[4] = v[7];
+    const float sum = below;
+    below = own;
+    own = above;
+    return sum;
+  }
+  __device__ __forceinline__ void skip() {
+    below = own;
+    own = 0.0f;
+  }
+};
 
-__device__ __forceinline__ bool interior(int i, int j, int k, const Box& b) {
-  return !(i == 0 || j == 0 || k == 0 || i + 1 >= b.bx || j + 1 >= b.by || k + 1 >= b.bz);
-}
-
-// The primal and dual kernels run 32x8 (x, y) tiles, each thread marching through
-// `zchunk` planes of one (i, j) column: no index division, and the y/z neighbours of a
-// voxel are the tile's own recent loads (L1) rather than another block's (L2).
-constexpr int kTgvBX = 32, kTgvBY = 8;
-// Resident blocks per SM the primal and dual kernels are compiled for (their register
-// budgets: 85 registers a thread, no spills; the plane's values are held in registers).
-constexpr int kTgvPrimalBlocks = 3;
-constexpr int kTgvDualBlocks = 3;
+// Codes of a column's planes (0 outside the chunk's reach)
+#define TGV_COLUMN()                                                                          \
+  const int i = blockIdx.x * kTgvBX + threadIdx.x, j = blockIdx.y * kTgvBY + threadIdx.y;     \
+  if (i >= b.bx || j >= b.by) return;                                                         \
+  const unsigned bx = (unsigned)b.bx, sxy = bx * (unsigned)b.by;                              \
+  const int kbeg = blockIdx.z * zchunk;                                                       \
+  const int kend = min(b.bz, (int)(blockIdx.z + 1) * zchunk);                                 \
+  if (kbeg >= kend) return;                                                                   \
+  const unsigned col = (unsigned)j * bx + (unsigned)i;                                        \
+  const uint8_t* __restrict__ mk = A.mk;                                                      \
+  auto code_at = [&](int k) -> int { return k < kend ? mk[(unsigned)k * sxy + col] : 0; };
 
 // Dual update (tgv.rs:1157-1213).  q selects the buffers holding phi_, chi_, w_.
 // Every array is accessed through a restrict-qualified pointer (no two alias, and no
-// voxel reads what another voxel writes in the same launch); the two masks of the next
-// plane are fetched while the current plane computes, and every value a plane needs is
-// loaded into registers before its update, so a plane waits on one round of loads.  The
-// arithmetic is that of the reference, in its order.
-__global__ void __launch_bounds__(kTgvBX* kTgvBY, kTgvDualBlocks) k_tgv_dual(Box b, TgvArrays A, TgvScalars c, TgvConst K, int q,
+// voxel reads what another voxel writes in the same launch).  Values of the next plane
+// (chi_, phi_, w_ above the voxel) are carried over to it.  mask0 holds no voxel of the box's
+// faces (it is eroded from the volume's, and the box leaves two voxels around it), so its
+// voxels have all 26 neighbours and need no boundary case; the eroded mask's may lie on
+// them.  The arithmetic is that of the reference, in its order.
+__global__ void __launch_bounds__(kTgvBX* kTgvBY, kTgvBlocks) k_tgv_dual(Box b, TgvArrays A, TgvScalars c, TgvConst K, int q,
                                                              int zchunk, const TgvFlag* flag) {
   if (flag->done) return;
-  const long long sxy = (long long)b.bx * b.by;
   const float* __restrict__ phb = A.phi[q];
   const float* __restrict__ chb = A.chi[q];
   const float* __restrict__ wbx = A.w[q][0];
   const float* __restrict__ wby = A.w[q][1];
   const float* __restrict__ wbz = A.w[q][2];
-  const uint8_t* __restrict__ m0 = A.m0;
-  const uint8_t* __restrict__ me = A.me;
   const float* __restrict__ lphi = A.lphi;
   float* __restrict__ eta = A.eta;
   float* __restrict__ p0 = A.p[0];
@@ -441,104 +466,80 @@ __global__ void __launch_bounds__(kTgvBX* kTgvBY, kTgvDualBlocks) k_tgv_dual(Box
   float* __restrict__ q3 = A.q[3];
   float* __restrict__ q4 = A.q[4];
   float* __restrict__ q5 = A.q[5];
-  const int i = blockIdx.x * kTgvBX + threadIdx.x, j = blockIdx.y * kTgvBY + threadIdx.y;
-  if (i >= b.bx || j >= b.by) return;
-  const int kbeg = blockIdx.z * zchunk;
-  const int kend = min(b.bz, (int)(blockIdx.z + 1) * zchunk);
-  if (kbeg >= kend) return;
-  long long s = (long long)kbeg * sxy + (long long)j * b.bx + i;
-  uint8_t nm0 = m0[s], nme = me[s];
-  for (int k = kbeg; k < kend; ++k, s += sxy) {
-    const bool in0 = nm0 != 0, inm = nme != 0;
-    if (k + 1 < kend) {
-      nm0 = m0[s + sxy];
-      nme = me[s + sxy];
+  TGV_COLUMN()
+  Stencil27 S;
+  float cc[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};  // chi_ at plane k: centre, x-, x+, y-, y+
+  float phm = 0.0f, phc = 0.0f;                  // phi_ at k - 1 and k
+  float wc[3] = {0.0f, 0.0f, 0.0f};              // w_ at k
+  int c0 = code_at(kbeg), c1 = code_at(kbeg + 1), c2 = code_at(kbeg + 2);
+  {
+    const unsigned s = (unsigned)kbeg * sxy + col;
+    if (c0 & 1) S.add(chb, s - sxy, bx, K, cc);
+    if ((c0 | c1) & 1) S.add(chb, s, bx, K, cc);
+    if (c0 & 1) {
+      phm = phb[s - sxy];
+      phc = phb[s];
     }
-    if (!(in0 || inm)) continue;
-    // Every load of the plane first, into registers, then the update in the reference's
-    // order.  Neighbour offsets are clamped to the box, which gives exactly the values the
-    // Neumann Laplacian substitutes at its faces (the centre), and loads that the
-    // zero-on-the-far-face differences and the interior-only stencil never use.
-    const long long dxm = i > 0 ? -1 : 0, dxp = i + 1 < b.bx ? 1 : 0;
-    const long long dym = j > 0 ? -(long long)b.bx : 0, dyp = j + 1 < b.by ? (long long)b.bx : 0;
-    const long long dzm = k > 0 ? -sxy : 0, dzp = k + 1 < b.bz ? sxy : 0;
-    const long long ox[3] = {dxm, 0, dxp}, oy[3] = {dym, 0, dyp}, oz[3] = {dzm, 0, dzp};
-    float ch[27];  // chi_ at (i + di - 1, j + dj - 1, k + dk - 1): ch[(dk * 3 + dj) * 3 + di]
-    float ph[7];   // phi_: centre, x-, x+, y-, y+, z-, z+
-    float wc[3], wx[3], wy[3], wz[3];  // w_ at the voxel and its x+1, y+1, z+1 neighbours
-    float lph = 0.0f, et = 0.0f, pc[3], qc[6];
-#pragma unroll
-    for (int dk = 0; dk < 3; ++dk)
-#pragma unroll
-      for (int dj = 0; dj < 3; ++dj)
-#pragma unroll
-        for (int di = 0; di < 3; ++di) ch[(dk * 3 + dj) * 3 + di] = 0.0f;
+    if (c0 & 2) {
+      wc[0] = wbx[s];
+      wc[1] = wby[s];
+      wc[2] = wbz[s];
+    }
+  }
+  for (int k = kbeg; k < kend; ++k) {
+    const unsigned s = (unsigned)k * sxy + col;
+    const int c3 = code_at(k + 3);
+    const bool in0 = (c0 & 1) != 0;
+    float pc[3] = {0.0f, 0.0f, 0.0f}, qc[6], wx[3], wy[3], ph[4], lph = 0.0f, et = 0.0f;
+    float wz[3] = {0.0f, 0.0f, 0.0f}, phz = 0.0f;
+    if (c0 & 2) {
+      pc[0] = p0[s];
+      pc[1] = p1[s];
+      pc[2] = p2[s];
+    }
     if (in0) {
-#pragma unroll
-      for (int dk = 0; dk < 3; ++dk)
-#pragma unroll
-        for (int dj = 0; dj < 3; ++dj)
-#pragma unroll
-          for (int di = 0; di < 3; ++di) ch[(dk * 3 + dj) * 3 + di] = chb[s + ox[di] + oy[dj] + oz[dk]];
-      ph[0] = phb[s];
-      ph[1] = phb[s + dxm];
-      ph[2] = phb[s + dxp];
-      ph[3] = phb[s + dym];
-      ph[4] = phb[s + dyp];
-      ph[5] = phb[s + dzm];
-      ph[6] = phb[s + dzp];
       lph = lphi[s];
       et = eta[s];
-#pragma unroll
-      for (int t = 0; t < 6; ++t) qc[t] = A.q[t][s];
-      wx[0] = wbx[s + dxp];
-      wx[1] = wby[s + dxp];
-      wx[2] = wbz[s + dxp];
-      wy[0] = wbx[s + dyp];
-      wy[1] = wby[s + dyp];
-      wy[2] = wbz[s + dyp];
-      wz[0] = wbx[s + dzp];
-      wz[1] = wby[s + dzp];
-      wz[2] = wbz[s + dzp];
-    } else {
-      ch[13] = chb[s];
-      ch[14] = chb[s + dxp];
-      ch[16] = chb[s + dyp];
-      ch[22] = chb[s + dzp];
+      qc[0] = q0[s];
+      qc[1] = q1[s];
+      qc[2] = q2[s];
+      qc[3] = q3[s];
+      qc[4] = q4[s];
+      qc[5] = q5[s];
+      wx[0] = wbx[s + 1];
+      wx[1] = wby[s + 1];
+      wx[2] = wbz[s + 1];
+      wy[0] = wbx[s + bx];
+      wy[1] = wby[s + bx];
+      wy[2] = wbz[s + bx];
+      ph[0] = phb[s - 1];
+      ph[1] = phb[s + 1];
+      ph[2] = phb[s - bx];
+      ph[3] = phb[s + bx];
     }
-    wc[0] = wbx[s];
-    wc[1] = wby[s];
-    wc[2] = wbz[s];
-    pc[0] = p0[s];
-    pc[1] = p1[s];
-    pc[2] = p2[s];
-    const float cb = ch[13];
-    if (in0) {
-      const float a0 = ph[0];
-      const float t1 = c.hx2 * (ph[1] - 2.0f * a0 + ph[2]) + c.hy2 * (ph[3] - 2.0f * a0 + ph[4]) +
-                       c.hz2 * (ph[5] - 2.0f * a0 + ph[6]);
-      float t2 = 0.0f;
-      if (interior(i, j, k, b)) {
-        float sum = 0.0f;
-#pragma unroll
-        for (int dk = 0; dk < 3; ++dk)
-#pragma unroll
-          for (int dj = 0; dj < 3; ++dj)
-#pragma unroll
-            for (int di = 0; di < 3; ++di) sum += K.st[(di * 3 + dj) * 3 + dk] * ch[(dk * 3 + dj) * 3 + di];
-        t2 = sum;
+    if ((c0 | c1) & 1) phz = phb[s + sxy];
+    if ((c0 & 1) | (c1 & 2)) {
+      wz[0] = wbx[s + sxy];
+      wz[1] = wby[s + sxy];
+      wz[2] = wbz[s + sxy];
+    }
+    float cn[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f}, t2 = 0.0f;
+    if ((c0 | c1 | c2) & 1) t2 = S.add(chb, s + sxy, bx, K, cn);
+    else S.skip();
+    if (c0 & 2) {
+      const float cb = cc[0];
+      float gx = 0.0f, gy = 0.0f, gz = 0.0f;
+      if (in0) {
+        const float t1 = c.hx2 * (ph[0] - 2.0f * phc + ph[1]) + c.hy2 * (ph[2] - 2.0f * phc + ph[3]) +
+                         c.hz2 * (phm - 2.0f * phc + phz);
+        eta[s] = et + c.sigma * (-t1 + t2 - lph);
+        gx = c.sstep * ((cc[2] - cb) * c.hx);
+        gy = c.sstep * ((cc[4] - cb) * c.hy);
+        gz = c.sstep * ((cn[0] - cb) * c.hz);
       }
-      et += c.sigma * (-t1 + t2 - lph);
-      eta[s] = et;
-    }
-    {
-      const float gx = i + 1 < b.bx ? (ch[14] - cb) * c.hx : 0.0f;
-      const float gy = j + 1 < b.by ? (ch[16] - cb) * c.hy : 0.0f;
-      const float gz = k + 1 < b.bz ? (ch[22] - cb) * c.hz : 0.0f;
-      const float s0 = in0 ? c.sstep : 0.0f, s1 = inm ? c.sstep : 0.0f;
-      float px = pc[0] + (s0 * gx - s1 * wc[0]);
-      float py = pc[1] + (s0 * gy - s1 * wc[1]);
-      float pz = pc[2] + (s0 * gz - s1 * wc[2]);
+      float px = pc[0] + (gx - c.sstep * wc[0]);
+      float py = pc[1] + (gy - c.sstep * wc[1]);
+      float pz = pc[2] + (gz - c.sstep * wc[2]);
       const float nrm = sqrtf(px * px + py * py + pz * pz);
       if (nrm > c.alpha1) {
         const float sc = c.alpha1 / nrm;
@@ -550,25 +551,16 @@ __global__ void __launch_bounds__(kTgvBX* kTgvBY, kTgvDualBlocks) k_tgv_dual(Box
       p1[s] = py;
       p2[s] = pz;
     }
-    if (in0) {
-      // symgrad (src/utils/gradient.rs:300-372), zero on the far faces
-      const float wx0 = wc[0], wy0 = wc[1], wz0 = wc[2];
-      float sxx = 0.0f, sxy_ = 0.0f, sxz = 0.0f, syy = 0.0f, syz = 0.0f, szz = 0.0f;
-      if (i + 1 < b.bx) {
-        sxx = (wx[0] - wx0) * c.hx;
-        sxy_ = ((wx[1] - wy0) * c.hx) * 0.5f;
-        sxz = ((wx[2] - wz0) * c.hx) * 0.5f;
-      }
-      if (j + 1 < b.by) {
-        syy = (wy[1] - wy0) * c.hy;
-        sxy_ += ((wy[0] - wx0) * c.hy) * 0.5f;
-        syz = ((wy[2] - wz0) * c.hy) * 0.5f;
-      }
-      if (k + 1 < b.bz) {
-        szz = (wz[2] - wz0) * c.hz;
-        sxz += ((wz[0] - wx0) * c.hz) * 0.5f;
-        syz += ((wz[1] - wy0) * c.hz) * 0.5f;
-      }
+    if (in0) {  // symgrad (src/utils/gradient.rs:300-372)
+      const float sxx = (wx[0] - wc[0]) * c.hx;
+      float sxy_ = ((wx[1] - wc[1]) * c.hx) * 0.5f;
+      float sxz = ((wx[2] - wc[2]) * c.hx) * 0.5f;
+      const float syy = (wy[1] - wc[1]) * c.hy;
+      sxy_ += ((wy[0] - wc[0]) * c.hy) * 0.5f;
+      float syz = ((wy[2] - wc[2]) * c.hy) * 0.5f;
+      const float szz = (wz[2] - wc[2]) * c.hz;
+      sxz += ((wz[0] - wc[0]) * c.hz) * 0.5f;
+      syz += ((wz[1] - wc[1]) * c.hz) * 0.5f;
       float qq[6] = {qc[0] + c.sstep * sxx, qc[1] + c.sstep * sxy_, qc[2] + c.sstep * sxz,
                      qc[3] + c.sstep * syy, qc[4] + c.sstep * syz, qc[5] + c.sstep * szz};
       const float fro = sqrtf(qq[0] * qq[0] + qq[3] * qq[3] + qq[5] * qq[5] +
@@ -585,148 +577,142 @@ __global__ void __launch_bounds__(kTgvBX* kTgvBY, kTgvDualBlocks) k_tgv_dual(Box
       q4[s] = qq[4];
       q5[s] = qq[5];
     }
+#pragma unroll
+    for (int t = 0; t < 5; ++t) cc[t] = cn[t];
+#pragma unroll
+    for (int t = 0; t < 3; ++t) wc[t] = wz[t];
+    phm = phc;
+    phc = phz;
+    c0 = c1;
+    c1 = c2;
+    c2 = c3;
   }
 }
 
 // Primal update and extrapolation (tgv.rs:1215-1271).  Buffers [1-q] hold the current
 // iterate x (read), [q] the extrapolation consumed by the dual step (overwritten with
-// x_new); [1-q] then receives 2 x_new - x.  Restrict-qualified pointers, the next
-// plane's masks fetched ahead and the plane's values loaded before the update, as in
-// k_tgv_dual.
-__global__ void __launch_bounds__(kTgvBX* kTgvBY, kTgvPrimalBlocks) k_tgv_primal(Box b, TgvArrays A, TgvScalars c,
+// x_new); [1-q] then receives 2 x_new - x.  Outside the eroded mask every variable stays
+// zero, and phi and chi outside mask0, so those voxels are neither read nor written.
+__global__ void __launch_bounds__(kTgvBX* kTgvBY, kTgvBlocks) k_tgv_primal(Box b, TgvArrays A, TgvScalars c,
                                                                               TgvConst K, int q, int zchunk,
                                                                               const TgvFlag* flag) {
   if (flag->done) return;
-  const long long sxy = (long long)b.bx * b.by;
-  const uint8_t* __restrict__ m0 = A.m0;
-  const uint8_t* __restrict__ me = A.me;
   const float* __restrict__ etab = A.eta;
   const float* __restrict__ p0 = A.p[0];
   const float* __restrict__ p1 = A.p[1];
   const float* __restrict__ p2 = A.p[2];
-  const float* __restrict__ qb[6] = {A.q[0], A.q[1], A.q[2], A.q[3], A.q[4], A.q[5]};
-  const float* __restrict__ phr = A.phi[1 - q];
-  float* __restrict__ phw = A.phi[q];
-  float* __restrict__ phx = A.phi[1 - q];
-  const float* __restrict__ chr = A.chi[1 - q];
-  float* __restrict__ chw = A.chi[q];
-  float* __restrict__ chx = A.chi[1 - q];
-  // eta and q are only ever updated inside mask0 (k_tgv_dual) and start at zero, so
-  // m0*eta = eta and m0*q = q
-  auto mq = [&](int comp, long long t) { return qb[comp][t]; };
-  const int i = blockIdx.x * kTgvBX + threadIdx.x, j = blockIdx.y * kTgvBY + threadIdx.y;
-  if (i >= b.bx || j >= b.by) return;
-  const int kbeg = blockIdx.z * zchunk;
-  const int kend = min(b.bz, (int)(blockIdx.z + 1) * zchunk);
-  if (kbeg >= kend) return;
-  long long s = (long long)kbeg * sxy + (long long)j * b.bx + i;
-  uint8_t nm0 = m0[s], nme = me[s];
-  for (int k = kbeg; k < kend; ++k, s += sxy) {
-    const bool in0 = nm0 != 0, inm = nme != 0;
-    if (k + 1 < kend) {
-      nm0 = m0[s + sxy];
-      nme = me[s + sxy];
+  const float* __restrict__ q0 = A.q[0];
+  const float* __restrict__ q1 = A.q[1];
+  const float* __restrict__ q2 = A.q[2];
+  const float* __restrict__ q3 = A.q[3];
+  const float* __restrict__ q4 = A.q[4];
+  const float* __restrict__ q5 = A.q[5];
+  // a voxel reads x in [1-q] before it writes either buffer there, and no other voxel reads them
+  float* phw = A.phi[q];
+  float* phx = A.phi[1 - q];
+  float* chw = A.chi[q];
+  float* chx = A.chi[1 - q];
+  TGV_COLUMN()
+  Stencil27 S;
+  float ec[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f}, em = 0.0f;  // eta at plane k (as cc above) and k - 1
+  float pz = 0.0f, qz[3] = {0.0f, 0.0f, 0.0f};              // mask0 p2; q2, q4, q5 at k - 1
+  int c0 = code_at(kbeg), c1 = code_at(kbeg + 1), c2 = code_at(kbeg + 2);
+  {
+    const unsigned s = (unsigned)kbeg * sxy + col;
+    if (c0 & 1) {
+      S.add(etab, s - sxy, bx, K, ec);
+      em = ec[0];
     }
-    // every load of the plane first (clamped neighbour offsets give the values the
-    // Neumann faces substitute), then the update in the reference's order
-    const long long dxm = i > 0 ? -1 : 0, dxp = i + 1 < b.bx ? 1 : 0;
-    const long long dym = j > 0 ? -(long long)b.bx : 0, dyp = j + 1 < b.by ? (long long)b.bx : 0;
-    const long long dzm = k > 0 ? -sxy : 0, dzp = k + 1 < b.bz ? sxy : 0;
-    const long long ox[3] = {dxm, 0, dxp}, oy[3] = {dym, 0, dyp}, oz[3] = {dzm, 0, dzp};
-    float e27[27];  // eta at (i + di - 1, j + dj - 1, k + dk - 1): e27[(dk * 3 + dj) * 3 + di]
-    float pc[3] = {0.0f, 0.0f, 0.0f}, pm[3] = {0.0f, 0.0f, 0.0f};  // p at the voxel; p_a at the voxel - e_a
-    float mm[3] = {0.0f, 0.0f, 0.0f};  // mask0 at the voxel - e_a (1 or 0)
-    float qc[6], qx[3], qy[3], qz[3];  // q at the voxel; (q0,q1,q2)(x-1), (q1,q3,q4)(y-1), (q2,q4,q5)(z-1)
-#pragma unroll
-    for (int t = 0; t < 27; ++t) e27[t] = 0.0f;
-    if (in0) {
-#pragma unroll
-      for (int dk = 0; dk < 3; ++dk)
-#pragma unroll
-        for (int dj = 0; dj < 3; ++dj)
-#pragma unroll
-          for (int di = 0; di < 3; ++di) e27[(dk * 3 + dj) * 3 + di] = etab[s + ox[di] + oy[dj] + oz[dk]];
-      pm[0] = p0[s + dxm];
-      pm[1] = p1[s + dym];
-      pm[2] = p2[s + dzm];
-      mm[0] = m0[s + dxm] ? 1.0f : 0.0f;
-      mm[1] = m0[s + dym] ? 1.0f : 0.0f;
-      mm[2] = m0[s + dzm] ? 1.0f : 0.0f;
-    }
-    if (in0 || inm) {
-      pc[0] = p0[s];
-      pc[1] = p1[s];
-      pc[2] = p2[s];
-    }
-    if (inm) {
-#pragma unroll
-      for (int t = 0; t < 6; ++t) qc[t] = mq(t, s);
-      qx[0] = mq(0, s + dxm);
-      qx[1] = mq(1, s + dxm);
-      qx[2] = mq(2, s + dxm);
-      qy[0] = mq(1, s + dym);
-      qy[1] = mq(3, s + dym);
-      qy[2] = mq(4, s + dym);
-      qz[0] = mq(2, s + dzm);
-      qz[1] = mq(4, s + dzm);
-      qz[2] = mq(5, s + dzm);
-    }
-    const float phi_old = phr[s];
-    const float chi_old = chr[s];
-    float wn[3], wo[3];
-#pragma unroll
-    for (int comp = 0; comp < 3; ++comp) wo[comp] = wn[comp] = A.w[1 - q][comp][s];
-    // phi
-    float lap = 0.0f;
-    if (in0) {
-      const float a0 = e27[13];
-      lap = c.hx2 * (e27[12] - 2.0f * a0 + e27[14]) + c.hy2 * (e27[10] - 2.0f * a0 + e27[16]) +
-            c.hz2 * (e27[4] - 2.0f * a0 + e27[22]);
-    }
-    const float phi_new = (phi_old + c.tau * lap) / (1.0f + (inm ? c.tau : 0.0f));
-    // chi: bdiv_masked (src/utils/gradient.rs:497-565) minus the stencil of m0*eta
-    float t1 = 0.0f;
-    if (in0) {
-      const float gxt = 1.0f * pc[0] * c.hx - (i > 0 ? mm[0] * pm[0] * c.hx : 0.0f);
-      const float gyt = 1.0f * pc[1] * c.hy - (j > 0 ? mm[1] * pm[1] * c.hy : 0.0f);
-      const float gzt = 1.0f * pc[2] * c.hz - (k > 0 ? mm[2] * pm[2] * c.hz : 0.0f);
-      t1 = gxt + gyt + gzt;
-    }
-    float t2 = 0.0f;
-    if (in0 && interior(i, j, k, b)) {
-      float sum = 0.0f;
-#pragma unroll
-      for (int dk = 0; dk < 3; ++dk)
-#pragma unroll
-        for (int dj = 0; dj < 3; ++dj)
-#pragma unroll
-          for (int di = 0; di < 3; ++di) sum += K.st[(di * 3 + dj) * 3 + dk] * e27[(dk * 3 + dj) * 3 + di];
-      t2 = sum;
-    }
-    const float chi_new = chi_old + c.tstep * (t1 - t2);
-    // w: symdiv of m0*q (src/utils/gradient.rs:380-432), zero on the near faces
-    if (inm) {
-      const float bx0 = i > 0 ? qx[0] : 0.0f, bx1 = i > 0 ? qx[1] : 0.0f, bx2 = i > 0 ? qx[2] : 0.0f;
-      const float by1 = j > 0 ? qy[0] : 0.0f, by3 = j > 0 ? qy[1] : 0.0f, by4 = j > 0 ? qy[2] : 0.0f;
-      const float bz2 = k > 0 ? qz[0] : 0.0f, bz4 = k > 0 ? qz[1] : 0.0f, bz5 = k > 0 ? qz[2] : 0.0f;
-      const float dqx = (qc[0] - bx0) * c.hx + (qc[1] - by1) * c.hy + (qc[2] - bz2) * c.hz;
-      const float dqy = (qc[1] - bx1) * c.hx + (qc[3] - by3) * c.hy + (qc[4] - bz4) * c.hz;
-      const float dqz = (qc[2] - bx2) * c.hx + (qc[4] - by4) * c.hy + (qc[5] - bz5) * c.hz;
-      wn[0] += c.tstep * (pc[0] + dqx);
-      wn[1] += c.tstep * (pc[1] + dqy);
-      wn[2] += c.tstep * (pc[2] + dqz);
-    }
-    phw[s] = phi_new;
-    phx[s] = 2.0f * phi_new - phi_old;
-    chw[s] = chi_new;
-    chx[s] = 2.0f * chi_new - chi_old;
-#pragma unroll
-    for (int comp = 0; comp < 3; ++comp) {
-      A.w[q][comp][s] = wn[comp];
-      A.w[1 - q][comp][s] = 2.0f * wn[comp] - wo[comp];
+    if ((c0 | c1) & 1) S.add(etab, s, bx, K, ec);
+    if ((c0 & 2) && kbeg > 0 && (mk[s - sxy] & 1)) {
+      pz = p2[s - sxy];
+      qz[0] = q2[s - sxy];
+      qz[1] = q4[s - sxy];
+      qz[2] = q5[s - sxy];
     }
   }
+  for (int k = kbeg; k < kend; ++k) {
+    const unsigned s = (unsigned)k * sxy + col;
+    const int c3 = code_at(k + 3);
+    const bool in0 = (c0 & 1) != 0;
+    float pn[3] = {0.0f, 0.0f, 0.0f}, qn[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    float pmx = 0.0f, pmy = 0.0f, qx[3] = {0.0f, 0.0f, 0.0f}, qy[3] = {0.0f, 0.0f, 0.0f};
+    float phi_old = 0.0f, chi_old = 0.0f, wo[3] = {0.0f, 0.0f, 0.0f};
+    if (c0 & 2) {
+      // q is zero outside mask0
+      pn[0] = p0[s];
+      pn[1] = p1[s];
+      pn[2] = p2[s];
+      if (in0) {
+        qn[0] = q0[s];
+        qn[1] = q1[s];
+        qn[2] = q2[s];
+        qn[3] = q3[s];
+        qn[4] = q4[s];
+        qn[5] = q5[s];
+        phi_old = phx[s];
+        chi_old = chx[s];
+        const float px = p0[s - 1], py = p1[s - bx];
+        pmx = mk[s - 1] & 1 ? px : 0.0f;
+        pmy = mk[s - bx] & 1 ? py : 0.0f;
+      }
+      if (i > 0) {
+        qx[0] = q0[s - 1];
+        qx[1] = q1[s - 1];
+        qx[2] = q2[s - 1];
+      }
+      if (j > 0) {
+        qy[0] = q1[s - bx];
+        qy[1] = q3[s - bx];
+        qy[2] = q4[s - bx];
+      }
+#pragma unroll
+      for (int t = 0; t < 3; ++t) wo[t] = A.w[1 - q][t][s];
+    }
+    float en[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f}, t2 = 0.0f;
+    if ((c0 | c1 | c2) & 1) t2 = S.add(etab, s + sxy, bx, K, en);
+    else S.skip();
+    if (c0 & 2) {
+      if (in0) {
+        const float a0 = ec[0];
+        const float lap = c.hx2 * (ec[1] - 2.0f * a0 + ec[2]) + c.hy2 * (ec[3] - 2.0f * a0 + ec[4]) +
+                          c.hz2 * (em - 2.0f * a0 + en[0]);
+        const float phi_new = (phi_old + c.tau * lap) / (1.0f + c.tau);
+        // chi: bdiv_masked (src/utils/gradient.rs:497-565) minus the stencil of m0*eta
+        const float gxt = 1.0f * pn[0] * c.hx - pmx * c.hx;
+        const float gyt = 1.0f * pn[1] * c.hy - pmy * c.hy;
+        const float gzt = 1.0f * pn[2] * c.hz - pz * c.hz;
+        const float chi_new = chi_old + c.tstep * (gxt + gyt + gzt - t2);
+        phw[s] = phi_new;
+        phx[s] = 2.0f * phi_new - phi_old;
+        chw[s] = chi_new;
+        chx[s] = 2.0f * chi_new - chi_old;
+      }
+      // w: symdiv of q (src/utils/gradient.rs:380-432), zero on the near faces
+      const float dqx = (qn[0] - qx[0]) * c.hx + (qn[1] - qy[0]) * c.hy + (qn[2] - qz[0]) * c.hz;
+      const float dqy = (qn[1] - qx[1]) * c.hx + (qn[3] - qy[1]) * c.hy + (qn[4] - qz[1]) * c.hz;
+      const float dqz = (qn[2] - qx[2]) * c.hx + (qn[4] - qy[2]) * c.hy + (qn[5] - qz[2]) * c.hz;
+      const float wn[3] = {wo[0] + c.tstep * (pn[0] + dqx), wo[1] + c.tstep * (pn[1] + dqy),
+                           wo[2] + c.tstep * (pn[2] + dqz)};
+#pragma unroll
+      for (int t = 0; t < 3; ++t) {
+        A.w[q][t][s] = wn[t];
+        A.w[1 - q][t][s] = 2.0f * wn[t] - wo[t];
+      }
+    }
+    em = ec[0];
+#pragma unroll
+    for (int t = 0; t < 5; ++t) ec[t] = en[t];
+    pz = in0 ? pn[2] : 0.0f;
+    qz[0] = qn[2];
+    qz[1] = qn[4];
+    qz[2] = qn[5];
+    c0 = c1;
+    c1 = c2;
+    c2 = c3;
+  }
 }
+#undef TGV_COLUMN
 
 // Relative change of chi over mask0 at iteration `it` (tgv.rs:923-941, 1146-1154); sets
 // the flag below tol, else saves chi for the next check.
@@ -831,9 +817,10 @@ void tgv_device(qsm_ctx* ctx, const double* phase, const uint8_t* mask, const qs
   float* ph = F("phase");
   uint8_t* m0s = ws<uint8_t>(ctx, "tgv.m0s", (size_t)B);
   uint8_t* mes = ws<uint8_t>(ctx, "tgv.mes", (size_t)B);
+  uint8_t* mk = ws<uint8_t>(ctx, "tgv.mk", (size_t)B);
   {
     LaunchScope ls(ctx, "tgv_extract");
-    k_tgv_extract<<<grid1d(B), 256, 0, ctx->stream>>>(b, d.nx, d.ny, phase, m0f, mef, ph, m0s, mes);
+    k_tgv_extract<<<grid1d(B), 256, 0, ctx->stream>>>(b, d.nx, d.ny, phase, m0f, mef, ph, m0s, mes, mk);
     ls.done();
   }
   const float vsx = (float)d.vsx, vsy = (float)d.vsy, vsz = (float)d.vsz;
@@ -880,8 +867,7 @@ void tgv_device(qsm_ctx* ctx, const double* phase, const uint8_t* mask, const qs
   // state, zero initialised
   TgvArrays A;
   A.lphi = lphi;
-  A.m0 = m0s;
-  A.me = mes;
+  A.mk = mk;
   const char* names[] = {"eta", "px", "py", "pz", "qxx", "qxy", "qxz", "qyy", "qyz", "qzz", "phi0", "phi1",
                          "chi0", "chi1", "wx0", "wy0", "wz0", "wx1", "wy1", "wz1", "chi_prev"};
   float* buf[21];
@@ -904,9 +890,8 @@ void tgv_device(qsm_ctx* ctx, const double* phase, const uint8_t* mask, const qs
   // before iteration t the current iterate sits in [t % 2] and its extrapolation in
   // [(t + 1) % 2]; the dual step reads the extrapolation
   const unsigned gblocks = grid1d(B);
-  // primal/dual tiles: ~16 blocks per SM in all, each marching zchunk planes
   const unsigned tgx = (unsigned)((b.bx + kTgvBX - 1) / kTgvBX), tgy = (unsigned)((b.by + kTgvBY - 1) / kTgvBY);
-  const long long nzc = std::max<long long>(1, 16LL * sm_count(ctx) / ((long long)tgx * tgy));
+  const long long nzc = std::max<long long>(1, (long long)kTgvChunks * sm_count(ctx) / ((long long)tgx * tgy));
   const int zchunk = (int)((b.bz + nzc - 1) / nzc);
   const dim3 tgrid(tgx, tgy, (unsigned)((b.bz + zchunk - 1) / zchunk)), tblock(kTgvBX, kTgvBY);
   auto one_iter = [&](size_t t) {
