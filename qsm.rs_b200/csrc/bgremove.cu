@@ -232,7 +232,7 @@ void vsharp_impl(qsm_ctx* ctx, const GridDims& d, const double* field, const uin
     smv_erode_first(ctx, d, mask, std::vector<SmvSphere>(spheres.begin() + g0, spheres.begin() + g1), delta, first);
     {
       LaunchScope ls(ctx, "vsharp_rows");
-      k_row_hits<<<x_rows_grid(f.g), 256, 0, ctx->stream>>>(d.nx, d.ny * d.nz, first, hits);
+      k_row_hits<<<x_rows_grid(ctx, k_row_hits, f.g), 256, 0, ctx->stream>>>(d.nx, d.ny * d.nz, first, hits);
       ls.done();
     }
     for (size_t idx = g0; idx < g1; ++idx) {

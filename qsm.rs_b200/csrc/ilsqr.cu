@@ -973,14 +973,14 @@ void ilsqr_impl(qsm_ctx* ctx, const GridDims& d, const double* f, const uint8_t*
   T* wg = ws<T>(ctx, nm("wgrad"), (size_t)(3 * N));
   {
     LaunchScope ls(ctx, "ilsqr_fgrad_masked");
-    k_fgrad_masked<TD><<<grid1d(N), 256, 0, ctx->stream>>>(xfs, mask, d.nx, d.ny, d.nz, 1.0 / d.vsx, 1.0 / d.vsy,
+    k_fgrad_masked<TD><<<wave_grid(ctx, k_fgrad_masked<TD>, N), 256, 0, ctx->stream>>>(xfs, mask, d.nx, d.ny, d.nz, 1.0 / d.vsx, 1.0 / d.vsy,
                                                           1.0 / d.vsz, dwork);
     ls.done();
     const std::vector<double> tx = percentiles(ctx, dwork, mask, N, count, {50.0, 70.0});
     const std::vector<double> ty = percentiles(ctx, dwork + N, mask, N, count, {50.0, 70.0});
     const std::vector<double> tz = percentiles(ctx, dwork + 2 * N, mask, N, count, {50.0, 70.0});
     LaunchScope ls2(ctx, "ilsqr_grad_weights");
-    k_grad_weights<T><<<grid1d(N), 256, 0, ctx->stream>>>(N, dwork, mask, tx[0], tx[1], ty[0], ty[1], tz[0], tz[1], wg);
+    k_grad_weights<T><<<wave_grid(ctx, k_grad_weights<T>, N), 256, 0, ctx->stream>>>(N, dwork, mask, tx[0], tx[1], ty[0], ty[1], tz[0], tz[1], wg);
     ls2.done();
   }
   LsmrState* mst = ws<LsmrState>(ctx, nm("lsmr"), 1);
@@ -1024,7 +1024,7 @@ void ilsqr_impl(qsm_ctx* ctx, const GridDims& d, const double* f, const uint8_t*
   };
   {
     LaunchScope ls(ctx, "lsmr_grad");
-    k_lsmr_grad<double, T><<<grid1d(N), 256, 0, ctx->stream>>>(d.nx, d.ny, d.nz, hx, hy, hz, xlsqr, wg, u3, mst,
+    k_lsmr_grad<double, T><<<wave_grid(ctx, k_lsmr_grad<double, T>, N), 256, 0, ctx->stream>>>(d.nx, d.ny, d.nz, hx, hy, hz, xlsqr, wg, u3, mst,
                                                                 partials, 1);
     ls.done();
   }
@@ -1038,12 +1038,12 @@ void ilsqr_impl(qsm_ctx* ctx, const GridDims& d, const double* f, const uint8_t*
     mic_chain(LoadScaled<T>{vv, &mst->sv, d.nx}, StoreReal<T>{rq, d.nx, invn});
     {
       LaunchScope ls(ctx, "lsmr_grad");
-      k_lsmr_grad<T, T><<<grid1d(N), 256, 0, ctx->stream>>>(d.nx, d.ny, d.nz, hx, hy, hz, rq, wg, u3, mst, partials, 0);
+      k_lsmr_grad<T, T><<<wave_grid(ctx, k_lsmr_grad<T, T>, N), 256, 0, ctx->stream>>>(d.nx, d.ny, d.nz, hx, hy, hz, rq, wg, u3, mst, partials, 0);
       ls.done();
     }
     at_u(0);
     LaunchScope ls(ctx, "lsmr_update");
-    k_lsmr_update<T><<<grid1d(N), 256, 0, ctx->stream>>>(N, hh, hbar, xx, vv, mst, partials);
+    k_lsmr_update<T><<<wave_grid(ctx, k_lsmr_update<T>, N), 256, 0, ctx->stream>>>(N, hh, hbar, xx, vv, mst, partials);
     ls.done();
   });
 

@@ -241,9 +241,29 @@ template <typename T> cplx_t<T>* x_stage_c(qsm_ctx* ctx, const Fft3<T>& f) {
 // of its own around the plain kernel, except in small volumes, where the launch costs more
 // than the two-factor kernel (functor inside) loses.
 template <typename T> inline bool x_use_stage(const Fft3<T>& f) { return f.g.nvox() > (1LL << 20); }
-inline unsigned x_rows_grid(const Geom& g) {
-  const long long b = ((long long)g.nrows() + 7) / 8;
-  return (unsigned)(b < 1184 ? b : 1184);
+// Persistent grid: as many CTAs as fit on the device at once, capped by the work.
+template <class K> unsigned persistent_grid(qsm_ctx* ctx, K kernel, int threads, size_t smem, long long work) {
+  int per_sm = 0;
+  QSM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
+  if (per_sm < 1) throw QsmError(QSM_ERR_UNSUPPORTED_SIZE, "transform tile does not fit on an SM");
+  long long g = (long long)per_sm * sm_count(ctx);
+  if (g > work) g = work;
+  if (g < 1) g = 1;
+  return (unsigned)g;
+}
+
+// Grid of 256-thread blocks of an elementwise kernel over n elements: one full wave.  A grid
+// fixed at 16 blocks per SM left the last of three to four waves of the register-heavy
+// kernels mostly idle (48 registers: five blocks per SM, adjoint update at 160x192x160 111.6
+// us, 92.3 in one wave).
+template <class K> unsigned wave_grid(qsm_ctx* ctx, K kernel, long long n) {
+  return persistent_grid(ctx, kernel, 256, 0, (n + 255) / 256);
+}
+
+// One full wave: with 47 registers five blocks fit on an SM, and a fixed eight per SM ran
+// them in two waves, the second mostly idle.
+template <class K> unsigned x_rows_grid(qsm_ctx* ctx, K kernel, const Geom& g) {
+  return persistent_grid(ctx, kernel, 256, 0, ((long long)g.nrows() + 7) / 8);
 }
 
 // DEAD (compile-time kernels only): the pass reads ld's rows for the last time and drops
@@ -274,7 +294,7 @@ void run_x_r2c(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* spec, const Load& ld, 
   T* st = x_stage(ctx, f);
   {
     LaunchScope ls(ctx, "x_load");
-    k_x_load<T, T, Load><<<x_rows_grid(f.g), 256, 0, ctx->stream>>>(f.g, f.g.nx, ld, st, done);
+    k_x_load<T, T, Load><<<x_rows_grid(ctx, k_x_load<T, T, Load>, f.g), 256, 0, ctx->stream>>>(f.g, f.g.nx, ld, st, done);
     ls.done();
   }
   if (listed) x_plain_r2c<T>(ctx, f, st, spec, done);
@@ -310,7 +330,7 @@ void run_x_c2r(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* spec, const Stor
   if (listed) x_plain_c2r<T>(ctx, f, spec, buf, T(1), done);
   else run_x_c2r_rt<T>(ctx, f, spec, buf, T(1), done);
   LaunchScope ls(ctx, "x_store");
-  k_x_store<T, T, Store><<<x_rows_grid(f.g), 256, 0, ctx->stream>>>(f.g, f.g.nx, buf, st, done);
+  k_x_store<T, T, Store><<<x_rows_grid(ctx, k_x_store<T, T, Store>, f.g), 256, 0, ctx->stream>>>(f.g, f.g.nx, buf, st, done);
   ls.done();
 }
 
@@ -366,33 +386,22 @@ void run_x_full(qsm_ctx* ctx, const Fft3<T>& f, const Load& ld, const Mid& mid, 
   C* rows = x_stage_c(ctx, f);
   {
     LaunchScope ls(ctx, "x_load");
-    k_x_load<T, C, Load><<<x_rows_grid(f.g), 256, 0, ctx->stream>>>(f.g, f.g.pitch, ld, rows, done);
+    k_x_load<T, C, Load><<<x_rows_grid(ctx, k_x_load<T, C, Load>, f.g), 256, 0, ctx->stream>>>(f.g, f.g.pitch, ld, rows, done);
     ls.done();
   }
   if constexpr (D1 != 0) run_x_c2c_rt<T, D1>(ctx, f, rows, done);
   {
     LaunchScope ls(ctx, "x_mid");
-    k_x_mid<T, Mid><<<x_rows_grid(f.g), 256, 0, ctx->stream>>>(f.g, mid, rows, done);
+    k_x_mid<T, Mid><<<x_rows_grid(ctx, k_x_mid<T, Mid>, f.g), 256, 0, ctx->stream>>>(f.g, mid, rows, done);
     ls.done();
   }
   if constexpr (D2 != 0) run_x_c2c_rt<T, D2>(ctx, f, rows, done);
   LaunchScope ls(ctx, "x_store");
-  k_x_store<T, C, Store><<<x_rows_grid(f.g), 256, 0, ctx->stream>>>(f.g, f.g.pitch, rows, st, done);
+  k_x_store<T, C, Store><<<x_rows_grid(ctx, k_x_store<T, C, Store>, f.g), 256, 0, ctx->stream>>>(f.g, f.g.pitch, rows, st, done);
   ls.done();
 }
 
 template <typename T> inline int yz_cols() { return sizeof(T) == 4 ? 16 : 8; }
-
-// Persistent grid: as many CTAs as fit on the device at once, capped by the work.
-template <class K> unsigned persistent_grid(qsm_ctx* ctx, K kernel, int threads, size_t smem, long long work) {
-  int per_sm = 0;
-  QSM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
-  if (per_sm < 1) throw QsmError(QSM_ERR_UNSUPPORTED_SIZE, "transform tile does not fit on an SM");
-  long long g = (long long)per_sm * sm_count(ctx);
-  if (g > work) g = work;
-  if (g < 1) g = 1;
-  return (unsigned)g;
-}
 
 // Tile walk of a Y (axis 1) or Z (axis 2) pass with P-column tiles.  edge: walk a
 // narrow column remainder (at most P/4 columns) as edge tiles (TileWalk); only the

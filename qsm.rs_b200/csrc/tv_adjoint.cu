@@ -169,6 +169,7 @@ void tv_unrolled_impl(qsm_ctx* ctx, const GridDims& d, const double* f, const ui
   QSM_CUDA(cudaMemsetAsync(s, 0, sizeof(T) * N, ctx->stream));
   QSM_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned), ctx->stream));
   QSM_CUDA(cudaMemsetAsync(tbar, 0, sizeof(double), ctx->stream));
+  const unsigned gadj = wave_grid(ctx, k_tv_adj_update<T>, N);
   int cur = 0;           // vb[cur] holds vbar_j for the step about to run
   bool have_vbar = false;  // false: vbar_K = 0
   size_t j = K;
@@ -194,7 +195,7 @@ void tv_unrolled_impl(qsm_ctx* ctx, const GridDims& d, const double* f, const ui
       // adjoint of U_i from S_i = (y_i, u_{i-1})
       const State S = state(i);
       LaunchScope ls(ctx, "tv_adj_update");
-      k_tv_adj_update<T><<<g, 256, 0, ctx->stream>>>(d.nx, d.ny, d.nz, v.hx, v.hy, v.hz, v.thr, v.x0,
+      k_tv_adj_update<T><<<gadj, 256, 0, ctx->stream>>>(d.nx, d.ny, d.nz, v.hx, v.hy, v.hz, v.thr, v.x0,
                                                      S.y, S.u, have_vbar ? vb[cur] : nullptr, w, vb[1 - cur], partials, counter,
                                                      tbar);
       ls.done();
