@@ -9,6 +9,7 @@
 // truncation decisions are the reference's.
 #include "closed_form_ops.cuh"
 #include "functors.cuh"
+#include "plane.cuh"
 #include "solvers.h"
 
 #include <algorithm>
@@ -23,11 +24,9 @@ void closed_form_chain(qsm_ctx* ctx, const GridDims& d, const double* d_in, cons
   using C = cplx_t<T>;
   Fft3<T> f = make_fft3<T>(ctx, d);
   C* spec = ws<C>(ctx, "spec", (size_t)f.g.hsize());
-  run_x_r2c<T>(ctx, f, spec, LoadCast<double, T>{d_in, d.nx}, nullptr);
-  run_yz<T, -1, 1>(ctx, f, spec, spec, OpId<T>{}, nullptr);
+  run_xy_fwd<T>(ctx, f, spec, LoadCast<double, T>{d_in, d.nx}, nullptr);
   run_z_fused<T>(ctx, f, spec, spec, op, nullptr);
-  run_yz<T, +1, 1>(ctx, f, spec, spec, OpId<T>{}, nullptr);
-  run_x_c2r<T>(ctx, f, spec, StoreMaskedF64<T>{d_out, d_mask, d.nx, (T)(1.0 / (double)d.n)}, nullptr);
+  run_xy_inv<T>(ctx, f, spec, StoreMaskedF64<T>{d_out, d_mask, d.nx, (T)(1.0 / (double)d.n)}, nullptr);
 }
 
 template <class OpF, class OpD>

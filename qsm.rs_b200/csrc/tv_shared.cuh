@@ -4,6 +4,7 @@
 #pragma once
 
 #include "functors.cuh"
+#include "plane.cuh"
 #include "solvers.h"
 
 #include <algorithm>
@@ -708,6 +709,9 @@ void tv_alloc(qsm_ctx* ctx, TvVol<T>& v, const std::string& pre, const GridDims&
     const long long resident = 2LL * sm_count(ctx);
     const long long zc = std::max<long long>(1, 2 * resident / ((long long)gbxs * gby));
     v.zchunk_s = (int)std::min<long long>(d.nz, std::max<long long>(4, (d.nz + zc - 1) / zc));
+    // ... or fewer planes, while that leaves SMs without a block
+    while (v.zchunk_s > 1 && (long long)gbxs * gby * ((d.nz + v.zchunk_s - 1) / v.zchunk_s) < sm_count(ctx))
+      v.zchunk_s = (v.zchunk_s + 1) / 2;
     v.sgrid_s = dim3(gbxs, gby, (d.nz + v.zchunk_s - 1) / v.zchunk_s);
     v.staged = true;
     nblk = std::max(nblk, (size_t)v.sgrid_s.x * v.sgrid_s.y * v.sgrid_s.z);
@@ -785,11 +789,9 @@ template <typename T> void tv_step_launch(qsm_ctx* ctx, const TvVol<T>& v, int q
 // those passes drop their L2 lines rather than leave them to be written back to HBM
 // while the stencil streams.
 template <typename T> void tv_fft(qsm_ctx* ctx, const TvVol<T>& v, int q, const int* done) {
-  run_x_r2c<T, true, true>(ctx, v.f, v.spec, LoadCast<T, T>{v.div, v.d.nx}, done);
-  run_yz<T, -1, 1>(ctx, v.f, v.spec, v.spec, OpId<T>{}, done);
+  run_xy_fwd<T, true, true>(ctx, v.f, v.spec, LoadCast<T, T>{v.div, v.d.nx}, done);
   run_z_fused_m<T>(ctx, v.f, v.spec, v.spec, v.mult, done);
-  run_yz<T, +1, 1>(ctx, v.f, v.spec, v.spec, OpId<T>{}, done);
-  run_x_c2r<T, true, true>(ctx, v.f, v.spec, StoreReal<T>{v.yb[q], v.d.nx, v.scale}, done);
+  run_xy_inv<T, true, true>(ctx, v.f, v.spec, StoreReal<T>{v.yb[q], v.d.nx, v.scale}, done);
 }
 extern template void tv_fft<float>(qsm_ctx*, const TvVol<float>&, int, const int*);
 extern template void tv_fft<double>(qsm_ctx*, const TvVol<double>&, int, const int*);
