@@ -611,14 +611,15 @@ def bench_multi_echo(local, dev, seed=5):
     names = ("chi", "xsa", "xfs", "xlsqr")
     il_err = {v: {k: _errs(a, b) for k, a, b in zip(names, il_out[v], il_out["fp64"])}
               for v in ("mixed", "mixed_float_krylov")}
-    # the LSQR loop's passes run on full complex FP64 spectra (16 B per value) in the default mixed
-    # context: Z inverse with the dipole scale reads x and writes t, the fused X pass reads t and
-    # the weights and writes t, the Z forward epilogue reads t and the previous vector and writes
-    sd = 16
-    il_model = {"fft_z_inv": 2 * N * sd, "fft_y_inv": 2 * N * sd, "fft_y_fwd": 2 * N * sd,
-                "fft_x_lsqr": 2 * N * sd + N * 8, "fft_z_lsqr": 3 * N * sd}
-    il_roof = _dominant_roofline(prof_il, il_model, "LSQR passes on full complex FP64 spectra: read + write one "
-                                                    "spectrum (2*N*16 B), + weights (fused X), + previous vector (Z out)")
+    # the LSQR loop's passes run on FP64 half spectra (8 B per voxel) in the default mixed context:
+    # Z inverse with its scale (4 B per voxel) reads x and writes t, the weighted X pass reads t and
+    # the weights and writes t, the Z forward epilogue reads t, the scale and the previous vector
+    # and writes
+    sd = 8
+    il_model = {"fft_z_inv": 2 * N * sd + N * 4, "fft_y_inv": 2 * N * sd, "fft_y_fwd": 2 * N * sd,
+                "fft_x_lsqr": 2 * N * sd + N * 8, "fft_z_lsqr": 3 * N * sd + N * 4}
+    il_roof = _dominant_roofline(prof_il, il_model, "LSQR passes on FP64 half spectra: read + write one spectrum "
+                                                    "(2*N*8 B), + scale (Z), + weights (X), + previous vector (Z out)")
     cm = qsmgpu.Context(local, "mixed")
     sm = torch.cuda.ExternalStream(cm.stream_handle(), device=dev)
     wrapped = torch.remainder(phases[2] + np.pi, 2 * np.pi) - np.pi
@@ -653,16 +654,16 @@ def bench_multi_echo(local, dev, seed=5):
     V = int(box(m0).numel())
     V0 = int(box(m0).sum())
     Vm = int(box(m_eroded).sum())
-    # bytes per box voxel: dual reads both masks and chi; inside mask0 phi, lphi, eta (r+w), q (r+w);
-    # inside the eroded mask p (r+w) and w.  Primal reads both masks, phi, chi, w and writes phi, chi,
-    # w twice (iterate and extrapolation); inside mask0 eta and p; inside the eroded mask q.
-    tgv_model = {"tgv_dual": 6 * V + 64 * V0 + 36 * Vm, "tgv_primal": 62 * V + 16 * V0 + 24 * Vm}
+    # bytes per box voxel: both kernels read the mask code.  Dual: inside mask0 phi, chi, lphi, eta
+    # (r+w), q (r+w); inside the eroded mask p (r+w) and w.  Primal: inside mask0 eta, q, phi, chi and
+    # writes phi, chi twice (iterate and extrapolation); inside the eroded mask p, w and w twice.
+    tgv_model = {"tgv_dual": V + 68 * V0 + 36 * Vm, "tgv_primal": V + 52 * V0 + 48 * Vm}
     tgv_roof = _dominant_roofline(prof_tgv, tgv_model, "compulsory bytes per box voxel by mask membership: "
-                                                       "dual 6 + 64 (mask0) + 36 (eroded mask), primal 62 + 16 + 24")
+                                                       "dual 1 + 68 (mask0) + 36 (eroded mask), primal 1 + 52 + 48")
     return {"workload": "384x384x256 at 0.6 mm, 3 T, 4 echoes TE 4/12/20/28 ms, 40 cylinders chi 0.3-0.6 ppm; "
                         "synthetic phantom",
             "linear_fit_fp64": {"ms": round(t_fit, 3), "fit_kernel_alg_gb": round(fit_bytes / 1e9, 3),
-                                "note": "ms covers the fit kernel and the reliability percentile (radix select)"},
+                                "note": "ms covers the fit kernel and the reliability percentile (exact rank selection)"},
             "ilsqr_ms": il_ms, "ilsqr_errors_vs_fp64_gpu": il_err, "ilsqr_roofline_mixed": il_roof,
             "tgv_1000_iterations_ms": round(t_tgv, 2),
             "tgv_box": {"voxels": V, "mask0": V0, "eroded_mask": Vm}, "tgv_roofline": tgv_roof,

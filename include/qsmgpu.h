@@ -133,7 +133,8 @@ QSM_API qsm_status qsm_ctx_autotune_entry(const qsm_ctx* ctx, size_t i, char* ke
  * negative value cancels.  The context stays usable after the failed call. */
 QSM_API qsm_status qsm_ctx_inject_alloc_failure(qsm_ctx* ctx, long long after);
 /* 1 when every axis length of `grid` has a transform plan: lengths up to 4096 whose prime
- * factors are at most 13, and any length up to 2048 (a Bluestein transform). */
+ * factors are at most 13, and any length up to 2048 (dense factors or a Bluestein
+ * transform). */
 QSM_API int qsm_grid_supported(const qsm_grid* grid);
 
 /* ---------------------------------------------------------------- params --- */
@@ -471,7 +472,7 @@ QSM_API qsm_status qsm_run_bg_removal(qsm_ctx* ctx, const double* field_ppm, siz
 /* prctile (src/inversion/ilsqr.rs:937-946) of the values d_vals[i] with d_mask[i] != 0
  * (all n values when d_mask is NULL), for each of the np percents in p; results in
  * out[0..np) on the host.  The reference sorts the selected values; this computes the
- * same order statistics by radix selection.  Returns 0 for an empty selection, as the
+ * same order statistics by selection.  Returns 0 for an empty selection, as the
  * reference's prctile does. */
 QSM_API qsm_status qsm_prctile_device(qsm_ctx* ctx, const double* d_vals, const uint8_t* d_mask, size_t n,
                                       const double* p, size_t np, double* out);

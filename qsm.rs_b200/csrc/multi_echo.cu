@@ -8,7 +8,7 @@
 // is written with explicitly rounded double intrinsics (no fused multiply-add) in the
 // reference's evaluation order, so every output is the reference's float64 result bit
 // for bit.  The reliability threshold is an exact order statistic of the selected
-// residuals (radix selection), which the reference takes from a full sort.
+// residuals (select.cu), which the reference takes from a full sort.
 #include "common.cuh"
 #include "select.h"
 #include "solvers.h"

@@ -5,7 +5,7 @@
 // sampled brackets: 2048 sampled keys are sorted by one block, the two sample keys some
 // standard deviations around the rank's place bracket its value, and one pass over the
 // data counts the keys below and at the bracket's ends and collects those strictly
-// between them (about 7 %).  The next level does the same to what was collected, until it
+// between them (about a tenth).  The next level does the same to what was collected, until it
 // fits one block's sort, which reads the rank off.  The counts decide exactly whether the
 // rank lies below, at or between the bracket's ends, so the result is the order statistic
 // itself whatever the sample was; a bracket that misses it (or collects more than its
