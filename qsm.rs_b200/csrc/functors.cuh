@@ -25,17 +25,6 @@ template <typename Ta, typename T> struct LoadProduct {
   }
 };
 
-// value where mask != 0, else 0
-template <typename Tin, typename T> struct LoadMasked {
-  const Tin* p;
-  const uint8_t* mask;
-  int nx;
-  __device__ __forceinline__ T operator()(int row, int e) const {
-    const long long i = (long long)row * nx + e;
-    return mask[i] != 0 ? (T)p[i] : T(0);
-  }
-};
-
 // A loader that only reads an array of the working precision, and its array.
 template <typename T> struct PlainLoad<T, LoadCast<T, T>> : std::true_type {};
 

@@ -343,11 +343,6 @@ template <typename T> Fft3<T> make_fft3_full(qsm_ctx* ctx, const GridDims& d) {
   return f;
 }
 
-// Identity pointwise hook of k_x_full.
-template <typename T> struct MidId {
-  __device__ __forceinline__ cplx_t<T> operator()(cplx_t<T> v, int, int) const { return v; }
-};
-
 // X pass over full complex rows: load -> FFT(D1) -> mid -> FFT(D2) -> store.
 // W: a hot loop's pass; with both transforms it takes the compile-time kernel
 // (k_x_full_fx) for the lengths of QSM_FIXED_PLANS (FP64 384: 96 registers against the
