@@ -8,6 +8,13 @@
 
 namespace qsm {
 
+// Kernels that a grid's passes may take.  kAll: the fastest form of each length.  kBase and
+// kBaseWide: the compile-time passes of QSM_FIXED_PLANS (and QSM_FIXED_PLANS_WIDE) and
+// otherwise the run-time engine, whatever faster forms are added.  The forms of a length
+// differ in their roundings, so a solver whose single-precision map must not move by them
+// (restrict_forms) keeps to these.
+enum class PassForms { kAll, kBase, kBaseWide };
+
 template <typename T> struct Fft3 {
   Geom g;
   FftPlan1D px, py, pz;
@@ -16,7 +23,13 @@ template <typename T> struct Fft3 {
   const cplx_t<T>* twz;
   TwoFactor<T> tfx{}, tfy{}, tfz{};  // two-factor passes of each axis (n = 0: none)
   T* xstage = nullptr;  // buffer of the runtime-engine X passes (null: the context's own)
+  PassForms forms = PassForms::kAll;
 };
+
+template <typename T> void restrict_forms(Fft3<T>& f, PassForms forms) {
+  f.forms = forms;
+  f.tfx = f.tfy = f.tfz = TwoFactor<T>{};
+}
 
 // The two-factor form of a length (two_factor.cu), n = 0 when it has none.
 template <typename T> TwoFactor<T> make_two_factor(qsm_ctx* ctx, int n);
@@ -217,6 +230,10 @@ bool x_plain_r2c(qsm_ctx* ctx, const Fft3<T>& f, const T* in, cplx_t<T>* spec, c
 template <typename T>
 bool x_plain_c2r(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* spec, T* out, T scale, const int* done);
 bool plan_listed(const FftPlan1D& pl);
+// Whether the axis takes the compile-time passes of some list.
+template <typename T> inline bool axis_listed(const qsm_ctx* ctx, const Fft3<T>& f, const FftPlan1D& pl) {
+  return compiled_plans(ctx) && f.forms == PassForms::kAll && plan_listed(pl);
+}
 // Loaders and stores that are just such arrays (functors.cuh).
 template <typename T, class Load> struct PlainLoad : std::false_type {};
 template <typename T, class Store> struct PlainStore : std::false_type {};
@@ -271,7 +288,7 @@ template <class K> unsigned x_rows_grid(qsm_ctx* ctx, K kernel, const Geom& g) {
 template <typename T, bool W = false, bool DEAD = false, class Load>
 void run_x_r2c(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* spec, const Load& ld, const int* done) {
   if (run_x_r2c_fixed<T, W, DEAD>(ctx, f, spec, ld, done)) return;
-  const bool listed = compiled_plans(ctx) && plan_listed(f.px);
+  const bool listed = axis_listed(ctx, f, f.px);
   if constexpr (PlainLoad<T, Load>::value) {
     if (listed) {
       x_plain_r2c<T>(ctx, f, ld.p, spec, done);
@@ -306,7 +323,7 @@ void run_x_r2c(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* spec, const Load& ld, 
 template <typename T, bool W = false, bool DEAD = false, class Store>
 void run_x_c2r(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* spec, const Store& st, const int* done) {
   if (run_x_c2r_fixed<T, W, DEAD>(ctx, f, spec, st, done)) return;
-  const bool listed = compiled_plans(ctx) && plan_listed(f.px);
+  const bool listed = axis_listed(ctx, f, f.px);
   if constexpr (PlainStore<T, Store>::value) {
     if (listed) {
       x_plain_c2r<T>(ctx, f, spec, st.out, st.scale, done);
@@ -437,6 +454,12 @@ template <typename T> inline size_t dx_smem(int n, int P) {
 
 template <typename T> inline size_t yz_smem(int n, int P) {
   return (size_t)(((n + 7) & ~7) + 2 * (size_t)n * P) * sizeof(cplx_t<T>);
+}
+
+// shared memory of the multiplier Z pass: n multiplier rows, m tile-buffer rows (m = n except
+// for Bluestein plans)
+template <typename T> inline size_t zm_smem(int n, int m, int P) {
+  return yz_smem<T>(m, P) + 2 * (((size_t)n * P + 3) & ~(size_t)3) * sizeof(T);
 }
 
 // Columns per tile of the compile-time Y/Z passes: 128-byte tile rows (16 float or 8
@@ -605,6 +628,10 @@ template <typename T, int DIR, int AXIS>
 void run_yz_plain(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const int* done);
 template <typename T, int DIR, int AXIS>
 void run_yz_rt(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const int* done);
+// The run-time engine's multiplier Z pass in one kernel; false when no tile of it fits an SM.
+template <typename T>
+bool run_z_fused_m_rt(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const T* mult,
+                      const int* done);
 // Z forward -> precomputed real multiplier array (spectrum layout) -> Z inverse.
 template <typename T>
 void run_z_fused_m(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const T* mult,
@@ -671,7 +698,7 @@ void run_yz(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst
     if constexpr (W) {
       if (run_yz_op_fixed<T, DIR, AXIS, false>(ctx, f, src, dst, op, nullptr, nullptr, done, yz_name(AXIS, DIR))) return;
     }
-    const bool listed = compiled_plans(ctx) && plan_listed(AXIS == 1 ? f.py : f.pz);
+    const bool listed = axis_listed(ctx, f, AXIS == 1 ? f.py : f.pz);
     if (!listed && run_yz_tf<T, DIR, AXIS, false>(ctx, f, src, dst, op, nullptr, nullptr, done, yz_name(AXIS, DIR))) return;
     run_yz_hooks<T, DIR, AXIS>(ctx, f, src, dst, op, done);
   }
@@ -685,7 +712,7 @@ void run_yz_acc(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>*
   if constexpr (W) {
     if (run_yz_op_fixed<T, DIR, AXIS, true>(ctx, f, src, dst, op, partials, counter, done, name)) return;
   }
-  const bool listed = compiled_plans(ctx) && plan_listed(AXIS == 1 ? f.py : f.pz);
+  const bool listed = axis_listed(ctx, f, AXIS == 1 ? f.py : f.pz);
   if (!listed && run_yz_tf<T, DIR, AXIS, true>(ctx, f, src, dst, op, partials, counter, done, name)) return;
   // dst may be the op's old vector: the transform goes through a buffer of its own
   cplx_t<T>* t = x_stage_c(ctx, f);
@@ -715,20 +742,26 @@ void spec_multiplier(qsm_ctx* ctx, const Fft3<T>& f, const Op& op, T* out, const
 template <typename T, class Op>
 void run_z_fused(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const Op& op,
                  const int* done, bool array = true) {
-  if (array && compiled_plans(ctx) && plan_listed(f.pz)) {
+  if (array && (f.forms != PassForms::kAll || axis_listed(ctx, f, f.pz))) {
     T* m = ws_scratch<T>(ctx, sizeof(T) == 4 ? "z.mult32" : "z.mult64", (size_t)f.g.hsize());
     spec_multiplier<T>(ctx, f, op, m, done);
-    run_z_fused_m<T>(ctx, f, src, dst, m, done);
-    return;
+    if (f.forms == PassForms::kAll) {
+      run_z_fused_m<T>(ctx, f, src, dst, m, done);
+      return;
+    }
+    if (run_z_fused_m_rt<T>(ctx, f, src, dst, m, done)) return;
   }
   if (run_z_fused_tf(ctx, f, src, dst, op, done)) return;
-  run_yz_plain<T, -1, 2>(ctx, f, src, dst, done);
+  const bool rt = f.forms != PassForms::kAll;
+  if (rt) run_yz_rt<T, -1, 2>(ctx, f, src, dst, done);
+  else run_yz_plain<T, -1, 2>(ctx, f, src, dst, done);
   {
     LaunchScope ls(ctx, "z_mid");
     k_spec_mid<T, Op><<<spec_grid(f.g), 128, 0, ctx->stream>>>(f.g, dst, op, done);
     ls.done();
   }
-  run_yz_plain<T, +1, 2>(ctx, f, dst, dst, done);
+  if (rt) run_yz_rt<T, +1, 2>(ctx, f, dst, dst, done);
+  else run_yz_plain<T, +1, 2>(ctx, f, dst, dst, done);
 }
 
 // ---------------------------------------------------------------------------

@@ -46,6 +46,7 @@ bool run_yz_fixed(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T
       return launch_yz_fx<T, DIR, AXIS, FP>(ctx, f, shape, src, dst, done, true);                 \
     }
     QSM_FIXED_PLANS(QSM_TRY_YZ)
+    if (f.forms == PassForms::kBase) return false;
     QSM_FIXED_PLANS_WIDE(QSM_TRY_YZ)
 #undef QSM_TRY_YZ
     return false;
@@ -55,18 +56,13 @@ bool run_yz_fixed(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T
 template <typename T, int DIR, int AXIS>
 void run_yz_plain(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const int* done) {
   if (run_yz_fixed<T, DIR, AXIS>(ctx, f, src, dst, done)) return;
-  if (compiled_plans(ctx) && plan_listed(AXIS == 1 ? f.py : f.pz)) {
+  if (axis_listed(ctx, f, AXIS == 1 ? f.py : f.pz)) {
     if (more_yz_0<T, DIR, AXIS>(ctx, f, src, dst, done) || more_yz_1<T, DIR, AXIS>(ctx, f, src, dst, done) ||
         more_yz_2<T, DIR, AXIS>(ctx, f, src, dst, done) || more_yz_3<T, DIR, AXIS>(ctx, f, src, dst, done))
       return;
   }
   if (run_yz_tf<T, DIR, AXIS, false>(ctx, f, src, dst, OpId<T>{}, nullptr, nullptr, done, yz_name(AXIS, DIR))) return;
   run_yz_rt<T, DIR, AXIS>(ctx, f, src, dst, done);
-}
-
-// n multiplier rows, m tile-buffer rows (m = n except for Bluestein plans)
-template <typename T> inline size_t zm_smem(int n, int m, int P) {
-  return yz_smem<T>(m, P) + 2 * (((size_t)n * P + 3) & ~(size_t)3) * sizeof(T);
 }
 
 // One compile-time multiplier Z pass (k_z_fused_m_fx, FP a FixedPlan) in launch shape
@@ -160,13 +156,16 @@ void run_z_fused_m(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<
       if (launch_zm_fx<T, FP>(ctx, f, shape, src, dst, mult, done, true)) return;                 \
     }
     QSM_FIXED_PLANS(QSM_TRY_ZM)
-    QSM_FIXED_PLANS_WIDE(QSM_TRY_ZM)
+    if (f.forms != PassForms::kBase) {
+      QSM_FIXED_PLANS_WIDE(QSM_TRY_ZM)
+    }
 #undef QSM_TRY_ZM
-    if (plan_listed(pl) &&
+    if (axis_listed(ctx, f, pl) &&
         (more_zm_0<T>(ctx, f, src, dst, mult, done) || more_zm_1<T>(ctx, f, src, dst, mult, done) ||
          more_zm_2<T>(ctx, f, src, dst, mult, done) || more_zm_3<T>(ctx, f, src, dst, mult, done)))
       return;
   }
+  if (!tf_usable(ctx, f.tfz, tf_cols<T>()) && run_z_fused_m_rt<T>(ctx, f, src, dst, mult, done)) return;
   run_z_fused<T>(ctx, f, src, dst, OpMultArray<T>{mult}, done, false);
 }
 

@@ -37,6 +37,37 @@ void run_yz_rt(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* 
   ls.done();
 }
 
+// Tile width of the multiplier Z pass, 0 when no width fits (long axes).
+template <typename T, class K> int zm_tile_width(K kernel, int n, int m, int Tn) {
+  for (int p = yz_cols<T>(); p >= 16 / (int)sizeof(T); p /= 2) {
+    if (p * Tn > 1024 || zm_smem<T>(n, m, p) > 227u * 1024u) continue;
+    ensure_smem(kernel, zm_smem<T>(n, m, p));
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, p * Tn, zm_smem<T>(n, m, p)) != cudaSuccess) {
+      (void)cudaGetLastError();
+      continue;
+    }
+    if (per_sm >= 1) return p;
+  }
+  return 0;
+}
+
+template <typename T>
+bool run_z_fused_m_rt(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const T* mult,
+                      const int* done) {
+  const FftPlan1D& pl = f.pz;
+  auto kern = pl.m != pl.n ? k_z_fused_m<T, true> : k_z_fused_m<T, false>;
+  const int P = zm_tile_width<T>(kern, pl.n, pl.m, pl.T);
+  if (P == 0) return false;
+  const size_t smem = zm_smem<T>(pl.n, pl.m, P);
+  const TileWalk w = tile_walk(f, 2, P);
+  const unsigned grid = persistent_grid(ctx, kern, P * pl.T, smem, w.ntiles);
+  LaunchScope ls(ctx, "fft_z_fused");
+  kern<<<grid, dim3(P, pl.T), smem, ctx->stream>>>(f.g, pl, w, f.twz, src, dst, mult, done);
+  ls.done();
+  return true;
+}
+
 template <typename T>
 void run_x_r2c_rt(qsm_ctx* ctx, const Fft3<T>& f, const T* in, cplx_t<T>* spec, const int* done) {
   const int Tt = x_block_t(f.px.T);
@@ -94,6 +125,7 @@ bool plan_listed(const FftPlan1D& pl) {
   template void run_yz_rt<T, +1, 1>(qsm_ctx*, const Fft3<T>&, const cplx_t<T>*, cplx_t<T>*, const int*);       \
   template void run_yz_rt<T, -1, 2>(qsm_ctx*, const Fft3<T>&, const cplx_t<T>*, cplx_t<T>*, const int*);       \
   template void run_yz_rt<T, +1, 2>(qsm_ctx*, const Fft3<T>&, const cplx_t<T>*, cplx_t<T>*, const int*);       \
+  template bool run_z_fused_m_rt<T>(qsm_ctx*, const Fft3<T>&, const cplx_t<T>*, cplx_t<T>*, const T*, const int*); \
   template void run_x_r2c_rt<T>(qsm_ctx*, const Fft3<T>&, const T*, cplx_t<T>*, const int*);                   \
   template void run_x_c2r_rt<T>(qsm_ctx*, const Fft3<T>&, const cplx_t<T>*, T*, T, const int*);                \
   template void run_x_c2c_rt<T, -1>(qsm_ctx*, const Fft3<T>&, cplx_t<T>*, const int*);                         \

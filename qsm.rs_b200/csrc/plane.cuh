@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(kPlaneThreads)
 // 9.73 ms, 96x96x90 13.05 and 12.93, 128x128x80 16.6 and 17.3, 128x128x128 21.7 and 20.3,
 // 128x96x160 21.0 and 22.8).
 template <typename T> inline bool plane_usable(qsm_ctx* ctx, const Fft3<T>& f) {
-  if (!compiled_plans(ctx)) return false;
+  if (!compiled_plans(ctx) || f.forms != PassForms::kAll) return false;
   if (f.g.nx == 64 || f.g.ny == 64) return true;
   return 5LL * f.g.nz >= 3LL * sm_count(ctx) && f.g.nz <= sm_count(ctx);
 }

@@ -80,6 +80,23 @@ __global__ void __launch_bounds__(128)
   A[((size_t)z * ny + ky) * nxh + kx] = (z == 0 || 2 * z == nz ? 1.0 : 2.0) * s;
 }
 
+// The normalised sphere's image (src/kernels/smv.rs:19-67) as an X-pass input; the inclusion
+// test without fused multiply-adds, as the reference's.
+struct LoadSphere {
+  int nx, ny, nz;
+  double vsx, vsy, vsz, r2, norm;
+  static __device__ __forceinline__ double coord(int i, int n, double vs) { return (double)(i <= n / 2 ? i : i - n) * vs; }
+  __device__ __forceinline__ double operator()(int row, int e) const {
+    const int k = row / ny, j = row - k * ny;
+    const double dx = coord(e, nx, vsx), dy = coord(j, ny, vsy), dz = coord(k, nz, vsz);
+    return __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)) <= r2 ? norm : 0.0;
+  }
+};
+__global__ void k_one_minus_re(long long H, const double2* __restrict__ S, float* __restrict__ out) {
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < H; i += (long long)gridDim.x * blockDim.x)
+    out[i] = (float)(1.0 - S[i].x);
+}
+
 constexpr int kSmvZ = 16;   // kz per thread
 constexpr int kSmvZc = 32;  // planes of dz per shared-memory cosine table
 
@@ -540,6 +557,20 @@ void smv_multiplier(qsm_ctx* ctx, const Fft3<T>& f, const SmvSphere& s, SmvMult 
 }
 template void smv_multiplier<float>(qsm_ctx*, const Fft3<float>&, const SmvSphere&, SmvMult, double, float*);
 template void smv_multiplier<double>(qsm_ctx*, const Fft3<double>&, const SmvSphere&, SmvMult, double, double*);
+
+void smv_one_minus_transform(qsm_ctx* ctx, const GridDims& d, const SmvSphere& s, float* out) {
+  Fft3<double> f = make_fft3<double>(ctx, d);
+  restrict_forms(f, PassForms::kBase);
+  const long long H = f.g.hsize();
+  double2* S = ws<double2>(ctx, "smv.S", (size_t)H);
+  run_x_r2c<double>(ctx, f, S, LoadSphere{d.nx, d.ny, d.nz, d.vsx, d.vsy, d.vsz, s.r2, s.total > 0.0 ? 1.0 / s.total : 0.0},
+                    nullptr);
+  run_yz<double, -1, 1>(ctx, f, S, S, OpId<double>{}, nullptr);
+  run_yz<double, -1, 2>(ctx, f, S, S, OpId<double>{}, nullptr);
+  LaunchScope ls(ctx, "smv_spectrum");
+  k_one_minus_re<<<grid1d(H), 256, 0, ctx->stream>>>(H, S, out);
+  ls.done();
+}
 
 void smv_erode_first(qsm_ctx* ctx, const GridDims& d, const uint8_t* mask, const std::vector<SmvSphere>& spheres,
                      double delta, uint8_t* first) {

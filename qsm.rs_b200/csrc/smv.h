@@ -28,6 +28,11 @@ enum SmvMult {
 template <typename T>
 void smv_multiplier(qsm_ctx* ctx, const Fft3<T>& f, const SmvSphere& s, SmvMult kind, double threshold, T* out);
 
+// 1 - S in single precision from the transform of the sphere's image.  Its last bits differ
+// from the cosine sums', which flips a rounding to single precision somewhere in most large
+// spectra: for callers whose map must keep its roundings (restrict_forms).
+void smv_one_minus_transform(qsm_ctx* ctx, const GridDims& d, const SmvSphere& s, float* out);
+
 // Erosion by several spheres (mean of the mask over the sphere > delta), largest first:
 // first[i] = index of the first sphere that keeps voxel i, 255 when none does.  At most
 // 254 spheres.

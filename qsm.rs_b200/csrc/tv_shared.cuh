@@ -678,10 +678,11 @@ extern template void tv_tune<double>(qsm_ctx*, const TvVol<double>&);
 // tuning of a grid the context has not seen (tv_tune), which overwrites the new buffers.
 template <typename T>
 void tv_alloc(qsm_ctx* ctx, TvVol<T>& v, const std::string& pre, const GridDims& d, double thr, TvState* st,
-              const uint8_t* d_mask, double* d_out) {
+              const uint8_t* d_mask, double* d_out, PassForms forms = PassForms::kAll) {
   using C = cplx_t<T>;
   v.d = d;
   v.f = make_fft3<T>(ctx, d);
+  if (forms != PassForms::kAll) restrict_forms(v.f, forms);
   const long long N = d.n;
   const long long H = v.f.g.hsize();
   auto nm = [&](const char* s) { return pre + s; };
