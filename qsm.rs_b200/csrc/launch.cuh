@@ -31,10 +31,11 @@ template <typename T> void restrict_forms(Fft3<T>& f, PassForms forms) {
   f.tfx = f.tfy = f.tfz = TwoFactor<T>{};
 }
 
-// The two-factor form of a length (two_factor.cu), n = 0 when it has none.
-template <typename T> TwoFactor<T> make_two_factor(qsm_ctx* ctx, int n);
+// The two-factor form of a length on axis 0, 1 or 2 (two_factor.cu), n = 0 when it does not
+// take one.
+template <typename T> TwoFactor<T> make_two_factor(qsm_ctx* ctx, int n, int axis);
 // Its radices and blocks, and its host table (tw).
-template <typename T> TwoFactor<T> plan_two_factor(int n);
+template <typename T> TwoFactor<T> plan_two_factor(int n, int axis);
 template <typename T> std::vector<cplx_t<T>> two_factor_table(const TwoFactor<T>& ax);
 
 // Point each Bluestein plan at the chirp and kernel spectrum that follow the stage
@@ -62,9 +63,9 @@ template <typename T> Fft3<T> make_fft3(qsm_ctx* ctx, const GridDims& d) {
   f.twy = (const cplx_t<T>*)twiddle_table(ctx, f.py, dbl);
   f.twz = (const cplx_t<T>*)twiddle_table(ctx, f.pz, dbl);
   attach_tables(f);
-  f.tfx = make_two_factor<T>(ctx, d.nx);
-  f.tfy = make_two_factor<T>(ctx, d.ny);
-  f.tfz = make_two_factor<T>(ctx, d.nz);
+  f.tfx = make_two_factor<T>(ctx, d.nx, 0);
+  f.tfy = make_two_factor<T>(ctx, d.ny, 1);
+  f.tfz = make_two_factor<T>(ctx, d.nz, 2);
   return f;
 }
 
@@ -736,13 +737,13 @@ void spec_multiplier(qsm_ctx* ctx, const Fft3<T>& f, const Op& op, T* out, const
   ls.done();
 }
 
-// Z forward -> op.mid -> Z inverse, op.mid a real multiplier (v -> m v).  Listed lengths
-// evaluate it once into an array for the compile-time multiplier pass (`array` false where
-// no buffer may be allocated); else the two-factor kernel evaluates it in the pass.
+// Z forward -> op.mid -> Z inverse, op.mid a real multiplier (v -> m v).  The two-factor kernel
+// evaluates it in the pass; other lengths evaluate it once into an array for the multiplier
+// pass (`array` false where no buffer may be allocated).
 template <typename T, class Op>
 void run_z_fused(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const Op& op,
                  const int* done, bool array = true) {
-  if (array && (f.forms != PassForms::kAll || axis_listed(ctx, f, f.pz))) {
+  if (array && (axis_listed(ctx, f, f.pz) || !tf_usable(ctx, f.tfz, tf_cols<T>()))) {
     T* m = ws_scratch<T>(ctx, sizeof(T) == 4 ? "z.mult32" : "z.mult64", (size_t)f.g.hsize());
     spec_multiplier<T>(ctx, f, op, m, done);
     if (f.forms == PassForms::kAll) {

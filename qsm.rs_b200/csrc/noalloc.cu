@@ -141,7 +141,7 @@ extern "C" qsm_status qsm_tkd_device_noalloc(const double* d_local_field, const 
     // through the output buffer
     TwoFactor<double>* axes[3] = {&f.tfx, &f.tfy, &f.tfz};
     for (int a = 0; a < 3; ++a) {
-      TwoFactor<double> ax = plan_two_factor<double>(ns[a]);
+      TwoFactor<double> ax = plan_two_factor<double>(ns[a], a);
       if (ax.n == 0) continue;
       const std::vector<double2> h = two_factor_table(ax);
       const size_t bytes = round256(h.size() * sizeof(double2));
