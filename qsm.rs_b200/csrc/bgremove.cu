@@ -86,15 +86,6 @@ template <typename T> struct OpPoisson {
   }
 };
 
-// Multiplier array applied as a pass's elements are fetched.
-template <typename T> struct OpPreMult {
-  using C = cplx_t<T>;
-  const T* m;
-  static constexpr bool kNoPost = true;
-  __device__ __forceinline__ C pre(C v, int, int, int, long long idx) const { return cscale(v, __ldg(m + idx)); }
-  __device__ __forceinline__ C post(C v, int, int, int, long long) const { return v; }
-};
-
 // V-SHARP first-hit selection (src/bgremove/vsharp.rs:168-176): the voxels that this
 // radius is the first to keep
 template <typename T> struct StoreSelect {

@@ -108,4 +108,14 @@ __device__ __forceinline__ void block_sum2(double& a, double& b) {
   }
 }
 
+// ------------------------------------------------------------ k-space hooks --
+// Multiplier array applied as a pass's elements are fetched.
+template <typename T> struct OpPreMult {
+  using C = cplx_t<T>;
+  const T* m;
+  static constexpr bool kNoPost = true;
+  __device__ __forceinline__ C pre(C v, int, int, int, long long idx) const { return cscale(v, __ldg(m + idx)); }
+  __device__ __forceinline__ C post(C v, int, int, int, long long) const { return v; }
+};
+
 }  // namespace qsm

@@ -17,9 +17,14 @@
 // mask the decision is a count.  One exact distance transform to the nearest zero voxel
 // serves every sphere: a voxel further from all zeros than the radius (compared with the
 // sphere's own rounding, (dx^2 + dy^2) + dz^2) misses nothing.  Only where a sphere
-// tolerates missing voxels are the others counted, by row prefix sums, stopping at the
-// first count above the tolerance.  A mask with values above 1 is decided by its weighted
-// sum over the same rows.
+// tolerates missing voxels are the others counted: up to two on bit planes, 32 voxels a
+// thread; more (spheres from about 9500 voxels, 13 voxels of radius) and masks with values
+// above 1 by the sphere's sums of the mask through FP64 transforms, rounded to the whole
+// numbers that they are, whose cost depends neither on the radius nor on the values.  (Counting
+// voxel by voxel along the sphere's rows, V-SHARP of radii 12..1 mm took 33.9 ms at
+// 384x384x256 and 0.6 mm in double and 12.5 ms at 192x192x128 and 0.4 mm, now 14.2 and 2.9;
+// on a mask of threes 44.8 ms at 256x256x176 and 1 mm, now 5.2.)
+#include "functors.cuh"
 #include "smv.h"
 
 #include <algorithm>
@@ -146,10 +151,10 @@ struct ErodeState {
 };
 
 // One warp per row: distance in x to the row's nearest zero voxel (periodic, up to rx;
-// kNoZero beyond) and the row's prefix sums.
+// kNoZero beyond).
 __global__ void __launch_bounds__(256)
     k_smv_rows(int nx, int nrows, int rx, const uint8_t* __restrict__ mask, uint16_t* __restrict__ gx,
-               int* __restrict__ prefix, ErodeState* st) {
+               ErodeState* st) {
   extern __shared__ unsigned bits_all[];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int ext = nx + 2 * rx, words = (ext + 31) >> 5;
@@ -165,20 +170,10 @@ __global__ void __launch_bounds__(256)
       if (lane == 0) bits[w] = b;
     }
     __syncwarp();
-    int carry = 0;
-    if (lane == 0) prefix[(long long)row * (nx + 1)] = 0;
     for (int x0 = 0; x0 < nx; x0 += 32) {
       const int x = x0 + lane;
-      const int v = x < nx ? (int)m[x] : 0;
-      weighted |= v > 1;
-      int s = v;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, s, o);
-        if (lane >= o) s += t;
-      }
       if (x < nx) {
-        prefix[(long long)row * (nx + 1) + x + 1] = carry + s;
+        weighted |= m[x] > 1;
         const int j = x + rx, w0 = j >> 5, b0 = j & 31;
         int best = rx + 1;
         unsigned u = bits[w0] >> b0;  // zeros at or right of x
@@ -201,7 +196,6 @@ __global__ void __launch_bounds__(256)
         }
         gx[(long long)row * nx + x] = best <= rx ? (uint16_t)best : (uint16_t)kNoZero;
       }
-      carry += __shfl_sync(0xffffffffu, s, 31);
     }
     __syncwarp();
   }
@@ -266,7 +260,7 @@ __global__ void __launch_bounds__(256)
 // min over |dz| <= rz of d2 + dz^2, then the first sphere whose radius it exceeds
 __global__ void __launch_bounds__(256)
     k_smv_edt_z(int nx, int ny, int nz, int rz, double vsz, const double* __restrict__ d2, int ns,
-                const double* __restrict__ r2, const ErodeState* __restrict__ st, uint8_t* __restrict__ first) {
+                const double* __restrict__ r2, uint8_t* __restrict__ first) {
   extern __shared__ __align__(16) double tab[];
   double* sz = tab;           // dz^2
   double* sr = tab + rz + 1;  // r^2
@@ -279,7 +273,6 @@ __global__ void __launch_bounds__(256)
   const long long p = (long long)blockIdx.x * 256 + threadIdx.x, sxy = (long long)nx * ny;
   const int z0 = blockIdx.y * kEdtU;
   if (p >= sxy) return;
-  const bool weighted = st->weighted != 0;
   const double inf = __longlong_as_double(0x7ff0000000000000ll);
   double m[kEdtU];
   double any = 0.0;
@@ -310,13 +303,11 @@ __global__ void __launch_bounds__(256)
   for (int u = 0; u < kEdtU; ++u) {
     if (z0 + u >= nz) break;
     int f = 255;
-    if (!weighted) {
-      for (int s = 0; s < ns; ++s)
-        if (m[u] > sr[s]) {
-          f = s;
-          break;
-        }
-    }
+    for (int s = 0; s < ns; ++s)
+      if (m[u] > sr[s]) {
+        f = s;
+        break;
+      }
     first[(z0 + u) * sxy + p] = (uint8_t)f;
   }
 }
@@ -408,14 +399,13 @@ __device__ __forceinline__ void smv_row_sum(const ErodeSphere& E, int y, int z, 
 }
 
 // Tolerances of one or two missing voxels, 32 voxels per thread: saturating counts of the
-// sphere's zeros in three bit planes, summed over its rows.  (The per-voxel count below took
-// 2.2 ms at 256x256x176 for V-SHARP's three tolerant radii: every warp along a boundary
-// walked all 450 rows.)
+// sphere's zeros in three bit planes, summed over its rows.  (A count per voxel took 2.2 ms
+// at 256x256x176 for V-SHARP's three tolerant radii: every warp along a boundary walked all
+// 450 rows.)
 __global__ void __launch_bounds__(128)
     k_smv_count_bits(int nx, int ny, int nz, int wpr, int ns, const ErodeSphere* __restrict__ spheres,
                      const int4* __restrict__ rows, const unsigned* __restrict__ planes,
-                     const ErodeState* __restrict__ st, uint8_t* __restrict__ first) {
-  if (st->weighted != 0) return;
+                     uint8_t* __restrict__ first) {
   const long long nrows = (long long)ny * nz, plane = nrows * wpr;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= plane) return;
@@ -441,57 +431,18 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-// Voxels that a sphere tolerating more than two missing voxels may still keep (0/1 masks),
-// or every voxel of a weighted mask: sums of the sphere's rows by their prefix sums.
-__global__ void __launch_bounds__(256)
-    k_smv_count(int nx, int ny, int nz, int ns, int tolerant, const ErodeSphere* __restrict__ spheres,
-                const int4* __restrict__ rows, const int* __restrict__ prefix, const ErodeState* __restrict__ st,
-                uint8_t* __restrict__ first) {
-  const bool weighted = st->weighted != 0;
-  if (!weighted && !tolerant) return;
-  const int x = blockIdx.x * 32 + (threadIdx.x & 31);
-  const int y = blockIdx.y * 8 + (threadIdx.x >> 5), z = blockIdx.z;
-  if (x >= nx || y >= ny) return;
-  const long long i = ((long long)z * ny + y) * nx + x;
-  const int have = first[i];
-  const int lim = have < ns ? have : ns;
-  for (int s = 0; s < lim; ++s) {
-    const ErodeSphere E = spheres[s];
-    if (!weighted && E.total - E.need <= 2) continue;
-    long long sum = 0;
-    long long seen = 0;
-    bool keep = false;
-    for (int r = 0; r < E.count; ++r) {
-      const int4 q = __ldg(rows + E.begin + r);
-      int yy = y + q.x, zz = z + q.y;
-      yy = yy < 0 ? yy + ny : (yy >= ny ? yy - ny : yy);
-      zz = zz < 0 ? zz + nz : (zz >= nz ? zz - nz : zz);
-      const int* P = prefix + ((long long)zz * ny + yy) * (nx + 1);
-      int v;
-      if (q.w >= nx) {
-        v = P[nx];
-      } else {
-        const int a = x - q.z, b = a + q.w;  // run [a, b)
-        if (a < 0) v = P[nx] - P[a + nx] + P[b];
-        else if (b > nx) v = P[nx] - P[a] + P[b - nx];
-        else v = P[b] - P[a];
-      }
-      sum += v;
-      seen += q.w;
-      if (!weighted) {
-        if (seen - sum > E.total - E.need) break;  // too many missing
-        keep = r + 1 == E.count;
-      } else if (sum >= E.need) {
-        keep = true;
-        break;
-      }
-    }
-    if (keep) {
-      first[i] = (uint8_t)s;
-      return;
-    }
+// The voxels that a sphere keeps by its sum of the mask (v / N times the sphere's voxels, a
+// whole number), where no earlier sphere does.
+struct StoreErode {
+  uint8_t* first;
+  int nx, index;
+  double scale, need;
+  __device__ __forceinline__ void operator()(int row, int e, double v) {
+    const long long i = (long long)row * nx + e;
+    if (rint(v * scale) >= need && (int)first[i] > index) first[i] = (uint8_t)index;
   }
-}
+  __device__ __forceinline__ void finish() {}
+};
 
 }  // namespace
 
@@ -572,16 +523,38 @@ void smv_one_minus_transform(qsm_ctx* ctx, const GridDims& d, const SmvSphere& s
   ls.done();
 }
 
+// Spheres of `es` in `list` on top of what `first` holds, by transforms.
+static void erode_by_transform(qsm_ctx* ctx, const GridDims& d, const uint8_t* mask,
+                               const std::vector<SmvSphere>& spheres, const std::vector<ErodeSphere>& es,
+                               const std::vector<int>& list, uint8_t* first) {
+  Fft3<double> f = make_fft3<double>(ctx, d);
+  const size_t H = (size_t)f.g.hsize();
+  double2* F = ws<double2>(ctx, "smv.F", H);
+  double2* t = ws<double2>(ctx, "smv.S", H);
+  double* m = ws<double>(ctx, "smv.m64", H);
+  run_x_r2c<double>(ctx, f, F, LoadCast<uint8_t, double>{mask, d.nx}, nullptr);
+  run_yz<double, -1, 1>(ctx, f, F, F, OpId<double>{}, nullptr);
+  run_yz<double, -1, 2>(ctx, f, F, F, OpId<double>{}, nullptr);
+  for (int s : list) {
+    const ErodeSphere& e = es[(size_t)s];
+    smv_multiplier<double>(ctx, f, spheres[(size_t)s], kSmvS, 0.0, m);
+    run_yz<double, +1, 2, true>(ctx, f, F, t, OpPreMult<double>{m}, nullptr);
+    run_yz<double, +1, 1>(ctx, f, t, t, OpId<double>{}, nullptr);
+    run_x_c2r<double>(ctx, f, t, StoreErode{first, d.nx, s, (double)e.total / (double)d.n, (double)e.need}, nullptr);
+  }
+}
+
 void smv_erode_first(qsm_ctx* ctx, const GridDims& d, const uint8_t* mask, const std::vector<SmvSphere>& spheres,
                      double delta, uint8_t* first) {
   const int ns = (int)spheres.size();
   if (ns < 1 || ns > 254) throw QsmError(QSM_ERR_INVALID_ARGUMENT, "smv_erode_first: 1 to 254 spheres");
   const long long N = d.n;
   const int nrows = d.ny * d.nz;
-  int rx = 0, ry = 0, rz = 0, tolerant = 0, lbits = -1;
+  int rx = 0, ry = 0, rz = 0, lbits = -1;
   std::vector<double> r2;
   std::vector<ErodeSphere> es;
-  std::vector<int4> rows;
+  std::vector<int4> rows;        // of the spheres that bit planes count
+  std::vector<int> all, tolerant;  // spheres; those tolerating more than two missing voxels
   for (const SmvSphere& s : spheres) {
     rx = std::max(rx, s.half[0]);
     ry = std::max(ry, s.dy);
@@ -594,47 +567,55 @@ void smv_erode_first(qsm_ctx* ctx, const GridDims& d, const uint8_t* mask, const
     while (need > 0 && (double)(need - 1) / s.total > delta) --need;
     while (!((double)need / s.total > delta)) ++need;
     e.need = need;
-    if (e.total - e.need > 2) tolerant = 1;
-    else if (e.need < e.total) lbits = std::max(lbits, s.half[0]);
     e.begin = (int)rows.size();
-    for (int z = 0; z <= s.dz; ++z)
-      for (int y = 0; y <= s.dy; ++y) {
-        const int L = s.half[(size_t)z * (s.dy + 1) + y];
-        if (L < 0) break;  // the same for larger |y|
-        const int len = std::min(2 * L + 1, d.nx);
-        for (int sy = 0; sy < ((y == 0 || 2 * y == d.ny) ? 1 : 2); ++sy)
-          for (int sz = 0; sz < ((z == 0 || 2 * z == d.nz) ? 1 : 2); ++sz)
-            rows.push_back(make_int4(sy ? -y : y, sz ? -z : z, L, len));
+    e.count = 0;
+    const long long tol = e.total - e.need;
+    all.push_back((int)es.size());
+    if (tol > 2) tolerant.push_back((int)es.size());
+    if (tol == 1 || tol == 2) {
+      lbits = std::max(lbits, s.half[0]);
+      for (int z = 0; z <= s.dz; ++z)
+        for (int y = 0; y <= s.dy; ++y) {
+          const int L = s.half[(size_t)z * (s.dy + 1) + y];
+          if (L < 0) break;  // the same for larger |y|
+          for (int sy = 0; sy < ((y == 0 || 2 * y == d.ny) ? 1 : 2); ++sy)
+            for (int sz = 0; sz < ((z == 0 || 2 * z == d.nz) ? 1 : 2); ++sz)
+              rows.push_back(make_int4(sy ? -y : y, sz ? -z : z, L, 0));
+        }
+      e.count = (int)rows.size() - e.begin;
+      // a fixed shuffle, so that the rows cut by a nearby boundary come up early: xorshift64
+      // with its author's example seed (G. Marsaglia, Xorshift RNGs, 2003)
+      unsigned long long rnd = 88172645463325252ull;
+      for (int i = e.count - 1; i > 0; --i) {
+        rnd ^= rnd << 13;
+        rnd ^= rnd >> 7;
+        rnd ^= rnd << 17;
+        std::swap(rows[(size_t)(e.begin + i)], rows[(size_t)(e.begin + (int)(rnd % (unsigned long long)(i + 1)))]);
       }
-    e.count = (int)rows.size() - e.begin;
-    // a fixed shuffle: the rows cut by a nearby boundary come up early
-    unsigned long long rnd = 88172645463325252ull;
-    for (int i = e.count - 1; i > 0; --i) {
-      rnd ^= rnd << 13;
-      rnd ^= rnd >> 7;
-      rnd ^= rnd << 17;
-      std::swap(rows[(size_t)(e.begin + i)], rows[(size_t)(e.begin + (int)(rnd % (unsigned long long)(i + 1)))]);
     }
     es.push_back(e);
   }
   uint16_t* gx = ws<uint16_t>(ctx, "smv.gx", (size_t)N);
-  double* d2 = ws<double>(ctx, "smv.d2", (size_t)N);
-  int* prefix = ws<int>(ctx, "smv.prefix", (size_t)nrows * (d.nx + 1));
-  double* dr2 = ws<double>(ctx, "smv.r2", 254);
-  ErodeSphere* des = ws<ErodeSphere>(ctx, "smv.spheres", 254);
-  int4* drows = ws<int4>(ctx, "smv.rows", rows.size());
   ErodeState* st = ws<ErodeState>(ctx, "smv.state", 1);
-  h2d(ctx, dr2, r2.data(), r2.size() * sizeof(double));
-  h2d(ctx, des, es.data(), es.size() * sizeof(ErodeSphere));
-  h2d(ctx, drows, rows.data(), rows.size() * sizeof(int4));
   QSM_CUDA(cudaMemsetAsync(st, 0, sizeof(ErodeState), ctx->stream));
   {
     const size_t smem = (size_t)8 * ((d.nx + 2 * rx + 31) / 32) * sizeof(unsigned);
     const int blocks = std::min((nrows + 7) / 8, 8 * sm_count(ctx));
     LaunchScope ls(ctx, "smv_rows");
-    k_smv_rows<<<blocks, 256, smem, ctx->stream>>>(d.nx, nrows, rx, mask, gx, prefix, st);
+    k_smv_rows<<<blocks, 256, smem, ctx->stream>>>(d.nx, nrows, rx, mask, gx, st);
     ls.done();
   }
+  ErodeState h{};
+  d2h(ctx, &h, st, sizeof(h));
+  sync(ctx);
+  if (h.weighted) {
+    QSM_CUDA(cudaMemsetAsync(first, 255, (size_t)N, ctx->stream));
+    erode_by_transform(ctx, d, mask, spheres, es, all, first);
+    return;
+  }
+  double* d2 = ws<double>(ctx, "smv.d2", (size_t)N);
+  double* dr2 = ws<double>(ctx, "smv.r2", 254);
+  h2d(ctx, dr2, r2.data(), r2.size() * sizeof(double));
   {
     const size_t smem = (size_t)(rx + ry + 2) * sizeof(double);
     LaunchScope ls(ctx, "smv_edt_y");
@@ -646,14 +627,18 @@ void smv_erode_first(qsm_ctx* ctx, const GridDims& d, const uint8_t* mask, const
     const size_t smem = (size_t)(rz + 1 + ns) * sizeof(double);
     LaunchScope ls(ctx, "smv_edt_z");
     k_smv_edt_z<<<dim3((unsigned)(((long long)d.nx * d.ny + 255) / 256), (d.nz + kEdtU - 1) / kEdtU), 256, smem,
-                  ctx->stream>>>(d.nx, d.ny, d.nz, rz, d.vsz, d2, ns, dr2, st, first);
+                  ctx->stream>>>(d.nx, d.ny, d.nz, rz, d.vsz, d2, ns, dr2, first);
     ls.done();
   }
   if (lbits >= 0) {
     const int wpr = (d.nx + 31) / 32, pad = (lbits + 31) / 32, words = wpr + 2 * pad + 1;
     const long long total = (long long)nrows * wpr;
-    unsigned* bits = ws<unsigned>(ctx, "smv.bits", (size_t)nrows * words);
-    unsigned* planes = ws<unsigned>(ctx, "smv.planes", (size_t)3 * (lbits + 1) * total);
+    unsigned* bits = ws_scratch<unsigned>(ctx, "smv.bits", (size_t)nrows * words);
+    unsigned* planes = ws_scratch<unsigned>(ctx, "smv.planes", (size_t)3 * (lbits + 1) * total);
+    ErodeSphere* des = ws<ErodeSphere>(ctx, "smv.spheres", 254);
+    int4* drows = ws_scratch<int4>(ctx, "smv.rows", rows.size());
+    h2d(ctx, des, es.data(), es.size() * sizeof(ErodeSphere));
+    h2d(ctx, drows, rows.data(), rows.size() * sizeof(int4));
     {
       LaunchScope ls(ctx, "smv_planes");
       k_smv_bits<<<16 * sm_count(ctx), 256, 0, ctx->stream>>>(d.nx, nrows, words, pad, mask, bits);
@@ -663,13 +648,10 @@ void smv_erode_first(qsm_ctx* ctx, const GridDims& d, const uint8_t* mask, const
     }
     LaunchScope ls(ctx, "smv_count_bits");
     k_smv_count_bits<<<(unsigned)((total + 127) / 128), 128, 0, ctx->stream>>>(d.nx, d.ny, d.nz, wpr, ns, des, drows,
-                                                                               planes, st, first);
+                                                                               planes, first);
     ls.done();
   }
-  LaunchScope ls(ctx, "smv_count");
-  k_smv_count<<<dim3((d.nx + 31) / 32, (d.ny + 7) / 8, d.nz), 256, 0, ctx->stream>>>(d.nx, d.ny, d.nz, ns, tolerant,
-                                                                                    des, drows, prefix, st, first);
-  ls.done();
+  if (!tolerant.empty()) erode_by_transform(ctx, d, mask, spheres, es, tolerant, first);
 }
 
 }  // namespace qsm
