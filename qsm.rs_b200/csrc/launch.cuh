@@ -629,7 +629,9 @@ template <typename T, int DIR, int AXIS>
 void run_yz_plain(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const int* done);
 template <typename T, int DIR, int AXIS>
 void run_yz_rt(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const int* done);
-// The run-time engine's multiplier Z pass in one kernel; false when no tile of it fits an SM.
+// The run-time engine's multiplier Z pass in one kernel; false when no tile of it fits an SM,
+// which z_mult_fits says beforehand.
+template <typename T> bool z_mult_fits(const FftPlan1D& pl);
 template <typename T>
 bool run_z_fused_m_rt(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const T* mult,
                       const int* done);

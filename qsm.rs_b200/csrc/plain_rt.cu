@@ -52,6 +52,11 @@ template <typename T, class K> int zm_tile_width(K kernel, int n, int m, int Tn)
   return 0;
 }
 
+template <typename T> bool z_mult_fits(const FftPlan1D& pl) {
+  auto kern = pl.m != pl.n ? k_z_fused_m<T, true> : k_z_fused_m<T, false>;
+  return zm_tile_width<T>(kern, pl.n, pl.m, pl.T) > 0;
+}
+
 template <typename T>
 bool run_z_fused_m_rt(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const T* mult,
                       const int* done) {
@@ -125,6 +130,7 @@ bool plan_listed(const FftPlan1D& pl) {
   template void run_yz_rt<T, +1, 1>(qsm_ctx*, const Fft3<T>&, const cplx_t<T>*, cplx_t<T>*, const int*);       \
   template void run_yz_rt<T, -1, 2>(qsm_ctx*, const Fft3<T>&, const cplx_t<T>*, cplx_t<T>*, const int*);       \
   template void run_yz_rt<T, +1, 2>(qsm_ctx*, const Fft3<T>&, const cplx_t<T>*, cplx_t<T>*, const int*);       \
+  template bool z_mult_fits<T>(const FftPlan1D&);                                                             \
   template bool run_z_fused_m_rt<T>(qsm_ctx*, const Fft3<T>&, const cplx_t<T>*, cplx_t<T>*, const T*, const int*); \
   template void run_x_r2c_rt<T>(qsm_ctx*, const Fft3<T>&, const T*, cplx_t<T>*, const int*);                   \
   template void run_x_c2r_rt<T>(qsm_ctx*, const Fft3<T>&, const cplx_t<T>*, T*, T, const int*);                \

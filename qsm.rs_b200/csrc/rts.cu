@@ -98,7 +98,8 @@ template <typename T>
 void rts_impl(qsm_ctx* ctx, const GridDims& d, const double* f, const uint8_t* mask, const double bdir[3],
               const qsm_rts_params& p, qsm_progress_fn progress, void* user, double* out) {
   const std::string pre = sizeof(T) == 4 ? "rts32." : "rts64.";
-  if ((size_t)plan_or_throw(d.nz).m * 36 * sizeof(T) / sizeof(float) > 227u * 1024u && d.nz > 1024)
+  // refused as ever: lengths whose multiplier pass the run-time engine cannot hold in one kernel
+  if (!z_mult_fits<T>(plan_or_throw(d.nz)))
     throw QsmError(QSM_ERR_UNSUPPORTED_SIZE, "z axis too long for the RTS multiplier tiles");
   TvState* st = ws<TvState>(ctx, pre + "state", 1);
   TvVol<T> v;
