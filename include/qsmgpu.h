@@ -130,7 +130,9 @@ QSM_API qsm_status qsm_ctx_autotune_entry(const qsm_ctx* ctx, size_t i, char* ke
 /* Fault injection for callers' error-path tests: after `after` more successful device
  * allocations, the context's next allocation fails with QSM_ERR_ALLOC (the failure is
  * simulated on the host; nothing reaches the GPU), then allocations succeed again.  A
- * negative value cancels.  The context stays usable after the failed call. */
+ * negative value cancels.  The context stays usable after the failed call.  The page-locked
+ * slots of large host copies, made once, count as one allocation; without them, and without
+ * the key buffers of order statistics, a call does its work in another way. */
 QSM_API qsm_status qsm_ctx_inject_alloc_failure(qsm_ctx* ctx, long long after);
 /* 1 when every axis length of `grid` has a transform plan: lengths up to 4096 whose prime
  * factors are at most 13, and any length up to 2048 (dense factors or a Bluestein

@@ -10,13 +10,23 @@
 
 namespace qsm {
 
-cudaError_t ctx_malloc(qsm_ctx* ctx, void** p, size_t bytes) {
+namespace {
+// Whether the allocation about to be made is the one that is to fail.
+bool injected_failure(qsm_ctx* ctx) {
   if (ctx->alloc_fail_after == 0) {
     ctx->alloc_fail_after = -1;  // one injected failure, then allocations succeed again
+    return true;
+  }
+  if (ctx->alloc_fail_after > 0) ctx->alloc_fail_after--;
+  return false;
+}
+}  // namespace
+
+cudaError_t ctx_malloc(qsm_ctx* ctx, void** p, size_t bytes) {
+  if (injected_failure(ctx)) {
     *p = nullptr;
     return cudaErrorMemoryAllocation;
   }
-  if (ctx->alloc_fail_after > 0) ctx->alloc_fail_after--;
   return cudaMalloc(p, bytes);
 }
 
@@ -267,17 +277,20 @@ bool pageable(const void* p) {
   return at.type == cudaMemoryTypeUnregistered;
 }
 
-void ensure_pinned(qsm_ctx* ctx) {
-  if (!ctx->pinned && cudaHostAlloc(&ctx->pinned, 2 * kStageThreads * kStageChunk, cudaHostAllocDefault) != cudaSuccess) {
+// False when the pinned slots cannot be had; the copy then goes through the driver's own.
+bool ensure_pinned(qsm_ctx* ctx) {
+  if (!ctx->pinned && (injected_failure(ctx) || cudaHostAlloc(&ctx->pinned, 2 * kStageThreads * kStageChunk,
+                                                              cudaHostAllocDefault) != cudaSuccess)) {
     (void)cudaGetLastError();
     ctx->pinned = nullptr;
-    throw QsmError(QSM_ERR_ALLOC, "pinned staging allocation failed");
+    return false;
   }
   while (ctx->pinned_ev.size() < 2 * (size_t)kStageThreads) {
     cudaEvent_t e = nullptr;
     QSM_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     ctx->pinned_ev.push_back(e);
   }
+  return true;
 }
 
 // work(worker) on kStageThreads threads (worker 0 here, and those that cannot be started);
@@ -304,7 +317,11 @@ template <class F> void stage_workers(qsm_ctx* ctx, const F& work) {
 }  // namespace
 
 void staged_h2d(qsm_ctx* ctx, void* dst, const void* src, size_t bytes) {
-  ensure_pinned(ctx);
+  if (!ensure_pinned(ctx)) {
+    QSM_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    sync(ctx);
+    return;
+  }
   const uint8_t* s = static_cast<const uint8_t*>(src);
   uint8_t* d = static_cast<uint8_t*>(dst);
   stage_workers(ctx, [&](int w) -> cudaError_t {
@@ -325,7 +342,11 @@ void staged_h2d(qsm_ctx* ctx, void* dst, const void* src, size_t bytes) {
 }
 
 void staged_d2h(qsm_ctx* ctx, void* dst, const void* src, size_t bytes) {
-  ensure_pinned(ctx);
+  if (!ensure_pinned(ctx)) {
+    QSM_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    sync(ctx);
+    return;
+  }
   const uint8_t* s = static_cast<const uint8_t*>(src);
   uint8_t* d = static_cast<uint8_t*>(dst);
   stage_workers(ctx, [&](int w) -> cudaError_t {

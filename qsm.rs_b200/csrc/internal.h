@@ -142,8 +142,9 @@ cudaError_t ctx_malloc(qsm_ctx* ctx, void** p, size_t bytes);
 // Staged copies: kStageThreads host threads, each taking every kStageThreads-th chunk
 // through its own two pinned slots, so that the host copies run side by side and under the
 // DMA.  (One pageable cudaMemcpyAsync per buffer: 18 ms for a 58 MB volume in and out with its
-// mask, 7 GB/s; staged 5 ms.)  staged_h2d returns when the source has been read,
-// staged_d2h when the destination is written.
+// mask, 7 GB/s; staged 5 ms.)  Where the 16 MB of slots cannot be had they are plain copies.
+// staged_h2d returns when the source has been read, staged_d2h when the destination is
+// written.
 constexpr int kStageThreads = 8;
 constexpr size_t kStageChunk = (size_t)1 << 20;
 constexpr size_t kStageMin = (size_t)4 << 20;
