@@ -416,8 +416,9 @@ long long count_selected(qsm_ctx* ctx, const uint8_t* mask, long long n) {
 
 namespace {
 
-// The sampled brackets; false when a bracket missed its rank (the caller then runs the
-// radix passes).  count: values selected by the mask.
+// The sampled brackets; false when a bracket missed its rank or their key buffers (4 bytes a
+// value) cannot be had: the caller then runs the radix passes.  count: values selected by the
+// mask.
 bool bracket_ranks(qsm_ctx* ctx, const double* vals, const uint8_t* mask, long long n, long long count,
                    const std::vector<long long>& ranks, std::vector<double>& out) {
   BrkState h{};
@@ -435,8 +436,13 @@ bool bracket_ranks(qsm_ctx* ctx, const double* vals, const uint8_t* mask, long l
   const long long cap = std::max<long long>(kBrkSample, n / 8);
   BrkState* st = ws<BrkState>(ctx, "sel.brk", 1);
   unsigned long long* buf[2];
-  for (int i = 0; i < 2; ++i)
-    buf[i] = ws<unsigned long long>(ctx, i ? "sel.keys1" : "sel.keys0", (size_t)cap * kBrkMaxGroups);
+  try {
+    for (int i = 0; i < 2; ++i)
+      buf[i] = ws<unsigned long long>(ctx, i ? "sel.keys1" : "sel.keys0", (size_t)cap * kBrkMaxGroups);
+  } catch (const QsmError& e) {  // the radix passes need no such buffers
+    if (e.code != QSM_ERR_ALLOC) throw;
+    return false;
+  }
   h2d(ctx, st, &h, sizeof(h));
   const size_t smem = kBrkSample * sizeof(unsigned long long);
   raise_smem_limit(reinterpret_cast<const void*>(k_sel_bracket), ctx->device, smem);

@@ -1,12 +1,15 @@
 """Calls whose larger buffers cannot be had: the staged host copies without their page-locked
-slots.  The failure is simulated on the host (qsm_ctx_inject_alloc_failure); the call then
-does without, with the same result."""
+slots, and order statistics without their key buffers.  The failure is simulated on the host
+(qsm_ctx_inject_alloc_failure); the call then does without, with the same result.  And which
+of its two ways a selection takes, seen by the kernels that ran: brackets where they can hold
+the ranks, the radix passes where the sample misses them."""
 import numpy as np
 import pytest
 import torch
 
 import qsmgpu
 from qsmgpu import Grid, inversion
+from oracle import qsm_oracle as O
 
 pytestmark = pytest.mark.gpu
 
@@ -25,3 +28,67 @@ def test_host_calls_without_pinned_slots():
         np.testing.assert_array_equal(inversion.tkd(f, m, grid, (0, 0, 1), p, ctx=ctx), want)
         # the failure was taken by the slots, and the next copies have them
         np.testing.assert_array_equal(inversion.tkd(f, m, grid, (0, 0, 1), p, ctx=ctx), want)
+
+
+PERCENTS = [0.1, 30.0, 60.0, 99.9]
+
+
+def selection(n, kind):
+    rng = np.random.default_rng(n)
+    v = rng.standard_normal(n)
+    if kind == "few":
+        v = np.round(v)
+    elif kind == "equal":
+        v = np.full(n, -0.25)
+    elif kind == "sorted":
+        v = np.sort(v)
+    return v
+
+
+def percentiles(ctx, v, m):
+    """The library's values, the oracle's, and whether the radix passes ran."""
+    dv = torch.from_numpy(v).cuda()
+    dm = torch.from_numpy(m).cuda() if m is not None else None
+    torch.cuda.synchronize()
+    ctx.set_profiling(True)
+    try:
+        ctx.profile_reset()
+        got = inversion.prctile_device(ctx, dv.data_ptr(), dm.data_ptr() if m is not None else 0, v.size, PERCENTS)
+        kernels = ctx.profile()
+    finally:
+        ctx.set_profiling(False)
+    sel = np.sort(v if m is None else v[m > 0])
+    return got, [O.prctile(sel, p) for p in PERCENTS], "select_hist" in kernels
+
+
+@pytest.mark.parametrize("kind", ["normal", "few", "equal", "sorted"])
+@pytest.mark.parametrize("n,keep", [(2048, 1.0), (2049, 1.0), (30011, 1.0), (300007, 0.5), (3000017, 0.3), (6000000, 1.0)])
+def test_brackets_hold_the_ranks(ctx64, kind, n, keep):
+    v = selection(n, kind)
+    m = (np.random.default_rng(n + 1).random(n) < keep).astype(np.uint8) if keep < 1.0 else None
+    got, want, radix = percentiles(ctx64, v, m)
+    np.testing.assert_array_equal(got, want)
+    assert not radix
+
+
+def test_radix_passes_where_the_sample_misses(ctx64):
+    """3000 selected values in one stretch of 3 million: two or three of the 2048 sampled
+    places lie in it, too few to set a bracket."""
+    v = selection(3000017, "normal")
+    m = np.zeros(v.size, np.uint8)
+    m[1000000:1003000] = 1
+    got, want, radix = percentiles(ctx64, v, m)
+    np.testing.assert_array_equal(got, want)
+    assert radix
+
+
+@pytest.mark.parametrize("after", [2, 3])
+def test_order_statistics_without_key_buffers(after):
+    """A masked selection makes the count, the bracket state and two key buffers."""
+    v = selection(300007, "normal")
+    m = (np.random.default_rng(4).random(v.size) < 0.5).astype(np.uint8)
+    with qsmgpu.Context(0, "f64") as ctx:
+        ctx.inject_alloc_failure(after)
+        got, want, radix = percentiles(ctx, v, m)
+        np.testing.assert_array_equal(got, want)
+        assert radix
