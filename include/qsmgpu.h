@@ -304,8 +304,9 @@ QSM_API qsm_status qsm_ilsqr_device(qsm_ctx* ctx, const double* d_local_field, c
  * src/inversion/ilsqr.rs:988-1010: y = D * FFT(w * Re(IFFT(D * x))), D the dipole kernel
  * of (grid, bdir).  x and y are full complex spectra of nx*ny*nz values (interleaved re,
  * im; Fortran order; 16-byte aligned device memory), w is real (nx*ny*nz values).  Runs
- * the five passes of the solver's own loop, in float in a mixed context (whatever its
- * Krylov precision) and in double otherwise. */
+ * the five half-spectrum passes of the solver's own loop between a folding and an unfolding
+ * of the full spectra, in float in a mixed context (whatever its Krylov precision) and in
+ * double otherwise. */
 QSM_API qsm_status qsm_ilsqr_lsqr_operator_device(qsm_ctx* ctx, const qsm_grid* grid, const double bdir[3],
                                                   const double* d_weights, const double* d_x, double* d_y);
 /* inversion::tgv_qsm — src/inversion/tgv.rs:1045-1299: susceptibility (ppm) from WRAPPED

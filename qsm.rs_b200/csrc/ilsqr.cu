@@ -160,27 +160,6 @@ __global__ void k_dipole_pow(KSpace K, int nx, int ny, int nz, double n_exp, dou
   }
 }
 
-// ==================================================== loaders, stores, mids ==
-template <typename T> struct LoadSpecRow {  // full-spectrum row element
-  const cplx_t<T>* s;
-  int pitch;
-  __device__ __forceinline__ cplx_t<T> operator()(int row, int e) const { return s[(long long)row * pitch + e]; }
-};
-template <typename T> struct StoreSpecRow {
-  cplx_t<T>* s;
-  int pitch;
-  __device__ __forceinline__ void operator()(int row, int e, cplx_t<T> v) { s[(long long)row * pitch + e] = v; }
-  __device__ __forceinline__ void finish() {}
-};
-// w * Re(v)/N as a real row element (lsqr_step's apply_a, ilsqr.rs:1000-1003)
-template <typename T> struct MidWeightRe {
-  const T* w;
-  int nx;
-  T invn;
-  __device__ __forceinline__ cplx_t<T> operator()(cplx_t<T> v, int row, int e) const {
-    return mk<cplx_t<T>>(w[(long long)row * nx + e] * (v.x * invn), T(0));
-  }
-};
 // ====================================================================== LSQR ==
 struct LsqrState {
   int done;   // every later kernel returns at once
@@ -192,7 +171,7 @@ struct LsqrState {
   double rho_bar, phi_bar, bnorm, t1, t2, tol;
 };
 
-// The scalar recurrence after the norm of an application's output (modes as OpLsqrOut).
+// The scalar recurrence after the norm of an application's output (modes as OpLsqrHalf).
 __device__ inline void lsqr_last(LsqrState* st, int mode, double total) {
   const double nrm = sqrt(total);
   if (mode == 0 || mode == 2) {
@@ -230,65 +209,6 @@ __device__ __forceinline__ double dip(const KSpace& K, int ix, int iy, int iz) {
   return K.dipole(__ldg(K.fx + ix), __ldg(K.fy + iy), __ldg(K.fz + iz));
 }
 
-// pre: (x * s) * D(k), s = the input vector's deferred scale
-template <typename T> struct OpScaleD {
-  using C = cplx_t<T>;
-  KSpace K;
-  const double* s;
-  // the dipole evaluation runs over a staged tile (k_pass_yz_st_op): inside the first
-  // stage's direct loads it lengthened their latency chain (309 against 256 us in float)
-  static constexpr bool kStagedPre = true;
-  __device__ __forceinline__ C pre(C v, int ix, int iy, int iz, long long) const {
-    return cscale(cscale(v, (T)*s), (T)dip(K, ix, iy, iz));
-  }
-  __device__ __forceinline__ C post(C v, int, int, int, long long) const { return v; }
-};
-
-// Z forward epilogue of an A application.  mode 0: u = A v - alpha*u (then beta);
-// 1: v = A u - beta*v (then alpha and the rotation); 2: b (then beta = ||b||);
-// 3: v = A^H u (then alpha; alpha*beta = 0 ends the solve with x = 0).
-template <typename T> struct OpLsqrOut {
-  using C = cplx_t<T>;
-  KSpace K;
-  const C* old;
-  LsqrState* st;
-  int mode;
-  // the compile-time pass stages `old` through shared memory (k_pass_yz_dx_old)
-  static constexpr bool kReadsOld = true;
-  struct Scalars {
-    double coef, sc;
-  };
-  __device__ __forceinline__ C pre(C v, int, int, int, long long) const { return v; }
-  __device__ __forceinline__ C post(C v, int ix, int iy, int iz, long long idx, double& acc) const {
-    C r = cscale(v, (T)dip(K, ix, iy, iz));
-    if (mode <= 1) {
-      const double coef = mode == 0 ? -st->alpha : -st->beta;
-      const double sc = mode == 0 ? st->su : st->sv;
-      const C o = cscale(old[idx], (T)sc);
-      r = cadd(r, cscale(o, (T)coef));
-    }
-    acc += (double)r.x * (double)r.x + (double)r.y * (double)r.y;
-    return r;
-  }
-  __device__ __forceinline__ const C* old_src() const { return mode <= 1 ? old : nullptr; }
-  __device__ __forceinline__ Scalars scalars() const {
-    if (mode > 1) return Scalars{0.0, 0.0};
-    return Scalars{mode == 0 ? -st->alpha : -st->beta, mode == 0 ? st->su : st->sv};
-  }
-  // post() with the old value and the scalars already in hand (same arithmetic)
-  __device__ __forceinline__ C post_old(C v, int ix, int iy, int iz, long long, C oldv, const Scalars& s,
-                                        double& acc) const {
-    C r = cscale(v, (T)dip(K, ix, iy, iz));
-    if (mode <= 1) {
-      const C o = cscale(oldv, (T)s.sc);
-      r = cadd(r, cscale(o, (T)s.coef));
-    }
-    acc += (double)r.x * (double)r.x + (double)r.y * (double)r.y;
-    return r;
-  }
-  __device__ void last(double total) const { lsqr_last(st, mode, total); }
-};
-
 // v * s * m: the input of A, s its deferred scale
 template <typename T> struct OpScaleM {
   using C = cplx_t<T>;
@@ -301,7 +221,9 @@ template <typename T> struct OpScaleM {
   __device__ __forceinline__ C post(C v, int, int, int, long long) const { return v; }
 };
 
-// Z forward epilogue of an application of A on half spectra; modes as OpLsqrOut.
+// Z forward epilogue of an application of A.  mode 0: u = A v - alpha*u (then beta);
+// 1: v = A u - beta*v (then alpha and the rotation); 2: b (then beta = ||b||);
+// 3: v = A^H u (then alpha; alpha*beta = 0 ends the solve with x = 0).
 template <typename T> struct OpLsqrHalf {
   using C = cplx_t<T>;
   const T* m;
@@ -309,6 +231,7 @@ template <typename T> struct OpLsqrHalf {
   const C* old;
   LsqrState* st;
   int mode;
+  // the compile-time pass stages `old` through shared memory (k_pass_yz_dx_old)
   static constexpr bool kReadsOld = true;
   static constexpr bool kNoPre = true;
   struct Scalars {
@@ -437,6 +360,32 @@ void run_x_weight(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* spec, const T* w, T
   }
   run_x_c2r<T>(ctx, f, spec, StoreReal<T>{img, f.g.nx, invn}, done);
   run_x_r2c<T>(ctx, f, spec, LoadProduct<T, T>{img, w, f.g.nx}, done);
+}
+
+// What an application of A works with.
+template <typename T> struct LsqrOperator {
+  const Fft3<T>* f;
+  const T* m;  // OpHalfD
+  const T* w;
+  T invn;
+  cplx_t<T>* t;  // a half spectrum
+  T* img;        // a real volume
+  LsqrState* st;
+  double* partials;
+  unsigned* counter;
+};
+// dst = A(s x) with the epilogue of `mode` (OpLsqrHalf): h -> m FFT(w IFFT(m h)) on half spectra.
+template <typename T>
+void lsqr_apply(qsm_ctx* ctx, const LsqrOperator<T>& a, const cplx_t<T>* x, const double* s, cplx_t<T>* dst,
+                const cplx_t<T>* old, int mode) {
+  const Fft3<T>& f = *a.f;
+  const int* done = &a.st->done;
+  run_yz<T, +1, 2, true>(ctx, f, x, a.t, OpScaleM<T>{a.m, s}, done);
+  run_yz<T, +1, 1>(ctx, f, a.t, a.t, OpId<T>{}, done);
+  run_x_weight<T>(ctx, f, a.t, a.w, a.invn, a.img, done);
+  run_yz<T, -1, 1>(ctx, f, a.t, a.t, OpId<T>{}, done);
+  run_yz_acc<T, -1, 2, true>(ctx, f, a.t, dst, OpLsqrHalf<T>{a.m, f.g.nx, old, a.st, mode}, a.partials, a.counter, done,
+                             "fft_z_lsqr");
 }
 
 template <typename T>
@@ -878,17 +827,9 @@ void ilsqr_impl(qsm_ctx* ctx, const GridDims& d, const double* f, const uint8_t*
   run_yz<T, -1, 1>(ctx, fh, t, t, OpId<T>{}, nullptr);
   run_yz_acc<T, -1, 2, true>(ctx, fh, t, ub, OpLsqrHalf<T>{mult, d.nx, nullptr, lst, 2}, partials, counter, nullptr,
                              "fft_z_lsqr");
-  // y = A(s*x) written to dst with the given epilogue mode
-  auto apply_a = [&](const C* x, const double* s, C* dst, const C* old, int mode) {
-    run_yz<T, +1, 2, true>(ctx, fh, x, t, OpScaleM<T>{mult, s}, ldone);
-    run_yz<T, +1, 1>(ctx, fh, t, t, OpId<T>{}, ldone);
-    run_x_weight<T>(ctx, fh, t, wl, invn, img, ldone);
-    run_yz<T, -1, 1>(ctx, fh, t, t, OpId<T>{}, ldone);
-    run_yz_acc<T, -1, 2, true>(ctx, fh, t, dst, OpLsqrHalf<T>{mult, d.nx, old, lst, mode}, partials, counter, ldone,
-                               "fft_z_lsqr");
-  };
+  const LsqrOperator<T> A{&fh, mult, wl, invn, t, img, lst, partials, counter};
   // v = A^H u, alpha; w = v
-  apply_a(ub, &lst->su, vb, nullptr, 3);
+  lsqr_apply<T>(ctx, A, ub, &lst->su, vb, nullptr, 3);
   {
     LaunchScope ls(ctx, "lsqr_init");
     k_lsqr_init_w<T><<<grid1d(NH), 256, 0, ctx->stream>>>(NH, vb, wb, lst);
@@ -896,8 +837,8 @@ void ilsqr_impl(qsm_ctx* ctx, const GridDims& d, const double* f, const uint8_t*
   }
   const unsigned ugrid = grid1d(NH);
   run_iterations(ctx, 50, ldone, [&]() {  // maxit_lsqr, ilsqr.rs:967
-    apply_a(vb, &lst->sv, ub, ub, 0);
-    apply_a(ub, &lst->su, vb, vb, 1);
+    lsqr_apply<T>(ctx, A, vb, &lst->sv, ub, ub, 0);
+    lsqr_apply<T>(ctx, A, ub, &lst->su, vb, vb, 1);
     LaunchScope ls(ctx, "lsqr_update");
     k_lsqr_update<T><<<ugrid, 256, 0, ctx->stream>>>(NH, xb, wb, vb, lst, partials);
     ls.done();
@@ -1058,32 +999,41 @@ void ilsqr_impl(qsm_ctx* ctx, const GridDims& d, const double* f, const uint8_t*
 }
 
 // ---------------------------------------------------- the LSQR operator alone ----
-// Contiguous complex double rows (nx values) <-> full-spectrum rows (pitch values).
+// The operator takes any full spectrum x, but A sees only the real image of D x: with
+// Y(k) = (D(k) x(k) + conj(D(-k) x(-k))) / 2 that is h = Y / m (0 where m is, for there
+// D(k) = D(-k) = 0), and A's h = m G is y = D G.
 template <typename T>
-__global__ void k_rows_to_pitch(long long nrows, int nx, int pitch, const double2* __restrict__ in,
-                                cplx_t<T>* __restrict__ out) {
-  const long long total = nrows * pitch;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long row = i / pitch;
-    const int e = (int)(i - row * pitch);
+__global__ void __launch_bounds__(128)
+    k_lsqr_fold(Geom g, KSpace K, const T* __restrict__ m, const double2* __restrict__ x, cplx_t<T>* __restrict__ h) {
+  const int iy = blockIdx.x, iz = blockIdx.y;
+  const int my = iy ? g.ny - iy : 0, mz = iz ? g.nz - iz : 0;
+  const long long row = ((long long)iz * g.ny + iy) * g.pitch;
+  const double2* xa = x + ((long long)iz * g.ny + iy) * g.nx;
+  const double2* xb = x + ((long long)mz * g.ny + my) * g.nx;
+  for (int ix = threadIdx.x; ix < g.pitch; ix += blockDim.x) {
     cplx_t<T> v = mk<cplx_t<T>>(T(0), T(0));
-    if (e < nx) {
-      const double2 a = in[row * nx + e];
-      v = mk<cplx_t<T>>((T)a.x, (T)a.y);
+    if (ix < g.nxh && m[row + ix] != T(0)) {
+      const int mx = ix ? g.nx - ix : 0;
+      const double da = dip(K, ix, iy, iz), db = dip(K, mx, my, mz), r = 0.5 / (double)m[row + ix];
+      const double2 a = xa[ix], b = xb[mx];
+      v = mk<cplx_t<T>>((T)((da * a.x + db * b.x) * r), (T)((da * a.y - db * b.y) * r));
     }
-    out[i] = v;
+    h[row + ix] = v;
   }
 }
 template <typename T>
-__global__ void k_pitch_to_rows(long long nrows, int nx, int pitch, const cplx_t<T>* __restrict__ in,
-                                double2* __restrict__ out) {
-  const long long total = nrows * nx;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long row = i / nx;
-    const cplx_t<T> v = in[row * pitch + (i - row * nx)];
-    out[i] = make_double2((double)v.x, (double)v.y);
+__global__ void __launch_bounds__(128)
+    k_lsqr_unfold(Geom g, KSpace K, const T* __restrict__ m, const cplx_t<T>* __restrict__ h, double2* __restrict__ y) {
+  const int iy = blockIdx.x, iz = blockIdx.y;
+  const int my = iy ? g.ny - iy : 0, mz = iz ? g.nz - iz : 0;
+  const long long rowa = ((long long)iz * g.ny + iy) * g.pitch, rowb = ((long long)mz * g.ny + my) * g.pitch;
+  for (int ix = threadIdx.x; ix < g.nx; ix += blockDim.x) {
+    const bool own = ix < g.nxh;
+    const long long i = own ? rowa + ix : rowb + (g.nx - ix);
+    const double mm = (double)m[i];
+    const double r = mm != 0.0 ? dip(K, ix, iy, iz) / mm : 0.0;
+    const cplx_t<T> v = h[i];
+    y[((long long)iz * g.ny + iy) * g.nx + ix] = make_double2(r * (double)v.x, own ? r * (double)v.y : -r * (double)v.y);
   }
 }
 template <typename T>
@@ -1093,46 +1043,39 @@ __global__ void k_cast_real(long long n, const double* __restrict__ in, T* __res
 }
 
 // y = D * FFT(w * Re(IFFT(D * x))): one application of lsqr_step's operator
-// (src/inversion/ilsqr.rs:988-1010) with the five passes of the solver's own loop.
+// (src/inversion/ilsqr.rs:988-1010) by the solver's own (lsqr_apply).
 template <typename T>
 void lsqr_operator_impl(qsm_ctx* ctx, const GridDims& d, const double bdir[3], const double* w, const double2* x,
                         double2* y) {
   using C = cplx_t<T>;
   const std::string pre = sizeof(T) == 4 ? "ilop32." : "ilop64.";
-  Fft3<T> ff = make_fft3_full<T>(ctx, d);
-  KSpace K = make_kspace(ctx, d, bdir);
-  const long long N = d.n, NF = ff.g.hsize(), nrows = (long long)d.ny * d.nz;
-  C* xin = ws<C>(ctx, pre + "x", (size_t)NF);
-  C* t = ws<C>(ctx, pre + "t", (size_t)NF);
-  C* yo = ws<C>(ctx, pre + "y", (size_t)NF);
-  T* wl = ws<T>(ctx, pre + "w", (size_t)N);
+  const Fft3<T> f = make_fft3<T>(ctx, d);
+  const KSpace K = make_kspace(ctx, d, bdir);
+  const size_t N = (size_t)d.n, NH = (size_t)f.g.hsize();
+  C* h = ws<C>(ctx, pre + "h", NH);
+  C* out = ws<C>(ctx, pre + "y", NH);
+  T* m = ws<T>(ctx, pre + "m", NH);
+  T* wl = ws<T>(ctx, pre + "w", N);
   LsqrState* st = ws<LsqrState>(ctx, pre + "state", 1);
-  double* partials = ws<double>(ctx, pre + "partials", (size_t)kMaxPersistentBlocks * 4);
-  unsigned* counter = ws<unsigned>(ctx, pre + "counter", 1);
+  const LsqrOperator<T> A{&f, m, wl, (T)(1.0 / (double)d.n), ws<C>(ctx, pre + "t", NH), ws<T>(ctx, pre + "img", N), st,
+                          ws<double>(ctx, pre + "partials", std::max(x_partials(f, 1), (size_t)kMaxPersistentBlocks * 4)),
+                          ws<unsigned>(ctx, pre + "counter", 1)};
   LsqrState init{};
   init.su = 1.0;
-  init.sv = 1.0;
   h2d(ctx, st, &init, sizeof(init));
-  QSM_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned), ctx->stream));
+  QSM_CUDA(cudaMemsetAsync(A.counter, 0, sizeof(unsigned), ctx->stream));
+  spec_multiplier<T>(ctx, f, OpHalfD<T>{K, 0}, m, nullptr);
+  const dim3 rows((unsigned)d.ny, (unsigned)d.nz);
   {
     LaunchScope ls(ctx, "ilsqr_op_pack");
-    k_rows_to_pitch<T><<<grid1d(NF), 256, 0, ctx->stream>>>(nrows, d.nx, ff.g.pitch, x, xin);
+    k_cast_real<T><<<grid1d(d.n), 256, 0, ctx->stream>>>(d.n, w, wl);
+    k_lsqr_fold<T><<<rows, 128, 0, ctx->stream>>>(f.g, K, m, x, h);
     ls.done();
-    LaunchScope ls2(ctx, "ilsqr_op_weights");
-    k_cast_real<T><<<grid1d(N), 256, 0, ctx->stream>>>(N, w, wl);
-    ls2.done();
   }
-  const T invn = (T)(1.0 / (double)N);
-  run_yz<T, +1, 2>(ctx, ff, xin, t, OpScaleD<T>{K, &st->su}, nullptr);
-  run_yz<T, +1, 1>(ctx, ff, t, t, OpId<T>{}, nullptr);
-  run_x_full<T, +1, -1, true>(ctx, ff, LoadSpecRow<T>{t, ff.g.pitch}, MidWeightRe<T>{wl, d.nx, invn},
-                              StoreSpecRow<T>{t, ff.g.pitch}, nullptr, "fft_x_lsqr");
-  run_yz<T, -1, 1>(ctx, ff, t, t, OpId<T>{}, nullptr);
-  run_yz_acc<T, -1, 2, true>(ctx, ff, t, yo, OpLsqrOut<T>{K, nullptr, st, 2}, partials, counter, nullptr,
-                             "fft_z_lsqr");
+  lsqr_apply<T>(ctx, A, h, &st->su, out, nullptr, 3);
   {
     LaunchScope ls(ctx, "ilsqr_op_unpack");
-    k_pitch_to_rows<T><<<grid1d(nrows * d.nx), 256, 0, ctx->stream>>>(nrows, d.nx, ff.g.pitch, yo, y);
+    k_lsqr_unfold<T><<<rows, 128, 0, ctx->stream>>>(f.g, K, m, out, y);
     ls.done();
   }
   sync(ctx);

@@ -239,14 +239,12 @@ template <typename T> inline bool axis_listed(const qsm_ctx* ctx, const Fft3<T>&
 template <typename T, class Load> struct PlainLoad : std::false_type {};
 template <typename T, class Store> struct PlainStore : std::false_type {};
 
-// Runtime-engine X passes over plain arrays (real rows, half spectra, full complex rows),
+// Runtime-engine X passes over plain arrays (real rows and half spectra),
 // compiled once (plain_rt.cu).
 template <typename T>
 void run_x_r2c_rt(qsm_ctx* ctx, const Fft3<T>& f, const T* in, cplx_t<T>* spec, const int* done);
 template <typename T>
 void run_x_c2r_rt(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* spec, T* out, T scale, const int* done);
-template <typename T, int DIR>
-void run_x_c2c_rt(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* rows, const int* done);
 
 // Buffers of the runtime-engine X passes, between the caller's functor and the engine.
 template <typename T> T* x_stage(qsm_ctx* ctx, const Fft3<T>& f) {
@@ -349,68 +347,6 @@ void run_x_c2r(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* spec, const Stor
   else run_x_c2r_rt<T>(ctx, f, spec, buf, T(1), done);
   LaunchScope ls(ctx, "x_store");
   k_x_store<T, T, Store><<<x_rows_grid(ctx, k_x_store<T, T, Store>, f.g), 256, 0, ctx->stream>>>(f.g, f.g.nx, buf, st, done);
-  ls.done();
-}
-
-// Transform bundle for full complex spectra (complex-to-complex along x too): every
-// x column is valid, rows padded to a multiple of 4 values.
-template <typename T> Fft3<T> make_fft3_full(qsm_ctx* ctx, const GridDims& d) {
-  Fft3<T> f = make_fft3<T>(ctx, d);
-  f.g.nxh = d.nx;
-  f.g.pitch = (d.nx + 3) / 4 * 4;
-  return f;
-}
-
-// X pass over full complex rows: load -> FFT(D1) -> mid -> FFT(D2) -> store.
-// W: a hot loop's pass; with both transforms it takes the compile-time kernel
-// (k_x_full_fx) for the lengths of QSM_FIXED_PLANS (FP64 384: 96 registers against the
-// runtime engine's 130, two blocks per SM instead of one).
-template <typename T, int D1, int D2, bool W = false, class Load, class Mid, class Store>
-void run_x_full(qsm_ctx* ctx, const Fft3<T>& f, const Load& ld, const Mid& mid, const Store& st, const int* done,
-                const char* name) {
-  using C = cplx_t<T>;
-  if constexpr (W && D1 != 0 && D2 != 0) {
-    if (compiled_plans(ctx)) {
-#define QSM_TRY_XF(N_, T_, R0_, R1_, R2_)                                                          \
-    if (FixedPlan<N_, T_, R0_, R1_, R2_>::matches(f.px)) {                                         \
-      using FP = FixedPlan<N_, T_, R0_, R1_, R2_>;                                                 \
-      const int P = x_fx_pencils<FP>(ctx, f.g.nrows());                                            \
-      const size_t smem = (size_t)(x_tw_len<T>(N_) + P * x_rowlen<T>(N_)) * sizeof(C);            \
-      auto kern = k_x_full_fx<T, FP, D1, D2, Load, Mid, Store>;                                    \
-      ensure_smem(kern, smem);                                                                     \
-      LaunchScope ls(ctx, name);                                                                   \
-      kern<<<x_fx_blocks(f.g.nrows(), P), dim3(T_, P), smem, ctx->stream>>>(f.g, f.twx, ld, mid, st, done);   \
-      ls.done();                                                                                   \
-      return;                                                                                      \
-    }
-    QSM_FIXED_PLANS(QSM_TRY_XF)
-#undef QSM_TRY_XF
-    }
-  }
-  if (tf_usable(ctx, f.tfx, tf_x_stride<T>())) {
-    const size_t smem = tf_smem<T>(f.tfx.n, tf_x_stride<T>());
-    auto kern = k_x_full_tf<T, D1, D2, Load, Mid, Store>;
-    ensure_smem(kern, smem);
-    LaunchScope ls(ctx, name);
-    kern<<<tf_x_grid<T>(f.g.nrows()), kTfThreads, smem, ctx->stream>>>(f.g, f.tfx, ld, mid, st, done);
-    ls.done();
-    return;
-  }
-  C* rows = x_stage_c(ctx, f);
-  {
-    LaunchScope ls(ctx, "x_load");
-    k_x_load<T, C, Load><<<x_rows_grid(ctx, k_x_load<T, C, Load>, f.g), 256, 0, ctx->stream>>>(f.g, f.g.pitch, ld, rows, done);
-    ls.done();
-  }
-  if constexpr (D1 != 0) run_x_c2c_rt<T, D1>(ctx, f, rows, done);
-  {
-    LaunchScope ls(ctx, "x_mid");
-    k_x_mid<T, Mid><<<x_rows_grid(ctx, k_x_mid<T, Mid>, f.g), 256, 0, ctx->stream>>>(f.g, mid, rows, done);
-    ls.done();
-  }
-  if constexpr (D2 != 0) run_x_c2c_rt<T, D2>(ctx, f, rows, done);
-  LaunchScope ls(ctx, "x_store");
-  k_x_store<T, C, Store><<<x_rows_grid(ctx, k_x_store<T, C, Store>, f.g), 256, 0, ctx->stream>>>(f.g, f.g.pitch, rows, st, done);
   ls.done();
 }
 
@@ -550,13 +486,6 @@ bool launch_yz_op_fx(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* tw, const 
     if (grid > (unsigned)kMaxPersistentBlocks) return false;
     LaunchScope ls(ctx, name);
     kern<<<grid, dim3(P, FP::T), smem, ctx->stream>>>(f.g, w, tw, src, dst, op, partials, counter, done);
-    ls.done();
-  } else if constexpr (!ACC && StagedPre<Op>::value) {
-    auto kern = k_pass_yz_st_op<T, DIR, AXIS, FP, P, Op>;
-    const size_t smem = yz_smem<T>(FP::n, P);
-    if (!fx_launch_ok(ctx, kern, P * FP::T, smem, &grid, w.ntiles)) return false;
-    LaunchScope ls(ctx, name);
-    kern<<<grid, dim3(P, FP::T), smem, ctx->stream>>>(f.g, w, tw, src, dst, op, done);
     ls.done();
   } else {
     auto kern = k_pass_yz_dx_op<T, DIR, AXIS, FP, P, Op, ACC>;

@@ -148,36 +148,6 @@ __global__ void k_x_r2c(Geom g, const __grid_constant__ FftPlan1D pl, const cplx
   }
 }
 
-// ---------------------------------------------------------------------------
-// X transform of full complex rows in place (complex-to-complex spectra: [nz][ny][pitch]
-// with all nx columns valid).  One row per pencil; blockDim = (Tb, P).
-// ---------------------------------------------------------------------------
-template <typename T, int DIR, bool BL>
-__global__ void k_x_c2c(Geom g, const __grid_constant__ FftPlan1D pl, const cplx_t<T>* __restrict__ twg,
-                        cplx_t<T>* __restrict__ rows, const int* __restrict__ done) {
-  using C = cplx_t<T>;
-  if (done != nullptr && *done) return;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  C* tw = reinterpret_cast<C*>(smraw);
-  const int n = pl.n;
-  const int m = pl.m;  // slot length: n, or the Bluestein convolution length
-  const int rowlen = x_rowlen<T>(m);
-  C* sm = tw + m;
-  const int tid = threadIdx.x + threadIdx.y * blockDim.x;
-  for (int i = tid; i < m; i += blockDim.x * blockDim.y) tw[i] = twg[i];
-  const int t = threadIdx.x;
-  const long long row = (long long)blockIdx.x * blockDim.y + threadIdx.y;
-  const bool active = row < g.nrows() && t < pl.T;
-  C* sp = sm + threadIdx.y * rowlen;
-  SAPadded<PadG<T>::G> sa;
-  if (active)
-    for (int e = t; e < n; e += pl.T) sp[sa(e)] = rows[row * g.pitch + e];
-  __syncthreads();
-  fft_pencil<DIR, C, SAPadded<PadG<T>::G>, false, false, BL>(&pl, t, active, sp, sa, tw, nullptr, nullptr, 0, 0);
-  if (active)
-    for (int e = t; e < n; e += pl.T) rows[row * g.pitch + e] = sp[sa(e)];
-}
-
 // Elementwise halves of a runtime-engine X pass: the loader's rows to an array of row
 // pitch `pitch`, the mid hook over complex rows, and the array to the store functor.  A
 // warp takes whole rows.
@@ -190,17 +160,6 @@ __global__ void __launch_bounds__(256)
 #pragma unroll 4
     for (int e = lane; e < g.nx; e += 32) out[(long long)row * pitch + e] = ld(row, e);
 }
-template <typename T, class Mid>
-__global__ void __launch_bounds__(256)
-    k_x_mid(Geom g, Mid mid, cplx_t<T>* __restrict__ rows, const int* __restrict__ done) {
-  if (done != nullptr && *done) return;
-  const int lane = threadIdx.x & 31;
-  for (int row = blockIdx.x * 8 + (threadIdx.x >> 5); row < g.nrows(); row += gridDim.x * 8)
-    for (int e = lane; e < g.nx; e += 32) {
-      cplx_t<T>* q = rows + (long long)row * g.pitch + e;
-      *q = mid(*q, row, e);
-    }
-}
 template <typename T, typename V, class Store>
 __global__ void __launch_bounds__(256)
     k_x_store(Geom g, int pitch, const V* in, Store st0, const int* __restrict__ done) {
@@ -211,49 +170,6 @@ __global__ void __launch_bounds__(256)
 #pragma unroll 4
     for (int e = lane; e < g.nx; e += 32) st(row, e, __ldcg(in + (long long)row * pitch + e));
   }
-  st.finish();
-}
-
-// Compile-time X pass over full complex rows with both transforms (FP a FixedPlan), per
-// row load -> FFT(D1) -> mid -> FFT(D2) -> store:
-//   Load : C operator()(int row, int e)
-//   Mid  : C operator()(C v, int row, int e)
-//   Store: void operator()(int row, int e, C v); void finish()
-// The first transform's first stage fetches through the loader, its last stage applies the
-// mid hook and passes the values in registers to the second transform (the reversed plan),
-// whose last stage hands its values straight to the store functor.  Every element of a row is fetched
-// in the first stage, before any store of that row, so the loader and the store may
-// address the same rows.
-template <typename T, class FP, int D1, int D2, class Load, class Mid, class Store>
-__global__ void k_x_full_fx(Geom g, const cplx_t<T>* __restrict__ twg, Load ld, Mid mid, Store st0,
-                            const int* __restrict__ done) {
-  using C = cplx_t<T>;
-  constexpr int N = FP::n, TT = FP::T;
-  static_assert(D1 != 0 && D2 != 0, "both transforms");
-  if (done != nullptr && *done) return;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  constexpr bool TWP = x_tw_padded<T>();
-  C* tw = reinterpret_cast<C*>(smraw);
-  C* sm = tw + x_tw_len<T>(N);
-  const int tid = threadIdx.x + threadIdx.y * blockDim.x;
-  for (int i = tid; i < N; i += blockDim.x * blockDim.y) tw[TWP ? tw_pad(i) : i] = twg[i];
-  const int t = threadIdx.x;
-  const int row = blockIdx.x * blockDim.y + threadIdx.y;
-  const bool active = row < g.nrows() && t < TT;
-  C* sp = sm + threadIdx.y * x_rowlen<T>(N);
-  SAPadded<x_pad<T, FP>()> sa;
-  Store st = st0;
-  auto fetch_g = [&](int e) -> C { return ld(row, e); };
-  auto emit_g = [&](int e, C v) { st(row, e, v); };
-  // The first transform's last stage applies the mid hook in registers and the second
-  // transform, the reversed plan, starts from them (FetchInRegs): no shared-memory round
-  // trip and no barrier between the two.
-  C v[kFftEmax];
-  auto hook = [&](int e, C x) -> C { return mid(x, row, e); };
-  EmitInRegs<decltype(hook)> keep{hook};
-  FetchInRegs in_regs;
-  FP::template run_v<D1, TWP>(v, t, active, sp, sa, tw, fetch_g, keep);
-  ReversePlan<FP>::type::template run_v<D2, TWP>(v, t, active, sp, sa, tw, in_regs, emit_g);
   st.finish();
 }
 
@@ -892,65 +808,6 @@ __global__ void __launch_bounds__(P* FP::T, yz_dx_min_blocks<T, P * FP::T>())
   if constexpr (ACC) {
     if (grid_sum_last<1>(acc, partials, counter) && tid == 0) op.last(acc[0]);
   }
-}
-
-// Ops whose pre hook is costly enough (a k-space evaluation per element) that it should
-// run on a staged tile rather than inside the first stage's loads (kStagedPre).
-template <class Op, class = void> struct StagedPre : std::false_type {};
-template <class Op> struct StagedPre<Op, std::void_t<decltype(Op::kStagedPre)>> : std::bool_constant<Op::kStagedPre> {};
-
-// Compile-time Y/Z operator pass in staged form: the tile is copied into shared memory
-// with cp.async, double-buffered so the next tile's copy overlaps this tile's work, the
-// pre hook runs over the staged tile, and the transform (FP) reads its first stage from
-// shared memory and hands each output to the post hook on its way to global memory.
-template <typename T, int DIR, int AXIS, class FP, int P, class Op>
-__global__ void __launch_bounds__(P* FP::T, yz_dx_min_blocks<T, P * FP::T>())
-    k_pass_yz_st_op(Geom g, TileWalk w, const cplx_t<T>* __restrict__ twg, const cplx_t<T>* src, cplx_t<T>* dst,
-                    Op op, const int* __restrict__ done) {
-  using C = cplx_t<T>;
-  constexpr int n = FP::n;
-  if (done != nullptr && *done) return;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  C* tw = reinterpret_cast<C*>(smraw);
-  C* buf0 = tw + ((n + 7) & ~7);
-  C* buf1 = buf0 + n * P;
-  const int tid = threadIdx.x + threadIdx.y * P;
-  for (int i = tid; i < n; i += P * FP::T) tw[i] = twg[i];
-  const int px = threadIdx.x;
-  const int t = threadIdx.y;
-  SAStridedC<P> sa;
-  int tile = blockIdx.x;
-  if (tile < w.ntiles) issue_tile(src, buf0, g, w, tile, n, P);
-  cp_async_commit();
-  for (int it = 0; tile < w.ntiles; tile += gridDim.x, ++it) {
-    C* cur = (it & 1) ? buf1 : buf0;
-    C* nxt = (it & 1) ? buf0 : buf1;
-    const int next = tile + gridDim.x;
-    if (next < w.ntiles) issue_tile(src, nxt, g, w, next, n, P);
-    cp_async_commit();
-    cp_async_wait<1>();
-    __syncthreads();
-    const int tx = tile % w.ntx, outer = tile / w.ntx;
-    const int col = tx * P + px;
-    const bool active = col < g.nxh;
-    const long long base = col + (long long)outer * w.ostride;
-    C* sp = cur + px;
-    if (active) {
-      for (int e = t; e < n; e += FP::T) {
-        const long long idx = base + e * w.estride;
-        sp[sa(e)] = (AXIS == 1) ? op.pre(sp[sa(e)], col, e, outer, idx) : op.pre(sp[sa(e)], col, outer, e, idx);
-      }
-    }
-    __syncthreads();
-    auto fetch = [&](int e) -> C { return sp[sa(e)]; };
-    auto emit = [&](int e, C v) {
-      const long long idx = base + e * w.estride;
-      dst[idx] = (AXIS == 1) ? op.post(v, col, e, outer, idx) : op.post(v, col, outer, e, idx);
-    };
-    // the transform ends with a block barrier, so the buffer may be refilled next
-    FP::template run<DIR>(t, active, sp, sa, tw, fetch, emit);
-  }
-  cp_async_wait<0>();
 }
 
 // Ops whose store epilogue reads a second array at the stored element (kReadsOld): the

@@ -97,21 +97,6 @@ void run_x_c2r_rt(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* spec, T* out,
   ls.done();
 }
 
-template <typename T, int DIR>
-void run_x_c2c_rt(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* rows, const int* done) {
-  if ((f.px.n + f.px.T - 1) / f.px.T > kFftEmax)
-    throw QsmError(QSM_ERR_UNSUPPORTED_SIZE, "x length outside the per-thread register budget");
-  const int Tt = x_block_t(f.px.T);
-  const int P = x_pencils_per_block<T>(f.px.T);
-  const size_t smem = (size_t)(f.px.m + P * x_rowlen<T>(f.px.m)) * sizeof(cplx_t<T>);
-  auto kern = f.px.m != f.px.n ? k_x_c2c<T, DIR, true> : k_x_c2c<T, DIR, false>;
-  ensure_smem(kern, smem);
-  const long long blocks = ((long long)f.g.nrows() + P - 1) / P;
-  LaunchScope ls(ctx, "fft_x_c2c");
-  kern<<<(unsigned)blocks, dim3(Tt, P), smem, ctx->stream>>>(f.g, f.px, f.twx, rows, done);
-  ls.done();
-}
-
 bool plan_listed(const FftPlan1D& pl) {
 #define QSM_LISTED(N_, T_, R0_, R1_, R2_) \
   if (FixedPlan<N_, T_, R0_, R1_, R2_>::matches(pl)) return true;
@@ -133,9 +118,7 @@ bool plan_listed(const FftPlan1D& pl) {
   template bool z_mult_fits<T>(const FftPlan1D&);                                                             \
   template bool run_z_fused_m_rt<T>(qsm_ctx*, const Fft3<T>&, const cplx_t<T>*, cplx_t<T>*, const T*, const int*); \
   template void run_x_r2c_rt<T>(qsm_ctx*, const Fft3<T>&, const T*, cplx_t<T>*, const int*);                   \
-  template void run_x_c2r_rt<T>(qsm_ctx*, const Fft3<T>&, const cplx_t<T>*, T*, T, const int*);                \
-  template void run_x_c2c_rt<T, -1>(qsm_ctx*, const Fft3<T>&, cplx_t<T>*, const int*);                         \
-  template void run_x_c2c_rt<T, +1>(qsm_ctx*, const Fft3<T>&, cplx_t<T>*, const int*);
+  template void run_x_c2r_rt<T>(qsm_ctx*, const Fft3<T>&, const cplx_t<T>*, T*, T, const int*);
 QSM_RT(float)
 QSM_RT(double)
 #undef QSM_RT

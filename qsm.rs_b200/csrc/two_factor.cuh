@@ -506,48 +506,4 @@ __global__ void __launch_bounds__(kTfThreads, tf_min_blocks<T>())
   st.finish();
 }
 
-// Full complex rows, one per pencil: load -> FFT(D1) -> mid -> FFT(D2) -> store (a
-// direction of 0 skips that transform), as k_x_full.
-template <typename T, int D1, int D2, class Load, class Mid, class Store>
-__global__ void __launch_bounds__(kTfThreads, tf_min_blocks<T>())
-    k_x_full_tf(Geom g, const __grid_constant__ TwoFactor<T> ax, Load ld, Mid mid, Store st0,
-                const int* __restrict__ done) {
-  using C = cplx_t<T>;
-  if (done != nullptr && *done) return;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  C* sm = reinterpret_cast<C*>(smraw);
-  constexpr int P = tf_cols<T>(), S = tf_x_stride<T>();
-  const int n = ax.n;
-  tf_load_table(ax, sm + 2 * n * S);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int nrows = g.nrows();
-  Store st = st0;
-  for (int q0 = blockIdx.x * P; q0 < nrows; q0 += gridDim.x * P) {
-    for (int p = wid; p < P; p += kTfThreads / 32) {
-      const bool h = q0 + p < nrows;
-      tf_each<4>(
-          lane, 32, n, [&](int e) -> C { return h ? ld(q0 + p, e) : mk<C>(T(0), T(0)); },
-          [&](int e, C v) { sm[e * S + p] = v; });
-    }
-    __syncthreads();
-    int z = 0;
-    if constexpr (D1 != 0) z = tf_transform<T, D1>(ax, S, 0, n * S);
-    for (int p = wid; p < P; p += kTfThreads / 32) {
-      if (q0 + p >= nrows) break;
-      tf_each<4>(
-          lane, 32, n, [&](int e) -> C { return mid(sm[z + e * S + p], q0 + p, e); },
-          [&](int e, C v) { sm[z + e * S + p] = v; });
-    }
-    __syncthreads();
-    if constexpr (D2 != 0) z = tf_transform<T, D2>(ax, S, z, n * S - z);
-    for (int p = wid; p < P; p += kTfThreads / 32) {
-      if (q0 + p >= nrows) break;
-#pragma unroll 4
-      for (int e = lane; e < n; e += 32) st(q0 + p, e, sm[z + e * S + p]);
-    }
-    __syncthreads();
-  }
-  st.finish();
-}
-
 }  // namespace qsm
