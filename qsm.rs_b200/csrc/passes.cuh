@@ -885,11 +885,14 @@ template <int THREADS, int BUDGET = 512> constexpr int zm_min_blocks() {
 // Threads per SM the multiplier Z pass of length N is compiled for: 640 (five 128-thread
 // blocks, at most 102 registers) where that compiles without spills, as for the 176-point
 // benchmark axis (TV-ADMM 256x256x176: 2 us per iteration less); 512 for the lengths whose
-// plan spilled at 640 (ptxas: 4-92 bytes per thread).
+// plan spills at 640 (ptxas: 4-96 bytes per thread) and is the faster for it (128x128xN:
+// 252 26.9 to 22.9 us, 312 32.7 to 27.0, 360 34.6 to 27.8; 45 and 189 come out even, and 350
+// slower, 31.5 to 35.2).
 template <typename T, int N> constexpr int zm_budget() {
   if (sizeof(T) == 8) return 384;  // twice the registers per value (168 at 128 threads)
   return (N == 75 || N == 125 || N == 128 || N == 135 || N == 150 || N == 180 || N == 216 || N == 224 ||
-          N == 225 || N == 240 || N == 256)
+          N == 225 || N == 231 || N == 240 || N == 252 || N == 256 || N == 270 || N == 273 || N == 300 ||
+          N == 312 || N == 315 || N == 360)
              ? 512
              : 640;
 }
