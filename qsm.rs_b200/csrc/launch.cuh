@@ -138,8 +138,8 @@ template <typename T> struct OpMultArray {
 
 // Doubles that K sums per block of an X pass may fill (grid_sum_last), whichever kernel runs.
 template <typename T> inline size_t x_partials(const Fft3<T>& f, int K) {
-  // blocks of the runtime engine; the compile-time kernels' are half as large, with room for
-  // a pencil count that does not fill them
+  // blocks of the runtime engine; a compile-time block holds at least 64 threads of pencils
+  // (x_fx_pencils) to the engine's 256, so four times as many is the bound
   const long long b = 4 * x_blocks(f);
   return (size_t)(b > kMaxPersistentBlocks ? b : kMaxPersistentBlocks) * K;
 }
@@ -225,7 +225,7 @@ bool run_x_c2r_fixed(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* spec, cons
 }
 
 // Compile-time X passes between a real array and a half spectrum for every listed length
-// (plain_x32.cu, plain_x64.cu, more_*.cu); x_plain_has says whether the axis is one of them.
+// (plain_x32.cu, plain_x64.cu, more_*.cu); axis_listed says whether the axis is one of them.
 template <typename T>
 bool x_plain_r2c(qsm_ctx* ctx, const Fft3<T>& f, const T* in, cplx_t<T>* spec, const int* done);
 template <typename T>
@@ -255,7 +255,10 @@ template <typename T> cplx_t<T>* x_stage_c(qsm_ctx* ctx, const Fft3<T>& f) {
 }
 // A listed length with a functor that no compile-time kernel carries: the functor as a pass
 // of its own around the plain kernel, except in small volumes, where the launch costs more
-// than the two-factor kernel (functor inside) loses.
+// than the two-factor kernel (functor inside) loses.  TKD in double, functor inside against
+// its own pass: 49.8 and 55.3 us at 64x48x40, 68.0 and 69.3 at 96x90x88, 78.1 and 75.4 at
+// 100x100x110, 85.1 and 80.6 at 160x96x90, 192 and 167 at 256x160x120; iSMV, 50 iterations:
+// 2.12 and 2.08 ms at 72x64x60, 4.09 and 3.82 at 100x100x110, 13.8 and 11.7 at 256x160x120.
 template <typename T> inline bool x_use_stage(const Fft3<T>& f) { return f.g.nvox() > (1LL << 20); }
 // Persistent grid: as many CTAs as fit on the device at once, capped by the work.
 template <class K> unsigned persistent_grid(qsm_ctx* ctx, K kernel, int threads, size_t smem, long long work) {
@@ -569,19 +572,15 @@ template <typename T>
 void run_z_fused_m(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const T* mult,
                    const int* done);
 
-// Tune the launch shape of the compile-time Y/Z pass (DIR, AXIS) and of the multiplier
-// Z pass for grid f, running the candidates in place on `scratch` (a half spectrum of f
-// whose contents may be overwritten) and `mscratch` (a real half-spectrum array).  With
-// `chain`, each candidate is timed inside that sequence of launches instead (the solver's
-// own chain of passes, which looks the shape up under the same key), so that it is judged
-// where it runs: after the pass that fills the L2-resident spectrum, not back to back
-// with itself.  No-op when the lengths have no compile-time pass, the shapes are cached,
-// the autotuner is off or the stream is capturing.
+// Tune the launch shape of the compile-time Y/Z pass (DIR, AXIS) and of the multiplier Z
+// pass for grid f: each candidate is timed inside `chain`, the solver's own sequence of
+// passes (which looks the shape up under the same key), so that it is judged where it runs:
+// after the pass that fills the L2-resident spectrum, not back to back with itself.  No-op
+// when the lengths have no compile-time pass, the shapes are cached, the autotuner is off or
+// the stream is capturing.
 template <typename T, int DIR, int AXIS>
-void tune_yz_fixed(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* scratch, const std::function<void()>* chain = nullptr);
-template <typename T>
-void tune_z_fused_m(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* scratch, T* mscratch,
-                    const std::function<void()>* chain = nullptr);
+void tune_yz_fixed(qsm_ctx* ctx, const Fft3<T>& f, const std::function<void()>& chain);
+template <typename T> void tune_z_fused_m(qsm_ctx* ctx, const Fft3<T>& f, const std::function<void()>& chain);
 
 #define QSM_MORE_DECLARE(G_)                                                                                      \
   template <typename T, int DIR, int AXIS>                                                                        \

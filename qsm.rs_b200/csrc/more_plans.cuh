@@ -13,10 +13,10 @@ namespace qsm {
 
 #define QSM_MORE_YZ(N_, T_, R0_, R1_, R2_)                                                        \
   if (FixedPlan<N_, T_, R0_, R1_, R2_>::matches(AXIS == 1 ? f.py : f.pz) && fx_cols<T>() * T_ <= 1024) \
-    return launch_yz_fx<T, DIR, AXIS, FixedPlan<N_, T_, R0_, R1_, R2_>>(ctx, f, 0, src, dst, done, true);
+    return launch_yz_fx<T, DIR, AXIS, FixedPlan<N_, T_, R0_, R1_, R2_>>(ctx, f, 0, src, dst, done);
 #define QSM_MORE_ZM(N_, T_, R0_, R1_, R2_)                                                        \
   if (FixedPlan<N_, T_, R0_, R1_, R2_>::matches(f.pz) && kZmCols * T_ <= 1024)                     \
-    return launch_zm_fx<T, FixedPlan<N_, T_, R0_, R1_, R2_>>(ctx, f, 0, src, dst, mult, done, true);
+    return launch_zm_fx<T, FixedPlan<N_, T_, R0_, R1_, R2_>>(ctx, f, 0, src, dst, mult, done);
 #define QSM_MORE_XR(N_, T_, R0_, R1_, R2_)                                                        \
   if (FixedPlan<N_, T_, R0_, R1_, R2_>::matches(f.px))                                             \
     return launch_x_r2c_fx<T, FixedPlan<N_, T_, R0_, R1_, R2_>, false>(ctx, f, spec, LoadCast<T, T>{in, f.g.nx}, done);

@@ -1,4 +1,4 @@
-// The four 3D-FFT pass kernels the solvers are built from.
+// The 3D-FFT pass kernels the solvers are built from.
 //
 // Spectra use the half-spectrum layout of a real-to-complex transform along x:
 // complex [nz][ny][pitch] with x' in [0, nx/2] valid (Fortran order like the
@@ -7,16 +7,16 @@
 // (src/fft.rs:514-540); with real-symmetric (Nyquist-averaged) multipliers the
 // half-spectrum chain computes the same values on half the bytes.
 //
-//   k_x_r2c   : two real rows per complex pencil (z = a + i b), forward FFT along x,
-//               split into the two half spectra.  A loader functor produces the
-//               real input on the fly (cast from f64, masked, stencil, kernel image).
-//   k_pass_yz : C2C along y or z.  Persistent CTAs walk P-column tiles (128-byte rows);
-//               each tile is staged into shared memory with cp.async, double
-//               buffered so that the next tile's copy overlaps this tile's transform.
-//               Optional pre/post pointwise hooks.
-//   k_z_fused : same tiling; forward z FFT -> pointwise multiplier -> inverse z FFT.
-//   k_x_c2r   : rebuild two Hermitian rows, inverse FFT along x, hand each real
-//               value to a store functor (scale, mask, selection).
+//   k_x_r2c     : two real rows per complex pencil (z = a + i b), forward FFT along x, split
+//                 into the two half spectra.
+//   k_pass_yz   : C2C along y or z.  Persistent CTAs walk P-column tiles (128-byte rows);
+//                 each tile is staged into shared memory with cp.async, double buffered so
+//                 that the next tile's copy overlaps this tile's transform.
+//   k_z_fused_m : same tiling; forward z FFT -> multiplier array -> inverse z FFT.
+//   k_x_c2r     : rebuild two Hermitian rows, inverse FFT along x.
+//
+// These are the run-time engine's, over plain arrays; k_*_fx and k_pass_yz_dx* are their
+// compile-time forms, where loaders, operators and stores are functors of the pass.
 #pragma once
 
 #include "fft_engine.cuh"
@@ -766,7 +766,7 @@ __global__ void __launch_bounds__(P* FP::T, yz_dx_min_blocks<T, P * FP::T>())
 // k_pass_yz_dx with the pass's operator applied as elements are fetched (op.pre) and
 // stored (op.post), for passes that carry one (k-space scalings, fused LSQR epilogues).
 // ACC: op.post also adds to a per-thread FP64 sum that is reduced over the grid at the
-// end (grid_sum_last) and handed to op.last, as in k_pass_yz_acc.  The element order of
+// end (grid_sum_last) and handed to op.last.  The element order of
 // that sum follows the fixed plan's last stage, so the total is deterministic for a
 // given launch shape.
 template <typename T, int DIR, int AXIS, class FP, int P, class Op, bool ACC>

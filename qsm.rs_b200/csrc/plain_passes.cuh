@@ -9,10 +9,8 @@
 namespace qsm {
 
 // One compile-time Y/Z pass (k_pass_yz_dx, FP a FixedPlan) in launch shape `shape`.
-// scoped: count and (when profiling) time the launch under the pass's name.
 template <typename T, int DIR, int AXIS, class FP>
-bool launch_yz_fx(qsm_ctx* ctx, const Fft3<T>& f, int shape, const cplx_t<T>* src, cplx_t<T>* dst,
-                  const int* done, bool scoped) {
+bool launch_yz_fx(qsm_ctx* ctx, const Fft3<T>& f, int shape, const cplx_t<T>* src, cplx_t<T>* dst, const int* done) {
   const cplx_t<T>* tw = (AXIS == 1) ? f.twy : f.twz;
   auto kern = k_pass_yz_dx<T, DIR, FP, fx_cols<T>()>;
   const size_t smem = dx_smem<T>(FP::n, fx_cols<T>());
@@ -21,11 +19,7 @@ bool launch_yz_fx(qsm_ctx* ctx, const Fft3<T>& f, int shape, const cplx_t<T>* sr
   if (!fx_launch_ok(ctx, kern, fx_cols<T>() * FP::T, smem, &grid, w.ntiles, (shape & kTuneBlockPerTile) != 0,
                     tune_bpsm(shape)))
     return false;
-  if (!scoped) {
-    kern<<<grid, dim3(fx_cols<T>(), FP::T), smem, ctx->stream>>>(f.g, w, tw, src, dst, done);
-    return true;
-  }
-  LaunchScope ls(ctx, AXIS == 1 ? (DIR < 0 ? "fft_y_fwd" : "fft_y_inv") : (DIR < 0 ? "fft_z_fwd" : "fft_z_inv"));
+  LaunchScope ls(ctx, yz_name(AXIS, DIR));
   kern<<<grid, dim3(fx_cols<T>(), FP::T), smem, ctx->stream>>>(f.g, w, tw, src, dst, done);
   ls.done();
   return true;
@@ -43,7 +37,7 @@ bool run_yz_fixed(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T
     if (FixedPlan<N_, T_, R0_, R1_, R2_>::matches(pl) && fx_cols<T>() * T_ <= 1024) {                   \
       using FP = FixedPlan<N_, T_, R0_, R1_, R2_>;                                                \
       const int shape = tuned_shape(ctx, yz_tune_key<T>("yz_fx", f, AXIS, DIR));                  \
-      return launch_yz_fx<T, DIR, AXIS, FP>(ctx, f, shape, src, dst, done, true);                 \
+      return launch_yz_fx<T, DIR, AXIS, FP>(ctx, f, shape, src, dst, done);                       \
     }
     QSM_FIXED_PLANS(QSM_TRY_YZ)
     if (f.forms == PassForms::kBase) return false;
@@ -66,10 +60,10 @@ void run_yz_plain(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T
 }
 
 // One compile-time multiplier Z pass (k_z_fused_m_fx, FP a FixedPlan) in launch shape
-// `shape`; scoped as in launch_yz_fx.
+// `shape`.
 template <typename T, class FP>
 bool launch_zm_fx(qsm_ctx* ctx, const Fft3<T>& f, int shape, const cplx_t<T>* src, cplx_t<T>* dst, const T* mult,
-                  const int* done, bool scoped) {
+                  const int* done) {
   auto kfx = k_z_fused_m_fx<T, FP, kZmCols>;
   const size_t smem = zm_smem<T>(FP::n, FP::n, kZmCols);
   const TileWalk w = tile_walk(f, 2, kZmCols, (shape & kTuneEdge) != 0);
@@ -77,10 +71,6 @@ bool launch_zm_fx(qsm_ctx* ctx, const Fft3<T>& f, int shape, const cplx_t<T>* sr
   if (!fx_launch_ok(ctx, kfx, kZmCols * FP::T, smem, &grid, w.ntiles, (shape & kTuneBlockPerTile) != 0,
                     tune_bpsm(shape)))
     return false;
-  if (!scoped) {
-    kfx<<<grid, dim3(kZmCols, FP::T), smem, ctx->stream>>>(f.g, w, f.twz, src, dst, mult, done);
-    return true;
-  }
   LaunchScope ls(ctx, "fft_z_fused");
   kfx<<<grid, dim3(kZmCols, FP::T), smem, ctx->stream>>>(f.g, w, f.twz, src, dst, mult, done);
   ls.done();
@@ -88,7 +78,7 @@ bool launch_zm_fx(qsm_ctx* ctx, const Fft3<T>& f, int shape, const cplx_t<T>* sr
 }
 
 template <typename T, int DIR, int AXIS>
-void tune_yz_fixed(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* scratch, const std::function<void()>* chain) {
+void tune_yz_fixed(qsm_ctx* ctx, const Fft3<T>& f, const std::function<void()>& chain) {
   {
     if (!compiled_plans(ctx)) return;
     const std::string key = yz_tune_key<T>("yz_fx", f, AXIS, DIR);
@@ -101,12 +91,7 @@ void tune_yz_fixed(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* scratch, const std
       const size_t smem = dx_smem<T>(FP::n, fx_cols<T>());                                             \
       ensure_smem(kern, smem);                                                                    \
       const auto cands = yz_candidates(f, fx_cols<T>(), kern, fx_cols<T>() * FP::T, smem);                  \
-      if (chain != nullptr)                                                                       \
-        autotune_pick(ctx, key, cands, [&](int c) { ctx->tuned[key] = TuneRec{c, {}}; (*chain)(); }, 3, 4); \
-      else                                                                                        \
-        autotune_pick(ctx, key, cands, [&](int c) {                                               \
-          launch_yz_fx<T, DIR, AXIS, FP>(ctx, f, c, scratch, scratch, nullptr, false);             \
-        });                                                                                       \
+      autotune_pick(ctx, key, cands, [&](int c) { ctx->tuned[key] = TuneRec{c, {}}; chain(); }, 3, 4); \
       return;                                                                                     \
     }
     QSM_FIXED_PLANS(QSM_TUNE_YZ)
@@ -116,8 +101,7 @@ void tune_yz_fixed(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* scratch, const std
 }
 
 template <typename T>
-void tune_z_fused_m(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* scratch, T* mscratch,
-                    const std::function<void()>* chain) {
+void tune_z_fused_m(qsm_ctx* ctx, const Fft3<T>& f, const std::function<void()>& chain) {
   {
     if (!compiled_plans(ctx)) return;
     const std::string key = yz_tune_key<T>("zm_fx", f, 2, -1);
@@ -130,12 +114,7 @@ void tune_z_fused_m(qsm_ctx* ctx, const Fft3<T>& f, cplx_t<T>* scratch, T* mscra
       const size_t smem = zm_smem<T>(FP::n, FP::n, kZmCols);                                      \
       ensure_smem(kfx, smem);                                                                     \
       const auto cands = yz_candidates(f, kZmCols, kfx, kZmCols * FP::T, smem);                   \
-      if (chain != nullptr)                                                                       \
-        autotune_pick(ctx, key, cands, [&](int c) { ctx->tuned[key] = TuneRec{c, {}}; (*chain)(); }, 3, 4); \
-      else                                                                                        \
-        autotune_pick(ctx, key, cands, [&](int c) {                                               \
-          launch_zm_fx<T, FP>(ctx, f, c, scratch, scratch, mscratch, nullptr, false);              \
-        });                                                                                       \
+      autotune_pick(ctx, key, cands, [&](int c) { ctx->tuned[key] = TuneRec{c, {}}; chain(); }, 3, 4); \
       return;                                                                                     \
     }
     QSM_FIXED_PLANS(QSM_TUNE_ZM)
@@ -153,7 +132,7 @@ void run_z_fused_m(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<
     if (FixedPlan<N_, T_, R0_, R1_, R2_>::matches(pl) && kZmCols * T_ <= 1024) {                   \
       using FP = FixedPlan<N_, T_, R0_, R1_, R2_>;                                                \
       const int shape = tuned_shape(ctx, yz_tune_key<T>("zm_fx", f, 2, -1));                      \
-      if (launch_zm_fx<T, FP>(ctx, f, shape, src, dst, mult, done, true)) return;                 \
+      if (launch_zm_fx<T, FP>(ctx, f, shape, src, dst, mult, done)) return;                       \
     }
     QSM_FIXED_PLANS(QSM_TRY_ZM)
     if (f.forms != PassForms::kBase) {

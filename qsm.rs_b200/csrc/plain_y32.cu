@@ -7,7 +7,7 @@ template void run_yz_plain<float, -1, 1>(qsm_ctx*, const Fft3<float>&, const cpl
 template void run_yz_plain<float, +1, 1>(qsm_ctx*, const Fft3<float>&, const cplx_t<float>*, cplx_t<float>*, const int*);
 template void run_yz_plain<float, -1, 2>(qsm_ctx*, const Fft3<float>&, const cplx_t<float>*, cplx_t<float>*, const int*);
 template void run_yz_plain<float, +1, 2>(qsm_ctx*, const Fft3<float>&, const cplx_t<float>*, cplx_t<float>*, const int*);
-template void tune_yz_fixed<float, -1, 1>(qsm_ctx*, const Fft3<float>&, cplx_t<float>*, const std::function<void()>*);
-template void tune_yz_fixed<float, +1, 1>(qsm_ctx*, const Fft3<float>&, cplx_t<float>*, const std::function<void()>*);
+template void tune_yz_fixed<float, -1, 1>(qsm_ctx*, const Fft3<float>&, const std::function<void()>&);
+template void tune_yz_fixed<float, +1, 1>(qsm_ctx*, const Fft3<float>&, const std::function<void()>&);
 
 }  // namespace qsm

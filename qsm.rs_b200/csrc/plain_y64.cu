@@ -7,7 +7,7 @@ template void run_yz_plain<double, -1, 1>(qsm_ctx*, const Fft3<double>&, const c
 template void run_yz_plain<double, +1, 1>(qsm_ctx*, const Fft3<double>&, const cplx_t<double>*, cplx_t<double>*, const int*);
 template void run_yz_plain<double, -1, 2>(qsm_ctx*, const Fft3<double>&, const cplx_t<double>*, cplx_t<double>*, const int*);
 template void run_yz_plain<double, +1, 2>(qsm_ctx*, const Fft3<double>&, const cplx_t<double>*, cplx_t<double>*, const int*);
-template void tune_yz_fixed<double, -1, 1>(qsm_ctx*, const Fft3<double>&, cplx_t<double>*, const std::function<void()>*);
-template void tune_yz_fixed<double, +1, 1>(qsm_ctx*, const Fft3<double>&, cplx_t<double>*, const std::function<void()>*);
+template void tune_yz_fixed<double, -1, 1>(qsm_ctx*, const Fft3<double>&, const std::function<void()>&);
+template void tune_yz_fixed<double, +1, 1>(qsm_ctx*, const Fft3<double>&, const std::function<void()>&);
 
 }  // namespace qsm

@@ -161,6 +161,7 @@ struct BrkState {
   BrkGroup g[kBrkMaxGroups];
 };
 
+// lowbias32, a published 32-bit integer hash (C. Wellons, hash-prospector, 2018)
 __device__ __forceinline__ unsigned hash32(unsigned x) {
   x ^= x >> 16;
   x *= 0x7feb352du;

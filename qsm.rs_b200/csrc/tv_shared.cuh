@@ -816,9 +816,9 @@ template <typename T> void tv_tune(qsm_ctx* ctx, const TvVol<T>& v) {
     tv_step_launch(ctx, v, 0, 0);
     tv_fft(ctx, v, 0, nullptr);
   };
-  tune_yz_fixed<T, -1, 1>(ctx, v.f, v.spec, &chain);
-  tune_yz_fixed<T, +1, 1>(ctx, v.f, v.spec, &chain);
-  tune_z_fused_m<T>(ctx, v.f, v.spec, v.mult, &chain);
+  tune_yz_fixed<T, -1, 1>(ctx, v.f, chain);
+  tune_yz_fixed<T, +1, 1>(ctx, v.f, chain);
+  tune_z_fused_m<T>(ctx, v.f, chain);
 }
 
 template <typename T> void tv_iter(qsm_ctx* ctx, const TvVol<T>& v, int q) {

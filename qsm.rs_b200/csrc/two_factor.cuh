@@ -263,7 +263,8 @@ __device__ __forceinline__ void tf_each(int first, int step, int total, const F&
   for (; i < total; i += step) put(i, f(i));
 }
 
-// Y/Z pass (IsPlainOp: no hooks; ACC: the post hook accumulates, as k_pass_yz_acc).  The
+// Y/Z pass (IsPlainOp: no hooks; ACC: the post hook also sums one FP64
+// value per element, which the last block hands to op.last).  The
 // tile is staged by cp.async; the next tile's copy starts as soon as the first stage has
 // read this one, under the second stage and the stores.
 template <typename T, int DIR, int AXIS, class Op, bool ACC>
