@@ -293,25 +293,30 @@ bool ensure_pinned(qsm_ctx* ctx) {
   return true;
 }
 
-// work(worker) on kStageThreads threads (worker 0 here, and those that cannot be started);
-// the first CUDA error of any is thrown.
-template <class F> void stage_workers(qsm_ctx* ctx, const F& work) {
+// Threads of a staged copy: one for each kStageShare bytes.
+int stage_threads(size_t bytes) {
+  return (int)std::min<size_t>(std::max<size_t>((bytes + kStageShare - 1) / kStageShare, 1), kStageThreads);
+}
+
+// work(worker) on `workers` threads (worker 0 here, and those that cannot be started); the
+// first CUDA error of any is thrown.
+template <class F> void stage_workers(qsm_ctx* ctx, int workers, const F& work) {
   cudaError_t err[kStageThreads];
   auto run = [&](int w) {
     err[w] = cudaSetDevice(ctx->device);
     if (err[w] == cudaSuccess) err[w] = work(w);
   };
   std::vector<std::thread> th;
-  th.reserve(kStageThreads);
+  th.reserve((size_t)workers);
   int started = 1;
   try {
-    for (; started < kStageThreads; ++started) th.emplace_back(run, started);
+    for (; started < workers; ++started) th.emplace_back(run, started);
   } catch (const std::system_error&) {
   }
   run(0);
-  for (int w = started; w < kStageThreads; ++w) run(w);
+  for (int w = started; w < workers; ++w) run(w);
   for (auto& t : th) t.join();
-  for (int w = 0; w < kStageThreads; ++w)
+  for (int w = 0; w < workers; ++w)
     if (err[w] != cudaSuccess) throw QsmError(QSM_ERR_CUDA, std::string("staged copy: ") + cudaGetErrorString(err[w]));
 }
 }  // namespace
@@ -324,9 +329,10 @@ void staged_h2d(qsm_ctx* ctx, void* dst, const void* src, size_t bytes) {
   }
   const uint8_t* s = static_cast<const uint8_t*>(src);
   uint8_t* d = static_cast<uint8_t*>(dst);
-  stage_workers(ctx, [&](int w) -> cudaError_t {
+  const int workers = stage_threads(bytes);
+  stage_workers(ctx, workers, [&](int w) -> cudaError_t {
     int k = 0;
-    for (size_t off = (size_t)w * kStageChunk; off < bytes; off += kStageThreads * kStageChunk, k ^= 1) {
+    for (size_t off = (size_t)w * kStageChunk; off < bytes; off += workers * kStageChunk, k ^= 1) {
       const int slot = 2 * w + k;
       uint8_t* p = static_cast<uint8_t*>(ctx->pinned) + slot * kStageChunk;
       const size_t n = std::min(kStageChunk, bytes - off);
@@ -349,8 +355,9 @@ void staged_d2h(qsm_ctx* ctx, void* dst, const void* src, size_t bytes) {
   }
   const uint8_t* s = static_cast<const uint8_t*>(src);
   uint8_t* d = static_cast<uint8_t*>(dst);
-  stage_workers(ctx, [&](int w) -> cudaError_t {
-    const size_t step = kStageThreads * kStageChunk;
+  const int workers = stage_threads(bytes);
+  stage_workers(ctx, workers, [&](int w) -> cudaError_t {
+    const size_t step = workers * kStageChunk;
     auto issue = [&](size_t off, int k) -> cudaError_t {
       const int slot = 2 * w + k;
       cudaError_t e = cudaMemcpyAsync(static_cast<uint8_t*>(ctx->pinned) + slot * kStageChunk, s + off,

@@ -139,15 +139,21 @@ cudaError_t ctx_malloc(qsm_ctx* ctx, void** p, size_t bytes);
 
 // Host <-> device copies of the host-pointer entry points.  h2d and d2h hand pageable
 // buffers of kStageMin bytes and more to the staged copies, and others to cudaMemcpyAsync.
-// Staged copies: kStageThreads host threads, each taking every kStageThreads-th chunk
-// through its own two pinned slots, so that the host copies run side by side and under the
-// DMA.  (One pageable cudaMemcpyAsync per buffer: 18 ms for a 58 MB volume in and out with its
-// mask, 7 GB/s; staged 5 ms.)  Where the 16 MB of slots cannot be had they are plain copies.
-// staged_h2d returns when the source has been read, staged_d2h when the destination is
+// Staged copies: up to kStageThreads host threads, one for each kStageShare bytes, which take
+// the chunks in turn through two pinned slots each, so that the host copies run side by side
+// and under the DMA.  (One pageable cudaMemcpyAsync per buffer: 18 ms for a 58 MB volume in and
+// out with its mask, 7 GB/s; staged 5 ms.)  Starting the threads costs some 90 us, and pageable
+// copies are good for 20 GB/s up to some 20 MB: a volume in and out takes 0.66 ms plain and
+// 0.49 to 0.85 staged at 4.6 MB, 2.8 and 2.4 at 23 MB, 3.8 and 2.8 at 31 MB, 6.0 (14.7 into
+// fresh memory) and 3.9 (5.5) at 46 MB.  A device load of a 0.1, 4 and 19 MB NIfTI image takes
+// 31, 310 and 938 us; with eight threads whatever its size 124, 217 and 1470; through one pair
+// of 32 MB slots 39, 353 and 1468.  Where the 16 MB of slots cannot be had they are plain
+// copies.  staged_h2d returns when the source has been read, staged_d2h when the destination is
 // written.
 constexpr int kStageThreads = 8;
 constexpr size_t kStageChunk = (size_t)1 << 20;
-constexpr size_t kStageMin = (size_t)4 << 20;
+constexpr size_t kStageShare = (size_t)8 << 20;
+constexpr size_t kStageMin = (size_t)24 << 20;
 void staged_h2d(qsm_ctx* ctx, void* dst, const void* src, size_t bytes);
 void staged_d2h(qsm_ctx* ctx, void* dst, const void* src, size_t bytes);
 void h2d(qsm_ctx* ctx, void* dst, const void* src, size_t bytes);

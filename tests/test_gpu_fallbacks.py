@@ -8,15 +8,15 @@ import pytest
 import torch
 
 import qsmgpu
-from qsmgpu import Grid, inversion
+from qsmgpu import Grid, inversion, nifti
 from oracle import qsm_oracle as O
 
 pytestmark = pytest.mark.gpu
 
 
 def test_host_calls_without_pinned_slots():
-    """A host call of 8 MB makes the device volumes (field, mask, result), then the slots."""
-    grid = Grid.new(128, 128, 64)
+    """A host call of 26 MB makes the device volumes (field, mask, result), then the slots."""
+    grid = Grid.new(192, 128, 136)
     rng = np.random.default_rng(1)
     f = rng.standard_normal(grid.shape)
     m = (rng.random(grid.shape) < 0.5).astype(np.uint8)
@@ -28,6 +28,39 @@ def test_host_calls_without_pinned_slots():
         np.testing.assert_array_equal(inversion.tkd(f, m, grid, (0, 0, 1), p, ctx=ctx), want)
         # the failure was taken by the slots, and the next copies have them
         np.testing.assert_array_equal(inversion.tkd(f, m, grid, (0, 0, 1), p, ctx=ctx), want)
+
+
+
+# around the 24 MiB from which pageable copies are staged, and whole and broken shares of the
+# staging threads
+@pytest.mark.parametrize("dims", [(191, 128, 128), (192, 128, 128), (193, 128, 128), (256, 128, 128), (257, 128, 128),
+                                  (256, 256, 176)], ids=lambda d: "x".join(map(str, d)))
+def test_staged_copies_of_large_volumes_are_exact(ctx64, dims):
+    grid = Grid.new(*dims)
+    rng = np.random.default_rng(sum(dims))
+    f = rng.standard_normal(grid.shape)
+    m = (rng.random(grid.shape) < 0.5).astype(np.uint8)
+    p = inversion.TkdParams(0.2)
+    df, dm = torch.from_numpy(f).cuda(), torch.from_numpy(m).cuda()
+    out = torch.empty(grid.shape, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    inversion.tkd_device(ctx64, df.data_ptr(), dm.data_ptr(), grid, (0, 0, 1), p, out.data_ptr())
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(inversion.tkd(f, m, grid, (0, 0, 1), p, ctx=ctx64), out.cpu().numpy())
+
+
+@pytest.mark.parametrize("dims", [(32, 32, 32), (64, 64, 65), (128, 128, 129), (200, 180, 150)],
+                         ids=lambda d: "x".join(map(str, d)))
+def test_nifti_images_of_every_share(ctx64, dims):
+    """Float32 images of a part of a chunk to three shares, in and out of the device."""
+    n = dims[0] * dims[1] * dims[2]
+    v = np.random.default_rng(n).standard_normal(n).astype(np.float32).astype(np.float64)
+    raw = nifti.save_nifti(v, dims, (1.0, 1.0, 1.0), np.eye(4).ravel())
+    d = torch.empty(n, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    nifti.load_nifti_device(raw, d.data_ptr(), n, ctx=ctx64)
+    np.testing.assert_array_equal(d.cpu().numpy(), v)
+    assert nifti.save_nifti_device(d.data_ptr(), dims, (1.0, 1.0, 1.0), np.eye(4).ravel(), ctx=ctx64) == raw
 
 
 PERCENTS = [0.1, 30.0, 60.0, 99.9]
