@@ -385,8 +385,15 @@ struct TgvFlag {
 constexpr int kTgvBX = 32, kTgvBY = 4;
 constexpr int kTgvBlocks = 8;  // resident per SM
 // Chunks of z: enough that the tiles make about kTgvChunks blocks per SM, for the ends of the
-// ellipsoid's columns are idle (16: 227 us, 32: 210, 48: 203, 64 and 96: 204).
-constexpr int kTgvChunks = 48;
+// ellipsoid's columns are idle (16: 227 us, 32: 210, 48: 203, 64 and 96: 204); but a chunk
+// loads two planes more than it owns, so up to kTgvMinChunk planes while one wave of blocks
+// does not hold them all (200 iterations at 120x100x80, chunks of 1, 2, 3 and 4 planes: 6.35,
+// 5.57, 5.48, 5.28 ms; at 96x96x64 4.91, 4.73, 4.39, 4.62; at 144x160x120 15.0, 12.6, 11.6,
+// 11.2).  Boxes that need no more than a wave of single planes take the kernels' one-plane form
+// (ONE), whose loads go out together instead of plane by plane (2.64 instead of 2.89 ms at
+// 48x40x44, 2.56 and 2.86 at 37x53x41, 2.50 and 2.84 at 36x36x36).
+constexpr int kTgvChunks = 48, kTgvMinChunk = 4;
+constexpr int kTgvOneBlocks = 4;  // resident per SM, one-plane form (twice the registers)
 
 // Sums of the 27-point stencil (apply_stencil, tgv.rs:667-713; dk, dj, di order) along a
 // column: the nine values of a plane end the sum of the plane below, continue their own
@@ -398,10 +405,16 @@ struct Stencil27 {
   // x and y neighbours.
   __device__ __forceinline__ float add(const float* __restrict__ a, unsigned s, unsigned bx, const TgvConst& K, float c[5]) {
     float v[9];
+    plane(a, s, bx, v);
+    return add(v, K, c);
+  }
+  static __device__ __forceinline__ void plane(const float* __restrict__ a, unsigned s, unsigned bx, float v[9]) {
 #pragma unroll
     for (int dj = 0; dj < 3; ++dj)
 #pragma unroll
       for (int di = 0; di < 3; ++di) v[dj * 3 + di] = a[s + dj * bx - bx + di - 1];
+  }
+  __device__ __forceinline__ float add(const float v[9], const TgvConst& K, float c[5]) {
     float above = 0.0f;
 #pragma unroll
     for (int dj = 0; dj < 3; ++dj)
@@ -447,9 +460,11 @@ struct Stencil27 {
 // faces (it is eroded from the volume's, and the box leaves two voxels around it), so its
 // voxels have all 26 neighbours and need no boundary case; the eroded mask's may lie on
 // them.  The arithmetic is that of the reference, in its order.
-__global__ void __launch_bounds__(kTgvBX* kTgvBY, kTgvBlocks) k_tgv_dual(Box b, TgvArrays A, TgvScalars c, TgvConst K, int q,
+// ONE: chunks of one plane, every value loaded before the first is used.
+template <bool ONE>
+__global__ void __launch_bounds__(kTgvBX* kTgvBY, ONE ? kTgvOneBlocks : kTgvBlocks) k_tgv_dual(Box b, TgvArrays A, TgvScalars c, TgvConst K, int q,
                                                              int zchunk, const TgvFlag* flag) {
-  if (flag->done) return;
+  const int done = flag->done;
   const float* __restrict__ phb = A.phi[q];
   const float* __restrict__ chb = A.chi[q];
   const float* __restrict__ wbx = A.w[q][0];
@@ -472,7 +487,23 @@ __global__ void __launch_bounds__(kTgvBX* kTgvBY, kTgvBlocks) k_tgv_dual(Box b, 
   float phm = 0.0f, phc = 0.0f;                  // phi_ at k - 1 and k
   float wc[3] = {0.0f, 0.0f, 0.0f};              // w_ at k
   int c0 = code_at(kbeg), c1 = code_at(kbeg + 1), c2 = code_at(kbeg + 2);
-  {
+  if (done) return;  // read with the codes, not before them
+  float v0[9], v1[9], v2[9];  // ONE: the three planes of chi_
+  if constexpr (ONE) {
+    const unsigned s = (unsigned)kbeg * sxy + col;
+    if (c0 & 1) {
+      Stencil27::plane(chb, s - sxy, bx, v0);
+      Stencil27::plane(chb, s, bx, v1);
+      Stencil27::plane(chb, s + sxy, bx, v2);
+      phm = phb[s - sxy];
+      phc = phb[s];
+    }
+    if (c0 & 2) {
+      wc[0] = wbx[s];
+      wc[1] = wby[s];
+      wc[2] = wbz[s];
+    }
+  } else {
     const unsigned s = (unsigned)kbeg * sxy + col;
     if (c0 & 1) S.add(chb, s - sxy, bx, K, cc);
     if ((c0 | c1) & 1) S.add(chb, s, bx, K, cc);
@@ -524,8 +555,16 @@ __global__ void __launch_bounds__(kTgvBX* kTgvBY, kTgvBlocks) k_tgv_dual(Box b, 
       wz[2] = wbz[s + sxy];
     }
     float cn[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f}, t2 = 0.0f;
-    if ((c0 | c1 | c2) & 1) t2 = S.add(chb, s + sxy, bx, K, cn);
-    else S.skip();
+    if constexpr (ONE) {
+      if (in0) {
+        S.add(v0, K, cc);
+        S.add(v1, K, cc);
+        t2 = S.add(v2, K, cn);
+      }
+    } else {
+      if ((c0 | c1 | c2) & 1) t2 = S.add(chb, s + sxy, bx, K, cn);
+      else S.skip();
+    }
     if (c0 & 2) {
       const float cb = cc[0];
       float gx = 0.0f, gy = 0.0f, gz = 0.0f;
@@ -593,10 +632,11 @@ __global__ void __launch_bounds__(kTgvBX* kTgvBY, kTgvBlocks) k_tgv_dual(Box b, 
 // iterate x (read), [q] the extrapolation consumed by the dual step (overwritten with
 // x_new); [1-q] then receives 2 x_new - x.  Outside the eroded mask every variable stays
 // zero, and phi and chi outside mask0, so those voxels are neither read nor written.
-__global__ void __launch_bounds__(kTgvBX* kTgvBY, kTgvBlocks) k_tgv_primal(Box b, TgvArrays A, TgvScalars c,
+template <bool ONE>
+__global__ void __launch_bounds__(kTgvBX* kTgvBY, ONE ? kTgvOneBlocks : kTgvBlocks) k_tgv_primal(Box b, TgvArrays A, TgvScalars c,
                                                                               TgvConst K, int q, int zchunk,
                                                                               const TgvFlag* flag) {
-  if (flag->done) return;
+  const int done = flag->done;
   const float* __restrict__ etab = A.eta;
   const float* __restrict__ p0 = A.p[0];
   const float* __restrict__ p1 = A.p[1];
@@ -617,18 +657,29 @@ __global__ void __launch_bounds__(kTgvBX* kTgvBY, kTgvBlocks) k_tgv_primal(Box b
   float ec[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f}, em = 0.0f;  // eta at plane k (as cc above) and k - 1
   float pz = 0.0f, qz[3] = {0.0f, 0.0f, 0.0f};              // mask0 p2; q2, q4, q5 at k - 1
   int c0 = code_at(kbeg), c1 = code_at(kbeg + 1), c2 = code_at(kbeg + 2);
+  if (done) return;  // read with the codes, not before them
+  float v0[9], v1[9], v2[9];  // ONE: the three planes of eta
   {
     const unsigned s = (unsigned)kbeg * sxy + col;
-    if (c0 & 1) {
-      S.add(etab, s - sxy, bx, K, ec);
-      em = ec[0];
+    if constexpr (ONE) {
+      if (c0 & 1) {
+        Stencil27::plane(etab, s - sxy, bx, v0);
+        Stencil27::plane(etab, s, bx, v1);
+        Stencil27::plane(etab, s + sxy, bx, v2);
+      }
+    } else {
+      if (c0 & 1) {
+        S.add(etab, s - sxy, bx, K, ec);
+        em = ec[0];
+      }
+      if ((c0 | c1) & 1) S.add(etab, s, bx, K, ec);
     }
-    if ((c0 | c1) & 1) S.add(etab, s, bx, K, ec);
-    if ((c0 & 2) && kbeg > 0 && (mk[s - sxy] & 1)) {
-      pz = p2[s - sxy];
+    if ((c0 & 2) && kbeg > 0) {  // q is zero outside mask0
+      const float pm = p2[s - sxy];
       qz[0] = q2[s - sxy];
       qz[1] = q4[s - sxy];
       qz[2] = q5[s - sxy];
+      pz = mk[s - sxy] & 1 ? pm : 0.0f;
     }
   }
   for (int k = kbeg; k < kend; ++k) {
@@ -670,8 +721,17 @@ __global__ void __launch_bounds__(kTgvBX* kTgvBY, kTgvBlocks) k_tgv_primal(Box b
       for (int t = 0; t < 3; ++t) wo[t] = A.w[1 - q][t][s];
     }
     float en[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f}, t2 = 0.0f;
-    if ((c0 | c1 | c2) & 1) t2 = S.add(etab, s + sxy, bx, K, en);
-    else S.skip();
+    if constexpr (ONE) {
+      if (in0) {
+        S.add(v0, K, ec);
+        em = ec[0];
+        S.add(v1, K, ec);
+        t2 = S.add(v2, K, en);
+      }
+    } else {
+      if ((c0 | c1 | c2) & 1) t2 = S.add(etab, s + sxy, bx, K, en);
+      else S.skip();
+    }
     if (c0 & 2) {
       if (in0) {
         const float a0 = ec[0];
@@ -892,17 +952,22 @@ void tgv_device(qsm_ctx* ctx, const double* phase, const uint8_t* mask, const qs
   const unsigned gblocks = grid1d(B);
   const unsigned tgx = (unsigned)((b.bx + kTgvBX - 1) / kTgvBX), tgy = (unsigned)((b.by + kTgvBY - 1) / kTgvBY);
   const long long nzc = std::max<long long>(1, (long long)kTgvChunks * sm_count(ctx) / ((long long)tgx * tgy));
-  const int zchunk = (int)((b.bz + nzc - 1) / nzc);
+  const long long resident = (long long)kTgvBlocks * sm_count(ctx);
+  const long long fit = ((long long)tgx * tgy * b.bz + resident - 1) / resident;  // planes a thread for one wave
+  const int zchunk = std::max((int)((b.bz + nzc - 1) / nzc), (int)std::min<long long>(fit, kTgvMinChunk));
+  const bool one = zchunk == 1;
   const dim3 tgrid(tgx, tgy, (unsigned)((b.bz + zchunk - 1) / zchunk)), tblock(kTgvBX, kTgvBY);
   auto one_iter = [&](size_t t) {
     const int q = (int)((t + 1) % 2);
     {
       LaunchScope ls(ctx, "tgv_dual");
-      k_tgv_dual<<<tgrid, tblock, 0, ctx->stream>>>(b, A, c, K, q, zchunk, flag);
+      if (one) k_tgv_dual<true><<<tgrid, tblock, 0, ctx->stream>>>(b, A, c, K, q, zchunk, flag);
+      else k_tgv_dual<false><<<tgrid, tblock, 0, ctx->stream>>>(b, A, c, K, q, zchunk, flag);
       ls.done();
     }
     LaunchScope ls(ctx, "tgv_primal");
-    k_tgv_primal<<<tgrid, tblock, 0, ctx->stream>>>(b, A, c, K, q, zchunk, flag);
+    if (one) k_tgv_primal<true><<<tgrid, tblock, 0, ctx->stream>>>(b, A, c, K, q, zchunk, flag);
+    else k_tgv_primal<false><<<tgrid, tblock, 0, ctx->stream>>>(b, A, c, K, q, zchunk, flag);
     ls.done();
   };
   auto check = [&](size_t t) {
