@@ -23,6 +23,7 @@ template <typename T> struct Fft3 {
   const cplx_t<T>* twz;
   TwoFactor<T> tfx{}, tfy{}, tfz{};  // two-factor passes of each axis (n = 0: none)
   T* xstage = nullptr;  // buffer of the runtime-engine X passes (null: the context's own)
+  T* zstage = nullptr;  // multiplier array of run_z_fused (null: the context's own)
   PassForms forms = PassForms::kAll;
 };
 
@@ -674,7 +675,7 @@ template <typename T, class Op>
 void run_z_fused(qsm_ctx* ctx, const Fft3<T>& f, const cplx_t<T>* src, cplx_t<T>* dst, const Op& op,
                  const int* done, bool array = true) {
   if (array && (axis_listed(ctx, f, f.pz) || !tf_usable(ctx, f.tfz, tf_cols<T>()))) {
-    T* m = ws_scratch<T>(ctx, sizeof(T) == 4 ? "z.mult32" : "z.mult64", (size_t)f.g.hsize());
+    T* m = f.zstage ? f.zstage : ws_scratch<T>(ctx, sizeof(T) == 4 ? "z.mult32" : "z.mult64", (size_t)f.g.hsize());
     spec_multiplier<T>(ctx, f, op, m, done);
     if (f.forms == PassForms::kAll) {
       run_z_fused_m<T>(ctx, f, src, dst, m, done);

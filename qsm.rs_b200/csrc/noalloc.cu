@@ -137,10 +137,17 @@ extern "C" qsm_status qsm_tkd_device_noalloc(const double* d_local_field, const 
     K.by = bdir[1] / bn;
     K.bz = bdir[2] / bn;
 
-    // two-factor tables where they still fit; otherwise the runtime-engine X passes go
-    // through the output buffer
+    // until the last pass the output buffer holds the stage of X passes whose functors are
+    // passes of their own, and, where a half spectrum of reals fits it, the Z multiplier, which
+    // the Z pass copies 16 bytes at a time (128x128x128: 178 us with the dipole evaluated in a
+    // two-factor Z pass, 159 so)
+    f.xstage = d_out_chi;
+    if (f.g.hsize() <= d.n && reinterpret_cast<uintptr_t>(d_out_chi) % 16 == 0) f.zstage = d_out_chi;
+    // two-factor tables where a pass reads them and they still fit
+    const bool none[3] = {plan_listed(f.px) && x_use_stage(f), plan_listed(f.py), plan_listed(f.pz) && f.zstage != nullptr};
     TwoFactor<double>* axes[3] = {&f.tfx, &f.tfy, &f.tfz};
     for (int a = 0; a < 3; ++a) {
+      if (none[a]) continue;
       TwoFactor<double> ax = plan_two_factor<double>(ns[a], a);
       if (ax.n == 0) continue;
       const std::vector<double2> h = two_factor_table(ax);
@@ -151,13 +158,12 @@ extern "C" qsm_status qsm_tkd_device_noalloc(const double* d_local_field, const 
       cur += bytes;
       *axes[a] = ax;
     }
-    f.xstage = d_out_chi;
 
     // the same chain as qsm_tkd_device in double (src/inversion/tkd.rs:48-99); the
     // spectrum is fully written by the first pass, so nothing needs clearing
     run_x_r2c<double>(&local, f, spec, LoadCast<double, double>{d_local_field, d.nx}, nullptr);
     run_yz<double, -1, 1>(&local, f, spec, spec, OpId<double>{}, nullptr);
-    run_z_fused<double>(&local, f, spec, spec, OpTkd<double>{K, params->threshold, 0}, nullptr, false);
+    run_z_fused<double>(&local, f, spec, spec, OpTkd<double>{K, params->threshold, 0}, nullptr, f.zstage != nullptr);
     run_yz<double, +1, 1>(&local, f, spec, spec, OpId<double>{}, nullptr);
     run_x_c2r<double>(&local, f, spec, StoreMaskedF64<double>{d_out_chi, d_mask, d.nx, 1.0 / (double)d.n}, nullptr);
     QSM_CUDA(cudaStreamSynchronize(local.stream));
